@@ -755,6 +755,23 @@ int ott_conv_f32_forward(ott_ctx* ctx, const ott_conv_f32* c, const float* in_de
 
 int ott_conv_int8_kernel_kind(const ott_conv* c) { return c ? c->kind : OTT_ERR_INVALID; }
 
+namespace {
+// int8 NHWC input of a 3x3 depthwise layer: the multiply-adds can go to the tensor cores as the data lies, no byte transposes,
+// at one 128-row MMA per tap, 32 channels and 8 x 16 output pixels. That pays where the CUDA cores have the most transposing to
+// do per output - stride 2 (four input pixels per output) and fp32 output (whose stores the other kernel cannot coalesce) - on
+// launches long enough to amortise its longer pipeline (6 M outputs) and maps its tiles fit. Measured, tensor cores against
+// CUDA cores: 256 channels 56x56 stride 2, 64 images 15.7 / 20.2 us; 58 channels 80x80 stride 2, 256 images 27.1 / 43.2; 512
+// channels 28x28, fp32 out 57.8 / 64.9; but 128 channels 28x28 stride 2, 64 images 5.9 / 5.0 (too short), 58 channels 40x40
+// stride 2, 256 images 12.6 / 11.6 (20x20 outputs fill 52 % of their tiles), 256 channels 56x56 stride 1 41.1 / 40.7.
+bool depthwise_on_tensor_cores(const ott_ctx* ctx, const ott_conv* c, const ConvShape& s, int out_dtype) {
+    if (!c->dw_umma || out_dtype == OTT_S32_NHWC || ctx->dw_tensor_cores == 0) return false;
+    if (ctx->dw_tensor_cores == 2) return true;
+    if (s.sh == 1 && out_dtype != OTT_F32_NCHW) return false;
+    const long tiles = (long)((s.oh + 15) / 16) * ((s.ow + 7) / 8), pixels = (long)s.oh * s.ow;
+    return pixels * 10 >= tiles * 128 * 7 && (double)s.n * pixels * (c->dw_plan.ncb_total * 32) >= 6e6;
+}
+}  // namespace
+
 const char* ott_conv_int8_kernel_name(const ott_ctx* ctx, const ott_conv* c, int in_dtype, int out_dtype, int h, int w) {
     if (!ctx || !c) return "";
     const ott_conv_desc& d = c->d;
@@ -766,10 +783,8 @@ const char* ott_conv_int8_kernel_name(const ott_ctx* ctx, const ott_conv* c, int
     s.kh = d.kh; s.kw = d.kw; s.sh = d.sh; s.sw = d.sw; s.ph = d.ph; s.pw = d.pw; s.dh = d.dh; s.dw = d.dw;
     if (c->kind == OTT_KERNEL_DENSE_UMMA) return "dense_umma_kernel";
     if (c->kind == OTT_KERNEL_DENSE_DIRECT) return dense_stem_supports(s, in_dtype, out_dtype) ? "dense_stem_kernel" : "dense_direct_kernel";
-    const bool gathered = !c->src_channels.empty();
-    const bool tc_wins = c->dw_plan.ncb_total <= 2 || (long)s.h * s.w >= 2048;
-    if (c->dw_umma && (ctx->dw_tensor_cores == 2 || (ctx->dw_tensor_cores == 1 && tc_wins)) && !gathered && in_dtype == OTT_S8_NHWC && out_dtype != OTT_S32_NHWC)
-        return "dw_umma_kernel";
+    s.n = 1 << 20;  // the choice for a batch that fills the GPU
+    if (in_dtype == OTT_S8_NHWC && depthwise_on_tensor_cores(ctx, c, s, out_dtype)) return "dw_umma_kernel";
     if (c->w_tiled_dev && depthwise_tiled_supports(s, out_dtype)) return "depthwise_tiled_kernel";
     return "depthwise_kernel";
 }
@@ -993,30 +1008,30 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
 
     uint32_t* status = status_word_dev ? status_word_dev : ctx->status_dev;
     PlaneGather groups8;  // depthwise over gathered int8 input: where each 16-channel group lies
-    if (gathered && c->kind == OTT_KERNEL_DEPTHWISE && c->gather_group == 32) {
+    const bool dw_tensor = c->kind == OTT_KERNEL_DEPTHWISE && in_dtype == OTT_S8_NHWC && (!gathered || c->gather_group == 32) &&
+                           depthwise_on_tensor_cores(ctx, c, s, out_dtype);
+    if (gathered && c->kind == OTT_KERNEL_DEPTHWISE) {
         for (int i = 0; i < n_sources; ++i)
             if (!sources[i]) return ctx->fail(OTT_ERR_INVALID, "null source tensor");
         in_dev = sources[0];
-    } else if (gathered && c->kind == OTT_KERNEL_DEPTHWISE) {
+    }
+    if (gathered && c->kind == OTT_KERNEL_DEPTHWISE && !dw_tensor) {
         if (!c->w_tiled_dev || !depthwise_tiled_supports(s, out_dtype)) return ctx->fail(OTT_ERR_UNSUPPORTED, "gathered depthwise layer: tiled kernel only");
         for (int i = 0; i < n_sources; ++i) {
-            if (!sources[i]) return ctx->fail(OTT_ERR_INVALID, "null source tensor");
             groups8.base[i] = reinterpret_cast<const float*>(sources[i]);
             groups8.img_stride[i] = nhwc_channels(c->src_channels[(size_t)i]);
         }
-        for (size_t g = 0; g < c->block_x.size(); ++g) groups8.ref[g] = ((uint32_t)c->block_src[g] << 24) | c->block_x[g];
+        // a layer laid out in 32-channel groups: two 16-channel groups each; a second one past the end of its tensor belongs to
+        // zero filters only and repeats the first
+        const int per = c->gather_group / 16;
+        for (size_t g = 0; g < c->block_x.size(); ++g)
+            for (int j = 0; j < per; ++j) {
+                const int x = c->block_x[g] + 16 * j, end = nhwc_channels(c->src_channels[c->block_src[g]]);
+                groups8.ref[g * per + j] = ((uint32_t)c->block_src[g] << 24) | (uint32_t)(x < end ? x : c->block_x[g]);
+            }
         gather = &groups8;
-        in_dev = sources[0];
     }
-    // int8 NHWC input: the multiply-adds can go to the tensor cores as the data lies, no byte transposes. Every tap costs one
-    // 128-row MMA per 32 channels and 8 x 16 pixel tile, so this wins for narrow layers (at most 64 channels) and for wide
-    // layers on input maps large enough for the tiles to fit well (256 channels, 56 x 56, 64 images: stride 1 41.8 us against
-    // 49.1, stride 2 16.3 against 22.2; 116 channels on 20 x 20 lose, 18.5 against 13.6 and 10.5 against 9.2); elsewhere the CUDA cores do.
-    // A layer with gathered input that was laid out in 32-channel groups always runs here (its groups are the MMA's K blocks).
-    const bool dw_tc_wins = c->dw_plan.ncb_total <= 2 || (long)s.h * s.w >= 2048;
-    const bool dw_gathered_tc = gathered && c->kind == OTT_KERNEL_DEPTHWISE && c->gather_group == 32;
-    if (c->kind == OTT_KERNEL_DEPTHWISE && c->dw_umma && in_dtype == OTT_S8_NHWC && out_dtype != OTT_S32_NHWC &&
-        (dw_gathered_tc || (!gathered && (ctx->dw_tensor_cores == 2 || (ctx->dw_tensor_cores == 1 && dw_tc_wins))))) {
+    if (dw_tensor) {
         UmmaSources us{};
         if (gathered) {
             us.n_src = n_sources;

@@ -3,23 +3,29 @@
 // (Tensor/QuantizeX86.cpp:396-549) and requantize/dequantize epilogue (Tensor/QuantizeX86.cpp:1723-1870,
 // :851-903) fused into one pass over HBM.
 //
-// One CTA = one image x 32 channels x a band of TY output rows x TXO output columns.
+// One CTA = one image x 32 channels x a band of output rows x up to 64 (stride 2: 40) output columns.
 //  1. load: the input halo tile goes to shared memory as int8 *channel planes* (pixels of one channel are
-//     consecutive bytes). From fp32 NCHW it is quantized on the way (float4 loads along W); from int8 NHWC
-//     the 16-byte channel vectors of 4 neighbouring pixels are transposed in registers (4x4 byte transposes).
-//  2. compute: thread = (channel = lane, 4 consecutive output columns). Because pixels are consecutive
-//     bytes, one 32-bit window holds 4 horizontal taps of one channel and a dp4a against the packed filter
-//     row does 4 multiply-adds; the windows of the last K input rows stay in a register ring while the
-//     thread walks down the band. Sums are exact s32.
-//  3. epilogue in registers (epilogue.cuh). int8 results are packed 4 pixels to a word into shared-memory
-//     channel planes, transposed back to channel-innermost 16-byte vectors and stored along the NHWC
-//     channel axis; fp32 NCHW results are stored directly.
+//     consecutive bytes). From fp32 NCHW it is quantized on the way: a thread takes one 4-pixel word position of eight
+//     channels, so that the position's index arithmetic and bounds tests are paid once per eight words and eight 16-byte loads
+//     are in flight per thread. Words start on 16-byte boundaries of the tensor whatever the width is; a row's first pixel
+//     then lies `sh` (0..3) bytes into its first word, and the compute phase shifts each row by its own amount. From int8
+//     NHWC the 16-byte channel vectors of 4 neighbouring pixels are transposed in registers (4x4 byte transposes).
+//  2. compute: thread = (channel = lane, 4 consecutive output columns), walking down the band. Because pixels are consecutive bytes, one 32-bit window holds 4 horizontal taps of one channel and a dp4a does 4 multiply-adds; the
+//     windows of the last K input rows stay in registers while the thread walks down its rows. The fifth column of a 5x5
+//     filter would waste three quarters of a dp4a per row, so its bytes are collected down the column instead (one byte
+//     permute per row): 7 dp4a per output instead of 10. Sums are exact s32.
+//  3. epilogue in registers (epilogue.cuh). int8 results: a 4x4 byte transpose across four lanes (two shuffles) gives every
+//     lane four channels of one pixel; eight lanes write a pixel's 32 channels, one whole sector. fp32 NCHW results are
+//     stored directly. No staging buffer and no second barrier: warps leave one by one, and more CTAs fit an SM.
+// Bound by instruction issue on large fp32 inputs (the quantizer alone is 4 instructions per element) and by latency on small
+// maps, where the plan cuts the band and the rows per thread until the GPU has about two CTAs per SM.
 //
 // This header holds the kernel template; depthwise_tiled_k*s*.cu instantiate it per (kernel size, stride)
 // so the variants compile in parallel.
 #pragma once
 
 #include <mutex>
+#include <type_traits>
 
 #include "launch.cuh"
 #include "store.cuh"
@@ -27,49 +33,90 @@
 namespace ottk {
 namespace dwt {
 
-constexpr int CG = 32;  // channels per CTA (one warp's lanes)
+constexpr int CG = 32;  // channels per CTA: eight lanes of four channels
 constexpr int THREADS = 256;
+constexpr int LOAD_CH = 8;              // channels per load item (fp32 input)
 enum : int { EPI_S8 = 0, EPI_S8_HALF_AWAY = 1, EPI_F32 = 2 };
 
 struct Tile {
-    int ty, txo;      // output rows / columns per CTA (txo % 4 == 0)
-    int ir, rp, ps;   // input tile: rows, row pitch and plane stride in 32-bit words (ps odd)
-    int orp, ops;     // output staging planes: row pitch (= txo/4) and plane stride in words (ops odd)
+    int ty, nxq;          // output rows / groups of 4 output columns per CTA
+    int nrg, rpt;         // row groups per CTA and rows of one group (= per thread)
+    int ir, rp, ps;       // input tile: rows, row pitch and plane stride in 32-bit words (ps odd)
     int tiles_y, tiles_x, cgroups;
-    int threads;      // CTA size: one warp per group of 4 output columns, at most 8 warps
+    int threads;
+    uint32_t div_rp, div_nxq;  // ceil(2^20 / x): exact quotients for the small indices they are used on
 };
 
 template <int K, int S>
 struct Geo {
-    static constexpr int KK = (K + 3) / 4;               // packed filter words per filter row
-    static constexpr int NW = (3 * S + 4 * KK + 3) / 4;  // aligned words a thread needs per input row
+    static constexpr int KK = (K + 3) / 4;           // packed filter words per filter row
+    static constexpr int NRAW = S == 1 ? 3 : 4;      // aligned words under a thread's 4 outputs, in one input row
 };
 
-// Windows of one input row for the thread's 4 outputs: dstw[t][kk] = bytes [t*S + 4*kk, +4) counted from the
-// first input column of output 0. `sh` (0..3) is the byte offset of that column inside its aligned word.
+// The last K input rows under the thread's 4 outputs, as windows in registers: win[slot][t] = bytes [t*S, +4) of the row counted
+// from the first input column of output 0 (slot = input row % K), and for K = 5 the fifth column's bytes of the last four rows.
 template <int K, int S>
-__device__ __forceinline__ void load_row_windows(const uint32_t* __restrict__ p, int sh8, uint32_t dstw[4][Geo<K, S>::KK]) {
-    constexpr int KK = Geo<K, S>::KK, NW = Geo<K, S>::NW;
-    uint32_t raw[NW + 1], al[NW];
+struct RowRing {
+    static constexpr int NAL = Geo<K, S>::NRAW - 1;
+    uint32_t win[K][4], vert[4], al[NAL];
+    static __device__ __forceinline__ constexpr int tail_word(int t) { return S == 1 ? 1 : 1 + (t >> 1); }
+    static __device__ __forceinline__ constexpr int tail_byte(int t) { return S == 1 ? t : 2 * (t & 1); }
+
+    // `sh` = 8 * the byte offset of output 0's first column inside its aligned word (modulo 32)
+    __device__ __forceinline__ void load(uint32_t (&w)[4], const uint32_t* __restrict__ p, int sh) {
+        uint32_t raw[NAL + 1];
 #pragma unroll
-    for (int i = 0; i < NW + 1; ++i) raw[i] = p[i];
+        for (int i = 0; i < NAL + 1; ++i) raw[i] = p[i];
 #pragma unroll
-    for (int i = 0; i < NW; ++i) al[i] = __funnelshift_r(raw[i], raw[i + 1], sh8);
+        for (int i = 0; i < NAL; ++i) al[i] = __funnelshift_r(raw[i], raw[i + 1], sh);
 #pragma unroll
-    for (int t = 0; t < 4; ++t)
-#pragma unroll
-        for (int kk = 0; kk < KK; ++kk) {
-            const int bo = t * S + 4 * kk;  // compile-time after unrolling
-            const int wi = bo >> 2, bs = (bo & 3) * 8;
-            dstw[t][kk] = bs == 0 ? al[wi] : __funnelshift_r(al[wi], wi + 1 < NW ? al[wi + 1] : 0u, bs);
+        for (int t = 0; t < 4; ++t) {
+            const int wi = (t * S) >> 2, bs = ((t * S) & 3) * 8;  // compile-time after unrolling
+            w[t] = bs == 0 ? al[wi] : __funnelshift_r(al[wi], al[wi + 1], bs);
         }
-}
+    }
+    // the fifth column, oldest row in byte 0: drop the oldest row, append the row last loaded
+    __device__ __forceinline__ void push_tail() {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) vert[t] = __byte_perm(vert[t], al[tail_word(t)], 0x0321 | ((4 + tail_byte(t)) << 12));
+    }
+    __device__ __forceinline__ void prime(int r, const uint32_t* __restrict__ p, int sh) {
+        load(win[r % K], p, sh);
+        if (K == 5) {
+            if (r == 0) vert[0] = vert[1] = vert[2] = vert[3] = 0u;
+            push_tail();
+        }
+    }
+    // Loads the S rows that output row R (mod K) needs beyond those of the row before it and multiplies.
+    template <int R>
+    __device__ __forceinline__ void advance(const uint32_t* __restrict__& p, int rp, int& sh, int wmod8, const uint32_t (&wk)[K], uint32_t wv,
+                                            uint32_t w44, int (&acc)[4]) {
+        constexpr int base = (R * S) % K;
+#pragma unroll
+        for (int ky = K - S; ky < K; ++ky) {
+            if (K == 5 && ky > K - S) push_tail();  // (stride 2: the first of the two new rows)
+            load(win[(base + ky) % K], p, sh);
+            p += rp;
+            sh += wmod8;
+        }
+#pragma unroll
+        for (int ky = 0; ky < K; ++ky)
+#pragma unroll
+            for (int t = 0; t < 4; ++t) acc[t] = __dp4a((int)win[(base + ky) % K][t], (int)wk[ky], acc[t]);
+        if (K == 5) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                acc[t] = __dp4a((int)vert[t], (int)wv, acc[t]);
+                acc[t] = __dp4a((int)al[tail_word(t)], (int)(w44 << (8 * tail_byte(t))), acc[t]);
+            }
+            push_tail();
+        }
+    }
+};
 
 template <int EPI, int ACT>
-__device__ __forceinline__ int epi_s8(int acc, float si, float bi, float so, int has_bias, float p0) {
-    const float a = __int2float_rn(acc);
-    float v = has_bias ? __fmaf_rn(a, si, bi) : __fmul_rn(a, si);
-    v = activate_t<ACT>(v, p0);
+__device__ __forceinline__ int epi_s8(int acc, float si, float bi, float so, float p0) {
+    const float v = activate_t<ACT>(__fmaf_rn(__int2float_rn(acc), si, bi), p0);
     const float t = __fmul_rn(v, so);
     if (EPI == EPI_S8_HALF_AWAY) return float2int8(t, ROUND_HALF_AWAY);
     if (ACT == ACT_RELU || ACT == ACT_RELU6) return f2i8_nonneg(t);
@@ -78,16 +125,16 @@ __device__ __forceinline__ int epi_s8(int acc, float si, float bi, float so, int
 
 // Four accumulators of one channel -> four int8 in one word, the arithmetic as packed pairs (each lane rounds like epi_s8).
 template <int EPI, int ACT>
-__device__ __forceinline__ uint32_t epi_s8x4(const int (&acc)[4], float si, float bi, float so, int has_bias, float p0) {
+__device__ __forceinline__ uint32_t epi_s8x4(const int (&acc)[4], float si, float bi, float so, float p0) {
     if (EPI == EPI_S8_HALF_AWAY)
-        return pack_sat_s8x4(epi_s8<EPI, ACT>(acc[0], si, bi, so, has_bias, p0), epi_s8<EPI, ACT>(acc[1], si, bi, so, has_bias, p0),
-                             epi_s8<EPI, ACT>(acc[2], si, bi, so, has_bias, p0), epi_s8<EPI, ACT>(acc[3], si, bi, so, has_bias, p0));
+        return pack_sat_s8x4(epi_s8<EPI, ACT>(acc[0], si, bi, so, p0), epi_s8<EPI, ACT>(acc[1], si, bi, so, p0),
+                             epi_s8<EPI, ACT>(acc[2], si, bi, so, p0), epi_s8<EPI, ACT>(acc[3], si, bi, so, p0));
     const float2 s2 = make_float2(si, si), b2 = make_float2(bi, bi), o2 = make_float2(so, so);
     int q[4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const float2 a = make_float2(__int2float_rn(acc[2 * h]), __int2float_rn(acc[2 * h + 1]));
-        const float2 v = has_bias ? __ffma2_rn(a, s2, b2) : __fmul2_rn(a, s2);
+        const float2 v = __ffma2_rn(a, s2, b2);
         const float2 t = __fmul2_rn(make_float2(activate_t<ACT>(v.x, p0), activate_t<ACT>(v.y, p0)), o2);
         if (ACT == ACT_RELU || ACT == ACT_RELU6) {
             const float2 r = __fadd2_rn(t, make_float2(0.5f, 0.5f));
@@ -102,54 +149,24 @@ __device__ __forceinline__ uint32_t epi_s8x4(const int (&acc)[4], float si, floa
     return pack_sat_s8x4(q[0], q[1], q[2], q[3]);
 }
 
-// One output row for the thread. R = (output row index) % K selects, at compile time, which ring slots hold
-// the K input rows: input row r lives in slot r % K, and output row oy needs rows oy*S + ky.
-template <int K, int S, int EPI, int ACT, int R>
-__device__ __forceinline__ void row_step(int oy, const uint32_t* __restrict__ plane, const Tile& T, int xq, int sh8,
-                                         uint32_t (&win)[K][4][Geo<K, S>::KK], const uint32_t (&wk)[K][Geo<K, S>::KK],
-                                         float si, float bi, float so, const EpilogueParams& ep, uint32_t* __restrict__ oplane_s,
-                                         float* __restrict__ of32, int ow_left) {
-    constexpr int KK = Geo<K, S>::KK;
-    constexpr int base = (R * S) % K;
-    // the S rows this output row needs beyond those of the previous one
-#pragma unroll
-    for (int ky = K - S; ky < K; ++ky) load_row_windows<K, S>(plane + (oy * S + ky) * T.rp + xq * S, sh8, win[(base + ky) % K]);
-    int acc[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int ky = 0; ky < K; ++ky)
-#pragma unroll
-        for (int kk = 0; kk < KK; ++kk)
-#pragma unroll
-            for (int t = 0; t < 4; ++t) acc[t] = __dp4a((int)win[(base + ky) % K][t][kk], (int)wk[ky][kk], acc[t]);
-    if (EPI != EPI_F32) {
-        oplane_s[oy * T.orp + xq] = epi_s8x4<EPI, ACT>(acc, si, bi, so, ep.has_bias, ep.act_param0);
-    } else if (of32) {
-        float v[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const float a = __int2float_rn(acc[t]);
-            v[t] = activate_t<ACT>(ep.has_bias ? __fmaf_rn(a, si, bi) : __fmul_rn(a, si), ep.act_param0);
-        }
-        if (ow_left >= 4 && (reinterpret_cast<uintptr_t>(of32) & 15) == 0) {
-            *reinterpret_cast<float4*>(of32) = make_float4(v[0], v[1], v[2], v[3]);
-        } else {
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-                if (t < ow_left) of32[t] = v[t];
-        }
-    }
+// Quantize four pixels of one channel under either rounding rule.
+__device__ __forceinline__ uint32_t quantize_word(const float4& v, float sc, bool away) {
+    if (!away) return quantize4_pack(v.x, v.y, v.z, v.w, sc);
+    return pack4(quantize1(v.x, sc, ROUND_HALF_AWAY), quantize1(v.y, sc, ROUND_HALF_AWAY), quantize1(v.z, sc, ROUND_HALF_AWAY),
+                 quantize1(v.w, sc, ROUND_HALF_AWAY));
 }
 
 template <int K, int S, bool IN_F32, int EPI, int ACT>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, K == 3 ? 4 : 3)
 depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ PlaneGather G, const uint32_t* __restrict__ wq,
-                       const float* __restrict__ in_scales, int n_in_scales, EpilogueParams ep, void* __restrict__ out, ConvShape s, Tile T) {
+                       const float* __restrict__ in_scales, int n_in_scales, EpilogueParams ep, void* __restrict__ out, ConvShape s, Tile T,
+                       int aligned) {
     constexpr int KK = Geo<K, S>::KK;
     extern __shared__ uint32_t smem[];
+    __shared__ const float* ch_ptr[CG];
+    __shared__ float ch_scale[CG];
     pdl_launch_dependents();
-    pdl_wait();
-    uint32_t* tin = smem;                  // [32][ir][rp] (+pad): int8 channel planes of the input tile
-    uint32_t* tout = smem + CG * T.ps;     // [32][ty][orp] (+pad): int8 channel planes of the output tile
+    uint32_t* tin = smem;  // [32][ir][rp] (+pad): int8 channel planes of the input tile
 
     int b = blockIdx.x;
     const int cg = b % T.cgroups; b /= T.cgroups;
@@ -157,206 +174,275 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
     const int tyi = b % T.tiles_y;
     const int img = b / T.tiles_y;
     const int c0 = cg * CG;
-    const int oy0 = tyi * T.ty, ox0 = tx * T.txo;
+    const int oy0 = tyi * T.ty, ox0 = tx * T.nxq * 4;
     const int iy0 = oy0 * S - s.ph;
-    const int ix_first = ox0 * S - s.pw;                                   // first input column the tile needs
-    const int ix_al = (ix_first >= 0 ? ix_first : ix_first - 3) / 4 * 4;   // rounded down to a multiple of 4
-    const int sh8 = (ix_first - ix_al) * 8;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ix_first = ox0 * S - s.pw;  // first input column the tile needs
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
+
+    // the lane's channel: filter and epilogue constants (they do not depend on the previous kernel)
+    const int c = c0 + lane;
+    const bool c_ok = c < s.cout_pad;
+    uint32_t wk[K], wv = 0u, w44 = 0u;  // filter rows, first four columns; the fifth column's first four rows; its last row
+    {
+        uint32_t wd[K * KK];
+#pragma unroll
+        for (int i = 0; i < K * KK; ++i) wd[i] = c_ok ? __ldg(wq + (long)c * K * KK + i) : 0u;
+#pragma unroll
+        for (int ky = 0; ky < K; ++ky) wk[ky] = wd[ky * KK];
+        if (K == 5) {
+            wv = __byte_perm(__byte_perm(wd[1], wd[3], 0x0040), __byte_perm(wd[5], wd[7], 0x0040), 0x5410);
+            w44 = wd[9];
+        }
+    }
+    const float p_si = c_ok ? __ldg(ep.scale_in + c) : 0.f;
+    // fma(a, s, -0.0) is a * s to the last bit (sign of zero included), so a layer without bias needs no code of its own
+    const float p_bi = c_ok && ep.has_bias ? __ldg(ep.bias + c) : -0.0f;
+    const float p_so = c_ok && EPI != EPI_F32 ? __ldg(ep.scale_out + c) : 0.f;
+    if (IN_F32 && tid < CG && c0 + tid < s.cin) {
+        ch_ptr[tid] = G.plane(c0 + tid, img, (long)s.h * s.w);
+        ch_scale[tid] = n_in_scales == 1 ? __ldg(in_scales) : __ldg(in_scales + c0 + tid);
+    }
+    if (IN_F32) __syncthreads();
+    pdl_wait();
 
     // ---- 1. load the input tile ----
+    const int npos = T.ir * T.rp;
+    const int wmod = IN_F32 && !aligned ? s.w & 3 : 0;  // how the byte offset of a row's first pixel moves from row to row
     if (IN_F32) {
-        // warp = channel (4 per warp), lanes run over the (row, word) positions of the channel's plane
-        const bool vec_ok = (s.w % 4 == 0) && ep.rounding == ROUND_ADD_HALF_TRUNC;
-        const int per_plane = T.ir * T.rp;
-        const float inv_rp = 1.0f / (float)T.rp;
-        for (int cl = warp; cl < CG; cl += (int)blockDim.x / 32) {
-            const int c = c0 + cl;
-            uint32_t* dst = tin + cl * T.ps;
-            if (c >= s.cin) {
-                for (int i = lane; i < per_plane; i += 32) dst[i] = 0u;
-                continue;
-            }
-            const float sc = n_in_scales == 1 ? __ldg(in_scales) : __ldg(in_scales + c);
-            const float* xc = G.plane(c, img, (long)s.h * s.w);
-            if (vec_ok) {
-                // every aligned float4 is either wholly inside the image or wholly outside (w % 4 == 0, ix % 4 == 0);
-                // four independent loads per thread are issued before any is used
-                for (int i0 = lane; i0 < per_plane; i0 += 128) {
-                    float4 v[4];
+        const bool away = ep.rounding == ROUND_HALF_AWAY;
+        const int chunks = (min(CG, s.cin - c0) + LOAD_CH - 1) / LOAD_CH;
+        for (int i = tid, chunk = 0; ; i += (int)blockDim.x) {
+            while (i >= npos) { i -= npos; ++chunk; }
+            if (chunk >= chunks) break;
+            const int r = (int)(((uint32_t)i * T.div_rp) >> 20), xw = i - r * T.rp;
+            const int iy = iy0 + r, cl0 = chunk * LOAD_CH;
+            const bool row_ok = iy >= 0 && iy < s.h;
+            // (the planes past the last channel of an incomplete chunk repeat its last one: their filters are zero)
+            const int cl_last = min(CG, s.cin - c0) - 1;
+            uint32_t* dst = tin + cl0 * T.ps + i;
+            if (aligned) {
+                // every 16-byte word lies wholly inside the row or wholly outside
+                const int ix = (ix_first & ~3) + xw * 4;
+                if (row_ok && ix >= 0 && ix < s.w) {
+                    const int off = iy * s.w + ix;
+                    float4 v[LOAD_CH];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int i = i0 + 32 * u;
-                        const int r = (int)(((float)i + 0.5f) * inv_rp);
-                        const int xw = i - r * T.rp;
-                        const int iy = iy0 + r, ix = ix_al + xw * 4;
-                        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (i < per_plane && iy >= 0 && iy < s.h && ix >= 0 && ix < s.w)
-                            v[u] = __ldg(reinterpret_cast<const float4*>(xc + (long)iy * s.w + ix));
-                    }
+                    for (int k = 0; k < LOAD_CH; ++k) v[k] = __ldg(reinterpret_cast<const float4*>(ch_ptr[min(cl0 + k, cl_last)] + off));
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int i = i0 + 32 * u;
-                        if (i < per_plane) dst[i] = quantize4_pack(v[u].x, v[u].y, v[u].z, v[u].w, sc);
-                    }
+                    for (int k = 0; k < LOAD_CH; ++k) dst[k * T.ps] = quantize_word(v[k], ch_scale[min(cl0 + k, cl_last)], away);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < LOAD_CH; ++k) dst[k * T.ps] = 0u;
                 }
             } else {
-                int r = lane / T.rp, xw = lane - r * T.rp;
-                for (int i = lane; i < per_plane; i += 32) {
-                    const int iy = iy0 + r, ix = ix_al + xw * 4;
-                    uint32_t word = 0;
-                    if (iy >= 0 && iy < s.h && ix + 3 >= 0 && ix < s.w) {
-                        const float* row = xc + (long)iy * s.w;
-                        int q[4] = {0, 0, 0, 0};
+                // the word that starts on a 16-byte boundary of the tensor: whole words inside the row are one load, words that
+                // reach over a row's end take their pixels one by one
+                float4 v[LOAD_CH];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (ix + j >= 0 && ix + j < s.w) q[j] = quantize1(__ldg(row + ix + j), sc, ep.rounding);
-                        word = pack4(q[0], q[1], q[2], q[3]);
+                for (int k = 0; k < LOAD_CH; ++k) {
+                    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (row_ok) {
+                        const float* row = ch_ptr[min(cl0 + k, cl_last)] + iy * s.w;
+                        const int sh = ((int)(reinterpret_cast<uintptr_t>(row) >> 2) + ix_first) & 3;
+                        const int ix = ix_first - sh + xw * 4;
+                        if (ix >= 0 && ix + 3 < s.w) {
+                            v[k] = __ldg(reinterpret_cast<const float4*>(row + ix));
+                        } else {
+                            if (ix >= 0 && ix < s.w) v[k].x = __ldg(row + ix);
+                            if (ix + 1 >= 0 && ix + 1 < s.w) v[k].y = __ldg(row + ix + 1);
+                            if (ix + 2 >= 0 && ix + 2 < s.w) v[k].z = __ldg(row + ix + 2);
+                            if (ix + 3 >= 0 && ix + 3 < s.w) v[k].w = __ldg(row + ix + 3);
+                        }
                     }
-                    dst[i] = word;
-                    xw += 32;
-                    while (xw >= T.rp) { xw -= T.rp; ++r; }
                 }
+#pragma unroll
+                for (int k = 0; k < LOAD_CH; ++k) dst[k * T.ps] = quantize_word(v[k], ch_scale[min(cl0 + k, cl_last)], away);
             }
         }
     } else {
         // Each 16-channel group is read from one tensor: the layer's own input, or (a layer created with gathered input)
         // 16 channels of one of several source tensors, named by the table: ref = (tensor << 24) | first channel, and
         // img_stride[tensor] = that tensor's channel stride.
-        const int half = threadIdx.x & 1;  // blockDim.x is even: a thread stays on its half
-        const int c = c0 + half * 16;
-        const int8_t* x = static_cast<const int8_t*>(xin) + (long)img * s.h * s.w * s.cin_pad + c;
+        const int half = tid & 1;  // blockDim.x is even: a thread stays on its half
+        const int ch = c0 + half * 16;
+        const int8_t* x = static_cast<const int8_t*>(xin) + (long)img * s.h * s.w * s.cin_pad + ch;
         long pitch = s.cin_pad;
-        if (G.base[0] != nullptr && c < s.cin_pad) {
-            const uint32_t ref = G.ref[c >> 4];
+        if (G.base[0] != nullptr && ch < s.cin_pad) {
+            const uint32_t ref = G.ref[ch >> 4];
             pitch = (long)G.img_stride[ref >> 24];
             x = reinterpret_cast<const int8_t*>(G.base[ref >> 24]) + (long)img * s.h * s.w * pitch + (ref & 0xFFFFFFu);
         }
-        const int items = T.ir * T.rp * 2;  // (pixel quad, 16-channel half)
-        for (int i = threadIdx.x; i < items; i += (int)blockDim.x) {
-            const int xw = (i >> 1) % T.rp;
-            const int r = (i >> 1) / T.rp;
-            const int iy = iy0 + r, ix = ix_al + xw * 4;
-            uint4 v[4];
+        if (ch < s.cin_pad) {
+            for (int i = tid >> 1; i < npos; i += (int)blockDim.x >> 1) {  // one pixel quad
+                const int r = (int)(((uint32_t)i * T.div_rp) >> 20), xw = i - r * T.rp;
+                const int iy = iy0 + r, ix = (ix_first & ~3) + xw * 4;
+                const bool row_ok = iy >= 0 && iy < s.h;
+                uint4 v[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                v[j] = make_uint4(0, 0, 0, 0);
-                if (c < s.cin_pad && iy >= 0 && iy < s.h && ix + j >= 0 && ix + j < s.w)
-                    v[j] = __ldg(reinterpret_cast<const uint4*>(x + ((long)iy * s.w + ix + j) * pitch));
+                for (int j = 0; j < 4; ++j) {
+                    v[j] = make_uint4(0, 0, 0, 0);
+                    if (row_ok && ix + j >= 0 && ix + j < s.w) v[j] = __ldg(reinterpret_cast<const uint4*>(x + ((long)iy * s.w + ix + j) * pitch));
+                }
+                uint32_t* dst = tin + (half * 16) * T.ps + i;
+                uint32_t o[4];
+                transpose4x4(v[0].x, v[1].x, v[2].x, v[3].x, o);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) dst[(0 + k) * T.ps] = o[k];
+                transpose4x4(v[0].y, v[1].y, v[2].y, v[3].y, o);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) dst[(4 + k) * T.ps] = o[k];
+                transpose4x4(v[0].z, v[1].z, v[2].z, v[3].z, o);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) dst[(8 + k) * T.ps] = o[k];
+                transpose4x4(v[0].w, v[1].w, v[2].w, v[3].w, o);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) dst[(12 + k) * T.ps] = o[k];
             }
-            uint32_t* dst = tin + (half * 16) * T.ps + r * T.rp + xw;
-            uint32_t o[4];
-            transpose4x4(v[0].x, v[1].x, v[2].x, v[3].x, o);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dst[(0 + k) * T.ps] = o[k];
-            transpose4x4(v[0].y, v[1].y, v[2].y, v[3].y, o);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dst[(4 + k) * T.ps] = o[k];
-            transpose4x4(v[0].z, v[1].z, v[2].z, v[3].z, o);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dst[(8 + k) * T.ps] = o[k];
-            transpose4x4(v[0].w, v[1].w, v[2].w, v[3].w, o);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dst[(12 + k) * T.ps] = o[k];
         }
     }
     __syncthreads();
 
     // ---- 2. compute + 3. epilogue ----
-    const int c = c0 + lane;
-    const bool c_ok = c < s.cout_pad;
-    uint32_t wk[K][KK];
-#pragma unroll
-    for (int ky = 0; ky < K; ++ky)
-#pragma unroll
-        for (int kk = 0; kk < KK; ++kk) wk[ky][kk] = c_ok ? __ldg(wq + ((long)c * K + ky) * KK + kk) : 0u;
-    const float p_si = c_ok ? __ldg(ep.scale_in + c) : 0.f;
-    const float p_bi = c_ok ? __ldg(ep.bias + c) : 0.f;
-    const float p_so = c_ok ? __ldg(ep.scale_out + c) : 0.f;
-    const uint32_t* plane = tin + lane * T.ps;
-    uint32_t* oplane_s = tout + lane * T.ops;
     const int rows_out = min(T.ty, s.oh - oy0);
     const long oplane = (long)s.oh * s.ow;
-
-    for (int xq = warp; xq < T.txo / 4; xq += (int)blockDim.x / 32) {
-        const int ox = ox0 + xq * 4;
-        if (ox >= s.ow) break;
-        uint32_t win[K][4][KK];
-        // prime the ring with the first K-S input rows (slot = row % K)
+    const uint32_t* plane = tin + lane * T.ps;
+    // byte offset of the tile's first input column in its first aligned word, times 8; row r's is wmod8 * r further (mod 32: the
+    // funnel shifts take their amount modulo 32)
+    int sh8 = ix_first * 8;
+    if (IN_F32 && !aligned && c < s.cin) sh8 += ((int)(reinterpret_cast<uintptr_t>(ch_ptr[lane]) >> 2) + iy0 * wmod) * 8;
+    const int wmod8 = wmod * 8;
+    // int8 output: after the exchange below lane 4k + p holds pixel p's channels 4k .. 4k + 3
+    const int px = lane & 3, cq = c0 + (lane & ~3);
+    const uint32_t sel_a = px < 2 ? 0x5410u : 0x3276u, sel_b = (px & 1) == 0 ? 0x6240u : 0x3715u;
+    for (int item = warp; item < T.nxq * T.nrg; item += nwarps) {
+        const int rg = (int)(((uint32_t)item * T.div_nxq) >> 20), xq = item - rg * T.nxq;
+        const int ox = ox0 + xq * 4, r0 = rg * T.rpt;
+        const int nrows = min(T.rpt, rows_out - r0);
+        if (ox >= s.ow || nrows <= 0) continue;  // warp-uniform
+        RowRing<K, S> ring;
+        const uint32_t* p = plane + r0 * S * T.rp + xq * S;
+        int sh = sh8 + r0 * S * wmod8;
 #pragma unroll
-        for (int r = 0; r < K - S; ++r) load_row_windows<K, S>(plane + r * T.rp + xq * S, sh8, win[r % K]);
-        float* of32 = nullptr;
-        if (EPI == EPI_F32 && c < s.cout)
-            of32 = reinterpret_cast<float*>(out) + ((long)img * s.cout + c) * oplane + (long)oy0 * s.ow + ox;
-        const int ow_left = s.ow - ox;
-#define OTT_DW_STEP(R)                                                                                                  \
-    if (oy + R < rows_out)                                                                                              \
-        row_step<K, S, EPI, ACT, R>(oy + R, plane, T, xq, sh8, win, wk, p_si, p_bi, p_so, ep, oplane_s,                  \
-                                    of32 ? of32 + (long)(oy + R) * s.ow : nullptr, ow_left);
-        for (int oy = 0; oy < rows_out; oy += K) {
-            OTT_DW_STEP(0) OTT_DW_STEP(1) OTT_DW_STEP(2)
-            if (K > 3) { OTT_DW_STEP(3) OTT_DW_STEP(4) }
+        for (int r = 0; r < K - S; ++r) {
+            ring.prime(r, p, sh);
+            p += T.rp;
+            sh += wmod8;
         }
-#undef OTT_DW_STEP
-    }
-    if (EPI != EPI_F32) {
-        __syncthreads();
-        // planes -> channel-innermost: a thread takes 4 pixels x 16 channels (16 words), transposes, stores 4 x 16 B
-        int8_t* o = reinterpret_cast<int8_t*>(out);
-        const int items = rows_out * T.orp * 2;
-        for (int i = threadIdx.x; i < items; i += (int)blockDim.x) {
-            const int half = i & 1;
-            const int xq = (i >> 1) % T.orp, oy = (i >> 1) / T.orp;
-            const int cc = c0 + half * 16;
-            const int ox = ox0 + xq * 4;
-            if (ox >= s.ow || cc >= s.cout_pad) continue;
-            const uint32_t* src = tout + (half * 16) * T.ops + oy * T.orp + xq;
-            uint32_t px[4][4];  // [pixel][word of 4 channels]
+        int8_t* o8 = nullptr;
+        float* of = nullptr;
+        bool store_ok;
+        if (EPI == EPI_F32) {
+            of = reinterpret_cast<float*>(out) + ((long)img * s.cout + c) * oplane + (long)(oy0 + r0) * s.ow + ox;
+            store_ok = c < s.cout;
+        } else {
+            o8 = reinterpret_cast<int8_t*>(out) + (((long)img * s.oh + oy0 + r0) * s.ow + ox + px) * s.cout_pad + cq;
+            store_ok = ox + px < s.ow && cq < s.cout_pad;
+        }
+        const int ow_left = s.ow - ox;
+        const long row_step = EPI == EPI_F32 ? (long)s.ow : (long)s.ow * s.cout_pad;
+        auto step = [&](auto rc) {
+            constexpr int R = decltype(rc)::value;  // output row modulo K: fixes the ring slots at compile time
+            int acc[4] = {0, 0, 0, 0};
+            ring.template advance<R>(p, T.rp, sh, wmod8, wk, wv, w44, acc);
+            if (EPI != EPI_F32) {
+                uint32_t w = epi_s8x4<EPI, ACT>(acc, p_si, p_bi, p_so, ep.act_param0);
+                w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 2), sel_a);
+                w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 1), sel_b);
+                if (store_ok) *reinterpret_cast<uint32_t*>(o8) = w;
+                o8 += row_step;
+            } else {
+                float v[4];
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                uint32_t t4[4];
-                transpose4x4(src[(g * 4 + 0) * T.ops], src[(g * 4 + 1) * T.ops], src[(g * 4 + 2) * T.ops], src[(g * 4 + 3) * T.ops], t4);
+                for (int t = 0; t < 4; ++t) v[t] = activate_t<ACT>(__fmaf_rn(__int2float_rn(acc[t]), p_si, p_bi), ep.act_param0);
+                if (store_ok) {
+                    if (ow_left >= 4 && (reinterpret_cast<uintptr_t>(of) & 15) == 0) {
+                        *reinterpret_cast<float4*>(of) = make_float4(v[0], v[1], v[2], v[3]);
+                    } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) px[j][g] = t4[j];
+                        for (int t = 0; t < 4; ++t)
+                            if (t < ow_left) of[t] = v[t];
+                    }
+                }
+                of += row_step;
             }
-            int8_t* dst = o + (((long)img * s.oh + oy0 + oy) * s.ow + ox) * s.cout_pad + cc;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (ox + j < s.ow) *reinterpret_cast<uint4*>(dst + (long)j * s.cout_pad) = make_uint4(px[j][0], px[j][1], px[j][2], px[j][3]);
+        };
+        for (int oy = 0; oy < nrows; oy += K) {
+            step(std::integral_constant<int, 0>{});
+            if (oy + 1 < nrows) step(std::integral_constant<int, 1>{});
+            if (oy + 2 < nrows) step(std::integral_constant<int, 2>{});
+            if (K > 3) {
+                if (oy + 3 < nrows) step(std::integral_constant<int, 3>{});
+                if (oy + 4 < nrows) step(std::integral_constant<int, 4>{});
+            }
         }
     }
 }
 
-template <int K, int S>
+// Tile of a layer. Columns: equal tiles of at most 64 (stride 2: 40) outputs. Warps share the (column group, row group) items.
+// Rows: bands of equal height, as many rows as a channel plane of kPlaneWords words holds at most. Which number of bands is
+// best depends on how the CTAs fall on the SMs, so each is rated by the larger of what bounds it: the instructions of the SM with most CTAs (about 2.5 per cycle are
+// issued), or the latency of one CTA (memory round trip, then one warp's dependent instructions at six cycles each) times the
+// waves. The instruction counts are those of the inner loops: 26 per fp32 word loaded and quantized, 7 per 32 int8 quads
+// loaded and transposed, 46 / 75 per warp and output row of a 3x3 / 5x5 filter, 12 per row that only fills the ring.
+constexpr int kPlaneWords = 384, kSms = 148;
+template <int K, int S, bool IN_F32>
 inline Tile plan_tile(const ConvShape& s) {
-    constexpr int NW = Geo<K, S>::NW;
     Tile T{};
-    const int ow4 = (s.ow + 3) / 4 * 4;
-    T.txo = S == 1 ? (ow4 < 64 ? ow4 : 64) : (ow4 < 32 ? ow4 : 32);
-    const int ty_max = S == 1 ? (K == 3 ? 14 : 12) : (K == 3 ? 7 : 6);
-    // bands of equal height (20 rows -> 10 + 10, not 14 + 6), so no CTA is mostly idle
-    const int bands = (s.oh + ty_max - 1) / ty_max;
-    T.ty = (s.oh + bands - 1) / bands;
+    const int ow4 = (s.ow + 3) / 4, max_nxq = S == 1 ? 16 : 10;
+    T.tiles_x = (ow4 + max_nxq - 1) / max_nxq;
+    T.nxq = (ow4 + T.tiles_x - 1) / T.tiles_x;
+    T.rp = (T.nxq - 1) * S + Geo<K, S>::NRAW;
+    T.cgroups = (s.cout_pad + CG - 1) / CG;
+    const int ty_max = (kPlaneWords / T.rp - K) / S + 1;
+    const long per_band = (long)s.n * T.tiles_x * T.cgroups;
+    // a throughput-bound launch wants every warp to have the same work, a latency-bound one as many warps as there are
+    const int widths[2] = {T.nxq > 8 ? (T.nxq + 1) / 2 : T.nxq > 2 ? T.nxq : 2, THREADS / 32};
+    double best = 0;
+    for (int bands = (s.oh + ty_max - 1) / ty_max; bands <= s.oh; ++bands) {
+        const int ty = (s.oh + bands - 1) / bands, tiles_y = (s.oh + ty - 1) / ty;
+        if (tiles_y < bands) continue;  // no band is lower than with fewer of them
+        const long ctas = per_band * tiles_y;
+        const int npos = ((ty - 1) * S + K) * T.rp;
+        for (int w : widths) {
+            int nrg = 1;
+            while (T.nxq * nrg < w && ty > 2 * nrg) ++nrg;
+            const int rpt = (ty + nrg - 1) / nrg;
+            nrg = (ty + rpt - 1) / rpt;
+            const int passes = (T.nxq * nrg + w - 1) / w;
+            const double instr = npos * (IN_F32 ? 26.0 : 7.0) + passes * w * (rpt * (K == 3 ? 46.0 : 75.0) + (K - S) * 12.0);
+            int resident = 65536 / ((K == 3 ? 64 : 80) * 32 * w);
+            const int by_smem = 224 * 1024 / (CG * 4 * npos + 2048);
+            if (by_smem < resident) resident = by_smem;
+            const double waves = (double)ctas / ((double)kSms * resident);
+            const double busy = (double)((ctas + kSms - 1) / kSms) * instr / 2.5;
+            const double chain = (waves <= 1.0 ? 1.0 : waves + 0.5) * (1800.0 + 6.0 * instr / w);
+            const double score = busy > chain ? busy : chain;
+            if (T.ty != 0 && score >= best) continue;
+            best = score;
+            T.ty = ty; T.tiles_y = tiles_y; T.nrg = nrg; T.rpt = rpt; T.threads = 32 * w;
+        }
+        if (ty <= 2) break;
+    }
     T.ir = (T.ty - 1) * S + K;
-    T.rp = (T.txo / 4 - 1) * S + NW + 1 + 1;  // +1 realignment word, +1 because the tile origin is rounded down
     T.ps = T.ir * T.rp;
     if (T.ps % 2 == 0) T.ps += 1;
-    T.orp = T.txo / 4;
-    T.ops = T.ty * T.orp;
-    if (T.ops % 2 == 0) T.ops += 1;
-    T.tiles_y = (s.oh + T.ty - 1) / T.ty;
-    T.tiles_x = (s.ow + T.txo - 1) / T.txo;
-    T.cgroups = (s.cout_pad + CG - 1) / CG;
-    const int nxq = T.txo / 4;
-    T.threads = 32 * (nxq < 8 ? nxq : 8);
+    T.div_rp = ((1u << 20) + T.rp - 1) / T.rp;
+    T.div_nxq = ((1u << 20) + T.nxq - 1) / T.nxq;
     return T;
 }
 
 template <int K, int S, bool IN_F32, int EPI, int ACT>
 cudaError_t launch_t(cudaStream_t stream, const ConvShape& s, const void* x, const PlaneGather& G, const uint32_t* wq, const float* in_scales,
                      int n_in_scales, const EpilogueParams& ep, void* out) {
-    const Tile T = plan_tile<K, S>(s);
-    const size_t smem = ((size_t)CG * T.ps + (EPI != EPI_F32 ? (size_t)CG * T.ops : 0)) * 4;
+    const Tile T = plan_tile<K, S, IN_F32>(s);
+    const size_t smem = (size_t)CG * T.ps * 4;
+    // fp32 rows whose 16-byte words never cross a row's end: a width that is a multiple of 4 and 16-byte aligned planes
+    int aligned = s.w % 4 == 0 ? 1 : 0;
+    for (int i = 0, last = -1; IN_F32 && i < s.cin && aligned; ++i) {
+        const int b = (int)(G.ref[i] >> 24);
+        if (b != last && ((reinterpret_cast<uintptr_t>(G.base[b]) & 15) != 0 || G.img_stride[b] % 4 != 0)) aligned = 0;
+        last = b;
+    }
     auto kernel = depthwise_tiled_kernel<K, S, IN_F32, EPI, ACT>;
     static std::mutex mu;  // several host threads may drive different GPUs through this function at once
     static bool attr_set[64] = {};
@@ -372,7 +458,7 @@ cudaError_t launch_t(cudaStream_t stream, const ConvShape& s, const void* x, con
     }
     const long blocks = (long)s.n * T.tiles_y * T.tiles_x * T.cgroups;
     if (blocks == 0) return cudaSuccess;
-    return launch_overlapped(kernel, dim3((unsigned)blocks), dim3(T.threads), smem, stream, x, G, wq, in_scales, n_in_scales, ep, out, s, T);
+    return launch_overlapped(kernel, dim3((unsigned)blocks), dim3(T.threads), smem, stream, x, G, wq, in_scales, n_in_scales, ep, out, s, T, aligned);
 }
 
 template <int K, int S, bool IN_F32, int EPI>
