@@ -30,7 +30,7 @@ struct StemParams {
 template <int S, int OUT, int ACT>
 __global__ void __launch_bounds__(ST_TX * ST_TY)
 dense_stem_kernel(const float* __restrict__ x, const __grid_constant__ StemParams P, float in_scale, int has_bias, float act_p0,
-                  int rounding, void* __restrict__ out, ConvShape s, int tiles_x, int tiles_y) {
+                  uint32_t half, void* __restrict__ out, ConvShape s, int tiles_x, int tiles_y) {
     constexpr int IW = (ST_TX - 1) * S + 3, IH = (ST_TY - 1) * S + 3;  // input halo tile
     constexpr int RP = (IW + 3 + 3) / 4 + 1;                            // words per row (tile origin rounded down to 4)
     __shared__ uint32_t tin[3][IH][RP];
@@ -46,7 +46,7 @@ dense_stem_kernel(const float* __restrict__ x, const __grid_constant__ StemParam
 
     // ---- 1. quantize the halo tile ----
     const float* ximg = x + (long)img * 3 * s.h * s.w;
-    const bool vec_ok = (s.w % 4 == 0) && rounding == ROUND_ADD_HALF_TRUNC;
+    const bool vec_ok = s.w % 4 == 0;
     for (int i = threadIdx.x; i < 3 * IH * RP; i += ST_TX * ST_TY) {
         const int xw = i % RP, r = (i / RP) % IH, c = i / (RP * IH);
         const int iy = iy0 + r, ix = ix_al + xw * 4;
@@ -55,12 +55,12 @@ dense_stem_kernel(const float* __restrict__ x, const __grid_constant__ StemParam
             const float* row = ximg + ((long)c * s.h + iy) * s.w;
             if (vec_ok && ix >= 0 && ix + 3 < s.w) {
                 const float4 v = __ldg(reinterpret_cast<const float4*>(row + ix));
-                word = quantize4_pack(v.x, v.y, v.z, v.w, in_scale);
+                word = quantize4_pack(v.x, v.y, v.z, v.w, in_scale, half);
             } else {
                 int q[4] = {0, 0, 0, 0};
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (ix + j >= 0 && ix + j < s.w) q[j] = quantize1(__ldg(row + ix + j), in_scale, rounding);
+                    if (ix + j >= 0 && ix + j < s.w) q[j] = quantize1(__ldg(row + ix + j), in_scale, half);
                 word = pack4(q[0], q[1], q[2], q[3]);
             }
         }
@@ -112,7 +112,7 @@ dense_stem_kernel(const float* __restrict__ x, const __grid_constant__ StemParam
             if (OUT == DT_F32_NCHW) {
                 if (valid && co < s.cout) of32[(long)co * oplane] = v;
             } else {
-                qv[j] = float2int8(__fmul_rn(v, P.scale_out[co]), rounding);
+                qv[j] = float2int8(__fmul_rn(v, P.scale_out[co]), half);
             }
         }
         if (OUT == DT_S8_NHWC && valid) *reinterpret_cast<uint32_t*>(os8 + g * 4) = pack4(qv[0], qv[1], qv[2], qv[3]);
@@ -147,11 +147,11 @@ constexpr uint32_t SPM_TMEM_COLS = 128;       // 4 accumulators of 32 columns
 template <int S, int ACT, bool OUT8, bool C24>
 __global__ void __launch_bounds__(256)
 dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ StemParams P, float in_scale, int has_bias_arg, float act_p0,
-                           int rounding_arg, void* __restrict__ out_any, ConvShape s_arg, int ph_out, int pw_out, int tiles_x, int tiles_y, int pad_zero,
+                           uint32_t half_arg, void* __restrict__ out_any, ConvShape s_arg, int ph_out, int pw_out, int tiles_x, int tiles_y, int pad_zero,
                            uint32_t* __restrict__ status) {
     using namespace umma;
     const int has_bias = C24 ? 1 : has_bias_arg;
-    const int rounding = C24 ? (int)ROUND_ADD_HALF_TRUNC : rounding_arg;
+    const uint32_t half = C24 ? kHalfTrunc : half_arg;
     ConvShape s = s_arg;
     if (C24) { s.cout = 24; s.cout_pad = 32; }
     constexpr int IW = (SP_CX - 1) * S + 3, IH = (SP_CY - 1) * S + 3;
@@ -210,7 +210,7 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
     // quantized input halo tile, as int8 channel planes. All of a thread's loads are issued before the first is used: the CTA
     // runs its phases one after the other, so this phase's DRAM latency must be paid once, not once per loop trip.
     const float* ximg = x + (long)img * 3 * s.h * s.w;
-    const bool vec_ok = (s.w % 4 == 0) && rounding == ROUND_ADD_HALF_TRUNC;
+    const bool vec_ok = s.w % 4 == 0;
     constexpr int TIN_WORDS = 3 * IH * RP, TIN_TRIPS = (TIN_WORDS + 255) / 256;
     if (vec_ok) {
         float4 v[TIN_TRIPS];
@@ -227,7 +227,7 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
 #pragma unroll
         for (int u = 0; u < TIN_TRIPS; ++u) {
             const int i = threadIdx.x + 256 * u;
-            if (i < TIN_WORDS) (&tin[0][0][0])[i] = quantize4_pack(v[u].x, v[u].y, v[u].z, v[u].w, in_scale);
+            if (i < TIN_WORDS) (&tin[0][0][0])[i] = quantize4_pack(v[u].x, v[u].y, v[u].z, v[u].w, in_scale, half);
         }
     } else {
         for (int i = threadIdx.x; i < TIN_WORDS; i += 256) {
@@ -239,7 +239,7 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
                 int q[4] = {0, 0, 0, 0};
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (ix + j >= 0 && ix + j < s.w) q[j] = quantize1(__ldg(row + ix + j), in_scale, rounding);
+                    if (ix + j >= 0 && ix + j < s.w) q[j] = quantize1(__ldg(row + ix + j), in_scale, half);
                 word = pack4(q[0], q[1], q[2], q[3]);
             }
             (&tin[0][0][0])[i] = word;
@@ -369,11 +369,11 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
                 const float soa[4] = {so.x, so.y, so.z, so.w};
                 int qv[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float t = __fmul_rn(y[j], soa[j]);
-                    // after ReLU / ReLU6 t >= 0 (scales are positive): trunc(t + 0.5), the saturating pack clamps at 127
-                    qv[j] = 4 * q4 + j >= s.cout ? 0
-                            : ((ACT == ACT_RELU || ACT == ACT_RELU6) && rounding == ROUND_ADD_HALF_TRUNC) ? f2i8_nonneg(t) : float2int8(t, rounding);
+                for (int j = 0; j < 4; j += 2) {
+                    // after ReLU / ReLU6 nothing is negative (scales are positive); the saturating pack clamps at 127
+                    const int2 r = round2_act<ACT>(__fmul2_rn(make_float2(y[j], y[j + 1]), make_float2(soa[j], soa[j + 1])), half);
+                    qv[j] = 4 * q4 + j >= s.cout ? 0 : r.x;
+                    qv[j + 1] = 4 * q4 + j + 1 >= s.cout ? 0 : r.y;
                 }
                 *reinterpret_cast<uint32_t*>(static_cast<int8_t*>(out_any) + (((long)img * ph_out + py) * pw_out + px) * s.cout_pad + 4 * q4) =
                     pack_sat_s8x4(qv[0], qv[1], qv[2], qv[3]);
@@ -398,7 +398,7 @@ cudaError_t launch_act(cudaStream_t stream, const float* x, const StemParams& P,
     if (blocks == 0) return cudaSuccess;
     const dim3 grid((unsigned)blocks), block(ST_TX * ST_TY);
 #define OTT_STEM_LAUNCH(ACT) \
-    dense_stem_kernel<S, OUT, ACT><<<grid, block, 0, stream>>>(x, P, in_scale, ep.has_bias, ep.act_param0, ep.rounding, out, s, tiles_x, tiles_y)
+    dense_stem_kernel<S, OUT, ACT><<<grid, block, 0, stream>>>(x, P, in_scale, ep.has_bias, ep.act_param0, half_bits(ep.rounding), out, s, tiles_x, tiles_y)
     switch (ep.act_type) {
         case ACT_RELU: OTT_STEM_LAUNCH(ACT_RELU); break;
         case ACT_LRELU: OTT_STEM_LAUNCH(ACT_LRELU); break;
@@ -447,7 +447,7 @@ static cudaError_t launch_pool_s(cudaStream_t stream, const float* x, const Stem
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);            \
         if (e != cudaSuccess) return e;                                                                                   \
         e = launch_overlapped(kernel, dim3((unsigned)blocks), dim3(256), smem, stream, x, P, in_scale, ep.has_bias, ep.act_param0,        \
-                              ep.rounding, out, s, ph_out, pw_out, tiles_x, tiles_y, pad_zero, status);                    \
+                              half_bits(ep.rounding), out, s, ph_out, pw_out, tiles_x, tiles_y, pad_zero, status);                    \
         if (e != cudaSuccess) return e;                                                                                   \
     }
     switch (ep.act_type) {

@@ -75,7 +75,14 @@ __host__ __device__ inline SmemLayout smem_layout(const UmmaPlan& p) {
 // BUILD 1: compiled for two resident CTAs per SM (at most 102 registers per thread), which small layers need to hide latency;
 // BUILD 2: 576 threads (sixteen epilogue warps) for wide tiles with one CTA per SM; BUILD 0: 320 threads, one CTA per SM;
 // the one-CTA-per-SM plans of large layers use the build without that register limit.
-template <int OUT, int ACT, bool BIAS, int ROUND, int BUILD>
+//
+// A launch whose CTAs have one tile each is a serial chain (previous kernel -> activations -> MMAs -> epilogue -> end), so what
+// does not need the data stays off it: the producer has its first coordinates, its barrier's byte count and its descriptors
+// ready before it waits for the previous kernel and then issues the copy at once (stage and tap counters walk; the divisions
+// they replaced took 700 of the 1000 cycles between that wait and the first copy), the MMA issuer and the teardown wait for no
+// kernel at all, the epilogue warps work out their pixel before they wait for the accumulator, and tensor memory is freed
+// while the last rows are still being requantized.
+template <int OUT, int ACT, int BUILD>
 __global__ void __launch_bounds__(BUILD == 2 ? 64 + 32 * 16 : kMaxThreads, BUILD == 1 ? 2 : 1)
 dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant__ CUtensorMap tmB, const UmmaPlan P,
                   const ConvShape s, const EpilogueParams ep, void* __restrict__ out, uint32_t* __restrict__ status,
@@ -127,7 +134,7 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
             const int c = n_tile * P.bn + i;
             const bool in = c < s.cout_pad;
             sp[i] = in ? ep.scale_in[c] : 0.f;
-            sp[P.bn + i] = in ? ep.bias[c] : 0.f;
+            sp[P.bn + i] = in ? bias_or_neutral(ep, c) : 0.f;
             sp[2 * P.bn + i] = in ? ep.scale_out[c] : 0.f;
         }
     }
@@ -141,46 +148,49 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_wait();  // from here on the kernel reads activations and writes outputs: the previous kernel must be complete
 
     if (warp == 0) {
         if (lane == 0) {
             // ---- TMA producer (activations; the weights were requested during set-up) ----
-            uint32_t it = 0;
-            bool ok = true;
+            uint32_t st = 0, phase = 1;  // stage, and the parity that says it is free (the first round finds every stage free)
+            bool ok = true, waited = false;
+            const uint32_t load_bytes = P.gather && P.gather_whole ? (uint32_t)(kTileM * P.bkc * P.nkb)
+                                        : P.halo                    ? (uint32_t)(halo_w * halo_h * P.bkc)
+                                                                    : (uint32_t)kTileM * P.bkc;
             for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
-                int img, y0, x0;
-                if (P.flat) {
-                    img = 0; y0 = 0; x0 = m * kTileM;
-                } else {
-                    const int per_img = P.tiles_x * P.tiles_y;
-                    img = m / per_img;
-                    const int r = m - img * per_img;
-                    y0 = (r / P.tiles_x) * P.th * s.sh - s.ph;
-                    x0 = (r % P.tiles_x) * P.tw * s.sw - s.pw;
+                int img = 0, y0 = 0, x0 = m * kTileM;
+                if (!P.flat) {
+                    img = (int)fast_div((uint32_t)m, P.div_img);
+                    const int r = m - img * P.tiles_x * P.tiles_y, ty = (int)fast_div((uint32_t)r, P.div_tx);
+                    y0 = ty * P.th * s.sh - s.ph;
+                    x0 = (r - ty * P.tiles_x) * P.tw * s.sw - s.pw;
                 }
-                for (int kb = 0; kb < loads_per_tile; ++kb, ++it) {
-                    const uint32_t st = it % P.stages, ph = (it / P.stages) & 1u;
-                    if (!mbar_wait(bar_empty + 8u * st, ph ^ 1u, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
+                int cb = 0, kx = 0, ky = 0;  // per-tap loads: channel block and tap of the next box
+                for (int kb = 0; kb < loads_per_tile; ++kb) {
+                    const uint32_t full = bar_full + 8u * st, dst = sA + st * a_stage_bytes;
+                    if (!mbar_wait(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
+                    mbar_expect_tx(full, load_bytes);
+                    if (!waited) {
+                        pdl_wait();  // from here on the kernel reads what the previous one wrote
+                        waited = true;
+                    }
                     if (P.gather && P.gather_whole) {
-                        mbar_expect_tx(bar_full + 8u * st, (uint32_t)(kTileM * P.bkc * P.nkb));
                         for (int g = 0; g < P.nkb; ++g)
-                            tma_load_4d(&maps.tm[maps.block_src[g]], bar_full + 8u * st, sA + st * a_stage_bytes + (uint32_t)(g * kTileM * P.bkc),
-                                        (int)maps.block_x[g], x0, 0, 0);
+                            tma_load_4d(&maps.tm[maps.block_src[g]], full, dst + (uint32_t)(g * kTileM * P.bkc), (int)maps.block_x[g], x0, 0, 0);
                     } else if (P.gather) {
                         // K block kb = 32 channels of one of the source tensors (channels past that tensor's end arrive as zeros)
-                        mbar_expect_tx(bar_full + 8u * st, (uint32_t)kTileM * P.bkc);
-                        tma_load_4d(&maps.tm[maps.block_src[kb]], bar_full + 8u * st, sA + st * a_stage_bytes, (int)maps.block_x[kb], x0, 0, 0);
+                        tma_load_4d(&maps.tm[maps.block_src[kb]], full, dst, (int)maps.block_x[kb], x0, 0, 0);
                     } else if (P.halo) {
                         // the (8 + kw - 1) x (16 + kh - 1) pixels under the tile, one channel block; out-of-image pixels arrive as zeros
-                        mbar_expect_tx(bar_full + 8u * st, (uint32_t)(halo_w * halo_h * P.bkc));
-                        tma_load_4d(&maps.tm[0], bar_full + 8u * st, sA + st * a_stage_bytes, kb * P.bkc, x0, y0, img);
+                        tma_load_4d(&maps.tm[0], full, dst, kb * P.bkc, x0, y0, img);
                     } else {
-                        const int tap = kb / P.ncb, cb = kb - tap * P.ncb;
-                        const int ky = tap / s.kw, kx = tap - ky * s.kw;
-                        mbar_expect_tx(bar_full + 8u * st, (uint32_t)kTileM * P.bkc);
-                        tma_load_4d(&maps.tm[0], bar_full + 8u * st, sA + st * a_stage_bytes, cb * P.bkc, x0 + kx * s.dw, y0 + ky * s.dh, img);
+                        tma_load_4d(&maps.tm[0], full, dst, cb * P.bkc, x0 + kx * s.dw, y0 + ky * s.dh, img);
+                        if (++cb == P.ncb) {
+                            cb = 0;
+                            if (++kx == s.kw) { kx = 0; ++ky; }
+                        }
                     }
+                    if (++st == (uint32_t)P.stages) { st = 0; phase ^= 1u; }
                 }
             }
             if (!ok) {
@@ -194,15 +204,15 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
             // ---- MMA issuer ----
             bool ok = mbar_wait(bar_b, 0, abort_flag, status, 16u, P.wait_ns);
             tc_fence_after();
-            uint32_t it = 0, tile_i = 0;
+            pdl_wait();  // (no wait below is counted against its limit while the previous kernel still runs)
+            uint32_t st = 0, phase = 0, tile_i = 0;
             for (int m = m_first; ok && m < P.m_tiles; m += m_step, ++tile_i) {
                 const uint32_t buf = tile_i & acc_mask, use = tile_i >> acc_shift;
                 if (!mbar_wait(bar_tempty + 8u * buf, (use & 1u) ^ 1u, abort_flag, status, 4u, P.wait_ns)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d = tmem_base + buf * (uint32_t)P.acc_stride;
-                for (int kb = 0; kb < loads_per_tile; ++kb, ++it) {
-                    const uint32_t st = it % P.stages, ph = (it / P.stages) & 1u;
-                    if (!mbar_wait(bar_full + 8u * st, ph, abort_flag, status, 2u, P.wait_ns)) { ok = false; break; }
+                for (int kb = 0; kb < loads_per_tile; ++kb) {
+                    if (!mbar_wait(bar_full + 8u * st, phase, abort_flag, status, 2u, P.wait_ns)) { ok = false; break; }
                     tc_fence_after();
                     if (P.halo) {
                         // every filter tap reads the same halo tile through a view shifted by (ky, kx) pixels
@@ -268,62 +278,74 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
                         else steps(std::integral_constant<int, 1>{});
                     }
                     umma_commit(bar_empty + 8u * st);  // frees the A stage once these MMAs have read it
+                    if (++st == (uint32_t)P.stages) { st = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
                 umma_commit(bar_tfull + 8u * buf);  // accumulator complete
             }
+            // every accumulator read for the last time: the tensor memory can go back
+            for (uint32_t b = 0; ok && b <= acc_mask && b < tile_i; ++b)
+                ok = mbar_wait(bar_tempty + 8u * b, (((tile_i - 1 - b) >> acc_shift) & 1u), abort_flag, status, 4u, P.wait_ns);
+            if (!ok) *abort_flag = 1;
         }
+        __syncwarp();
+        // an aborted CTA frees the tensor memory only when all other warps have left (exited threads count as arrived)
+        if (*abort_flag) __syncthreads();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)P.tmem_cols) : "memory");
     } else {
         // ---- epilogue warps ----
         const int q = warp & 3;            // TMEM lane quarter this warp may read
         const int sub = (warp - 2) >> 2;   // which of the epi_warps/4 warps sharing that quarter
         const int col_step = 16 * (P.epi_warps / 4);
         const int row = q * 32 + lane;
+        const int row_y = row / P.tw, row_x = row - row_y * P.tw;
         const long plane = (long)s.oh * s.ow;
         const long total_pix = (long)s.n * plane;
         const float* s_si = reinterpret_cast<const float*>(base_ptr + L.params);
         const float* s_bi = s_si + P.bn;
         const float* s_so = s_bi + P.bn;
+        const uint32_t half = half_bits(ep.rounding);
         uint32_t tile_i = 0;
         bool ok = true;
+        pdl_wait();  // the outputs written below may still be read by the previous kernel
         for (int m = m_first; ok && m < P.m_tiles; m += m_step, ++tile_i) {
             const uint32_t buf = tile_i & acc_mask, use = tile_i >> acc_shift;
-            if (!mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
-            tc_fence_after();
             // which output pixel this thread's TMEM lane holds
             long pix;  // linear (img, oy, ox) index
+            long img = 0, inimg = 0;
             bool valid;
             if (P.flat) {
                 pix = (long)m * kTileM + row;
                 valid = pix < total_pix;
+                if (OUT == DT_F32_NCHW || (OUT == DT_S8_NHWC && mixed.out_f32 != nullptr)) {
+                    if (total_pix <= 0x7FFFFFFFl) {
+                        const uint32_t q32 = fast_div((uint32_t)pix, P.div_plane);
+                        img = (long)q32;
+                        inimg = pix - (long)q32 * plane;
+                    } else {
+                        img = pix / plane;
+                        inimg = pix - img * plane;
+                    }
+                }
             } else {
-                const int per_img = P.tiles_x * P.tiles_y;
-                const int img = m / per_img;
-                const int r = m - img * per_img;
-                const int oy = (r / P.tiles_x) * P.th + row / P.tw;
-                const int ox = (r % P.tiles_x) * P.tw + row % P.tw;
+                const int im = (int)fast_div((uint32_t)m, P.div_img);
+                const int r = m - im * P.tiles_x * P.tiles_y, ty = (int)fast_div((uint32_t)r, P.div_tx);
+                const int oy = ty * P.th + row_y, ox = (r - ty * P.tiles_x) * P.tw + row_x;
                 valid = oy < s.oh && ox < s.ow;
-                pix = (long)img * plane + (long)oy * s.ow + ox;
+                img = im;
+                inimg = (long)oy * s.ow + ox;
+                pix = img * plane + inimg;
             }
             const uint32_t taddr = tmem_base + buf * (uint32_t)P.acc_stride + ((uint32_t)(q * 32) << 16);
             int8_t* out_s8 = reinterpret_cast<int8_t*>(out) + pix * s.cout_pad + n_tile * P.bn;
             int32_t* out_s32 = reinterpret_cast<int32_t*>(out) + pix * s.cout_pad + n_tile * P.bn;
             float* out_f32 = nullptr;
-            if (OUT == DT_F32_NCHW || (OUT == DT_S8_NHWC && mixed.out_f32 != nullptr)) {
-                // (a 64-bit division costs about a hundred instructions per thread and tile; 32 bits cover any real tensor)
-                long img, inimg;
-                if (total_pix <= 0xFFFFFFFFll) {
-                    const uint32_t q32 = (uint32_t)pix / (uint32_t)plane;
-                    img = (long)q32;
-                    inimg = (long)((uint32_t)pix - q32 * (uint32_t)plane);
-                } else {
-                    img = pix / plane;
-                    inimg = pix - img * plane;
-                }
-                if (OUT == DT_S8_NHWC && mixed.plane_of_col != nullptr)
-                    out_f32 = mixed.out_f32 + img * mixed.f32_planes * plane + inimg;  // plane chosen per column below
-                else
-                    out_f32 = (OUT == DT_F32_NCHW ? reinterpret_cast<float*>(out) : mixed.out_f32) + (img * s.cout + n_tile * P.bn) * plane + inimg;
+            if (OUT == DT_F32_NCHW) {
+                out_f32 = reinterpret_cast<float*>(out) + (img * s.cout + n_tile * P.bn) * plane + inimg;
+            } else if (OUT == DT_S8_NHWC && mixed.out_f32 != nullptr) {
+                out_f32 = mixed.plane_of_col != nullptr ? mixed.out_f32 + img * mixed.f32_planes * plane + inimg  // plane chosen per column below
+                                                        : mixed.out_f32 + (img * s.cout + n_tile * P.bn) * plane + inimg;
             }
             // 16 accumulator columns -> 16 outputs of this thread's pixel. int8 results come back as 4 packed words in wds
             // (the caller stores them); the other output kinds are stored here.
@@ -346,7 +368,7 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
                         const float2 a = make_float2(__int2float_rn(v[g * 4 + 2 * h]), __int2float_rn(v[g * 4 + 2 * h + 1]));
                         const float2 s2 = h ? make_float2(si.z, si.w) : make_float2(si.x, si.y);
                         const float2 b2 = h ? make_float2(bi.z, bi.w) : make_float2(bi.x, bi.y);
-                        const float2 t = BIAS ? __ffma2_rn(a, s2, b2) : __fmul2_rn(a, s2);
+                        const float2 t = __ffma2_rn(a, s2, b2);
                         y[g * 4 + 2 * h] = activate_t<ACT>(t.x, ep.act_param0);
                         y[g * 4 + 2 * h + 1] = activate_t<ACT>(t.y, ep.act_param0);
                     }
@@ -383,19 +405,9 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
                         for (int h = 0; h < 2; ++h) {
                             const float2 t = __fmul2_rn(make_float2(y[g * 4 + 2 * h], y[g * 4 + 2 * h + 1]),
                                                         h ? make_float2(so.z, so.w) : make_float2(so.x, so.y));
-                            if (ROUND == ROUND_HALF_AWAY) {
-                                qv[2 * h] = float2int8(t.x, ROUND_HALF_AWAY);
-                                qv[2 * h + 1] = float2int8(t.y, ROUND_HALF_AWAY);
-                            } else if (ACT == ACT_RELU || ACT == ACT_RELU6) {
-                                // t >= 0 (or -0): trunc(t + 0.5), the upper clamp is the saturating pack
-                                const float2 r = __fadd2_rn(t, make_float2(0.5f, 0.5f));
-                                qv[2 * h] = __float2int_rz(r.x);
-                                qv[2 * h + 1] = __float2int_rz(r.y);
-                            } else {
-                                const float2 r = __fadd2_rn(t, make_float2(half_signed(t.x), half_signed(t.y)));
-                                qv[2 * h] = __float2int_rz(fmaxf(r.x, -127.5f));
-                                qv[2 * h + 1] = __float2int_rz(fmaxf(r.y, -127.5f));
-                            }
+                            const int2 rq = round2_act<ACT>(t, half);
+                            qv[2 * h] = rq.x;
+                            qv[2 * h + 1] = rq.y;
                         }
                         wds[g] = pack_sat_s8x4(qv[0], qv[1], qv[2], qv[3]);
                     }
@@ -404,6 +416,9 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
             // Chunks of 32 columns: two TMEM loads in flight, and int8 rows leave as one 32-byte store per thread, a whole
             // DRAM sector (two 16-byte stores from different warps would each touch half of it).
             const bool wide_ok = OUT == DT_S8_NHWC && ((s.cout_pad | (n_tile * P.bn)) & 31) == 0;
+            if (!mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
+            tc_fence_after();
+            if (sub * 32 >= P.bn && lane == 0) mbar_arrive(bar_tempty + 8u * buf);  // a narrow tile has no columns for this warp
             for (int col0 = sub * 32; col0 < P.bn; col0 += 2 * col_step) {
                 int va[16], vb[16];
                 const bool two = col0 + 16 < P.bn;
@@ -412,6 +427,11 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
                 if (two) tmem_ld16(taddr + (uint32_t)(col0 + 16), vb);
                 tmem_wait_ld16(va);
                 tmem_wait_ld16(vb);
+                if (col0 + 2 * col_step >= P.bn) {  // this warp's last columns: the accumulator may be overwritten from here on
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_tempty + 8u * buf);
+                }
                 if (!valid) continue;
                 uint32_t wa[4], wb[4];
                 const bool a_ok = n_tile * P.bn + col0 < s.cout_pad, b_ok = two && n_tile * P.bn + col0 + 16 < s.cout_pad;
@@ -441,18 +461,7 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
                     }
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_tempty + 8u * buf);
         }
-    }
-
-    // ---- teardown (every path ends here) ----
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)P.tmem_cols) : "memory");
     }
 }
 
@@ -477,7 +486,7 @@ CUtensorMapSwizzle swizzle_for(int bkc) {
     return bkc == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (bkc == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
-template <int OUT, int ACT, bool BIAS, int ROUND, int BUILD>
+template <int OUT, int ACT, int BUILD>
 const char* launch_variant(cudaStream_t stream, int sm_count, const KernelMaps& maps, const CUtensorMap& tmB, const UmmaPlan& p,
                            const ConvShape& s, const EpilogueParams& ep, void* out, uint32_t* status, const UmmaMixedOut& mixed) {
     // per-device, per-instantiation set-up; several host threads may drive different GPUs through this function at once
@@ -486,7 +495,7 @@ const char* launch_variant(cudaStream_t stream, int sm_count, const KernelMaps& 
     static int regs_per_thread[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    auto kernel = dense_umma_kernel<OUT, ACT, BIAS, ROUND, BUILD>;
+    auto kernel = dense_umma_kernel<OUT, ACT, BUILD>;
     int regs = 128;
     if (dev >= 0 && dev < 64) {
         std::lock_guard<std::mutex> lock(mu);
@@ -688,28 +697,29 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaPlan&
                 swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
     if (r != CUDA_SUCCESS) return "cuTensorMapEncodeTiled(activations) failed";
+    p.div_img = make_fast_div((uint32_t)(p.tiles_x * p.tiles_y));
+    p.div_tx = make_fast_div((uint32_t)p.tiles_x);
+    p.div_plane = make_fast_div((uint32_t)(s.oh * s.ow));
 
     const CUtensorMap& tmB = *reinterpret_cast<const CUtensorMap*>(weight_map);
     const char* err = nullptr;
-#define OTT_UMMA_LAUNCH(OUT, ACT, BIAS, ROUND)                                                                       \
-    err = p.ctas_per_sm > 1   ? launch_variant<OUT, ACT, BIAS, ROUND, 1>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed) \
-          : p.epi_warps == 16 ? launch_variant<OUT, ACT, BIAS, ROUND, 2>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed) \
-                              : launch_variant<OUT, ACT, BIAS, ROUND, 0>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed)
-#define OTT_UMMA_ACT(OUT, BIAS, ROUND)                                   \
-    switch (ep.act_type) {                                               \
-        case ACT_RELU: OTT_UMMA_LAUNCH(OUT, ACT_RELU, BIAS, ROUND); break;   \
-        case ACT_LRELU: OTT_UMMA_LAUNCH(OUT, ACT_LRELU, BIAS, ROUND); break; \
-        case ACT_RELU6: OTT_UMMA_LAUNCH(OUT, ACT_RELU6, BIAS, ROUND); break; \
-        default: OTT_UMMA_LAUNCH(OUT, ACT_NONE, BIAS, ROUND); break;         \
+#define OTT_UMMA_LAUNCH(OUT, ACT)                                                                                     \
+    err = p.ctas_per_sm > 1   ? launch_variant<OUT, ACT, 1>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed) \
+          : p.epi_warps == 16 ? launch_variant<OUT, ACT, 2>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed) \
+                              : launch_variant<OUT, ACT, 0>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed)
+#define OTT_UMMA_ACT(OUT)                                \
+    switch (ep.act_type) {                               \
+        case ACT_RELU: OTT_UMMA_LAUNCH(OUT, ACT_RELU); break;   \
+        case ACT_LRELU: OTT_UMMA_LAUNCH(OUT, ACT_LRELU); break; \
+        case ACT_RELU6: OTT_UMMA_LAUNCH(OUT, ACT_RELU6); break; \
+        default: OTT_UMMA_LAUNCH(OUT, ACT_NONE); break;         \
     }
     if (out_dtype == DT_S32_NHWC) {
-        OTT_UMMA_LAUNCH(DT_S32_NHWC, ACT_NONE, false, ROUND_ADD_HALF_TRUNC);
+        OTT_UMMA_LAUNCH(DT_S32_NHWC, ACT_NONE);
     } else if (out_dtype == DT_F32_NCHW) {
-        if (ep.has_bias) { OTT_UMMA_ACT(DT_F32_NCHW, true, ROUND_ADD_HALF_TRUNC) } else { OTT_UMMA_ACT(DT_F32_NCHW, false, ROUND_ADD_HALF_TRUNC) }
-    } else if (ep.rounding == ROUND_HALF_AWAY) {
-        if (ep.has_bias) { OTT_UMMA_ACT(DT_S8_NHWC, true, ROUND_HALF_AWAY) } else { OTT_UMMA_ACT(DT_S8_NHWC, false, ROUND_HALF_AWAY) }
+        OTT_UMMA_ACT(DT_F32_NCHW)
     } else {
-        if (ep.has_bias) { OTT_UMMA_ACT(DT_S8_NHWC, true, ROUND_ADD_HALF_TRUNC) } else { OTT_UMMA_ACT(DT_S8_NHWC, false, ROUND_ADD_HALF_TRUNC) }
+        OTT_UMMA_ACT(DT_S8_NHWC)
     }
 #undef OTT_UMMA_ACT
 #undef OTT_UMMA_LAUNCH

@@ -36,7 +36,7 @@ namespace dwt {
 constexpr int CG = 32;  // channels per CTA: eight lanes of four channels
 constexpr int THREADS = 256;
 constexpr int LOAD_CH = 8;              // channels per load item (fp32 input)
-enum : int { EPI_S8 = 0, EPI_S8_HALF_AWAY = 1, EPI_F32 = 2 };
+enum : int { EPI_S8 = 0, EPI_F32 = 1 };
 
 struct Tile {
     int ty, nxq;          // output rows / groups of 4 output columns per CTA
@@ -114,46 +114,17 @@ struct RowRing {
     }
 };
 
-template <int EPI, int ACT>
-__device__ __forceinline__ int epi_s8(int acc, float si, float bi, float so, float p0) {
-    const float v = activate_t<ACT>(__fmaf_rn(__int2float_rn(acc), si, bi), p0);
-    const float t = __fmul_rn(v, so);
-    if (EPI == EPI_S8_HALF_AWAY) return float2int8(t, ROUND_HALF_AWAY);
-    if (ACT == ACT_RELU || ACT == ACT_RELU6) return f2i8_nonneg(t);
-    return f2i8_lo_clamped(t);
-}
-
-// Four accumulators of one channel -> four int8 in one word, the arithmetic as packed pairs (each lane rounds like epi_s8).
-template <int EPI, int ACT>
-__device__ __forceinline__ uint32_t epi_s8x4(const int (&acc)[4], float si, float bi, float so, float p0) {
-    if (EPI == EPI_S8_HALF_AWAY)
-        return pack_sat_s8x4(epi_s8<EPI, ACT>(acc[0], si, bi, so, p0), epi_s8<EPI, ACT>(acc[1], si, bi, so, p0),
-                             epi_s8<EPI, ACT>(acc[2], si, bi, so, p0), epi_s8<EPI, ACT>(acc[3], si, bi, so, p0));
+// Four accumulators of one channel -> four int8 in one word, the arithmetic as packed pairs.
+template <int ACT>
+__device__ __forceinline__ uint32_t epi_s8x4(const int (&acc)[4], float si, float bi, float so, float p0, uint32_t half) {
     const float2 s2 = make_float2(si, si), b2 = make_float2(bi, bi), o2 = make_float2(so, so);
-    int q[4];
+    int2 q[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        const float2 a = make_float2(__int2float_rn(acc[2 * h]), __int2float_rn(acc[2 * h + 1]));
-        const float2 v = __ffma2_rn(a, s2, b2);
-        const float2 t = __fmul2_rn(make_float2(activate_t<ACT>(v.x, p0), activate_t<ACT>(v.y, p0)), o2);
-        if (ACT == ACT_RELU || ACT == ACT_RELU6) {
-            const float2 r = __fadd2_rn(t, make_float2(0.5f, 0.5f));
-            q[2 * h] = __float2int_rz(r.x);
-            q[2 * h + 1] = __float2int_rz(r.y);
-        } else {
-            const float2 r = __fadd2_rn(t, make_float2(half_signed(t.x), half_signed(t.y)));
-            q[2 * h] = __float2int_rz(fmaxf(r.x, -127.5f));
-            q[2 * h + 1] = __float2int_rz(fmaxf(r.y, -127.5f));
-        }
+        const float2 v = __ffma2_rn(make_float2(__int2float_rn(acc[2 * h]), __int2float_rn(acc[2 * h + 1])), s2, b2);
+        q[h] = round2_act<ACT>(__fmul2_rn(make_float2(activate_t<ACT>(v.x, p0), activate_t<ACT>(v.y, p0)), o2), half);
     }
-    return pack_sat_s8x4(q[0], q[1], q[2], q[3]);
-}
-
-// Quantize four pixels of one channel under either rounding rule.
-__device__ __forceinline__ uint32_t quantize_word(const float4& v, float sc, bool away) {
-    if (!away) return quantize4_pack(v.x, v.y, v.z, v.w, sc);
-    return pack4(quantize1(v.x, sc, ROUND_HALF_AWAY), quantize1(v.y, sc, ROUND_HALF_AWAY), quantize1(v.z, sc, ROUND_HALF_AWAY),
-                 quantize1(v.w, sc, ROUND_HALF_AWAY));
+    return pack_sat_s8x4(q[0].x, q[0].y, q[1].x, q[1].y);
 }
 
 template <int K, int S, bool IN_F32, int EPI, int ACT>
@@ -195,8 +166,8 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
         }
     }
     const float p_si = c_ok ? __ldg(ep.scale_in + c) : 0.f;
-    // fma(a, s, -0.0) is a * s to the last bit (sign of zero included), so a layer without bias needs no code of its own
-    const float p_bi = c_ok && ep.has_bias ? __ldg(ep.bias + c) : -0.0f;
+    const float p_bi = c_ok ? bias_or_neutral(ep, c) : 0.f;
+    const uint32_t half = half_bits(ep.rounding);
     const float p_so = c_ok && EPI != EPI_F32 ? __ldg(ep.scale_out + c) : 0.f;
     if (IN_F32 && tid < CG && c0 + tid < s.cin) {
         ch_ptr[tid] = G.plane(c0 + tid, img, (long)s.h * s.w);
@@ -209,7 +180,6 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
     const int npos = T.ir * T.rp;
     const int wmod = IN_F32 && !aligned ? s.w & 3 : 0;  // how the byte offset of a row's first pixel moves from row to row
     if (IN_F32) {
-        const bool away = ep.rounding == ROUND_HALF_AWAY;
         const int chunks = (min(CG, s.cin - c0) + LOAD_CH - 1) / LOAD_CH;
         for (int i = tid, chunk = 0; ; i += (int)blockDim.x) {
             while (i >= npos) { i -= npos; ++chunk; }
@@ -229,7 +199,7 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
 #pragma unroll
                     for (int k = 0; k < LOAD_CH; ++k) v[k] = __ldg(reinterpret_cast<const float4*>(ch_ptr[min(cl0 + k, cl_last)] + off));
 #pragma unroll
-                    for (int k = 0; k < LOAD_CH; ++k) dst[k * T.ps] = quantize_word(v[k], ch_scale[min(cl0 + k, cl_last)], away);
+                    for (int k = 0; k < LOAD_CH; ++k) dst[k * T.ps] = quantize4_pack(v[k].x, v[k].y, v[k].z, v[k].w, ch_scale[min(cl0 + k, cl_last)], half);
                 } else {
 #pragma unroll
                     for (int k = 0; k < LOAD_CH; ++k) dst[k * T.ps] = 0u;
@@ -256,7 +226,7 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
                     }
                 }
 #pragma unroll
-                for (int k = 0; k < LOAD_CH; ++k) dst[k * T.ps] = quantize_word(v[k], ch_scale[min(cl0 + k, cl_last)], away);
+                for (int k = 0; k < LOAD_CH; ++k) dst[k * T.ps] = quantize4_pack(v[k].x, v[k].y, v[k].z, v[k].w, ch_scale[min(cl0 + k, cl_last)], half);
             }
         }
     } else {
@@ -345,7 +315,7 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
             int acc[4] = {0, 0, 0, 0};
             ring.template advance<R>(p, T.rp, sh, wmod8, wk, wv, w44, acc);
             if (EPI != EPI_F32) {
-                uint32_t w = epi_s8x4<EPI, ACT>(acc, p_si, p_bi, p_so, ep.act_param0);
+                uint32_t w = epi_s8x4<ACT>(acc, p_si, p_bi, p_so, ep.act_param0, half);
                 w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 2), sel_a);
                 w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 1), sel_b);
                 if (store_ok) *reinterpret_cast<uint32_t*>(o8) = w;
@@ -479,9 +449,6 @@ cudaError_t launch_ks(cudaStream_t stream, const ConvShape& s, const void* x, co
     if (out_dtype == DT_F32_NCHW)
         return f32in ? launch_act<K, S, true, EPI_F32>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out)
                      : launch_act<K, S, false, EPI_F32>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);
-    if (ep.rounding == ROUND_HALF_AWAY)
-        return f32in ? launch_act<K, S, true, EPI_S8_HALF_AWAY>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out)
-                     : launch_act<K, S, false, EPI_S8_HALF_AWAY>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);
     return f32in ? launch_act<K, S, true, EPI_S8>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out)
                  : launch_act<K, S, false, EPI_S8>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);
 }

@@ -96,7 +96,7 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
     for (int i = threadIdx.x; i < P.cols; i += (int)blockDim.x) {
         const bool in = c_base + i < G.cpad;
         sp[i] = in ? ep.scale_in[c_base + i] : 0.f;
-        sp[P.cols + i] = in ? ep.bias[c_base + i] : 0.f;
+        sp[P.cols + i] = in ? bias_or_neutral(ep, c_base + i) : 0.f;
         sp[2 * P.cols + i] = in ? ep.scale_out[c_base + i] : 0.f;
     }
     if (warp == 1) {

@@ -9,6 +9,7 @@
 //   requantize  q = float2int8(v * scale_out)             Tensor/QuantizeX86.cpp:1723-1870
 //   float2int8  trunc(v + copysign(0.5, v)), clamp ±127   Tensor/VecIntrinsic.hpp:71-95   (rounding 0)
 //               round half away from zero, clamp ±127     Tensor/QuantizeX86.cpp:18-23    (rounding 1)
+//   no bias     fma(a, s, -0.0) is a * s to the last bit, the sign of zero included: bias_or_neutral below
 //   quantize    q = float2int8(x * scale)                 Tensor/QuantizeX86.cpp:396-549
 #pragma once
 
@@ -37,6 +38,9 @@ __device__ __forceinline__ float dequant(int acc, float scale_in, float bias, in
     return has_bias ? __fmaf_rn(a, scale_in, bias) : __fmul_rn(a, scale_in);
 }
 
+// the bias of a channel, or the value that makes the fma a plain product in a layer without bias
+__device__ __forceinline__ float bias_or_neutral(const EpilogueParams& ep, int c) { return ep.has_bias ? ep.bias[c] : -0.0f; }
+
 template <int ACT>
 __device__ __forceinline__ float activate_t(float v, float p0) {
     if (ACT == ACT_RELU) return v > 0.f ? v : 0.f;
@@ -54,41 +58,36 @@ __device__ __forceinline__ float activate(float v, int act, float p0) {
     }
 }
 
-// copysign(0.5, v) as one logic instruction: (bits(v) & 0x80000000) | bits(0.5). Written as lop3 with both constants in
+// Both int8 rounding rules are trunc(v + copysign(h, v)): h = 0.5 is the packed path's rule as it stands; with h = 0.5 - 2^-25,
+// the largest fp32 below one half, the same sum rounds half away from zero. (frac(v) >= 0.5: the exact sum lies at most 2^-25
+// below the next integer n and rounds to n, at n = 1 by ties-to-even; frac(v) < 0.5: it lies below n by more than half a step of
+// fp32 there. Checked for every fp32 value up to 2^23 in magnitude.) So the rule is a constant, not code of its own.
+constexpr uint32_t kHalfTrunc = 0x3F000000u, kHalfAway = 0x3EFFFFFFu;
+__host__ __device__ __forceinline__ uint32_t half_bits(int rounding) { return rounding == ROUND_HALF_AWAY ? kHalfAway : kHalfTrunc; }
+
+// copysign(h, v) as one logic instruction: (bits(v) & 0x80000000) | bits(h). Written as lop3 with both constants in
 // registers; the compiler's own form takes two instructions per value (a logic instruction carries one immediate).
-__device__ __forceinline__ float half_signed(float v) {
+__device__ __forceinline__ float half_signed(float v, uint32_t h) {
     uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(__float_as_uint(v)), "r"(0x80000000u), "r"(0x3F000000u));
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(__float_as_uint(v)), "r"(0x80000000u), "r"(h));
     return __uint_as_float(r);
 }
 
 // float -> int in [-127,127], kept as int so four of them can be packed by the caller.
-__device__ __forceinline__ int float2int8(float v, int rounding) {
-    int i;
-    if (rounding == ROUND_HALF_AWAY) {
-        const float t = truncf(v);
-        const float frac = __fsub_rn(v, t);  // exact
-        i = __float2int_rz(t);
-        if (fabsf(frac) >= 0.5f) i += (v < 0.f) ? -1 : 1;
-    } else {
-        const float adj = __fadd_rn(v, half_signed(v));
-        i = __float2int_rz(adj);
-    }
-    return max(-127, min(127, i));
-}
+__device__ __forceinline__ int float2int8(float v, uint32_t h) { return max(-127, min(127, __float2int_rz(__fadd_rn(v, half_signed(v, h))))); }
 
 __device__ __forceinline__ int requant(int acc, float scale_in, float bias, float scale_out, const EpilogueParams& ep) {
     float v = dequant(acc, scale_in, bias, ep.has_bias);
     v = activate(v, ep.act_type, ep.act_param0);
-    return float2int8(__fmul_rn(v, scale_out), ep.rounding);
+    return float2int8(__fmul_rn(v, scale_out), half_bits(ep.rounding));
 }
 
 __device__ __forceinline__ float dequant_act(int acc, float scale_in, float bias, const EpilogueParams& ep) {
     return activate(dequant(acc, scale_in, bias, ep.has_bias), ep.act_type, ep.act_param0);
 }
 
-__device__ __forceinline__ int quantize1(float x, float scale, int rounding) {
-    return float2int8(__fmul_rn(x, scale), rounding);
+__device__ __forceinline__ int quantize1(float x, float scale, uint32_t h) {
+    return float2int8(__fmul_rn(x, scale), h);
 }
 
 // ---- fast forms used by the hot loops (same results as the functions above) ----
@@ -105,24 +104,30 @@ __device__ __forceinline__ uint32_t pack_sat_s8x4(int a, int b, int c, int d) {
     return pack_sat_s8x2(b, a, pack_sat_s8x2(d, c, 0));
 }
 
-// float2int8 with rounding 0, clamped below at -127 only: trunc(max(adj, -127.5)) == max(trunc(adj), -127).
-// The clamp at +127 is left to pack_sat_s8x4.
-__device__ __forceinline__ int f2i8_lo_clamped(float v) {
-    return __float2int_rz(fmaxf(__fadd_rn(v, half_signed(v)), -127.5f));
+// two values -> trunc(v + copysign(h, v)), clamped below at -127 only (trunc(max(adj, -127.5)) == max(trunc(adj), -127)); the
+// clamp at +127 is left to pack_sat_s8x4
+__device__ __forceinline__ int2 round2(float2 v, uint32_t h) {
+    const float2 r = __fadd2_rn(v, make_float2(half_signed(v.x, h), half_signed(v.y, h)));
+    return make_int2(__float2int_rz(fmaxf(r.x, -127.5f)), __float2int_rz(fmaxf(r.y, -127.5f)));
 }
 
-// the same for v >= 0 (after ReLU / ReLU6): copysign(0.5, v) is +0.5; v == -0 truncates to 0 either way
-__device__ __forceinline__ int f2i8_nonneg(float v) { return __float2int_rz(__fadd_rn(v, 0.5f)); }
+// the same for v >= 0 (after ReLU / ReLU6): copysign(h, v) is +h; v == -0 truncates to 0 either way
+__device__ __forceinline__ int2 round2_nonneg(float2 v, uint32_t h) {
+    const float2 r = __fadd2_rn(v, make_float2(__uint_as_float(h), __uint_as_float(h)));
+    return make_int2(__float2int_rz(r.x), __float2int_rz(r.y));
+}
 
-// quantize 4 floats with one scale (rounding 0) and pack them, x in byte 0
-__device__ __forceinline__ uint32_t quantize4_pack(float x, float y, float z, float w, float scale) {
-    // the multiplies and the additions of +-0.5 as packed pairs (same IEEE operations, half the instructions)
+template <int ACT>
+__device__ __forceinline__ int2 round2_act(float2 v, uint32_t h) {
+    return ACT == ACT_RELU || ACT == ACT_RELU6 ? round2_nonneg(v, h) : round2(v, h);
+}
+
+// quantize 4 floats with one scale and pack them, x in byte 0
+__device__ __forceinline__ uint32_t quantize4_pack(float x, float y, float z, float w, float scale, uint32_t h) {
+    // the multiplies and the additions of +-h as packed pairs (same IEEE operations, half the instructions)
     const float2 sc = make_float2(scale, scale);
-    const float2 a = __fmul2_rn(make_float2(x, y), sc), b = __fmul2_rn(make_float2(z, w), sc);
-    const float2 ra = __fadd2_rn(a, make_float2(half_signed(a.x), half_signed(a.y)));
-    const float2 rb = __fadd2_rn(b, make_float2(half_signed(b.x), half_signed(b.y)));
-    return pack_sat_s8x4(__float2int_rz(fmaxf(ra.x, -127.5f)), __float2int_rz(fmaxf(ra.y, -127.5f)), __float2int_rz(fmaxf(rb.x, -127.5f)),
-                         __float2int_rz(fmaxf(rb.y, -127.5f)));
+    const int2 a = round2(__fmul2_rn(make_float2(x, y), sc), h), b = round2(__fmul2_rn(make_float2(z, w), sc), h);
+    return pack_sat_s8x4(a.x, a.y, b.x, b.y);
 }
 
 // 4x4 byte transpose: inputs are 4 words of 4 bytes; o[i] byte j = input j byte i

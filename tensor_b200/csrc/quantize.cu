@@ -22,7 +22,7 @@ __device__ __forceinline__ int qt_row(int p) { return (p & 3) * 33 + (p >> 2); }
 
 __global__ void __launch_bounds__(QT_THREADS)
 quantize_nchw_to_nhwc_kernel(const __grid_constant__ PlaneGather G, int8_t* __restrict__ out, const float* __restrict__ scales,
-                             int n_scales, int c, int cpad, int hw, int tiles_p, int tiles_c, int rounding, int out_stride, int scale_base, int flat,
+                             int n_scales, int c, int cpad, int hw, int tiles_p, int tiles_c, uint32_t half, int out_stride, int scale_base, int flat,
                              long total_px) {
     __shared__ uint32_t tile[4 * 33 * QT_PITCH];
     pdl_launch_dependents();
@@ -51,7 +51,7 @@ quantize_nchw_to_nhwc_kernel(const __grid_constant__ PlaneGather G, int8_t* __re
         uint32_t cw[4];  // channel i: its 4 pixels packed
         float4 v[4];
         float sc[4];
-        const bool fast = vec_ok && gp + 3 < px_end && c0 + cword * 4 + 3 < c && rounding == ROUND_ADD_HALF_TRUNC;
+        const bool fast = vec_ok && gp + 3 < px_end && c0 + cword * 4 + 3 < c;
         if (fast) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -60,7 +60,7 @@ quantize_nchw_to_nhwc_kernel(const __grid_constant__ PlaneGather G, int8_t* __re
                 v[i] = __ldg(reinterpret_cast<const float4*>(G.plane(cg, img, hw) + p));
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) cw[i] = quantize4_pack(v[i].x, v[i].y, v[i].z, v[i].w, sc[i]);
+            for (int i = 0; i < 4; ++i) cw[i] = quantize4_pack(v[i].x, v[i].y, v[i].z, v[i].w, sc[i], half);
         } else {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -71,7 +71,7 @@ quantize_nchw_to_nhwc_kernel(const __grid_constant__ PlaneGather G, int8_t* __re
                     const float* row = G.plane(cg, img, hw);
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        if (gp + j < px_end) q[j] = quantize1(__ldg(row + p + j), s, rounding);
+                        if (gp + j < px_end) q[j] = quantize1(__ldg(row + p + j), s, half);
                 }
                 cw[i] = pack4(q[0], q[1], q[2], q[3]);
             }
@@ -111,7 +111,7 @@ cudaError_t launch_quantize_nchw_to_nhwc(cudaStream_t stream, const PlaneGather&
     const int tiles_p = flat ? (int)((total_px + QT_P - 1) / QT_P) : (hw + QT_P - 1) / QT_P, tiles_c = (cpad + QT_C - 1) / QT_C;
     const long blocks = (long)(flat ? 1 : n) * tiles_p * tiles_c;
     return launch_overlapped(quantize_nchw_to_nhwc_kernel, dim3((unsigned)blocks), dim3(QT_THREADS), 0, stream, src, out, scales_dev, n_scales, c, cpad,
-                             hw, tiles_p, tiles_c, rounding, cpad, 0, flat, total_px);
+                             hw, tiles_p, tiles_c, half_bits(rounding), cpad, 0, flat, total_px);
 }
 
 // A plain tensor of any channel count: the plane table holds kGatherMaxChannels entries, so wider tensors are
@@ -133,7 +133,7 @@ cudaError_t launch_quantize_dense(cudaStream_t stream, const float* x, int c_tot
         const int tiles_c = (chunk_pad + QT_C - 1) / QT_C;
         const long blocks = (long)(flat ? 1 : n) * tiles_p * tiles_c;
         cudaError_t e = launch_overlapped(quantize_nchw_to_nhwc_kernel, dim3((unsigned)blocks), dim3(QT_THREADS), 0, stream, g, out + base, scales_dev,
-                                          n_scales, chunk, chunk_pad, hw, tiles_p, tiles_c, rounding, cpad, base, flat, total_px);
+                                          n_scales, chunk, chunk_pad, hw, tiles_p, tiles_c, half_bits(rounding), cpad, base, flat, total_px);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -24,15 +24,9 @@ __device__ __forceinline__ void requant16(const int (&v)[16], const float* __res
             const float2 t = __ffma2_rn(a, h ? make_float2(si.z, si.w) : make_float2(si.x, si.y), h ? make_float2(bi.z, bi.w) : make_float2(bi.x, bi.y));
             const float2 y = make_float2(activate_t<ACT>(t.x, p0), activate_t<ACT>(t.y, p0));
             const float2 u = __fmul2_rn(y, h ? make_float2(so.z, so.w) : make_float2(so.x, so.y));
-            if (ACT == ACT_RELU || ACT == ACT_RELU6) {
-                const float2 r = __fadd2_rn(u, make_float2(0.5f, 0.5f));
-                qv[2 * h] = __float2int_rz(r.x);
-                qv[2 * h + 1] = __float2int_rz(r.y);
-            } else {
-                const float2 r = __fadd2_rn(u, make_float2(half_signed(u.x), half_signed(u.y)));
-                qv[2 * h] = __float2int_rz(fmaxf(r.x, -127.5f));
-                qv[2 * h + 1] = __float2int_rz(fmaxf(r.y, -127.5f));
-            }
+            const int2 r = round2_act<ACT>(u, kHalfTrunc);
+            qv[2 * h] = r.x;
+            qv[2 * h + 1] = r.y;
         }
         wds[g] = pack_sat_s8x4(qv[0], qv[1], qv[2], qv[3]);
     }
@@ -129,15 +123,9 @@ __device__ __forceinline__ void store_accumulator_row(uint32_t taddr, int ncols,
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const float2 u = __fmul2_rn(make_float2(y[g * 4 + 2 * h], y[g * 4 + 2 * h + 1]), h ? make_float2(o4.z, o4.w) : make_float2(o4.x, o4.y));
-                    if (ACT == ACT_RELU || ACT == ACT_RELU6) {
-                        const float2 rr = __fadd2_rn(u, make_float2(0.5f, 0.5f));
-                        qv[2 * h] = __float2int_rz(rr.x);
-                        qv[2 * h + 1] = __float2int_rz(rr.y);
-                    } else {
-                        const float2 rr = __fadd2_rn(u, make_float2(half_signed(u.x), half_signed(u.y)));
-                        qv[2 * h] = __float2int_rz(fmaxf(rr.x, -127.5f));
-                        qv[2 * h + 1] = __float2int_rz(fmaxf(rr.y, -127.5f));
-                    }
+                    const int2 r = round2_act<ACT>(u, kHalfTrunc);
+                    qv[2 * h] = r.x;
+                    qv[2 * h + 1] = r.y;
                 }
                 wds[half][g] = pack_sat_s8x4(qv[0], qv[1], qv[2], qv[3]);
             }
