@@ -657,8 +657,17 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
     if (rc == OTT_OK) rc = upload(ctx, scale_out.data(), sizeof(float) * c->cout_pad, (void**)&c->scale_out_dev);
     if (rc == OTT_OK) rc = upload(ctx, in_scales, sizeof(float) * n_in_scales, (void**)&c->in_scales_dev);
     if (rc == OTT_OK && c->kind == OTT_KERNEL_DENSE_UMMA) {
-        const char* err = umma_encode_weight_map(c->plan, c->w_dev, c->weight_map);
-        if (err) rc = ctx->fail(OTT_ERR_CUDA, "%s", err);
+        int smem_optin = 0;
+        cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+        UmmaVariant v;
+        v.plan = c->plan;
+        c->umma.push_back(v);
+        for (int bn : kUmmaNarrow)
+            if (umma_narrow_plan(c->plan, bn, d->cout, smem_optin, &v.plan)) c->umma.push_back(v);
+        for (UmmaVariant& u : c->umma) {
+            const char* err = umma_encode_weight_map(u.plan, c->w_dev, u.weight_map);
+            if (err) rc = ctx->fail(OTT_ERR_CUDA, "%s", err);
+        }
     }
     // host staging vectors die at return: make sure the uploads have consumed them
     if (rc == OTT_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = ctx->fail(OTT_ERR_CUDA, "upload failed");
@@ -1100,7 +1109,7 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
                     us.block_src[kb] = c->block_src[kb];
                 }
             }
-            const char* err = launch_dense_umma(ctx->stream, ctx->sm_count, c->plan, c->weight_map, s, x, ep, out_dev, out_dtype, status,
+            const char* err = launch_dense_umma(ctx->stream, ctx->sm_count, c->umma.data(), (int)c->umma.size(), s, x, ep, out_dev, out_dtype, status,
                                                 gathered ? &us : nullptr, mixed, ctx->wait_limit_ns);
             if (err) return ctx->fail(OTT_ERR_CUDA, "%s: %s", err, cudaGetErrorString(cudaGetLastError()));
             break;

@@ -28,6 +28,7 @@ struct ott_conv {
     std::vector<float> scale_in_host, bias_host, scale_out_host;
     float in_scale0 = 1.f;
     ottk::UmmaPlan plan{};
+    std::vector<ottk::UmmaVariant> umma;  // tensor-core layers: `plan` and the narrower ones, each with its weight map
     // a layer whose input channels are gathered from several int8 tensors (ott_conv_int8_create_gathered): which K block is
     // which 32 channels of which source, and the channel count every source tensor must have
     std::vector<uint16_t> block_x;
@@ -39,7 +40,6 @@ struct ott_conv {
     std::vector<int> position;
     int stored_channels = 0;
     int gather_group = 16;  // channels per group of that order: 16 (CUDA-core kernel) or 32 (tensor-core kernel)
-    alignas(128) unsigned char weight_map[128];
     // depthwise 3x3 (stride 1 / 2, pad 1) with int8 input: the tensor-core kernel's plan, diagonal weight panel and its TMA descriptor
     bool dw_umma = false;
     ottk::DwPlan dw_plan{};

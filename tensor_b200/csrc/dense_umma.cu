@@ -297,7 +297,8 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
         // ---- epilogue warps ----
         const int q = warp & 3;            // TMEM lane quarter this warp may read
         const int sub = (warp - 2) >> 2;   // which of the epi_warps/4 warps sharing that quarter
-        const int col_step = 16 * (P.epi_warps / 4);
+        const int chunk = P.bn <= 32 ? 16 : 32;  // columns a warp takes at a time
+        const int col_step = chunk * (P.epi_warps / 4);
         const int row = q * 32 + lane;
         const int row_y = row / P.tw, row_x = row - row_y * P.tw;
         const long plane = (long)s.oh * s.ow;
@@ -418,16 +419,16 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
             const bool wide_ok = OUT == DT_S8_NHWC && ((s.cout_pad | (n_tile * P.bn)) & 31) == 0;
             if (!mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
             tc_fence_after();
-            if (sub * 32 >= P.bn && lane == 0) mbar_arrive(bar_tempty + 8u * buf);  // a narrow tile has no columns for this warp
-            for (int col0 = sub * 32; col0 < P.bn; col0 += 2 * col_step) {
+            if (sub * chunk >= P.bn && lane == 0) mbar_arrive(bar_tempty + 8u * buf);  // a narrow tile has no columns for this warp
+            for (int col0 = sub * chunk; col0 < P.bn; col0 += col_step) {
                 int va[16], vb[16];
-                const bool two = col0 + 16 < P.bn;
+                const bool two = chunk == 32 && col0 + 16 < P.bn;
                 __syncwarp();  // tcgen05.ld is warp-collective
                 tmem_ld16(taddr + (uint32_t)col0, va);
                 if (two) tmem_ld16(taddr + (uint32_t)(col0 + 16), vb);
                 tmem_wait_ld16(va);
                 tmem_wait_ld16(vb);
-                if (col0 + 2 * col_step >= P.bn) {  // this warp's last columns: the accumulator may be overwritten from here on
+                if (col0 + col_step >= P.bn) {  // this warp's last columns: the accumulator may be overwritten from here on
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_tempty + 8u * buf);
@@ -529,6 +530,49 @@ const char* launch_variant(cudaStream_t stream, int sm_count, const KernelMaps& 
 
 static int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
+// What follows from the width of the weight panel (p.bn, p.n_tiles): pipeline depth, tensor memory, shared memory, CTAs per SM.
+static bool plan_panel(UmmaPlan& p, int smem_budget) {
+    const bool whole = p.gather_whole != 0;
+    const long a_stage = p.a_stage_bytes, k_total = p.k_total;
+    const long left = (long)smem_budget - 1024 /*alignment slack*/ - 4096 /*barriers + epilogue parameters*/ - (long)p.bn * k_total;
+    p.stages = (int)(left / a_stage);
+    if (p.stages > 8) p.stages = 8;
+    // Small layers (few k-blocks, narrow panels) are latency-bound with one CTA per SM: keep the pipeline short so that
+    // several CTAs fit an SM and overlap each other's TMA / MMA / epilogue latencies.
+    if ((p.nkb <= 2 || whole) && p.stages > 4) p.stages = 4;
+    if (whole && p.stages > 2) p.stages = 2;  // two whole tiles in flight, and room for a second CTA on the SM
+    // a halo stage feeds all the taps of a whole pixel tile and channel block: three are a deep enough pipeline
+    if (p.halo && p.stages > 3) p.stages = 3;
+    if (p.stages < 2) return false;
+    // two accumulators of bn columns each; TMEM allocations are powers of two >= 32 columns
+    p.acc_stride = p.bn <= 32 ? 32 : (p.bn <= 64 ? 64 : (p.bn <= 128 ? 128 : 256));
+    // narrow tiles finish quickly; four accumulators let the MMA issuer run three tiles ahead of the epilogue
+    p.acc_bufs = p.acc_stride <= 64 ? 4 : 2;
+    p.tmem_cols = p.acc_bufs * p.acc_stride;
+    // instruction descriptor: D=s32 (2<<4), A=B=signed int8 (1<<7, 1<<10), both K-major, N>>3 at bit 17, M>>4 at bit 24
+    p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+    SmemLayout L = smem_layout(p);
+    p.smem_bytes = (int)L.total + 1024;
+    // CTAs per SM: TMEM has 512 columns per SM and the hardware scheduler does not account for them, so the shared-memory
+    // request is padded until no more CTAs fit an SM than TMEM can serve (a CTA that cannot get its columns would wait
+    // inside tcgen05.alloc for a neighbour to finish).
+    // eight epilogue warps, two per TMEM lane quarter (sixteen for wide single-CTA tiles, below)
+    p.epi_warps = 8;
+    int by_tmem = 512 / p.tmem_cols;
+    int by_smem = smem_budget / p.smem_bytes;
+    p.ctas_per_sm = by_tmem < by_smem ? by_tmem : by_smem;
+    if (p.ctas_per_sm > 4) p.ctas_per_sm = 4;
+    if (p.ctas_per_sm < 1) p.ctas_per_sm = 1;
+    // Wide tiles with one CTA per SM: sixteen epilogue warps (four per lane quarter, 576 threads, the build without a register
+    // cap). Requantizing a 128 x 256 tile costs the CUDA cores as much as its MMAs cost the tensor pipe, and eight warps reach
+    // only two thirds of the SM's requantize rate (measured: 512 -> 1024: 1660 -> 1837 TOP/s; 256 -> 512: 881 -> 1025; with
+    // 128-column tiles it loses, 3x3 128 -> 128: 1938 -> 1865).
+    if (p.ctas_per_sm == 1 && p.bn > 128) p.epi_warps = 16;
+    const int min_smem = smem_budget / (p.ctas_per_sm + 1) + 1;
+    if (p.smem_bytes < min_smem) p.smem_bytes = min_smem;
+    return true;
+}
+
 bool umma_plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, int dw, int smem_budget, UmmaPlan* plan, int bkc_override,
                      bool whole_tile_stages) {
     UmmaPlan p{};
@@ -561,44 +605,18 @@ bool umma_plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, 
     p.bn = round_up((cout_pad + p.n_tiles - 1) / p.n_tiles, 16);
     if (p.bkc == 32) p.bn = round_up(p.bn, 32);  // keeps every weight tile on a 1 KiB boundary
     if (p.bn > 256 || (long)p.bn * k_total > avail) return false;
-    const long left = (long)smem_budget - 1024 - 4096 - (long)p.bn * k_total;
-    p.stages = (int)(left / a_stage);
-    if (p.stages > 8) p.stages = 8;
-    // Small layers (few k-blocks, narrow panels) are latency-bound with one CTA per SM: keep the pipeline short so that
-    // several CTAs fit an SM and overlap each other's TMA / MMA / epilogue latencies.
-    if ((p.nkb <= 2 || whole) && p.stages > 4) p.stages = 4;
-    if (whole && p.stages > 2) p.stages = 2;  // two whole tiles in flight, and room for a second CTA on the SM
-    // a halo stage feeds all the taps of a whole pixel tile and channel block: three are a deep enough pipeline
-    if (p.halo && p.stages > 3) p.stages = 3;
-    if (p.stages < 2) return false;
-    // two accumulators of bn columns each; TMEM allocations are powers of two >= 32 columns
-    p.acc_stride = p.bn <= 32 ? 32 : (p.bn <= 64 ? 64 : (p.bn <= 128 ? 128 : 256));
-    // narrow tiles finish quickly; four accumulators let the MMA issuer run three tiles ahead of the epilogue
-    p.acc_bufs = p.acc_stride <= 64 ? 4 : 2;
-    p.tmem_cols = p.acc_bufs * p.acc_stride;
-    // instruction descriptor: D=s32 (2<<4), A=B=signed int8 (1<<7, 1<<10), both K-major, N>>3 at bit 17, M>>4 at bit 24
-    p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
     p.k_total = (int)k_total;
     p.cout_rows = p.n_tiles * p.bn;
-    SmemLayout L = smem_layout(p);
-    p.smem_bytes = (int)L.total + 1024;
-    // CTAs per SM: TMEM has 512 columns per SM and the hardware scheduler does not account for them, so the shared-memory
-    // request is padded until no more CTAs fit an SM than TMEM can serve (a CTA that cannot get its columns would wait
-    // inside tcgen05.alloc for a neighbour to finish).
-    // eight epilogue warps, two per TMEM lane quarter (sixteen for wide single-CTA tiles, below)
-    p.epi_warps = 8;
-    int by_tmem = 512 / p.tmem_cols;
-    int by_smem = smem_budget / p.smem_bytes;
-    p.ctas_per_sm = by_tmem < by_smem ? by_tmem : by_smem;
-    if (p.ctas_per_sm > 4) p.ctas_per_sm = 4;
-    if (p.ctas_per_sm < 1) p.ctas_per_sm = 1;
-    // Wide tiles with one CTA per SM: sixteen epilogue warps (four per lane quarter, 576 threads, the build without a register
-    // cap). Requantizing a 128 x 256 tile costs the CUDA cores as much as its MMAs cost the tensor pipe, and eight warps reach
-    // only two thirds of the SM's requantize rate (measured: 512 -> 1024: 1660 -> 1837 TOP/s; 256 -> 512: 881 -> 1025; with
-    // 128-column tiles it loses, 3x3 128 -> 128: 1938 -> 1865).
-    if (p.ctas_per_sm == 1 && p.bn > 128) p.epi_warps = 16;
-    const int min_smem = smem_budget / (p.ctas_per_sm + 1) + 1;
-    if (p.smem_bytes < min_smem) p.smem_bytes = min_smem;
+    if (!plan_panel(p, smem_budget)) return false;
+    *plan = p;
+    return true;
+}
+
+bool umma_narrow_plan(const UmmaPlan& base, int bn, int cout, int smem_budget, UmmaPlan* plan) {
+    UmmaPlan p = base;
+    p.bn = bn;
+    p.n_tiles = (nhwc_channels(cout) + bn - 1) / bn;
+    if (bn >= base.bn || p.n_tiles <= base.n_tiles || !plan_panel(p, smem_budget)) return false;
     *plan = p;
     return true;
 }
@@ -628,13 +646,18 @@ const char* umma_encode_weight_map(const UmmaPlan& p, const int8_t* w_dev, void*
     return r == CUDA_SUCCESS ? nullptr : "cuTensorMapEncodeTiled(weights) failed";
 }
 
-const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaPlan& plan_in, const void* weight_map,
-                              const ConvShape& s, const int8_t* x, const EpilogueParams& ep, void* out, int out_dtype,
-                              uint32_t* status, const UmmaSources* sources, const UmmaMixedOut* mixed_in, unsigned long long wait_limit_ns) {
+const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVariant* variants, int n_variants, const ConvShape& s,
+                              const int8_t* x, const EpilogueParams& ep, void* out, int out_dtype, uint32_t* status,
+                              const UmmaSources* sources, const UmmaMixedOut* mixed_in, unsigned long long wait_limit_ns) {
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return "cuTensorMapEncodeTiled entry point not available";
-    UmmaPlan p = plan_in;
-    p.wait_ns = wait_limit_ns;
+    // The tiling of the pixels is the same for every variant. A launch with fewer tiles than SMs is bound by the chain of one
+    // tile, most of which (MMAs, requantize, stores) shrinks with the panel: take the widest panels that put a CTA on every SM,
+    // or the narrowest, as long as all the CTAs are resident at once. Measured: 232 -> 232 on 10x10, one image 4.2 us with one
+    // panel of 240 columns, 2.9 with 32; but 717 -> 152 on 102 tiles 20.5 us with one panel and 23.4 with two that do not fit an
+    // SM together; with more tiles than SMs every extra panel only reads the activations once more.
+    UmmaPlan p = variants[0].plan;
+    const UmmaVariant* chosen = variants;
     const long pixels = (long)s.n * s.oh * s.ow;
     if (pixels == 0) return nullptr;
     KernelMaps km;  // only the entries the plan uses are filled in
@@ -697,11 +720,19 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaPlan&
                 swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
     if (r != CUDA_SUCCESS) return "cuTensorMapEncodeTiled(activations) failed";
+    for (int i = 1; i < n_variants && (long)p.m_tiles * chosen->plan.n_tiles < sm_count; ++i)
+        if ((long)p.m_tiles * variants[i].plan.n_tiles <= (long)sm_count * variants[i].plan.ctas_per_sm) chosen = variants + i;
+    {
+        const UmmaPlan tiling = p;
+        p = chosen->plan;
+        p.flat = tiling.flat; p.tw = tiling.tw; p.th = tiling.th; p.tiles_x = tiling.tiles_x; p.tiles_y = tiling.tiles_y; p.m_tiles = tiling.m_tiles;
+    }
+    p.wait_ns = wait_limit_ns;
     p.div_img = make_fast_div((uint32_t)(p.tiles_x * p.tiles_y));
     p.div_tx = make_fast_div((uint32_t)p.tiles_x);
     p.div_plane = make_fast_div((uint32_t)(s.oh * s.ow));
 
-    const CUtensorMap& tmB = *reinterpret_cast<const CUtensorMap*>(weight_map);
+    const CUtensorMap& tmB = *reinterpret_cast<const CUtensorMap*>(chosen->weight_map);
     const char* err = nullptr;
 #define OTT_UMMA_LAUNCH(OUT, ACT)                                                                                     \
     err = p.ctas_per_sm > 1   ? launch_variant<OUT, ACT, 1>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed) \

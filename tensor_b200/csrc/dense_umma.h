@@ -47,6 +47,16 @@ struct UmmaPlan {
 bool umma_plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, int dw, int smem_budget, UmmaPlan* plan,
                      int bkc_override = 0, bool whole_tile_stages = false);
 
+// The same layer over narrower weight panels of bn columns, for launches with few pixel tiles; false where it makes no difference.
+bool umma_narrow_plan(const UmmaPlan& base, int bn, int cout, int smem_budget, UmmaPlan* plan);
+
+// A plan and the tensor map that cuts the packed weights into its panels. A layer has its widest one and the narrower ones.
+struct UmmaVariant {
+    UmmaPlan plan{};
+    alignas(128) unsigned char weight_map[128];
+};
+constexpr int kUmmaNarrow[] = {128, 64, 32};
+
 // A 1x1 layer whose input channels are spread over several int8 NHWC tensors (each written by one producer layer): K block
 // kb of the implicit GEMM is the 32 channels starting at block_x[kb] of tensor block_src[kb]. The layer's weights are laid
 // out to match (zero for channels of a block that belong to another reader).
@@ -84,9 +94,10 @@ const char* umma_encode_weight_map(const UmmaPlan& p, const int8_t* w_dev, void*
 // Launch. Returns NULL or an error text.
 // sources: NULL, or where the K blocks of a plan with gather > 0 come from (x is then unused). mixed: NULL, or the fp32 side
 // output of an int8 launch.
-const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaPlan& plan, const void* weight_map,
-                              const ConvShape& s, const int8_t* x, const EpilogueParams& ep, void* out, int out_dtype,
-                              uint32_t* status, const UmmaSources* sources = nullptr, const UmmaMixedOut* mixed = nullptr,
+// variants: the layer's plans, widest panels first; which one runs depends on the number of pixel tiles.
+const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVariant* variants, int n_variants, const ConvShape& s,
+                              const int8_t* x, const EpilogueParams& ep, void* out, int out_dtype, uint32_t* status,
+                              const UmmaSources* sources = nullptr, const UmmaMixedOut* mixed = nullptr,
                               unsigned long long wait_limit_ns = 2000000000ull);
 
 }  // namespace ottk
