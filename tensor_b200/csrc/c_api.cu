@@ -25,8 +25,17 @@ int upload(ott_ctx* ctx, const void* host, size_t bytes, void** dev) {
     return OTT_OK;
 }
 
-int check_status_word(ott_ctx* ctx) {
-    OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(ctx->status_host, ctx->status_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+bool is_pinned(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost;
+}
+
+int check_status_word(ott_ctx* ctx, bool copied = false) {
+    if (!copied) OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(ctx->status_host, ctx->status_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     OTT_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
     for (cudaStream_t a : ctx->aux_stream)
         if (a) OTT_CUDA_CHECK(ctx, cudaStreamSynchronize(a));
@@ -49,6 +58,64 @@ size_t dtype_bytes(int dtype, int n, int c, int h, int w) {
 }
 
 }  // namespace
+
+int ctx_upload(ott_ctx* ctx, const HostCopy& copy) {
+    if (is_pinned(copy.host)) {
+        OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(copy.dev, copy.host, copy.bytes, cudaMemcpyHostToDevice, ctx->stream));
+        return OTT_OK;
+    }
+    HostStaging& ring = ctx->upload;
+    OTT_CUDA_CHECK(ctx, ring.ready());
+    for (size_t at = 0; at < copy.bytes; at += HostStaging::kPiece) {
+        const size_t len = std::min(HostStaging::kPiece, copy.bytes - at);
+        const int slot = ring.next;
+        ring.next = (slot + 1) % HostStaging::kSlots;
+        OTT_CUDA_CHECK(ctx, cudaEventSynchronize(ring.done[slot]));  // (an event never recorded counts as complete)
+        char* stage = ring.mem + slot * HostStaging::kPiece;
+        std::memcpy(stage, static_cast<const char*>(copy.host) + at, len);
+        OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(static_cast<char*>(copy.dev) + at, stage, len, cudaMemcpyHostToDevice, ctx->stream));
+        OTT_CUDA_CHECK(ctx, cudaEventRecord(ring.done[slot], ctx->stream));
+    }
+    return OTT_OK;
+}
+
+int ctx_download_and_sync(ott_ctx* ctx, const HostCopy* copies, int n) {
+    HostStaging& ring = ctx->download;
+    struct Piece {
+        char* dst;
+        size_t len;
+    } pending[HostStaging::kSlots];
+    // pieces [first, issued) are under way, piece i in slot i % kSlots
+    long first = 0, issued = 0;
+    auto retire = [&]() -> int {
+        const int slot = (int)(first % HostStaging::kSlots);
+        OTT_CUDA_CHECK(ctx, cudaEventSynchronize(ring.done[slot]));
+        std::memcpy(pending[slot].dst, ring.mem + slot * HostStaging::kPiece, pending[slot].len);
+        ++first;
+        return OTT_OK;
+    };
+    for (int i = 0; i < n; ++i) {
+        if (is_pinned(copies[i].host)) {
+            OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(copies[i].host, copies[i].dev, copies[i].bytes, cudaMemcpyDeviceToHost, ctx->stream));
+            continue;
+        }
+        OTT_CUDA_CHECK(ctx, ring.ready());
+        for (size_t at = 0; at < copies[i].bytes; at += HostStaging::kPiece) {
+            if (issued - first == HostStaging::kSlots)
+                if (const int rc = retire()) return rc;
+            const int slot = (int)(issued % HostStaging::kSlots);
+            pending[slot] = Piece{static_cast<char*>(copies[i].host) + at, std::min(HostStaging::kPiece, copies[i].bytes - at)};
+            OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(ring.mem + slot * HostStaging::kPiece, static_cast<char*>(copies[i].dev) + at, pending[slot].len,
+                                                cudaMemcpyDeviceToHost, ctx->stream));
+            OTT_CUDA_CHECK(ctx, cudaEventRecord(ring.done[slot], ctx->stream));
+            ++issued;
+        }
+    }
+    OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(ctx->status_host, ctx->status_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    while (first < issued)
+        if (const int rc = retire()) return rc;
+    return check_status_word(ctx, true);
+}
 
 extern "C" {
 
@@ -111,8 +178,9 @@ int ott_ctx_destroy(ott_ctx* ctx) {
     delete ctx->alloc;
     if (ctx->status_dev) cudaFree(ctx->status_dev);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
-    if (ctx->stage_in) cudaFreeHost(ctx->stage_in);
-    if (ctx->stage_out) cudaFreeHost(ctx->stage_out);
+    ctx->upload.release();
+    ctx->download.release();
+    if (ctx->detect_mem) cudaFreeHost(ctx->detect_mem);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return OTT_OK;
@@ -1136,11 +1204,11 @@ int ott_conv_int8_forward_host(ott_ctx* ctx, const ott_conv* c, const void* in_h
         (void)cudaGetLastError();
         return ctx->fail(OTT_ERR_ALLOC, "device allocation failed");
     }
-    OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(din.p, in_host, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
-    int rc = ott_conv_int8_forward(ctx, c, din.p, in_dtype, n, h, w, dout.p, out_dtype, nullptr);
+    int rc = ctx_upload(ctx, HostCopy{const_cast<void*>(in_host), din.p, in_bytes});
+    if (rc == OTT_OK) rc = ott_conv_int8_forward(ctx, c, din.p, in_dtype, n, h, w, dout.p, out_dtype, nullptr);
     if (rc != OTT_OK) return rc;
-    OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(out_host, dout.p, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    return check_status_word(ctx);
+    const HostCopy back{out_host, dout.p, out_bytes};
+    return ctx_download_and_sync(ctx, &back, 1);
 }
 
 }  // extern "C"

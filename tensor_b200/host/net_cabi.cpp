@@ -3,6 +3,7 @@
 #include <sstream>
 
 #include "../../include/otter_b200_net.h"
+#include "../csrc/ctx.h"
 #include "otter_api.hpp"
 
 struct ott_net;
@@ -12,20 +13,25 @@ struct ott_net_graph {
     std::vector<otter::Tensor> outputs;  // device tensors the replays write
 };
 
-// What ott_net_forward keeps between calls with host buffers of one shape: the device input buffer and one captured forward
-// per chunk of the batch (the chunks differ in where they read the input).
+// What the host-buffer calls keep between calls of one shape: the device input buffer and one captured forward per chunk of the
+// batch (the chunks differ in where they read the input). A batch of less than two chunks is one graph, captured when its shape
+// comes for the second time: a program that runs a shape once does not pay for a capture it never replays.
 struct HostPipeline {
     std::string key;
     void* dev_in = nullptr;
-    int chunk = 0;
     std::vector<ott_net_graph*> graphs;
+    bool plain = false;  // cannot be captured, or delivers a blob that has to be re-ordered on the host: runs layer by layer
 };
+constexpr size_t kMaxPipelines = 4;  // shapes kept; the oldest goes
 
 struct ott_net {
     otter::Net net;
     std::string error;
     std::vector<HostPipeline> pipelines;
+    void drop(HostPipeline& p);
     void drop_pipelines();
+    HostPipeline* pipeline(const std::string& key, bool* seen_before);
+    int build(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs);
     ~ott_net() { drop_pipelines(); }
 };
 
@@ -34,6 +40,17 @@ namespace {
 int fail(ott_net* n, int code, const std::string& what) {
     n->error = what;
     return code;
+}
+
+// everything a captured forward depends on besides the layers' parameters (which drop all pipelines when they change)
+std::string pipeline_key(const ott_net* net, const char* call, const char* input_blob, int n, int c, int h, int w, int n_out, const char* const* out_blobs) {
+    const ott_ctx* ctx = net->net.context();
+    char buf[160];
+    snprintf(buf, sizeof buf, "%s|%dx%dx%dx%d|%d|%d|%llu|", call, n, c, h, w, net->net.option.host_chunk, ctx->dw_tensor_cores, ctx->wait_limit_ns);
+    std::string key = buf;
+    key += input_blob;
+    for (int i = 0; i < n_out; ++i) key.append("|").append(out_blobs[i]);
+    return key;
 }
 
 void copy_str(const std::string& s, char* dst, int cap) {
@@ -79,6 +96,7 @@ int ott_net_set_option(ott_net* net, const char* key, int value) {
     if (!net || !key) return OTT_ERR_INVALID;
     otter::NetOption& o = net->net.option;
     const std::string k = key;
+    net->drop_pipelines();  // captured forwards were made under the old options
     if (k == "lightmode") o.lightmode = value != 0;
     else if (k == "use_packing_layout") o.use_packing_layout = value != 0;
     else if (k == "int8_rounding") o.int8_rounding = value;
@@ -242,56 +260,36 @@ int ott_net_forward(ott_net* net, const char* input_blob, const void* in, int in
                     const char* const* out_blobs, void* const* out_host) {
     if (!net || !input_blob || !in || n_out < 1 || !out_blobs) return OTT_ERR_INVALID;
     net->error.clear();
-    // Host in, host out, large batch: run the batch in chunks so that the upload of chunk i+1 and the download of chunk i-1
-    // overlap the kernels of chunk i (images are independent, so chunking changes no value). Each chunk's forward is a
-    // captured CUDA graph, kept for the next call with the same shape: a chunk then costs the host one launch instead of one
-    // per kernel, which is what allows chunks small enough to keep the fill and drain of the pipeline short.
+    // Host in, host out: the forward is a captured CUDA graph, kept for the next call with the same shape, so that the host pays
+    // for one launch instead of one per kernel (an image through ShuffleNetV2 costs the host 275 us to enqueue and the GPU 183 us
+    // to run). A large batch runs in chunks: the upload of chunk i+1 and the download of chunk i-1 overlap the kernels of chunk
+    // i (images are independent, so chunking changes no value).
     bool all_host_out = out_host != nullptr;
     for (int i = 0; all_host_out && i < n_out; ++i) all_host_out = out_host[i] != nullptr;
     const int chunk = net->net.option.host_chunk > 0 ? net->net.option.host_chunk : 64;
-    if (!in_on_device && all_host_out && n >= 2 * chunk) {
-        ott_ctx* ctx = net->net.context();
+    ott_ctx* ctx = net->net.context();
+    if (!in_on_device && all_host_out && n > 0 && c > 0 && h > 0 && w > 0 && ctx) {
         const size_t img_bytes = (size_t)c * h * w * sizeof(float);
-        std::string key = std::string(input_blob) + "|" + std::to_string(n) + "x" + std::to_string(c) + "x" + std::to_string(h) + "x" + std::to_string(w) +
-                          "|" + std::to_string(chunk);
-        for (int i = 0; i < n_out; ++i) key += std::string("|") + out_blobs[i];
-        HostPipeline* pipe = nullptr;
-        for (HostPipeline& p : net->pipelines)
-            if (p.key == key) pipe = &p;
-        int rc = OTT_OK;
-        if (!pipe) {
-            HostPipeline p;
-            p.key = key;
-            p.chunk = chunk;
-            if (ott_malloc(ctx, img_bytes * n, &p.dev_in) != OTT_OK) return fail(net, OTT_ERR_ALLOC, "device allocation for the input batch failed");
-            // the warm-up forward inside every capture reads the (not yet uploaded) buffer: give it defined contents
-            rc = ott_memset(ctx, p.dev_in, 0, img_bytes * n);
-            for (int b0 = 0; b0 < n && rc == OTT_OK; b0 += chunk) {
-                const int nb = n - b0 < chunk ? n - b0 : chunk;
-                ott_net_graph* g = nullptr;
-                rc = ott_net_capture(net, input_blob, static_cast<char*>(p.dev_in) + img_bytes * b0, nb, c, h, w, n_out, out_blobs, &g);
-                if (rc == OTT_OK) p.graphs.push_back(g);
-            }
-            bool dense = rc == OTT_OK;
-            for (size_t gi = 0; dense && gi < p.graphs.size(); ++gi)
-                for (const otter::Tensor& t : p.graphs[gi]->outputs) dense = dense && t.layout() == otter::Layout::NCHW;
-            if (!dense) {  // a capture failed, or an output is an int8 NHWC blob: this shape takes the plain path below
-                for (ott_net_graph* g : p.graphs) ott_net_graph_destroy(g);
-                ott_free(ctx, p.dev_in);
-                if (rc != OTT_OK && rc != OTT_ERR_UNSUPPORTED) return rc;
-                p.graphs.clear();
-                p.dev_in = nullptr;  // remembered, so that the next call does not try again
-            }
-            if (net->pipelines.size() >= 4) {  // a handful of shapes is kept; the oldest goes
-                for (ott_net_graph* g : net->pipelines.front().graphs) ott_net_graph_destroy(g);
-                if (net->pipelines.front().dev_in) ott_free(ctx, net->pipelines.front().dev_in);
-                net->pipelines.erase(net->pipelines.begin());
-            }
-            net->pipelines.push_back(std::move(p));
-            pipe = &net->pipelines.back();
-            rc = OTT_OK;
+        const bool chunked = n >= 2 * chunk;
+        bool seen = false;
+        HostPipeline* pipe = net->pipeline(pipeline_key(net, "forward", input_blob, n, c, h, w, n_out, out_blobs), &seen);
+        if (pipe->graphs.empty() && !pipe->plain && (chunked || seen)) {
+            const int rc = net->build(*pipe, input_blob, n, c, h, w, chunked ? chunk : n, n_out, out_blobs);
+            if (rc != OTT_OK) return rc;
         }
-        if (pipe && !pipe->graphs.empty()) {
+        if (!pipe->graphs.empty() && !chunked) {
+            int rc = ctx_upload(ctx, HostCopy{const_cast<void*>(in), pipe->dev_in, img_bytes * n});
+            if (rc == OTT_OK) rc = ott_net_graph_launch(pipe->graphs[0]);
+            if (rc != OTT_OK) return rc;
+            std::vector<HostCopy> back((size_t)n_out);
+            for (int i = 0; i < n_out; ++i) {
+                const otter::Tensor& t = pipe->graphs[0]->outputs[(size_t)i];
+                back[(size_t)i] = HostCopy{out_host[i], t.raw_data(), (size_t)t.numel() * otter::elementSize(t.scalar_type())};
+            }
+            return ctx_download_and_sync(ctx, back.data(), n_out);
+        }
+        if (!pipe->graphs.empty()) {
+            int rc = OTT_OK;
             size_t gi = 0;
             for (int b0 = 0; b0 < n && rc == OTT_OK; b0 += chunk, ++gi) {
                 const int nb = n - b0 < chunk ? n - b0 : chunk;
@@ -402,12 +400,57 @@ int ott_net_graph_destroy(ott_net_graph* graph) {
 
 }  // extern "C"
 
+void ott_net::drop(HostPipeline& p) {
+    for (ott_net_graph* g : p.graphs) ott_net_graph_destroy(g);
+    p.graphs.clear();
+    if (p.dev_in && net.context()) ott_free(net.context(), p.dev_in);
+    p.dev_in = nullptr;
+}
+
 void ott_net::drop_pipelines() {
-    for (HostPipeline& p : pipelines) {
-        for (ott_net_graph* g : p.graphs) ott_net_graph_destroy(g);
-        if (p.dev_in && net.context()) ott_free(net.context(), p.dev_in);
-    }
+    for (HostPipeline& p : pipelines) drop(p);
     pipelines.clear();
+}
+
+HostPipeline* ott_net::pipeline(const std::string& key, bool* seen_before) {
+    for (HostPipeline& p : pipelines)
+        if (p.key == key) {
+            *seen_before = true;
+            return &p;
+        }
+    *seen_before = false;
+    if (pipelines.size() >= kMaxPipelines) {
+        drop(pipelines.front());
+        pipelines.erase(pipelines.begin());
+    }
+    pipelines.emplace_back();
+    pipelines.back().key = key;
+    return &pipelines.back();
+}
+
+// Captures the pipeline's graphs. A failure to allocate is reported and may be tried again; any other failure to capture, or an
+// output that is not dense fp32 NCHW, makes the shape a plain one.
+int ott_net::build(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs) {
+    ott_ctx* ctx = net.context();
+    const size_t img_bytes = (size_t)c * h * w * sizeof(float);
+    if (ott_malloc(ctx, img_bytes * n, &p.dev_in) != OTT_OK) return fail(this, OTT_ERR_ALLOC, "device allocation for the input batch failed");
+    // the warm-up forward inside every capture reads the (not yet uploaded) buffer: give it defined contents
+    int rc = ott_memset(ctx, p.dev_in, 0, img_bytes * n);
+    for (int b0 = 0; b0 < n && rc == OTT_OK; b0 += chunk) {
+        ott_net_graph* g = nullptr;
+        rc = ott_net_capture(this, input_blob, static_cast<char*>(p.dev_in) + img_bytes * b0, n - b0 < chunk ? n - b0 : chunk, c, h, w, n_out, out_blobs, &g);
+        if (rc == OTT_OK) p.graphs.push_back(g);
+    }
+    bool dense = rc == OTT_OK;
+    for (size_t gi = 0; dense && gi < p.graphs.size(); ++gi)
+        for (const otter::Tensor& t : p.graphs[gi]->outputs) dense = dense && t.layout() == otter::Layout::NCHW;
+    if (dense) return OTT_OK;
+    drop(p);
+    if (rc == OTT_OK || rc == OTT_ERR_UNSUPPORTED) {
+        p.plain = true;
+        error.clear();
+    }
+    return p.plain ? OTT_OK : rc;
 }
 
 extern "C" {
@@ -416,15 +459,42 @@ int ott_net_forward_rows(ott_net* net, const char* input_blob, const void* in, i
                          float* out_host, int capacity_rows, int* rows, int* cols) {
     if (!net || !input_blob || !in || !out_blob || !out_host || !rows || !cols || capacity_rows < 0) return OTT_ERR_INVALID;
     net->error.clear();
-    otter::Extractor ex = net->net.create_extractor();
-    otter::Tensor x = in_on_device ? otter::Tensor::wrap(const_cast<void*>(in), (size_t)n * c * h * w * 4, otter::Device::CUDA, nullptr,
-                                                          {n, c, h, w}, otter::ScalarType::Float)
-                                   : otter::from_blob(const_cast<void*>(in), {n, c, h, w}, otter::ScalarType::Float);
-    int rc = ex.input(input_blob, x);
-    if (rc != 0) return fail(net, rc, "Extractor::input failed");
     otter::Tensor feat;
-    rc = ex.extract(out_blob, feat, 0);
-    if (rc != 0) return rc;
+    int rc = OTT_OK;
+    // From host memory: the blobs the layer reads come from a captured forward (see ott_net_forward); the layer itself, whose
+    // result has a size only it knows, runs behind the replay.
+    const int blob = net->net.find_blob_index_by_name(out_blob);
+    const otter::Layer* last = blob >= 0 && net->net.blob(blob).producer >= 0 ? net->net.layer(net->net.blob(blob).producer) : nullptr;
+    if (!in_on_device && last && last->type() == "NanodetPlusDetectionOutput" && n > 0 && c > 0 && h > 0 && w > 0 && net->net.context()) {
+        std::vector<std::string> names;
+        std::vector<const char*> outs;
+        for (int b : last->bottoms) names.push_back(net->net.blob(b).name);
+        for (const std::string& nm : names) outs.push_back(nm.c_str());
+        bool seen = false;
+        HostPipeline* pipe = net->pipeline(pipeline_key(net, "rows", input_blob, n, c, h, w, (int)outs.size(), outs.data()), &seen);
+        if (pipe->graphs.empty() && !pipe->plain && seen) {
+            rc = net->build(*pipe, input_blob, n, c, h, w, n, (int)outs.size(), outs.data());
+            if (rc != OTT_OK) return rc;
+        }
+        if (!pipe->graphs.empty()) {
+            rc = ctx_upload(net->net.context(), HostCopy{const_cast<void*>(in), pipe->dev_in, (size_t)n * c * h * w * sizeof(float)});
+            if (rc == OTT_OK) rc = ott_net_graph_launch(pipe->graphs[0]);
+            std::vector<otter::Tensor> tops(1);
+            if (rc == OTT_OK) rc = last->forward(pipe->graphs[0]->outputs, tops, net->net.option);
+            if (rc != OTT_OK) return fail(net, rc, std::string("forward of layer ") + last->name + " failed: " + ott_last_error(net->net.context()));
+            feat = tops[0];
+        }
+    }
+    if (!feat.defined()) {
+        otter::Extractor ex = net->net.create_extractor();
+        otter::Tensor x = in_on_device ? otter::Tensor::wrap(const_cast<void*>(in), (size_t)n * c * h * w * 4, otter::Device::CUDA, nullptr,
+                                                              {n, c, h, w}, otter::ScalarType::Float)
+                                       : otter::from_blob(const_cast<void*>(in), {n, c, h, w}, otter::ScalarType::Float);
+        rc = ex.input(input_blob, x);
+        if (rc != 0) return fail(net, rc, "Extractor::input failed");
+        rc = ex.extract(out_blob, feat, 0);
+        if (rc != 0) return rc;
+    }
     if (feat.dim() != 2 || feat.scalar_type() != otter::ScalarType::Float) return fail(net, OTT_ERR_INVALID, std::string(out_blob) + " is not a 2-D fp32 blob");
     *rows = (int)feat.size(0);
     *cols = (int)feat.size(1);

@@ -1,0 +1,70 @@
+"""GPU: the host-buffer forward replays a captured graph from the second call of a shape on: every call must equal the checker, with
+changing inputs and batch sizes, more shapes than are kept, parameters replaced in between, an int8 output blob (which is not
+captured), copies longer than the staging ring, and pinned buffers."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def small():
+    from graph_support import build_net, oracle_conv, oracle_conv_for_calibration
+    from graph_walk import calibrate, walk
+    from tensor_b200 import graphs
+    L = graphs.shufflenetv2_layers(40, 48, batch=1, stage_repeats=(2, 2, 2))
+    params = graphs.make_params(L, seed=21)
+    calibrate(L, params, np.random.default_rng(0).uniform(0, 1, size=(1, 3, 40, 48)).astype(np.float32), oracle_conv_for_calibration)
+    net = build_net(L, params)
+    yield net, params, lambda x, blob: walk(L, x, oracle_conv(params), want=[blob])[blob]
+    net.close()
+
+
+def test_every_call_of_a_shape(small):
+    net, params, want = small
+    rng = np.random.default_rng(1)
+    for n in (1, 2, 1, 2, 3, 1, 4, 5, 6, 1, 1, 6):  # six shapes, four of which are kept
+        x = rng.uniform(0, 1, size=(n, 3, 40, 48)).astype(np.float32)
+        assert np.array_equal(net.forward("data", x, ["conv5"])[0].view(np.int32), want(x, "conv5").view(np.int32)), n
+
+
+def test_replaced_parameters_take_effect(small):
+    net, params, want = small
+    x = np.random.default_rng(2).uniform(0, 1, size=(1, 3, 40, 48)).astype(np.float32)
+    for _ in range(3):
+        before = net.forward("data", x, ["conv5"])[0]
+    p = params["conv5"]
+    p["bias"] = p["bias"] + np.float32(0.25)
+    net.set_conv_params("conv5", p["weight"], p["bias"], p["w_scales"], p["in_scales"], p["out_scales"])
+    for _ in range(3):
+        after = net.forward("data", x, ["conv5"])[0]
+        assert np.array_equal(after.view(np.int32), want(x, "conv5").view(np.int32)) and not np.array_equal(after, before)
+
+
+def test_int8_blob_and_long_copies(small):
+    net, params, want = small
+    rng = np.random.default_rng(3)
+    for _ in range(3):
+        x = rng.uniform(0, 1, size=(1, 3, 40, 48)).astype(np.float32)
+        assert np.array_equal(net.forward("data", x, ["s2b0_r_pw1"])[0], want(x, "s2b0_r_pw1"))
+    for _ in range(3):
+        x = rng.uniform(0, 1, size=(120, 3, 40, 48)).astype(np.float32)  # 2.8 MB up, 2 MB down: more pieces than the ring has
+        assert np.array_equal(net.forward("data", x, ["conv5"])[0][[0, 59, 119]].view(np.int32), want(x[[0, 59, 119]], "conv5").view(np.int32))
+
+
+def test_pinned_buffers(small):
+    net, params, want = small
+    shape, out_shape = (2, 3, 40, 48), (2,) + net.blob_shape("conv5")[1:]
+    buf = [C.c_void_p(), C.c_void_p()]
+    for b, s in zip(buf, (shape, out_shape)):
+        assert net.lib.ott_host_alloc(int(np.prod(s)) * 4, C.byref(b)) == 0
+    x, y = (np.ctypeslib.as_array(C.cast(b, C.POINTER(C.c_float)), shape=s) for b, s in zip(buf, (shape, out_shape)))
+    for seed in range(3):
+        x[:] = np.random.default_rng(seed).uniform(0, 1, size=shape)
+        y[:] = -1
+        net.forward_raw("data", buf[0], False, shape, ["conv5"], [buf[1].value])
+        assert np.array_equal(y.view(np.int32), want(x, "conv5").view(np.int32))
+    for b in buf:
+        net.lib.ott_host_free(b)
