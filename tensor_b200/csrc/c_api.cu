@@ -1138,13 +1138,22 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
         ctx->launches += 1;
         return OTT_OK;
     }
-    DeviceBlock xq;  // scratch: the quantized activations when the input arrives as fp32
+    // scratch: the quantized activations when the input arrives as fp32 (taken whichever way this launch goes, so that what a call
+    // allocates depends on its shape alone)
+    DeviceBlock xq;
     const int8_t* x = static_cast<const int8_t*>(in_dev);
+    UmmaFloatInput f32;
+    const bool quant_inside = in_dtype == OTT_F32_NCHW && c->kind == OTT_KERNEL_DENSE_UMMA && c->n_in_scales == 1 &&
+                              umma_quantizes_inside(c->plan, s, ctx->sm_count) &&
+                              umma_float_input(static_cast<const float*>(in_dev), gather, d.cin, (long)h * w, c->in_scale0, &f32);
     if (in_dtype == OTT_F32_NCHW) {
         if (xq.alloc(ctx, (size_t)n * h * w * c->cin_pad) != cudaSuccess) {
             (void)cudaGetLastError();
             return ctx->fail(OTT_ERR_ALLOC, "scratch allocation for quantized activations failed");
         }
+        x = (const int8_t*)xq.p;
+    }
+    if (in_dtype == OTT_F32_NCHW && !quant_inside) {
         if (gather) {
             OTT_CUDA_CHECK(ctx, launch_quantize_nchw_to_nhwc(ctx->stream, *gather, (int8_t*)xq.p, c->in_scales_dev, c->n_in_scales, n, d.cin, h, w,
                                                               d.rounding));
@@ -1153,7 +1162,6 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
                                                        c->n_in_scales, n, d.cin, h, w, d.rounding));
         }
         ctx->launches += gather ? 1u : (uint64_t)((c->cin_pad + kGatherMaxChannels - 1) / kGatherMaxChannels);
-        x = (const int8_t*)xq.p;
     }
     switch (c->kind) {
         case OTT_KERNEL_DEPTHWISE:
@@ -1178,7 +1186,7 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
                 }
             }
             const char* err = launch_dense_umma(ctx->stream, ctx->sm_count, c->umma.data(), (int)c->umma.size(), s, x, ep, out_dev, out_dtype, status,
-                                                gathered ? &us : nullptr, mixed, ctx->wait_limit_ns);
+                                                gathered ? &us : nullptr, mixed, ctx->wait_limit_ns, quant_inside ? &f32 : nullptr);
             if (err) return ctx->fail(OTT_ERR_CUDA, "%s: %s", err, cudaGetErrorString(cudaGetLastError()));
             break;
         }

@@ -184,7 +184,6 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
     const int ix_al = (ix_first >= 0 ? ix_first : ix_first - 3) / 4 * 4;
     const int sh = ix_first - ix_al;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         abort_flag = 0;
@@ -199,6 +198,7 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
     if (warp == 7) {  // the warp that pools nothing (224 of the 256 threads do): its de-allocation below delays nobody
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(SPM_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        pdl_launch_dependents();  // not before this CTA has its tensor memory: see dense_umma.cu
     }
     // filters: row = output channel, 28 bytes of taps + 4 zero bytes, swizzled like the im2col rows
     if (threadIdx.x < 64) {

@@ -55,6 +55,57 @@ struct KernelMaps {
     uint8_t block_src[kUmmaMaxGatherBlocks];
 };
 
+// BUILD of the kernel, see dense_umma_kernel
+constexpr int kQuantBuild = 3, kQuantWarps = 8, kQuantRuns = 2;
+
+// fp32 input of a launch that quantizes on the way in (kQuantBuild)
+struct QuantSource {
+    // the input's channels as at most kQuantRuns runs of consecutive planes of a tensor (a Concat of two blobs is two runs):
+    // run i starts at channel first[i], whose plane is at base[i]; unused runs start past the last channel
+    const float* base[kQuantRuns];
+    long long img_stride[kQuantRuns];
+    int first[kQuantRuns];
+    float scale;
+    uint32_t half;           // rounding constant
+    int vec;                 // rows of four pixels are whole and 16-byte aligned
+    FastDiv div_halo;        // by the width of a halo tile
+    __device__ __forceinline__ const float* plane(int c, int img, int hw) const {
+        const int i = c >= first[1] ? 1 : 0;
+        return base[i] + (long long)img * img_stride[i] + (long long)(c - first[i]) * hw;
+    }
+};
+
+// Address of 16-byte chunk `chunk` of row `row` of an operand tile of bkc-byte rows at `tile` (1 KiB aligned): the swizzle TMA
+// applies for this row width.
+__device__ __forceinline__ uint32_t operand_chunk(uint32_t tile, int bkc, int row, int chunk) {
+    const uint32_t a = tile + (uint32_t)(row * bkc + chunk * 16);
+    return a ^ (((a >> 7) & ((uint32_t)(bkc >> 4) - 1u)) << 4);
+}
+
+__device__ __forceinline__ void store_chunk(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// The same position of 16 channels' planes: one load each, 4 bytes (V = float) or 16 (float4). A chunk that lies in one run walks its
+// planes; the address arithmetic of a run look-up per load costs more than the load.
+template <typename V>
+__device__ __forceinline__ void load16(V (&v)[16], const QuantSource& Q, int c0, int cin, int img, int hw, int p) {
+    if (c0 + 16 <= cin && (c0 >= Q.first[1] || c0 + 16 <= Q.first[1])) {
+        const float* ptr = Q.plane(c0, img, hw) + p;
+#pragma unroll
+        for (int j = 0; j < 16; ++j, ptr += hw) v[j] = __ldg(reinterpret_cast<const V*>(ptr));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = c0 + j < cin ? __ldg(reinterpret_cast<const V*>(Q.plane(c0 + j, img, hw) + p)) : V{};
+    }
+}
+__device__ __forceinline__ void quantize16(uint32_t addr, const float (&v)[16], const QuantSource& Q) {
+    uint32_t w[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) w[g] = quantize4_pack(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3], Q.scale, Q.half);
+    store_chunk(addr, w[0], w[1], w[2], w[3]);
+}
+
 struct SmemLayout {
     uint32_t b_panel, a_stages, bars, tmem_slot, abort_flag, params, total;
 };
@@ -82,13 +133,15 @@ __host__ __device__ inline SmemLayout smem_layout(const UmmaPlan& p) {
 // they replaced took 700 of the 1000 cycles between that wait and the first copy), the MMA issuer and the teardown wait for no
 // kernel at all, the epilogue warps work out their pixel before they wait for the accumulator, and tensor memory is freed
 // while the last rows are still being requantized.
+//
+// BUILD 3: fp32 NCHW input, quantized inside the kernel: warps 10..17 take the TMA producer's place, load the planes, quantize and
+// write the operand tiles (with TMA's swizzle) themselves. No int8 copy of the input crosses HBM and no second kernel runs.
 template <int OUT, int ACT, int BUILD>
-__global__ void __launch_bounds__(BUILD == 2 ? 64 + 32 * 16 : kMaxThreads, BUILD == 1 ? 2 : 1)
-dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant__ CUtensorMap tmB, const UmmaPlan P,
+__global__ void __launch_bounds__(BUILD >= 2 ? 64 + 32 * 16 : kMaxThreads, BUILD == 1 ? 2 : 1)
+dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuild, QuantSource, KernelMaps> maps, const __grid_constant__ CUtensorMap tmB, const UmmaPlan P,
                   const ConvShape s, const EpilogueParams ep, void* __restrict__ out, uint32_t* __restrict__ status,
                   const __grid_constant__ UmmaMixedOut mixed) {
     extern __shared__ uint8_t smem_raw[];
-    pdl_launch_dependents();
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
     const SmemLayout L = smem_layout(P);
@@ -109,11 +162,21 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
     // trip per tile instead of one per 32-channel block)
     const int loads_per_tile = P.halo ? P.ncb : (P.gather && P.gather_whole ? 1 : P.nkb);
 
+    // Tensor memory first, and only then may the next kernel start: a CTA of it that shared this SM and allocated before this one
+    // would hold the columns this one waits for while it waits for this kernel to end.
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
+                     "r"((uint32_t)P.tmem_cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        pdl_launch_dependents();
+    }
     if (threadIdx.x == 0) {
         prefetch_tensormap(&tmB);
-        for (int i = 0; i < (P.gather > 0 ? P.gather : 1); ++i) prefetch_tensormap(&maps.tm[i]);
+        if constexpr (BUILD != kQuantBuild)
+            for (int i = 0; i < (P.gather > 0 ? P.gather : 1); ++i) prefetch_tensormap(&maps.tm[i]);
         for (int i = 0; i < P.stages; ++i) {
-            mbar_init(bar_full + 8u * i, 1);
+            mbar_init(bar_full + 8u * i, BUILD == kQuantBuild ? kQuantWarps : 1);
             mbar_init(bar_empty + 8u * i, 1);
         }
         mbar_init(bar_b, 1);
@@ -138,18 +201,13 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
             sp[2 * P.bn + i] = in ? ep.scale_out[c] : 0.f;
         }
     }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
-                     "r"((uint32_t)P.tmem_cols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
+        if constexpr (BUILD != kQuantBuild)
         if (lane == 0) {
             // ---- TMA producer (activations; the weights were requested during set-up) ----
             uint32_t st = 0, phase = 1;  // stage, and the parity that says it is free (the first round finds every stage free)
@@ -293,6 +351,91 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
         if (*abort_flag) __syncthreads();
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)P.tmem_cols) : "memory");
+    } else if (BUILD == kQuantBuild && warp >= 2 + kMaxEpiWarps) {
+        if constexpr (BUILD == kQuantBuild) {
+            // ---- quantizers: warp q takes every eighth (16 channels, 32 pixels or pixel quads) item of a stage ----
+            const int qw = warp - (2 + kMaxEpiWarps), chunks = P.bkc >> 4, hw = s.h * s.w;
+            const long total_pix = (long)s.n * hw;
+            uint32_t st = 0, phase = 1;
+            int turn = qw;  // a stage of fewer than eight items starts with another warp each time
+            bool ok = true;
+            pdl_wait();
+            for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
+                int img = 0, y0 = 0, x0 = 0;
+                if (!P.flat) {
+                    img = (int)fast_div((uint32_t)m, P.div_img);
+                    const int r = m - img * P.tiles_x * P.tiles_y, ty = (int)fast_div((uint32_t)r, P.div_tx);
+                    y0 = ty * P.th - s.ph;
+                    x0 = (r - ty * P.tiles_x) * P.tw - s.pw;
+                }
+                for (int kb = 0; kb < loads_per_tile; ++kb) {
+                    if (!mbar_wait(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
+                    const uint32_t tile = sA + st * a_stage_bytes;
+                    if (P.flat && maps.vec) {
+                        const int ch = turn & 7, c0 = kb * P.bkc + ch * 16;
+                        const long gp = (long)m * kTileM + lane * 4;  // four pixels of one image
+                        if (ch < chunks && c0 < s.cin && gp < total_pix) {
+                            const int im = (int)fast_div((uint32_t)gp, P.div_plane), p = (int)(gp - (long)im * hw);
+                            float4 v[16];
+                            load16(v, maps, c0, s.cin, im, hw, p);
+                            uint32_t w[4][4];  // [group of four channels][pixel]
+#pragma unroll
+                            for (int g = 0; g < 4; ++g) {
+                                uint32_t cw[4];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const float4 f = v[4 * g + j];
+                                    cw[j] = quantize4_pack(f.x, f.y, f.z, f.w, maps.scale, maps.half);
+                                }
+                                transpose4x4(cw[0], cw[1], cw[2], cw[3], w[g]);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) store_chunk(operand_chunk(tile, P.bkc, lane * 4 + j, ch), w[0][j], w[1][j], w[2][j], w[3][j]);
+                        }
+                    } else {
+                        // pixel by pixel: flat tiles of any alignment, and halo tiles (out-of-image pixels are zeros)
+                        const int pixels = P.flat ? kTileM : halo_w * halo_h, items = ((pixels + 31) >> 5) * chunks, shift = 31 - __clz(chunks);
+                        for (int it = turn & 7; it < items; it += 2 * kQuantWarps) {
+                            float v[2][16];
+                            uint32_t dst[2];
+                            bool have[2];
+#pragma unroll
+                            for (int u = 0; u < 2; ++u) {
+                                const int item = it + u * kQuantWarps, ch = item & (chunks - 1), row = (item >> shift) * 32 + lane, c0 = kb * P.bkc + ch * 16;
+                                have[u] = item < items && row < pixels && c0 < s.cin;
+                                dst[u] = operand_chunk(tile, P.bkc, row, ch);
+                                int im = img, p;
+                                bool in;
+                                if (P.flat) {
+                                    const long gp = (long)m * kTileM + row;
+                                    in = gp < total_pix;
+                                    im = (int)fast_div((uint32_t)gp, P.div_plane);
+                                    p = (int)(gp - (long)im * hw);
+                                } else {
+                                    const int hy = (int)fast_div((uint32_t)row, maps.div_halo), iy = y0 + hy, ix = x0 + row - hy * halo_w;
+                                    in = iy >= 0 && iy < s.h && ix >= 0 && ix < s.w;
+                                    p = iy * s.w + ix;
+                                }
+                                if (have[u] && in) {
+                                    load16(v[u], maps, c0, s.cin, im, hw, p);
+                                } else {
+#pragma unroll
+                                    for (int j = 0; j < 16; ++j) v[u][j] = 0.f;
+                                }
+                            }
+#pragma unroll
+                            for (int u = 0; u < 2; ++u)
+                                if (have[u]) quantize16(dst[u], v[u], maps);
+                        }
+                    }
+                    turn += chunks;
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // these writes -> the MMA's reads
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_full + 8u * st);
+                    if (++st == (uint32_t)P.stages) { st = 0; phase ^= 1u; }
+                }
+            }
+        }
     } else {
         // ---- epilogue warps ----
         const int q = warp & 3;            // TMEM lane quarter this warp may read
@@ -306,6 +449,7 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
         const float* s_si = reinterpret_cast<const float*>(base_ptr + L.params);
         const float* s_bi = s_si + P.bn;
         const float* s_so = s_bi + P.bn;
+        const int c_base = n_tile * P.bn;  // the output channel of accumulator column 0
         const uint32_t half = half_bits(ep.rounding);
         uint32_t tile_i = 0;
         bool ok = true;
@@ -339,19 +483,19 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
                 pix = img * plane + inimg;
             }
             const uint32_t taddr = tmem_base + buf * (uint32_t)P.acc_stride + ((uint32_t)(q * 32) << 16);
-            int8_t* out_s8 = reinterpret_cast<int8_t*>(out) + pix * s.cout_pad + n_tile * P.bn;
-            int32_t* out_s32 = reinterpret_cast<int32_t*>(out) + pix * s.cout_pad + n_tile * P.bn;
+            int8_t* out_s8 = reinterpret_cast<int8_t*>(out) + pix * s.cout_pad + c_base;
+            int32_t* out_s32 = reinterpret_cast<int32_t*>(out) + pix * s.cout_pad + c_base;
             float* out_f32 = nullptr;
             if (OUT == DT_F32_NCHW) {
-                out_f32 = reinterpret_cast<float*>(out) + (img * s.cout + n_tile * P.bn) * plane + inimg;
+                out_f32 = reinterpret_cast<float*>(out) + (img * s.cout + c_base) * plane + inimg;
             } else if (OUT == DT_S8_NHWC && mixed.out_f32 != nullptr) {
                 out_f32 = mixed.plane_of_col != nullptr ? mixed.out_f32 + img * mixed.f32_planes * plane + inimg  // plane chosen per column below
-                                                        : mixed.out_f32 + (img * s.cout + n_tile * P.bn) * plane + inimg;
+                                                        : mixed.out_f32 + (img * s.cout + c_base) * plane + inimg;
             }
             // 16 accumulator columns -> 16 outputs of this thread's pixel. int8 results come back as 4 packed words in wds
             // (the caller stores them); the other output kinds are stored here.
             auto emit16 = [&](const int (&v)[16], int col0, uint32_t (&wds)[4]) {
-                const int c0 = n_tile * P.bn + col0;  // first global output channel of this chunk
+                const int c0 = c_base + col0;  // first global output channel of this chunk
                 if (OUT == DT_S32_NHWC) {
                     int4* o = reinterpret_cast<int4*>(out_s32 + col0);
 #pragma unroll
@@ -416,7 +560,7 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
             };
             // Chunks of 32 columns: two TMEM loads in flight, and int8 rows leave as one 32-byte store per thread, a whole
             // DRAM sector (two 16-byte stores from different warps would each touch half of it).
-            const bool wide_ok = OUT == DT_S8_NHWC && ((s.cout_pad | (n_tile * P.bn)) & 31) == 0;
+            const bool wide_ok = OUT == DT_S8_NHWC && ((s.cout_pad | (c_base)) & 31) == 0;
             if (!mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
             tc_fence_after();
             if (sub * chunk >= P.bn && lane == 0) mbar_arrive(bar_tempty + 8u * buf);  // a narrow tile has no columns for this warp
@@ -435,12 +579,12 @@ dense_umma_kernel(const __grid_constant__ KernelMaps maps, const __grid_constant
                 }
                 if (!valid) continue;
                 uint32_t wa[4], wb[4];
-                const bool a_ok = n_tile * P.bn + col0 < s.cout_pad, b_ok = two && n_tile * P.bn + col0 + 16 < s.cout_pad;
+                const bool a_ok = c_base + col0 < s.cout_pad, b_ok = two && c_base + col0 + 16 < s.cout_pad;
                 if (a_ok) emit16(va, col0, wa);
                 if (b_ok) emit16(vb, col0 + 16, wb);
                 if (OUT == DT_S8_NHWC && mixed.n_chunks > 0) {
                     // scattered output: each 16-column chunk has its own destination tensor
-                    const int ch = (n_tile * P.bn + col0) >> 4;
+                    const int ch = (c_base + col0) >> 4;
                     int8_t* da = a_ok ? mixed.dst[ch] : nullptr;
                     int8_t* db = b_ok ? mixed.dst[ch + 1] : nullptr;
                     if (da != nullptr && db != nullptr && ((mixed.pair_ok >> (ch >> 1)) & 1ull) != 0ull && (ch & 1) == 0) {
@@ -487,8 +631,8 @@ CUtensorMapSwizzle swizzle_for(int bkc) {
     return bkc == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (bkc == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
-template <int OUT, int ACT, int BUILD>
-const char* launch_variant(cudaStream_t stream, int sm_count, const KernelMaps& maps, const CUtensorMap& tmB, const UmmaPlan& p,
+template <int OUT, int ACT, int BUILD, typename Source>
+const char* launch_variant(cudaStream_t stream, int sm_count, const Source& maps, const CUtensorMap& tmB, const UmmaPlan& p,
                            const ConvShape& s, const EpilogueParams& ep, void* out, uint32_t* status, const UmmaMixedOut& mixed) {
     // per-device, per-instantiation set-up; several host threads may drive different GPUs through this function at once
     static std::mutex mu;
@@ -511,7 +655,7 @@ const char* launch_variant(cudaStream_t stream, int sm_count, const KernelMaps& 
     }
     // Tiles are dealt statically to the CTAs of the grid, so a grid larger than what is resident at once runs in waves.
     // The plan bounds residency by shared memory and TMEM; registers and threads are bounded here.
-    const int threads = 64 + 32 * p.epi_warps;
+    const int threads = 64 + 32 * (p.epi_warps + (BUILD == kQuantBuild ? kQuantWarps : 0));
     const int regs_per_warp = (regs * 32 + 255) / 256 * 256;
     int resident = 65536 / (regs_per_warp * (threads / 32));
     if (resident > 2048 / threads) resident = 2048 / threads;
@@ -646,9 +790,46 @@ const char* umma_encode_weight_map(const UmmaPlan& p, const int8_t* w_dev, void*
     return r == CUDA_SUCCESS ? nullptr : "cuTensorMapEncodeTiled(weights) failed";
 }
 
+// Describes an fp32 input for quantization inside the kernel; false when its planes are scattered over more runs than that takes.
+bool umma_float_input(const float* x, const PlaneGather* table, int cin, long hw, float scale, UmmaFloatInput* in) {
+    in->scale = scale;
+    in->n_runs = 0;
+    if (!table) {
+        in->base[0] = x;
+        in->img_stride[0] = (long long)cin * hw;
+        in->first[0] = 0;
+        in->n_runs = 1;
+        return true;
+    }
+    for (int c = 0; c < cin; ++c) {
+        if (c > 0 && table->ref[c] == table->ref[c - 1] + 1) continue;
+        if (in->n_runs == kQuantRuns) return false;
+        const int b = (int)(table->ref[c] >> 24);
+        in->base[in->n_runs] = table->base[b] + (long long)(table->ref[c] & 0xFFFFFFu) * hw;
+        in->img_stride[in->n_runs] = table->img_stride[b];
+        in->first[in->n_runs++] = c;
+    }
+    return true;
+}
+
+// The int8 copy of an fp32 input costs a kernel of its own (about 4 us of chain on a small launch) and an HBM round trip; inside the
+// convolution it costs every weight panel its own pass over the input, by eight warps. 1x1 layers whose images are whole pixel
+// quads win as long as there are at most two panels, or one wave of CTAs (us, copy -> inside: 192 -> 48 20x20 one image 7.9 ->
+// 4.8, 717 -> 152 18x20 x36 20.5 -> 13.6, 953 -> 160 16x60 x33 78.8 -> 39.5, 256 -> 512 28x28 x128 61.6 -> 55.5). Pixel-by-pixel
+// loads only pay on small launches (90 -> 77 31x33 x60: 18.3 -> 19.2), and for halo tiles only with one channel block (64 -> 64
+// 56x56 one image 8.5 -> 5.3; 100 -> 200 with two blocks 10.3 -> 14.5).
+bool umma_quantizes_inside(const UmmaPlan& p, const ConvShape& s, int sm_count) {
+    const bool flat = s.kh == 1 && s.kw == 1 && s.ph == 0 && s.pw == 0 && s.sh == 1 && s.sw == 1;
+    if ((!flat && !p.halo) || s.cin_pad <= 32 || (double)s.n * s.h * s.w > 2147483647.0) return false;
+    const long tiles = flat ? ((long)s.n * s.oh * s.ow + kTileM - 1) / kTileM : (long)s.n * ((s.ow + kHaloTw - 1) / kHaloTw) * ((s.oh + kHaloTh - 1) / kHaloTh);
+    const bool small = tiles * p.n_tiles <= sm_count;
+    if (!flat) return small && p.ncb == 1;
+    return small || (p.n_tiles <= 2 && (long)s.h * s.w % 4 == 0);
+}
+
 const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVariant* variants, int n_variants, const ConvShape& s,
                               const int8_t* x, const EpilogueParams& ep, void* out, int out_dtype, uint32_t* status,
-                              const UmmaSources* sources, const UmmaMixedOut* mixed_in, unsigned long long wait_limit_ns) {
+                              const UmmaSources* sources, const UmmaMixedOut* mixed_in, unsigned long long wait_limit_ns, const UmmaFloatInput* f32) {
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return "cuTensorMapEncodeTiled entry point not available";
     // The tiling of the pixels is the same for every variant. A launch with fewer tiles than SMs is bound by the chain of one
@@ -694,8 +875,9 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
         cuuint64_t dims[4] = {(cuuint64_t)s.cin_pad, (cuuint64_t)pixels, 1, 1};
         cuuint64_t strides[3] = {(cuuint64_t)s.cin_pad, (cuuint64_t)s.cin_pad * pixels, (cuuint64_t)s.cin_pad * pixels};
         cuuint32_t box[4] = {(cuuint32_t)p.bkc, (cuuint32_t)kTileM, 1, 1};
-        r = enc(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (!f32)
+            r = enc(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     } else {
         // rectangle of 128 output pixels with the least padding waste (halo mode: always 8 x 16)
         long best = -1;
@@ -716,8 +898,9 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
                              (cuuint32_t)(p.halo ? p.th + s.kh - 1 : (p.th - 1) * s.sh + 1), 1};
         estr[1] = (cuuint32_t)s.sw;
         estr[2] = (cuuint32_t)s.sh;
-        r = enc(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (!f32)
+            r = enc(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
     if (r != CUDA_SUCCESS) return "cuTensorMapEncodeTiled(activations) failed";
     for (int i = 1; i < n_variants && (long)p.m_tiles * chosen->plan.n_tiles < sm_count; ++i)
@@ -734,8 +917,27 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
 
     const CUtensorMap& tmB = *reinterpret_cast<const CUtensorMap*>(chosen->weight_map);
     const char* err = nullptr;
+    QuantSource qs;
+    if (f32) {
+        p.epi_warps = kMaxEpiWarps;
+        p.ctas_per_sm = 1;
+        p.smem_bytes = p.smem_bytes > 116 * 1024 ? p.smem_bytes : 116 * 1024;  // one CTA per SM: tensor memory is budgeted for one
+        qs.scale = f32->scale;
+        qs.half = half_bits(ep.rounding);
+        qs.div_halo = make_fast_div((uint32_t)(kHaloTw + s.kw - 1));
+        const long hw = (long)s.h * s.w;
+        qs.vec = hw % 4 == 0 ? 1 : 0;
+        for (int i = 0; i < kQuantRuns; ++i) {
+            const bool used = i < f32->n_runs;
+            qs.base[i] = used ? f32->base[i] : nullptr;
+            qs.img_stride[i] = used ? f32->img_stride[i] : 0;
+            qs.first[i] = used ? f32->first[i] : 1 << 30;
+            if (used && ((reinterpret_cast<uintptr_t>(qs.base[i]) & 15) != 0 || qs.img_stride[i] % 4 != 0)) qs.vec = 0;
+        }
+    }
 #define OTT_UMMA_LAUNCH(OUT, ACT)                                                                                     \
-    err = p.ctas_per_sm > 1   ? launch_variant<OUT, ACT, 1>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed) \
+    err = f32                 ? launch_variant<OUT, ACT, kQuantBuild>(stream, sm_count, qs, tmB, p, s, ep, out, status, mixed) \
+          : p.ctas_per_sm > 1 ? launch_variant<OUT, ACT, 1>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed) \
           : p.epi_warps == 16 ? launch_variant<OUT, ACT, 2>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed) \
                               : launch_variant<OUT, ACT, 0>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed)
 #define OTT_UMMA_ACT(OUT)                                \

@@ -91,6 +91,15 @@ void umma_pack_weights(const UmmaPlan& p, const int8_t* w_oihw, int cin, int cou
 // Encode the TMA descriptor of the packed weights (128 bytes written to map_out). Returns NULL or an error text.
 const char* umma_encode_weight_map(const UmmaPlan& p, const int8_t* w_dev, void* map_out);
 
+// fp32 NCHW input quantized inside the kernel (x of the launch is then unused), as runs of consecutive planes.
+struct UmmaFloatInput {
+    const float* base[2];
+    long long img_stride[2];
+    int first[2], n_runs;
+    float scale;
+};
+bool umma_float_input(const float* x, const PlaneGather* table, int cin, long hw, float scale, UmmaFloatInput* in);
+
 // Launch. Returns NULL or an error text.
 // sources: NULL, or where the K blocks of a plan with gather > 0 come from (x is then unused). mixed: NULL, or the fp32 side
 // output of an int8 launch.
@@ -98,6 +107,9 @@ const char* umma_encode_weight_map(const UmmaPlan& p, const int8_t* w_dev, void*
 const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVariant* variants, int n_variants, const ConvShape& s,
                               const int8_t* x, const EpilogueParams& ep, void* out, int out_dtype, uint32_t* status,
                               const UmmaSources* sources = nullptr, const UmmaMixedOut* mixed = nullptr,
-                              unsigned long long wait_limit_ns = 2000000000ull);
+                              unsigned long long wait_limit_ns = 2000000000ull, const UmmaFloatInput* f32 = nullptr);
+
+// whether a launch on fp32 input should quantize inside the kernel rather than read an int8 copy
+bool umma_quantizes_inside(const UmmaPlan& p, const ConvShape& s, int sm_count);
 
 }  // namespace ottk

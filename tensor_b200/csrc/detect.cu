@@ -6,7 +6,7 @@
 // later boxes it overlaps"), with the reference's formulas in the reference's operand order. The kept rows go straight into
 // pinned host memory (up to 16 MB of rows; what a crowded image of a huge batch has beyond its share is copied), so a call ends with one synchronisation and
 // no transfer. An image with more proposals than the CTA's shared memory holds (4096) is sorted and filtered on the host.
-// Bound by latency: the proposal kernel keeps sixteen class planes in flight per cell and takes all levels in one launch. 
+// Bound by latency: the proposal kernel keeps sixteen class planes in flight per cell and takes all levels in one launch. 32
 // images at 320x320, 29 boxes each: 114 -> 58 us a call.
 // Floating point: expf/division here and in the reference's -Ofast build round differently in the last place, so scores
 // agree to 1-2 ulp and box coordinates to about 1e-4 pixels; labels, order and counts are the same unless a score sits

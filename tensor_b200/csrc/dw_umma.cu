@@ -59,7 +59,6 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
                void* __restrict__ out, uint32_t* __restrict__ status) {
     constexpr int kEpiWarps = epi_warps_of(BUILD), kIssueWarps = issue_warps_of(BUILD);
     extern __shared__ uint8_t smem_raw[];
-    pdl_launch_dependents();
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t sW = base + P.w_off, sX = base + P.x_off;
@@ -103,6 +102,7 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"((uint32_t)P.tmem_cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        pdl_launch_dependents();  // not before this CTA has its tensor memory: see dense_umma.cu
     }
     tc_fence_before();
     __syncthreads();

@@ -60,7 +60,6 @@ __global__ void __launch_bounds__(kThreads, MULTI ? 2 : 1)
 dwpw_umma_kernel(const __grid_constant__ DwPwMaps maps, const __grid_constant__ CUtensorMap tmWdw, const __grid_constant__ CUtensorMap tmWpw, const DwPwPlan P,
                  const DwPwGeom G, const DwPwEpilogues ep, void* __restrict__ out, uint32_t* __restrict__ status, const __grid_constant__ UmmaMixedOut mixed) {
     extern __shared__ uint8_t smem_raw[];
-    pdl_launch_dependents();
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t sWdw = base + P.w_dw, sWpw = base + P.w_pw, sX = base + P.x, sY = base + P.y;
@@ -115,6 +114,7 @@ dwpw_umma_kernel(const __grid_constant__ DwPwMaps maps, const __grid_constant__ 
                      "r"((uint32_t)P.tmem_cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        pdl_launch_dependents();  // not before this CTA has its tensor memory: see dense_umma.cu
     }
     tc_fence_before();
     __syncthreads();

@@ -61,7 +61,6 @@ unit_umma_kernel(const __grid_constant__ UnitMaps maps, const __grid_constant__ 
                  const __grid_constant__ CUtensorMap tmW2, const UnitPlan P, const UnitGeom G, const UnitEpilogues ep, void* __restrict__ out,
                  uint32_t* __restrict__ status, const __grid_constant__ UmmaMixedOut mixed) {
     extern __shared__ uint8_t smem_raw[];
-    pdl_launch_dependents();
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t sW1 = base + P.w1, sWdw = base + P.wdw, sW2 = base + P.w2, sY1 = base + P.y1, sY2 = base + P.y2;
@@ -114,6 +113,7 @@ unit_umma_kernel(const __grid_constant__ UnitMaps maps, const __grid_constant__ 
                      "r"((uint32_t)P.tmem_cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        pdl_launch_dependents();  // not before this CTA has its tensor memory: see dense_umma.cu
     }
     tc_fence_before();
     __syncthreads();
