@@ -446,7 +446,7 @@ int ott_quantize_f32_nchw_to_s8_nhwc(ott_ctx* ctx, const float* x_dev, int n, in
     if (sc.alloc(ctx, sizeof(float) * n_scales) != cudaSuccess) return ctx->fail(OTT_ERR_ALLOC, "scale upload allocation failed");
     OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(sc.p, scales_host, sizeof(float) * n_scales, cudaMemcpyHostToDevice, ctx->stream));
     OTT_CUDA_CHECK(ctx, launch_quantize_dense(ctx->stream, x_dev, c, out_dev, (const float*)sc.p, n_scales, n, c, h, w, rounding));
-    ctx->launches += (uint64_t)((nhwc_channels(c) + kGatherMaxChannels - 1) / kGatherMaxChannels);
+    ctx->launches += 1;
     // the pageable scale array must stay readable until the copy has been issued; it has (pageable copies
     // are staged synchronously)
     return OTT_OK;
@@ -1161,7 +1161,7 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
             OTT_CUDA_CHECK(ctx, launch_quantize_dense(ctx->stream, static_cast<const float*>(in_dev), d.cin, (int8_t*)xq.p, c->in_scales_dev,
                                                        c->n_in_scales, n, d.cin, h, w, d.rounding));
         }
-        ctx->launches += gather ? 1u : (uint64_t)((c->cin_pad + kGatherMaxChannels - 1) / kGatherMaxChannels);
+        ctx->launches += 1;
     }
     switch (c->kind) {
         case OTT_KERNEL_DEPTHWISE:

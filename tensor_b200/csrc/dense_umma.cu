@@ -813,18 +813,19 @@ bool umma_float_input(const float* x, const PlaneGather* table, int cin, long hw
 }
 
 // The int8 copy of an fp32 input costs a kernel of its own (about 4 us of chain on a small launch) and an HBM round trip; inside the
-// convolution it costs every weight panel its own pass over the input, by eight warps. 1x1 layers whose images are whole pixel
-// quads win as long as there are at most two panels, or one wave of CTAs (us, copy -> inside: 192 -> 48 20x20 one image 7.9 ->
-// 4.8, 717 -> 152 18x20 x36 20.5 -> 13.6, 953 -> 160 16x60 x33 78.8 -> 39.5, 256 -> 512 28x28 x128 61.6 -> 55.5). Pixel-by-pixel
-// loads only pay on small launches (90 -> 77 31x33 x60: 18.3 -> 19.2), and for halo tiles only with one channel block (64 -> 64
-// 56x56 one image 8.5 -> 5.3; 100 -> 200 with two blocks 10.3 -> 14.5).
+// convolution it costs every weight panel its own pass over the input, by eight warps, and leaves the epilogue eight. 1x1 layers
+// whose images are whole pixel quads win with one panel that does not want sixteen epilogue warps, or with one wave of CTAs (us,
+// copy / inside: 192 -> 48 20x20 one image 7.9 / 4.8, 717 -> 152 18x20 x36 16.0 / 13.5, 953 -> 160 16x60 x33 41 / 39, 116 -> 116
+// 20x20 x256 17.5 / 16.1; but 256 -> 512 28x28 x128 52 / 55). Pixel-by-pixel loads only pay on small launches (90 -> 77 31x33 x60:
+// 12.5 / 19.2), and for halo tiles only with one channel block (64 -> 64 56x56 one image 8.5 / 5.3; 100 -> 200 with two blocks
+// 7.6 / 14.5).
 bool umma_quantizes_inside(const UmmaPlan& p, const ConvShape& s, int sm_count) {
     const bool flat = s.kh == 1 && s.kw == 1 && s.ph == 0 && s.pw == 0 && s.sh == 1 && s.sw == 1;
     if ((!flat && !p.halo) || s.cin_pad <= 32 || (double)s.n * s.h * s.w > 2147483647.0) return false;
     const long tiles = flat ? ((long)s.n * s.oh * s.ow + kTileM - 1) / kTileM : (long)s.n * ((s.ow + kHaloTw - 1) / kHaloTw) * ((s.oh + kHaloTh - 1) / kHaloTh);
     const bool small = tiles * p.n_tiles <= sm_count;
     if (!flat) return small && p.ncb == 1;
-    return small || (p.n_tiles <= 2 && (long)s.h * s.w % 4 == 0);
+    return small || (p.n_tiles == 1 && p.bn <= 192 && (long)s.h * s.w % 4 == 0);
 }
 
 const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVariant* variants, int n_variants, const ConvShape& s,

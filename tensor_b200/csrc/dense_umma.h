@@ -5,17 +5,6 @@
 
 namespace ottk {
 
-// Quotients by a divisor known at launch: n / d = (umulhi(n, mul) + n) >> shift for n < 2^31.
-struct FastDiv {
-    uint32_t mul, shift;
-};
-inline FastDiv make_fast_div(uint32_t d) {
-    uint32_t s = 0;
-    while ((1ull << s) < d) ++s;
-    return FastDiv{(uint32_t)((((1ull << s) - d) << 32) / d + 1), s};
-}
-__device__ __forceinline__ uint32_t fast_div(uint32_t n, FastDiv d) { return (__umulhi(n, d.mul) + n) >> d.shift; }
-
 // Fixed per layer at create time (tiling of K and N), completed per call (tiling of the pixels).
 struct UmmaPlan {
     // K: each filter tap is split into ncb channel blocks of bkc bytes (32/64/128 = the swizzle span)

@@ -13,6 +13,17 @@ __host__ __device__ inline int nhwc_channels(int c) { return (c + 15) & ~15; }
 
 enum : int { DT_F32_NCHW = 0, DT_S8_NHWC = 1, DT_S32_NHWC = 2 };
 
+// Quotients by a divisor known at launch: n / d = (umulhi(n, mul) + n) >> shift for n < 2^31.
+struct FastDiv {
+    uint32_t mul, shift;
+};
+inline FastDiv make_fast_div(uint32_t d) {
+    uint32_t s = 0;
+    while ((1ull << s) < d) ++s;
+    return FastDiv{(uint32_t)((((1ull << s) - d) << 32) / d + 1), s};
+}
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, FastDiv d) { return (__umulhi(n, d.mul) + n) >> d.shift; }
+
 // Shape of one convolution call (all kernels).
 struct ConvShape {
     int n, h, w, oh, ow;

@@ -72,7 +72,7 @@ extern "C" int ott_conv_int8_forward_noalloc(ott_ctx* ctx, const ott_conv* conv,
     // so nothing left in the array by an earlier call can leak into this one and nothing needs clearing.
     OTT_CUDA_CHECK(ctx, launch_quantize_dense(ctx->stream, in_f32_nchw_dev, conv->d.cin, reinterpret_cast<int8_t*>(scratch), conv->in_scales_dev,
                                                       conv->n_in_scales, n, conv->d.cin, h, w, conv->d.rounding));
-    ctx->launches += (uint64_t)((conv->cin_pad + kGatherMaxChannels - 1) / kGatherMaxChannels);  // one launch per 512-channel slice
+    ctx->launches += 1;
     // int8 input: this path of the ordinary forward launches the convolution kernel and takes no scratch
     return ott_conv_int8_forward(ctx, conv, scratch, OTT_S8_NHWC, n, h, w, out_dev, out_dtype, nullptr);
 }

@@ -3,9 +3,11 @@
 // Net::convert_layout (Tensor/Net.cpp:380-411).
 //
 // HBM-bound: 4 bytes read + 1 byte written per element. Each CTA moves a [64 channels x 128 pixels] tile
-// of one image: reads are float4 along W (the contiguous axis of NCHW), the channel/pixel transpose of
-// 4x4 blocks happens in registers, 32-bit words of 4 channels go through shared memory, and writes are
-// 16-byte groups of channels (the contiguous axis of NHWC).
+// of one image: reads are float4 along W (the contiguous axis of NCHW), eight of them in flight per thread, the channel/pixel
+// transpose of 4x4 blocks happens in registers, 32-bit words of 4 channels go through shared memory, and writes are
+// 16-byte groups of channels (the contiguous axis of NHWC). Tile coordinates are the grid's, the image of a pixel is a
+// multiply-shift quotient: with 64-bit divisions a thread spent more instructions on finding its 32 elements than on them
+// (17 per element; 64 channels 56x56 x256: 55.1 -> 41.6 us = 6.2 TB/s, 256 channels 28x28 x128: 31.1 -> 24.5).
 #include "kernels.h"
 #include "launch.cuh"
 
@@ -20,61 +22,68 @@ constexpr int QT_PITCH = 17;  // words per pixel row in shared memory (16 used):
 // four row groups, and the 32 lanes of a warp land in 32 consecutive rows of a group (no bank conflicts).
 __device__ __forceinline__ int qt_row(int p) { return (p & 3) * 33 + (p >> 2); }
 
-__global__ void __launch_bounds__(QT_THREADS)
-quantize_nchw_to_nhwc_kernel(const __grid_constant__ PlaneGather G, int8_t* __restrict__ out, const float* __restrict__ scales,
-                             int n_scales, int c, int cpad, int hw, int tiles_p, int tiles_c, uint32_t half, int out_stride, int scale_base, int flat,
-                             long total_px) {
+// A plain tensor's planes by arithmetic, a plane table's by look-up.
+struct DensePlanes {
+    const float* x;
+    long long img_stride;
+    __device__ __forceinline__ const float* plane(int c, int img, long hw) const { return x + (long long)img * img_stride + (long long)c * hw; }
+};
+
+static void advance_images(DensePlanes& g, int images) { g.x += (long long)images * g.img_stride; }
+static void advance_images(PlaneGather& g, int images) {
+    for (int i = 0; i < kGatherMaxBufs; ++i) g.base[i] += (long long)images * g.img_stride[i];
+}
+
+// Grid: x = pixel tile, y = channel tile, z = image (one when flat). flat: the pixel axis runs over all images (hw % 4 == 0, so a
+// thread's 4 pixels never straddle two images) and no tile is wasted on the tail of an image.
+template <typename Planes>
+__global__ void __launch_bounds__(QT_THREADS, 4)
+quantize_nchw_to_nhwc_kernel(const __grid_constant__ Planes G, int8_t* __restrict__ out, const float* __restrict__ scales, int n_scales, int c, int cpad,
+                             int hw, uint32_t half, int out_stride, int flat, int vec_ok, long total_px, FastDiv div_hw) {
     __shared__ uint32_t tile[4 * 33 * QT_PITCH];
     pdl_launch_dependents();
     pdl_wait();
-    const long tile_id = blockIdx.x;
-    const int tc = (int)(tile_id % tiles_c);
-    const int tp = (int)((tile_id / tiles_c) % tiles_p);
-    // flat: the pixel axis runs over all images (hw % 4 == 0, so a thread's 4 pixels never straddle two images) and no
-    // tile is wasted on the tail of an image; otherwise tiles are per image
-    const int img_tile = flat ? 0 : (int)(tile_id / ((long)tiles_c * tiles_p));
-    const int c0 = tc * QT_C;
-    const long p0 = (long)tp * QT_P;                     // first pixel of the tile (global when flat, in-image otherwise)
+    const int c0 = blockIdx.y * QT_C;
+    const long p0 = (long)blockIdx.x * QT_P;             // first pixel of the tile (global when flat, in-image otherwise)
     const long px_end = flat ? total_px : (long)hw;      // pixels beyond this do not exist
 
     // phase 1: a thread quantizes 4 consecutive pixels of 4 consecutive channels and packs, per pixel, the
     // 4 channels into one word. Lanes run along pixels (512 contiguous bytes per channel row per warp).
+    constexpr int PASSES = QT_C / 32;
     const int pq = threadIdx.x & 31, cq = threadIdx.x >> 5;
-    const bool vec_ok = (hw % 4 == 0);
     const long gp = p0 + pq * 4;
-    const int img = flat ? (int)(gp / hw) : img_tile;
+    const int img = flat ? (total_px <= 0x7FFFFFFFl ? (int)fast_div((uint32_t)gp, div_hw) : (int)(gp / hw)) : (int)blockIdx.z;
     const int p = flat ? (int)(gp - (long)img * hw) : (int)gp;
+    const bool vec = vec_ok && gp + 3 < px_end;
+    float4 v[PASSES][4];
 #pragma unroll
-    for (int pass = 0; pass < QT_C / 32; ++pass) {
-        if (c0 + 32 * pass >= cpad) break;  // narrow tensors: nothing of this half of the tile is ever stored
-        const int cword = cq + 8 * pass;
-        uint32_t cw[4];  // channel i: its 4 pixels packed
-        float4 v[4];
-        float sc[4];
-        const bool fast = vec_ok && gp + 3 < px_end && c0 + cword * 4 + 3 < c;
-        if (fast) {
+    for (int pass = 0; pass < PASSES; ++pass)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int cg = c0 + cword * 4 + i;
-                sc[i] = n_scales == 1 ? __ldg(scales) : __ldg(scales + scale_base + cg);
-                v[i] = __ldg(reinterpret_cast<const float4*>(G.plane(cg, img, hw) + p));
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) cw[i] = quantize4_pack(v[i].x, v[i].y, v[i].z, v[i].w, sc[i], half);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int cg = c0 + cword * 4 + i;
-                int q[4] = {0, 0, 0, 0};
-                if (cg < c) {
-                    const float s = n_scales == 1 ? __ldg(scales) : __ldg(scales + scale_base + cg);
-                    const float* row = G.plane(cg, img, hw);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (gp + j < px_end) q[j] = quantize1(__ldg(row + p + j), s, half);
+        for (int i = 0; i < 4; ++i) {
+            const int cg = c0 + (cq + 8 * pass) * 4 + i;
+            v[pass][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (cg < c) {
+                const float* row = G.plane(cg, img, hw) + p;
+                if (vec) {
+                    v[pass][i] = __ldg(reinterpret_cast<const float4*>(row));
+                } else {
+                    if (gp < px_end) v[pass][i].x = __ldg(row);
+                    if (gp + 1 < px_end) v[pass][i].y = __ldg(row + 1);
+                    if (gp + 2 < px_end) v[pass][i].z = __ldg(row + 2);
+                    if (gp + 3 < px_end) v[pass][i].w = __ldg(row + 3);
                 }
-                cw[i] = pack4(q[0], q[1], q[2], q[3]);
             }
+        }
+#pragma unroll
+    for (int pass = 0; pass < PASSES; ++pass) {
+        const int cword = cq + 8 * pass;
+        if (c0 + cword * 4 >= cpad) break;  // narrow tensors: nothing of these channels is ever stored
+        uint32_t cw[4];  // channel i: its 4 pixels packed
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int cg = c0 + cword * 4 + i;
+            const float sc = n_scales == 1 ? __ldg(scales) : (cg < c ? __ldg(scales + cg) : 0.f);
+            cw[i] = quantize4_pack(v[pass][i].x, v[pass][i].y, v[pass][i].z, v[pass][i].w, sc, half);
         }
         uint32_t pw[4];  // pixel j: its 4 channels packed
         transpose4x4(cw[0], cw[1], cw[2], cw[3], pw);
@@ -83,16 +92,32 @@ quantize_nchw_to_nhwc_kernel(const __grid_constant__ PlaneGather G, int8_t* __re
     }
     __syncthreads();
     // phase 2: 16-byte channel groups; consecutive threads -> consecutive groups of one pixel
-    int8_t* dst = out + (long)img_tile * hw * out_stride;
+    int8_t* dst = out + ((flat ? 0l : (long)blockIdx.z * hw) + p0) * out_stride + c0;
+#pragma unroll
     for (int i = threadIdx.x; i < QT_P * (QT_C / 16); i += QT_THREADS) {
         const int pl = i >> 2, g = i & 3;
-        const long pg = p0 + pl;
-        const int cg = c0 + g * 16;
-        if (pg < px_end && cg < cpad) {
+        if (p0 + pl < px_end && c0 + g * 16 < cpad) {
             const uint32_t* r = tile + qt_row(pl) * QT_PITCH + g * 4;
-            *reinterpret_cast<uint4*>(dst + pg * out_stride + cg) = make_uint4(r[0], r[1], r[2], r[3]);
+            *reinterpret_cast<uint4*>(dst + (long)pl * out_stride + g * 16) = make_uint4(r[0], r[1], r[2], r[3]);
         }
     }
+}
+
+template <typename Planes>
+static cudaError_t launch_quantize(cudaStream_t stream, const Planes& src, int8_t* out, int out_stride, const float* scales_dev, int n_scales, int vec_ok,
+                                   int n, int c, int cpad, int hw, int rounding) {
+    const int flat = hw % 4 == 0 ? 1 : 0;
+    const long total_px = (long)n * hw, span = flat ? total_px : hw;
+    for (int img0 = 0; img0 < (flat ? 1 : n); img0 += 65535) {  // (the grid's third dimension ends at 65535)
+        Planes part = src;
+        if (img0 > 0) advance_images(part, img0);
+        const dim3 grid((unsigned)((span + QT_P - 1) / QT_P), (unsigned)((cpad + QT_C - 1) / QT_C), (unsigned)(flat ? 1 : (n - img0 < 65535 ? n - img0 : 65535)));
+        const cudaError_t e = launch_overlapped(quantize_nchw_to_nhwc_kernel<Planes>, grid, dim3(QT_THREADS), 0, stream, part, out + (long)img0 * hw * out_stride,
+                                                scales_dev, n_scales, c, cpad, hw, half_bits(rounding), out_stride, flat, vec_ok, total_px,
+                                                make_fast_div((uint32_t)hw));
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 void gather_identity(PlaneGather* g, const float* x, int c, int c_total, long hw) {
@@ -106,37 +131,22 @@ cudaError_t launch_quantize_nchw_to_nhwc(cudaStream_t stream, const PlaneGather&
     const int hw = h * w, cpad = nhwc_channels(c);
     if (n == 0 || hw == 0) return cudaSuccess;
     if (c > kGatherMaxChannels) return cudaErrorInvalidValue;
-    const int flat = hw % 4 == 0 ? 1 : 0;
-    const long total_px = (long)n * hw;
-    const int tiles_p = flat ? (int)((total_px + QT_P - 1) / QT_P) : (hw + QT_P - 1) / QT_P, tiles_c = (cpad + QT_C - 1) / QT_C;
-    const long blocks = (long)(flat ? 1 : n) * tiles_p * tiles_c;
-    return launch_overlapped(quantize_nchw_to_nhwc_kernel, dim3((unsigned)blocks), dim3(QT_THREADS), 0, stream, src, out, scales_dev, n_scales, c, cpad,
-                             hw, tiles_p, tiles_c, half_bits(rounding), cpad, 0, flat, total_px);
+    bool aligned = hw % 4 == 0;  // four pixels of a plane are one 16-byte load
+    for (int i = 0, last = -1; i < c && aligned; ++i) {
+        const int b = (int)(src.ref[i] >> 24);
+        if (b != last) aligned = (reinterpret_cast<uintptr_t>(src.base[b]) & 15) == 0 && src.img_stride[b] % 4 == 0;
+        last = b;
+    }
+    return launch_quantize(stream, src, out, cpad, scales_dev, n_scales, aligned ? 1 : 0, n, c, cpad, hw, rounding);
 }
 
-// A plain tensor of any channel count: the plane table holds kGatherMaxChannels entries, so wider tensors are
-// quantized in channel chunks, each launch writing its slice of the NHWC rows.
+// a plain tensor of any channel count
 cudaError_t launch_quantize_dense(cudaStream_t stream, const float* x, int c_total, int8_t* out, const float* scales_dev, int n_scales,
                                   int n, int c, int h, int w, int rounding) {
     const int hw = h * w, cpad = nhwc_channels(c);
     if (n == 0 || hw == 0) return cudaSuccess;
-    const int flat = hw % 4 == 0 ? 1 : 0;
-    const long total_px = (long)n * hw;
-    const int tiles_p = flat ? (int)((total_px + QT_P - 1) / QT_P) : (hw + QT_P - 1) / QT_P;
-    for (int base = 0; base < cpad; base += kGatherMaxChannels) {
-        const int chunk_pad = cpad - base < kGatherMaxChannels ? cpad - base : kGatherMaxChannels;  // channels written by this launch
-        const int chunk = c - base < chunk_pad ? (c - base > 0 ? c - base : 0) : chunk_pad;          // of which real ones
-        PlaneGather g;
-        g.base[0] = x;
-        g.img_stride[0] = (long long)c_total * hw;
-        for (int i = 0; i < chunk; ++i) g.ref[i] = (uint32_t)(base + i);
-        const int tiles_c = (chunk_pad + QT_C - 1) / QT_C;
-        const long blocks = (long)(flat ? 1 : n) * tiles_p * tiles_c;
-        cudaError_t e = launch_overlapped(quantize_nchw_to_nhwc_kernel, dim3((unsigned)blocks), dim3(QT_THREADS), 0, stream, g, out + base, scales_dev,
-                                          n_scales, chunk, chunk_pad, hw, tiles_p, tiles_c, half_bits(rounding), cpad, base, flat, total_px);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    return launch_quantize(stream, DensePlanes{x, (long long)c_total * hw}, out, cpad, scales_dev, n_scales,
+                           hw % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? 1 : 0, n, c, cpad, hw, rounding);
 }
 
 // dst[img][c][p] = plane(c, img)[p]
