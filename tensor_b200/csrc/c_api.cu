@@ -2,6 +2,7 @@
 // ConvolutionLayer's create_pipeline_int8 / forward_int8 (Tensor/ConvolutionLayer.cpp:666-752, :754-847)
 // mapped onto the CUDA kernels. No CPU compute path exists here: every forward launches kernels.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <new>
@@ -614,6 +615,24 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
     c->bias_host = bias_p;
     c->scale_out_host = scale_out;
     c->in_scale0 = in_scales[0];
+    if (requant) {
+        c->one_scale_out = std::all_of(scale_out.begin(), scale_out.begin() + d->cout, [&](float v) { return v == scale_out[0]; }) ? 1 : 0;
+        // whether the clamp of the int8 output can stand for the activation (EpilogueParams::int8_pos): the largest sum the
+        // weights allow bounds what is requantized, and ReLU6 must have nothing to cut that the clamp would not
+        bool pos = d->act_type == ACT_RELU || d->act_type == ACT_RELU6;
+        const size_t per_cout = (size_t)(d->cin / d->groups) * d->kh * d->kw;
+        for (int p = 0; p < d->cout && pos; ++p) {
+            long sum = 0;
+            for (size_t i = 0; i < per_cout; ++i) sum += std::abs((int)w_oihw[p * per_cout + i]);
+            const double top = (128.0 * (double)sum * std::fabs((double)scale_in[p]) + std::fabs((double)bias_p[p])) * scale_out[p];
+            pos = scale_out[p] > 0.f && top < 32000.0;  // (false for NaN)
+            if (d->act_type == ACT_RELU6) {
+                const volatile float six = 6.f * scale_out[p], sum_h = six + (d->rounding == OTT_ROUND_HALF_AWAY ? 0x1.fffffep-2f : 0.5f);
+                pos = pos && sum_h >= 127.f;
+            }
+        }
+        c->int8_pos = pos ? 1 : 0;
+    }
     int rc = OTT_OK;
     std::vector<int8_t> wpacked;
     const int taps = d->kh * d->kw;
@@ -997,6 +1016,7 @@ int forward_maxpool_impl(ott_ctx* ctx, const ott_conv* c, const float* in_dev, i
     cudaSetDevice(ctx->device);
     EpilogueParams ep{};
     ep.scale_in = c->scale_in_dev; ep.bias = c->bias_dev; ep.scale_out = c->scale_out_dev;
+    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos;
     ep.has_bias = d.bias_term ? 1 : 0;
     ep.act_type = d.act_type; ep.act_param0 = d.act_param0; ep.rounding = d.rounding;
     OTT_CUDA_CHECK(ctx, launch_dense_stem_pool(ctx->stream, s, in_dev, c->w_host.data(), c->scale_in_host.data(), c->bias_host.data(),
@@ -1080,6 +1100,7 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
 
     EpilogueParams ep{};
     ep.scale_in = c->scale_in_dev; ep.bias = c->bias_dev; ep.scale_out = c->scale_out_dev;
+    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos;
     ep.has_bias = d.bias_term ? 1 : 0;
     ep.act_type = d.act_type; ep.act_param0 = d.act_param0; ep.rounding = d.rounding;
 

@@ -19,6 +19,7 @@
 namespace ottk {
 
 enum : int { ACT_NONE = 0, ACT_RELU = 1, ACT_LRELU = 2, ACT_RELU6 = 3 };
+constexpr int ACT_POS = 4;  // kernel builds only: int8 output whose activation the clamp to [0, 127] carries out, see EpilogueParams
 enum : int { ROUND_ADD_HALF_TRUNC = 0, ROUND_HALF_AWAY = 1 };
 
 // Per-layer epilogue parameters. Arrays are device pointers with one entry per (padded) output channel;
@@ -31,6 +32,11 @@ struct EpilogueParams {
     int act_type;
     float act_param0;
     int rounding;
+    int one_scale_out;       // every channel's scale_out is scale_out0
+    float scale_out0;
+    // ReLU, or ReLU6 where f(6) is 127 in every channel, and |v * scale_out| + 1 stays below 2^15 in every channel whatever the int8
+    // input is: float2int8(act(v) * scale_out) is trunc(v * scale_out + h) clamped to [0, 127], see requant4_pos
+    int int8_pos;
 };
 
 __device__ __forceinline__ float dequant(int acc, float scale_in, float bias, int has_bias) {
@@ -120,6 +126,19 @@ __device__ __forceinline__ int2 round2_nonneg(float2 v, uint32_t h) {
 template <int ACT>
 __device__ __forceinline__ int2 round2_act(float2 v, uint32_t h) {
     return ACT == ACT_RELU || ACT == ACT_RELU6 ? round2_nonneg(v, h) : round2(v, h);
+}
+
+// Four v * scale_out of an int8_pos layer -> four int8 of the activated values, a.x in byte 0. Adding 1.5 * 2^23 with rounding toward
+// zero leaves trunc(u + h) in the low bits of the sum (a floor below zero, which the clamp drops), so that neither the activation nor
+// a conversion to integer is an instruction of its own, and two values are clamped at a time: 2.3 logic instructions per value
+// less. Exact while |u| + h < 2^15, where the low 16 bits carry the sign.
+__device__ __forceinline__ uint32_t requant4_pos(float2 a, float2 b, uint32_t h) {
+    const float2 hh = make_float2(__uint_as_float(h), __uint_as_float(h)), magic = make_float2(12582912.f, 12582912.f);
+    const float2 ra = __fadd2_rz(__fadd2_rn(a, hh), magic), rb = __fadd2_rz(__fadd2_rn(b, hh), magic);
+    uint32_t pa = __byte_perm(__float_as_uint(ra.x), __float_as_uint(ra.y), 0x5410), pb = __byte_perm(__float_as_uint(rb.x), __float_as_uint(rb.y), 0x5410);
+    asm("min.relu.s16x2 %0, %0, %1;" : "+r"(pa) : "r"(0x007F007Fu));
+    asm("min.relu.s16x2 %0, %0, %1;" : "+r"(pb) : "r"(0x007F007Fu));
+    return __byte_perm(pa, pb, 0x6420);
 }
 
 // quantize 4 floats with one scale and pack them, x in byte 0
