@@ -60,6 +60,13 @@ struct KernelMaps {
 // shared memory, the same for all lanes, takes two passes of the data pipe that the output stores need too): a third fewer of
 // them, 64 -> 256 56x56 x128 without activation 51.9 -> 48.1 us. A test inside one build costs as much as it saves.
 constexpr int kOneScale = 8;
+// Compact builds: the output kind and the activation are arguments and nothing large is unrolled, so that every layer of a network's
+// small launches runs the same 39 KB of code. A specialised build is 60 to 110 KB, of which a launch runs about a third; when the
+// launch before it ran another build, its instructions come from L2 again: 20x20x116 -> 116, one image, us per launch, specialised /
+// compact: the same layer over and over 2.57 / 2.65, two activations in turn 3.20 / 2.63, five builds in turn 4.07 / 2.63.
+constexpr int kAnyOut = 7, kAnyAct = 7;
+constexpr int kCompactBuild = 4, kCompactQuantBuild = 5;
+constexpr __host__ __device__ bool build_quantizes(int build) { return build == 3 || build == kCompactQuantBuild; }
 constexpr int kQuantBuild = 3, kQuantWarps = 8, kQuantRuns = 2;
 
 // fp32 input of a launch that quantizes on the way in (kQuantBuild)
@@ -111,7 +118,7 @@ __device__ __forceinline__ void quantize16(uint32_t addr, const float (&v)[16], 
 }
 
 // columns of an accumulator an epilogue warp takes at a time
-__host__ __device__ __forceinline__ int epi_chunk(const UmmaPlan& p) { return p.bn <= 32 ? 16 : 32; }
+__host__ __device__ __forceinline__ int epi_chunk(const UmmaPlan& p) { return p.bn <= 32 || p.compact ? 16 : 32; }
 
 struct SmemLayout {
     uint32_t b_panel, a_stages, bars, tmem_slot, abort_flag, params, total;
@@ -141,15 +148,18 @@ __host__ __device__ inline SmemLayout smem_layout(const UmmaPlan& p) {
 // kernel at all, the epilogue warps work out their pixel before they wait for the accumulator, and tensor memory is freed
 // while the last rows are still being requantized.
 //
+// BUILDs 4 and 5: see kAnyOut.
+//
 // BUILD 3: fp32 NCHW input, quantized inside the kernel: warps 10..17 take the TMA producer's place, load the planes, quantize and
 // write the operand tiles (with TMA's swizzle) themselves. No int8 copy of the input crosses HBM and no second kernel runs.
 template <int OUT, int ACT_BUILD, int BUILD>
 __global__ void __launch_bounds__(BUILD >= 2 ? 64 + 32 * 16 : kMaxThreads, BUILD == 1 ? 2 : 1)
-dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuild, QuantSource, KernelMaps> maps, const __grid_constant__ CUtensorMap tmB, const UmmaPlan P,
+dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUILD), QuantSource, KernelMaps> maps, const __grid_constant__ CUtensorMap tmB, const UmmaPlan P,
                   const ConvShape s, const EpilogueParams ep, void* __restrict__ out, uint32_t* __restrict__ status,
                   const __grid_constant__ UmmaMixedOut mixed) {
     constexpr int ACT = ACT_BUILD & ~kOneScale;
-    constexpr bool ONE_SCALE = (ACT_BUILD & kOneScale) != 0;
+    constexpr bool ONE_SCALE = (ACT_BUILD & kOneScale) != 0, COMPACT = BUILD >= kCompactBuild, QUANT = build_quantizes(BUILD);
+    const auto writes = [&](int kind) { return OUT == kAnyOut ? P.out_kind == kind : OUT == kind; };
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -182,13 +192,16 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
     }
     if (threadIdx.x == 0) {
         prefetch_tensormap(&tmB);
-        if constexpr (BUILD != kQuantBuild)
+        if constexpr (!QUANT)
+#pragma unroll 1
             for (int i = 0; i < (P.gather > 0 ? P.gather : 1); ++i) prefetch_tensormap(&maps.tm[i]);
+#pragma unroll 1
         for (int i = 0; i < P.stages; ++i) {
-            mbar_init(bar_full + 8u * i, BUILD == kQuantBuild ? kQuantWarps : 1);
+            mbar_init(bar_full + 8u * i, QUANT ? kQuantWarps : 1);
             mbar_init(bar_empty + 8u * i, 1);
         }
         mbar_init(bar_b, 1);
+#pragma unroll 1
         for (int i = 0; i < P.acc_bufs; ++i) {
             mbar_init(bar_tfull + 8u * i, 1);
             mbar_init(bar_tempty + 8u * i, 4u * (uint32_t)((P.bn + epi_chunk(P) - 1) / epi_chunk(P)));  // one arrival per lane quarter and column chunk
@@ -198,10 +211,12 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         // the weight panel does not depend on the previous kernel: start loading it before waiting for that kernel
         mbar_expect_tx(bar_b, (uint32_t)P.nkb * b_tile_bytes);
+#pragma unroll 1
         for (int kb = 0; kb < P.nkb; ++kb) tma_load_2d(&tmB, bar_b, sB + kb * b_tile_bytes, kb * P.bkc, n_tile * P.bn);
     }
     {
         float* sp = reinterpret_cast<float*>(base_ptr + L.params);
+#pragma unroll 1
         for (int i = threadIdx.x; i < P.bn; i += (int)blockDim.x) {
             const int c = n_tile * P.bn + i;
             const bool in = c < s.cout_pad;
@@ -216,7 +231,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if constexpr (BUILD != kQuantBuild)
+        if constexpr (!QUANT)
         if (lane == 0) {
             // ---- TMA producer (activations; the weights were requested during set-up) ----
             uint32_t st = 0, phase = 1;  // stage, and the parity that says it is free (the first round finds every stage free)
@@ -242,6 +257,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
                         waited = true;
                     }
                     if (P.gather && P.gather_whole) {
+#pragma unroll 1
                         for (int g = 0; g < P.nkb; ++g)
                             tma_load_4d(&maps.tm[maps.block_src[g]], full, dst + (uint32_t)(g * kTileM * P.bkc), (int)maps.block_x[g], x0, 0, 0);
                     } else if (P.gather) {
@@ -289,7 +305,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
                         const uint64_t b0 = make_smem_desc(sB + kb * b_tile_bytes, P.bkc);
                         const uint32_t b_tap_step = ((uint32_t)P.ncb * b_tile_bytes) >> 4, a_px_step = (uint32_t)P.bkc >> 4;
                         uint32_t accumulate = kb != 0 ? 1u : 0u, a_row = 0, b_off = 0;
-                        if (s.kh == 3 && s.kw == 3) {
+                        if (!COMPACT && s.kh == 3 && s.kw == 3) {
                             // the common filter: all loops unrolled, every descriptor the base's low word plus a constant (the
                             // address field cannot carry), so that the one issuing thread spends its time issuing
                             const uint32_t a_lo = (uint32_t)a0, b_lo = (uint32_t)b0;
@@ -314,6 +330,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
                         for (int ky = 0; ky < s.kh; ++ky, a_row += (uint32_t)halo_w * a_px_step) {
                             uint32_t a_off = a_row;
                             for (int kx = 0; kx < s.kw; ++kx, a_off += a_px_step, b_off += b_tap_step) {
+#pragma unroll (COMPACT ? 1 : 4)
                                 for (int j = 0; j < P.bkc / 32; ++j) {
                                     umma_i8(d, a0 + a_off + 2u * j, b0 + b_off + 2u * j, P.idesc, accumulate);
                                     accumulate = 1u;
@@ -327,7 +344,9 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
                         const uint64_t a_hi = a0 & 0xFFFFFFFF00000000ull, b_hi = b0 & 0xFFFFFFFF00000000ull;
                         const uint32_t a_step = (uint32_t)(kTileM * P.bkc) >> 4, b_step = b_tile_bytes >> 4;
                         uint32_t ao = 0, bo = 0;
+#pragma unroll 1
                         for (int g = 0; g < P.nkb; ++g, ao += a_step, bo += b_step)
+#pragma unroll 1
                             for (int j = 0; j < P.bkc / 32; ++j)
                                 umma_i8(d, a_hi | (uint64_t)(a_lo + ao + 2u * j), b_hi | (uint64_t)(b_lo + bo + 2u * j), P.idesc, (g | j) != 0 ? 1u : 0u);
                     } else {
@@ -340,7 +359,10 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
 #pragma unroll
                             for (int j = 0; j < J; ++j) umma_i8(d, a_hi | (uint64_t)(a_lo + 2u * j), b_hi | (uint64_t)(b_lo + 2u * j), P.idesc, (kb | j) != 0 ? 1u : 0u);
                         };
-                        if (P.bkc == 128) steps(std::integral_constant<int, 4>{});
+                        if (COMPACT) {
+#pragma unroll 1
+                            for (int j = 0; j < P.bkc / 32; ++j) umma_i8(d, a_hi | (uint64_t)(a_lo + 2u * j), b_hi | (uint64_t)(b_lo + 2u * j), P.idesc, (kb | j) != 0 ? 1u : 0u);
+                        } else if (P.bkc == 128) steps(std::integral_constant<int, 4>{});
                         else if (P.bkc == 64) steps(std::integral_constant<int, 2>{});
                         else steps(std::integral_constant<int, 1>{});
                     }
@@ -360,8 +382,8 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
         if (*abort_flag) __syncthreads();
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)P.tmem_cols) : "memory");
-    } else if (BUILD == kQuantBuild && warp >= 2 + kMaxEpiWarps) {
-        if constexpr (BUILD == kQuantBuild) {
+    } else if (QUANT && warp >= 2 + kMaxEpiWarps) {
+        if constexpr (QUANT) {
             // ---- quantizers: warp q takes every eighth (16 channels, 32 pixels or pixel quads) item of a stage ----
             const int qw = warp - (2 + kMaxEpiWarps), chunks = P.bkc >> 4, hw = s.h * s.w;
             const long total_pix = (long)s.n * hw;
@@ -449,9 +471,9 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
         // ---- epilogue warps ----
         const int q = warp & 3;            // TMEM lane quarter this warp may read
         const int sub = (warp - 2) >> 2;   // which of the epi_warps/4 warps sharing that quarter
-        const int chunk = epi_chunk(P), n_chunks = (P.bn + chunk - 1) / chunk, nsub = P.epi_warps / 4;
+        const int chunk = COMPACT ? 16 : epi_chunk(P), n_chunks = (P.bn + chunk - 1) / chunk, nsub = P.epi_warps / 4;
         const int row = q * 32 + lane;
-        const int row_y = row / P.tw, row_x = row - row_y * P.tw;
+        const int row_y = row >> (31 - __clz(P.tw)), row_x = row & (P.tw - 1);  // (tw is a power of two)
         const long plane = (long)s.oh * s.ow;
         const long total_pix = (long)s.n * plane;
         const float* s_si = reinterpret_cast<const float*>(base_ptr + L.params);
@@ -475,7 +497,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
             if (P.flat) {
                 pix = (long)m * kTileM + row;
                 valid = pix < total_pix;
-                if (OUT == DT_F32_NCHW || (OUT == DT_S8_NHWC && mixed.out_f32 != nullptr)) {
+                if (writes(DT_F32_NCHW) || (writes(DT_S8_NHWC) && mixed.out_f32 != nullptr)) {
                     if (total_pix <= 0x7FFFFFFFl) {
                         const uint32_t q32 = fast_div((uint32_t)pix, P.div_plane);
                         img = (long)q32;
@@ -498,9 +520,9 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
             int8_t* out_s8 = reinterpret_cast<int8_t*>(out) + pix * s.cout_pad + c_base;
             int32_t* out_s32 = reinterpret_cast<int32_t*>(out) + pix * s.cout_pad + c_base;
             float* out_f32 = nullptr;
-            if (OUT == DT_F32_NCHW) {
+            if (writes(DT_F32_NCHW)) {
                 out_f32 = reinterpret_cast<float*>(out) + (img * s.cout + c_base) * plane + inimg;
-            } else if (OUT == DT_S8_NHWC && mixed.out_f32 != nullptr) {
+            } else if (writes(DT_S8_NHWC) && mixed.out_f32 != nullptr) {
                 out_f32 = mixed.plane_of_col != nullptr ? mixed.out_f32 + img * mixed.f32_planes * plane + inimg  // plane chosen per column below
                                                         : mixed.out_f32 + (img * s.cout + c_base) * plane + inimg;
             }
@@ -508,7 +530,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
             // (the caller stores them); the other output kinds are stored here.
             auto emit16 = [&](const int (&v)[16], int col0, uint32_t (&wds)[4]) {
                 const int c0 = c_base + col0;  // first global output channel of this chunk
-                if (OUT == DT_S32_NHWC) {
+                if (writes(DT_S32_NHWC)) {
                     int4* o = reinterpret_cast<int4*>(out_s32 + col0);
 #pragma unroll
                     for (int g = 0; g < 4; ++g) o[g] = make_int4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
@@ -530,7 +552,17 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
                         y[g * 4 + 2 * h + 1] = activate_t<ACT>(t.y, ep.act_param0);
                     }
                 }
-                if (OUT == DT_F32_NCHW) {
+                if (ACT == kAnyAct) {  // (activate_t<kAnyAct> left the values as they are)
+                    if (ep.act_type == ACT_LRELU) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) y[j] = activate_t<ACT_LRELU>(y[j], ep.act_param0);
+                    } else if (ep.act_type != ACT_NONE) {
+                        const float top = ep.act_type == ACT_RELU6 ? 6.f : __int_as_float(0x7F800000);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) y[j] = fminf(activate_t<ACT_RELU>(y[j], 0.f), top);
+                    }
+                }
+                if (writes(DT_F32_NCHW)) {
                     // one plane further per channel: a pointer that walks, and one bounds test per chunk where the chunk is whole
                     float* o = out_f32 + (long)col0 * plane;
                     if (c0 + 16 <= s.cout) {
@@ -572,7 +604,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
             };
             // Chunks of 32 columns: two TMEM loads in flight, and int8 rows leave as one 32-byte store per thread, a whole
             // DRAM sector (two 16-byte stores from different warps would each touch half of it).
-            const bool wide_ok = OUT == DT_S8_NHWC && ((s.cout_pad | (c_base)) & 31) == 0;
+            const bool wide_ok = writes(DT_S8_NHWC) && ((s.cout_pad | (c_base)) & 31) == 0;
             if (!mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) break;
             tc_fence_after();
             for (; ci < n_chunks; ci += nsub) {
@@ -593,7 +625,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
                 if (valid && a_ok) emit16(v, col0, wa);
                 if (valid && b_ok) emit16(v2, col0 + 16, wb);
                 if (!valid) continue;
-                if (OUT == DT_S8_NHWC && mixed.n_chunks > 0) {
+                if (writes(DT_S8_NHWC) && mixed.n_chunks > 0) {
                     // scattered output: each 16-column chunk has its own destination tensor
                     const int ch = (c_base + col0) >> 4;
                     int8_t* da = a_ok ? mixed.dst[ch] : nullptr;
@@ -606,7 +638,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<BUILD == kQuantBuil
                         if (da != nullptr) *reinterpret_cast<uint4*>(da + pix * mixed.pitch[ch]) = make_uint4(wa[0], wa[1], wa[2], wa[3]);
                         if (db != nullptr) *reinterpret_cast<uint4*>(db + pix * mixed.pitch[ch + 1]) = make_uint4(wb[0], wb[1], wb[2], wb[3]);
                     }
-                } else if (OUT == DT_S8_NHWC) {
+                } else if (writes(DT_S8_NHWC)) {
                     if (a_ok && b_ok && wide_ok) {
                         asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out_s8 + col0), "r"(wa[0]), "r"(wa[1]),
                                      "r"(wa[2]), "r"(wa[3]), "r"(wb[0]), "r"(wb[1]), "r"(wb[2]), "r"(wb[3])
@@ -666,7 +698,7 @@ const char* launch_variant(cudaStream_t stream, int sm_count, const Source& maps
     }
     // Tiles are dealt statically to the CTAs of the grid, so a grid larger than what is resident at once runs in waves.
     // The plan bounds residency by shared memory and TMEM; registers and threads are bounded here.
-    const int threads = 64 + 32 * (p.epi_warps + (BUILD == kQuantBuild ? kQuantWarps : 0));
+    const int threads = 64 + 32 * (p.epi_warps + (build_quantizes(BUILD) ? kQuantWarps : 0));
     const int regs_per_warp = (regs * 32 + 255) / 256 * 256;
     int resident = 65536 / (regs_per_warp * (threads / 32));
     if (resident > 2048 / threads) resident = 2048 / threads;
@@ -959,17 +991,29 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
         case ACT_RELU6: OTT_UMMA_LAUNCH(OUT, ACT_RELU6); break; \
         default: OTT_UMMA_LAUNCH(OUT, ACT_NONE); break;         \
     }
-    if (out_dtype == DT_S32_NHWC) {
+    // One more build in a chain of small launches is one more kernel whose code the SMs have to fetch (0.45 us per launch over a
+    // network on one image, where only some layers have one scale): from 2^25 outputs on the saved loads are worth several times that.
+    const bool one_scale = ep.one_scale_out && pixels * s.cout_pad >= (1l << 25);
+    // One tile per CTA: the launch is a chain whose longest part is fetching its own code, see kAnyOut. (Sixteen epilogue warps of
+    // sixteen columns each: the shortest code and the shortest chain; the quantizing build has room for eight.) Detector on one
+    // 416x416 image 488 -> 440 us, backbone on one 320x320 image 180 -> 168.
+    p.out_kind = out_dtype;
+    if ((long)p.m_tiles * p.n_tiles <= sm_count) {
+        p.compact = 1;
+        p.epi_warps = f32 ? kMaxEpiWarps : 2 * kMaxEpiWarps;
+        err = f32 ? launch_variant<kAnyOut, kAnyAct, kCompactQuantBuild>(stream, sm_count, qs, tmB, p, s, ep, out, status, mixed)
+                  : launch_variant<kAnyOut, kAnyAct, kCompactBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed);
+    } else if (out_dtype == DT_S32_NHWC) {
         OTT_UMMA_LAUNCH(DT_S32_NHWC, ACT_NONE);
     } else if (out_dtype == DT_F32_NCHW) {
         OTT_UMMA_ACT(DT_F32_NCHW)
-    } else if (ep.int8_pos && ep.one_scale_out) {
+    } else if (ep.int8_pos && one_scale) {
         OTT_UMMA_LAUNCH(DT_S8_NHWC, ACT_POS | kOneScale);
     } else if (ep.int8_pos) {
         OTT_UMMA_LAUNCH(DT_S8_NHWC, ACT_POS);
-    } else if (ep.one_scale_out && ep.act_type == ACT_NONE) {
+    } else if (one_scale && ep.act_type == ACT_NONE) {
         OTT_UMMA_LAUNCH(DT_S8_NHWC, ACT_NONE | kOneScale);
-    } else if (ep.one_scale_out && ep.act_type == ACT_LRELU) {
+    } else if (one_scale && ep.act_type == ACT_LRELU) {
         OTT_UMMA_LAUNCH(DT_S8_NHWC, ACT_LRELU | kOneScale);
     } else {
         OTT_UMMA_ACT(DT_S8_NHWC)

@@ -20,6 +20,8 @@ struct UmmaPlan {
     int epi_warps;   // epilogue warps per CTA: 8 or 16
     int ctas_per_sm; // resident CTAs per SM the launch is sized for (limited by TMEM columns and shared memory)
     // per call
+    int compact;     // the compact build runs it
+    int out_kind;    // DT_ of the output
     int halo;        // k x k layers: one TMA box per pixel tile and channel block holds the tile plus its halo; the taps read shifted views
     int a_stage_bytes;  // bytes of one activation stage (a 128-pixel tile, or a halo tile rounded up to 1 KiB)
     int flat;                          // 1x1: activations viewed as one [pixels, channels] matrix
