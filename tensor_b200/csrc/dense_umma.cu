@@ -44,6 +44,7 @@ constexpr int kMaxEpiWarps = 8;                     // 2 per TMEM lane quarter
 constexpr int kMaxThreads = 64 + 32 * kMaxEpiWarps;  // UmmaPlan::epi_warps is 4 or 8 (16 in the wide-tile build)
 constexpr int kTileM = 128;
 constexpr int kMaxAccBufs = 4;
+constexpr uint32_t kHalfSm = 113 * 1024;  // shared memory of a CTA that leaves room for another like it
 constexpr int kHaloTw = 8, kHaloTh = 16;  // pixel tile of the halo mode: 8 wide so that a tile row is one 8-row operand group
 using namespace umma;
 
@@ -153,12 +154,15 @@ __host__ __device__ inline SmemLayout smem_layout(const UmmaPlan& p) {
 // BUILD 3: fp32 NCHW input, quantized inside the kernel: warps 10..17 take the TMA producer's place, load the planes, quantize and
 // write the operand tiles (with TMA's swizzle) themselves. No int8 copy of the input crosses HBM and no second kernel runs.
 template <int OUT, int ACT_BUILD, int BUILD>
-__global__ void __launch_bounds__(BUILD >= 2 ? 64 + 32 * 16 : kMaxThreads, BUILD == 1 ? 2 : 1)
+__global__ void __launch_bounds__(BUILD == 2 || build_quantizes(BUILD) ? 64 + 32 * 16 : kMaxThreads, BUILD == 1 || BUILD == kCompactBuild ? 2 : 1)
 dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUILD), QuantSource, KernelMaps> maps, const __grid_constant__ CUtensorMap tmB, const UmmaPlan P,
                   const ConvShape s, const EpilogueParams ep, void* __restrict__ out, uint32_t* __restrict__ status,
                   const __grid_constant__ UmmaMixedOut mixed) {
     constexpr int ACT = ACT_BUILD & ~kOneScale;
     constexpr bool ONE_SCALE = (ACT_BUILD & kOneScale) != 0, COMPACT = BUILD >= kCompactBuild, QUANT = build_quantizes(BUILD);
+    // Pixels of a tile that are loaded and written: 128, or in a compact launch of a 1x1 layer fewer (the MMA's other rows read what
+    // the stage happens to hold and nobody reads their sums).
+    const int tile_rows = COMPACT ? P.tile_rows : kTileM;
     const auto writes = [&](int kind) { return OUT == kAnyOut ? P.out_kind == kind : OUT == kind; };
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -204,7 +208,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
 #pragma unroll 1
         for (int i = 0; i < P.acc_bufs; ++i) {
             mbar_init(bar_tfull + 8u * i, 1);
-            mbar_init(bar_tempty + 8u * i, 4u * (uint32_t)((P.bn + epi_chunk(P) - 1) / epi_chunk(P)));  // one arrival per lane quarter and column chunk
+            mbar_init(bar_tempty + 8u * i, (uint32_t)(tile_rows + 31) / 32u * (uint32_t)((P.bn + epi_chunk(P) - 1) / epi_chunk(P)));  // one arrival per lane quarter and column chunk
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -236,11 +240,11 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
             // ---- TMA producer (activations; the weights were requested during set-up) ----
             uint32_t st = 0, phase = 1;  // stage, and the parity that says it is free (the first round finds every stage free)
             bool ok = true, waited = false;
-            const uint32_t load_bytes = P.gather && P.gather_whole ? (uint32_t)(kTileM * P.bkc * P.nkb)
+            const uint32_t load_bytes = P.gather && P.gather_whole ? (uint32_t)(tile_rows * P.bkc * P.nkb)
                                         : P.halo                    ? (uint32_t)(halo_w * halo_h * P.bkc)
-                                                                    : (uint32_t)kTileM * P.bkc;
+                                                                    : (uint32_t)(tile_rows * P.bkc);
             for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
-                int img = 0, y0 = 0, x0 = m * kTileM;
+                int img = 0, y0 = 0, x0 = m * tile_rows;
                 if (!P.flat) {
                     img = (int)fast_div((uint32_t)m, P.div_img);
                     const int r = m - img * P.tiles_x * P.tiles_y, ty = (int)fast_div((uint32_t)r, P.div_tx);
@@ -404,8 +408,8 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                     const uint32_t tile = sA + st * a_stage_bytes;
                     if (P.flat && maps.vec) {
                         const int ch = turn & 7, c0 = kb * P.bkc + ch * 16;
-                        const long gp = (long)m * kTileM + lane * 4;  // four pixels of one image
-                        if (ch < chunks && c0 < s.cin && gp < total_pix) {
+                        const long gp = (long)m * tile_rows + lane * 4;  // four pixels of one image
+                        if (ch < chunks && c0 < s.cin && gp < total_pix && lane * 4 < tile_rows) {
                             const int im = (int)fast_div((uint32_t)gp, P.div_plane), p = (int)(gp - (long)im * hw);
                             float4 v[16];
                             load16(v, maps, c0, s.cin, im, hw, p);
@@ -425,7 +429,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                         }
                     } else {
                         // pixel by pixel: flat tiles of any alignment, and halo tiles (out-of-image pixels are zeros)
-                        const int pixels = P.flat ? kTileM : halo_w * halo_h, items = ((pixels + 31) >> 5) * chunks, shift = 31 - __clz(chunks);
+                        const int pixels = P.flat ? tile_rows : halo_w * halo_h, items = ((pixels + 31) >> 5) * chunks, shift = 31 - __clz(chunks);
                         for (int it = turn & 7; it < items; it += 2 * kQuantWarps) {
                             float v[2][16];
                             uint32_t dst[2];
@@ -438,7 +442,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                                 int im = img, p;
                                 bool in;
                                 if (P.flat) {
-                                    const long gp = (long)m * kTileM + row;
+                                    const long gp = (long)m * tile_rows + row;
                                     in = gp < total_pix;
                                     im = (int)fast_div((uint32_t)gp, P.div_plane);
                                     p = (int)(gp - (long)im * hw);
@@ -488,15 +492,15 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
         int ci = sub;  // this warp's next chunk, counted from the current tile's first
         pdl_wait();  // the outputs written below may still be read by the previous kernel
         for (int m = m_first; m < P.m_tiles; m += m_step, ++tile_i, ci -= n_chunks) {
-            if (ci >= n_chunks) continue;
+            if (ci >= n_chunks || q * 32 >= tile_rows) continue;
             const uint32_t buf = tile_i & acc_mask, use = tile_i >> acc_shift;
             // which output pixel this thread's TMEM lane holds
             long pix;  // linear (img, oy, ox) index
             long img = 0, inimg = 0;
             bool valid;
             if (P.flat) {
-                pix = (long)m * kTileM + row;
-                valid = pix < total_pix;
+                pix = (long)m * tile_rows + row;
+                valid = pix < total_pix && row < tile_rows;
                 if (writes(DT_F32_NCHW) || (writes(DT_S8_NHWC) && mixed.out_f32 != nullptr)) {
                     if (total_pix <= 0x7FFFFFFFl) {
                         const uint32_t q32 = fast_div((uint32_t)pix, P.div_plane);
@@ -896,33 +900,11 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
     p.flat = flat ? 1 : 0;
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = CUDA_SUCCESS;
-    if ((p.gather > 0) != (sources != nullptr)) return "gathered layer launched without its sources (or the reverse)";
-    if (p.gather > 0) {
-        if (!flat || sources->n_src != p.gather || p.nkb > kUmmaMaxGatherBlocks || p.bkc != kUmmaGatherBlock) return "bad gathered launch";
-        p.tw = kTileM; p.th = 1; p.tiles_x = (int)((pixels + kTileM - 1) / kTileM); p.tiles_y = 1;
+    if (flat) {
+        p.tw = p.tile_rows = kTileM; p.th = 1; p.tiles_x = (int)((pixels + kTileM - 1) / kTileM); p.tiles_y = 1;
         p.m_tiles = p.tiles_x;
-        for (int i = 0; i < sources->n_src && r == CUDA_SUCCESS; ++i) {
-            const cuuint64_t cp = (cuuint64_t)sources->src_cpad[i];
-            cuuint64_t dims[4] = {cp, (cuuint64_t)pixels, 1, 1};
-            cuuint64_t strides[3] = {cp, cp * pixels, cp * pixels};
-            cuuint32_t box[4] = {(cuuint32_t)p.bkc, (cuuint32_t)kTileM, 1, 1};
-            r = enc(&km.tm[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)sources->src[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        }
-        for (int kb = 0; kb < p.nkb; ++kb) {
-            km.block_x[kb] = sources->block_x[kb];
-            km.block_src[kb] = sources->block_src[kb];
-        }
-    } else if (flat) {
-        p.tw = kTileM; p.th = 1; p.tiles_x = (int)((pixels + kTileM - 1) / kTileM); p.tiles_y = 1;
-        p.m_tiles = p.tiles_x;
-        cuuint64_t dims[4] = {(cuuint64_t)s.cin_pad, (cuuint64_t)pixels, 1, 1};
-        cuuint64_t strides[3] = {(cuuint64_t)s.cin_pad, (cuuint64_t)s.cin_pad * pixels, (cuuint64_t)s.cin_pad * pixels};
-        cuuint32_t box[4] = {(cuuint32_t)p.bkc, (cuuint32_t)kTileM, 1, 1};
-        if (!f32)
-            r = enc(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     } else {
+        p.tile_rows = kTileM;
         // rectangle of 128 output pixels with the least padding waste (halo mode: always 8 x 16)
         long best = -1;
         for (int tw = 8; tw <= 128; tw *= 2) {
@@ -935,6 +917,46 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
         p.tiles_x = (s.ow + p.tw - 1) / p.tw;
         p.tiles_y = (s.oh + p.th - 1) / p.th;
         p.m_tiles = s.n * p.tiles_x * p.tiles_y;
+    }
+    for (int i = 1; i < n_variants && (long)p.m_tiles * chosen->plan.n_tiles < sm_count; ++i)
+        if ((long)p.m_tiles * variants[i].plan.n_tiles <= (long)sm_count * variants[i].plan.ctas_per_sm) chosen = variants + i;
+    {
+        const UmmaPlan tiling = p;
+        p = chosen->plan;
+        p.flat = tiling.flat; p.tw = tiling.tw; p.th = tiling.th; p.tiles_x = tiling.tiles_x; p.tiles_y = tiling.tiles_y; p.m_tiles = tiling.m_tiles;
+        p.tile_rows = tiling.tile_rows;
+    }
+    // SMs still idle: fewer pixels per tile. A tile's loads arrive a row at a time, and a gathered layer has a row of 32 bytes per pixel
+    // and K block (232 channels gathered in 15 blocks: 1900 rows for 128 pixels). 128 / 64 / 32 / 16 pixels at most: 116 -> 116 20x20
+    // 2.59 / 2.47 / 2.37 / 2.30 us, detector on one 416x416 image 450 / 433 / 429 / 427, backbone 169 / 164 / 160 / 159. A quantizing
+    // launch, whose CTAs have an SM to themselves, keeps 32 (116 -> 116: 3.8, with 16 4.4).
+    while (flat && p.tile_rows > (f32 ? 32 : 16) && (pixels + p.tile_rows / 2 - 1) / (p.tile_rows / 2) * p.n_tiles <= sm_count) {
+        p.tile_rows /= 2;
+        p.m_tiles = p.tiles_x = (int)((pixels + p.tile_rows - 1) / p.tile_rows);
+    }
+    if ((p.gather > 0) != (sources != nullptr)) return "gathered layer launched without its sources (or the reverse)";
+    if (p.gather > 0) {
+        if (!flat || sources->n_src != p.gather || p.nkb > kUmmaMaxGatherBlocks || p.bkc != kUmmaGatherBlock) return "bad gathered launch";
+        for (int i = 0; i < sources->n_src && r == CUDA_SUCCESS; ++i) {
+            const cuuint64_t cp = (cuuint64_t)sources->src_cpad[i];
+            cuuint64_t dims[4] = {cp, (cuuint64_t)pixels, 1, 1};
+            cuuint64_t strides[3] = {cp, cp * pixels, cp * pixels};
+            cuuint32_t box[4] = {(cuuint32_t)p.bkc, (cuuint32_t)p.tile_rows, 1, 1};
+            r = enc(&km.tm[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)sources->src[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        }
+        for (int kb = 0; kb < p.nkb; ++kb) {
+            km.block_x[kb] = sources->block_x[kb];
+            km.block_src[kb] = sources->block_src[kb];
+        }
+    } else if (flat) {
+        cuuint64_t dims[4] = {(cuuint64_t)s.cin_pad, (cuuint64_t)pixels, 1, 1};
+        cuuint64_t strides[3] = {(cuuint64_t)s.cin_pad, (cuuint64_t)s.cin_pad * pixels, (cuuint64_t)s.cin_pad * pixels};
+        cuuint32_t box[4] = {(cuuint32_t)p.bkc, (cuuint32_t)p.tile_rows, 1, 1};
+        if (!f32)
+            r = enc(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    } else {
         cuuint64_t dims[4] = {(cuuint64_t)s.cin_pad, (cuuint64_t)s.w, (cuuint64_t)s.h, (cuuint64_t)s.n};
         cuuint64_t strides[3] = {(cuuint64_t)s.cin_pad, (cuuint64_t)s.cin_pad * s.w, (cuuint64_t)s.cin_pad * s.w * s.h};
         // a strided layer's box spans (tw - 1) * sw + 1 columns of which the traversal takes every sw-th: tw land in shared memory
@@ -947,13 +969,6 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
                     swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
     if (r != CUDA_SUCCESS) return "cuTensorMapEncodeTiled(activations) failed";
-    for (int i = 1; i < n_variants && (long)p.m_tiles * chosen->plan.n_tiles < sm_count; ++i)
-        if ((long)p.m_tiles * variants[i].plan.n_tiles <= (long)sm_count * variants[i].plan.ctas_per_sm) chosen = variants + i;
-    {
-        const UmmaPlan tiling = p;
-        p = chosen->plan;
-        p.flat = tiling.flat; p.tw = tiling.tw; p.th = tiling.th; p.tiles_x = tiling.tiles_x; p.tiles_y = tiling.tiles_y; p.m_tiles = tiling.m_tiles;
-    }
     p.wait_ns = wait_limit_ns;
     p.div_img = make_fast_div((uint32_t)(p.tiles_x * p.tiles_y));
     p.div_tx = make_fast_div((uint32_t)p.tiles_x);
@@ -994,13 +1009,20 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
     // One more build in a chain of small launches is one more kernel whose code the SMs have to fetch (0.45 us per launch over a
     // network on one image, where only some layers have one scale): from 2^25 outputs on the saved loads are worth several times that.
     const bool one_scale = ep.one_scale_out && pixels * s.cout_pad >= (1l << 25);
-    // One tile per CTA: the launch is a chain whose longest part is fetching its own code, see kAnyOut. (Sixteen epilogue warps of
-    // sixteen columns each: the shortest code and the shortest chain; the quantizing build has room for eight.) Detector on one
-    // 416x416 image 488 -> 440 us, backbone on one 320x320 image 180 -> 168.
+    // One tile per CTA: the launch is a chain whose longest part is fetching its own code, see kAnyOut (detector on one 416x416 image
+    // 488 -> 440 us, backbone on one 320x320 image 180 -> 168). The next launch of such a chain sets itself up meanwhile where there is
+    // room for it on the same SMs, so the plan takes no more than one tile needs: eight epilogue warps at 96 registers, the stages of
+    // one tile, one accumulator (464 -> 1024 on 10x10, 128 CTAs: 4.6 -> 3.5 us).
     p.out_kind = out_dtype;
     if ((long)p.m_tiles * p.n_tiles <= sm_count) {
         p.compact = 1;
-        p.epi_warps = f32 ? kMaxEpiWarps : 2 * kMaxEpiWarps;
+        p.epi_warps = kMaxEpiWarps;
+        const int loads = p.halo ? p.ncb : (p.gather && p.gather_whole ? 1 : p.nkb);
+        if (p.stages > loads) p.stages = loads;
+        while (p.stages > 2 && smem_layout(p).total + 1024 > kHalfSm) --p.stages;
+        p.smem_bytes = (int)smem_layout(p).total + 1024;
+        p.acc_bufs = 2;  // (of which the one tile uses the first)
+        p.tmem_cols = p.acc_stride;
         err = f32 ? launch_variant<kAnyOut, kAnyAct, kCompactQuantBuild>(stream, sm_count, qs, tmB, p, s, ep, out, status, mixed)
                   : launch_variant<kAnyOut, kAnyAct, kCompactBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed);
     } else if (out_dtype == DT_S32_NHWC) {

@@ -27,6 +27,7 @@ struct UmmaPlan {
     int flat;                          // 1x1: activations viewed as one [pixels, channels] matrix
     int gather;                        // > 0: the K blocks come from this many int8 NHWC tensors (see UmmaSources)
     int gather_whole;                  // gathered layer whose pipeline stage holds all the K blocks of a pixel tile
+    int tile_rows;   // pixels of a tile (128, fewer in small launches of 1x1 layers)
     int tw, th, tiles_x, tiles_y, m_tiles;  // 128-pixel output rectangles (tw*th == 128)
     FastDiv div_img, div_tx, div_plane;     // by the tiles of an image, the tiles of a tile row, the pixels of an output plane
     unsigned long long wait_ns;        // limit of every mbarrier wait inside the kernel

@@ -28,3 +28,15 @@ def test_narrow_panels(ctx, cin, cout, h, w, k, stride):
         got, want = run_gpu(ctx, case, rounding), run_port(case, rounding)
         assert np.array_equal(got["acc"], want["acc"])
         assert np.array_equal(bits(got["y"]), bits(want["y"]))
+
+
+@pytest.mark.parametrize("pixels", [(1, 1), (3, 5), (4, 4), (1, 17), (1, 31), (4, 8), (3, 11), (7, 9), (5, 13), (1, 127), (3, 43), (20, 20)])
+@pytest.mark.parametrize("cin,cout", [(33, 40), (200, 70)])
+def test_few_pixels_per_tile(ctx, cin, cout, pixels):
+    from gpu_support import bits, run_gpu
+    for term, s8_input, act in ((101, True, ACT_RELU), (1, True, ACT_RELU6), (101, False, ACT_LRELU), (1, False, ACT_NONE)):
+        case = ConvCase(f"few_{pixels}", cin, cout, 1, 1, 0, n=1, h=pixels[0], w=pixels[1], bias_term=1, int8_scale_term=term, act_type=act, act_param0=0.1,
+                        s8_input=s8_input, seed=cin + pixels[1]).make()
+        got, want = run_gpu(ctx, case, ROUND_ADD_HALF_TRUNC), run_port(case, ROUND_ADD_HALF_TRUNC)
+        assert np.array_equal(got["acc"], want["acc"])
+        assert np.array_equal(bits(got["y"]), bits(want["y"]))
