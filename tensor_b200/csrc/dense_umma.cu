@@ -712,6 +712,8 @@ const char* launch_variant(cudaStream_t stream, int sm_count, const Source& maps
     if (per_n < 1) per_n = 1;
     if (per_n > p.m_tiles) per_n = p.m_tiles;
     const int grid = per_n * p.n_tiles;
+    // the compact plan holds one accumulator: a CTA with a second tile would compute it in columns that are not its own
+    if (p.compact && per_n < p.m_tiles) return "compact launch of more than one tile per CTA";
     if (launch_overlapped(kernel, dim3(grid), dim3(threads), (size_t)p.smem_bytes, stream, maps, tmB, p, s, ep, out, status, mixed) != cudaSuccess)
         return "dense_umma_kernel launch failed";
     return nullptr;
