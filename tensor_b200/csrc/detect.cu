@@ -6,7 +6,7 @@
 // later boxes it overlaps"), with the reference's formulas in the reference's operand order. The kept rows go straight into
 // pinned host memory (up to 16 MB of rows; what a crowded image of a huge batch has beyond its share is copied), so a call ends with one synchronisation and
 // no transfer. An image with more proposals than the CTA's shared memory holds (4096) is sorted and filtered on the host.
-// Bound by latency: the proposal kernel keeps sixteen class planes in flight per cell and takes all levels in one launch. 32
+// Bound by latency: the proposal kernel keeps forty class planes, then all the bins of a box in flight per cell and takes all levels in one launch. 32
 // images at 320x320, 29 boxes each: 114 -> 58 us a call.
 // Floating point: expf/division here and in the reference's -Ofast build round differently in the last place, so scores
 // agree to 1-2 ulp and box coordinates to about 1e-4 pixels; labels, order and counts are the same unless a score sits
@@ -27,7 +27,7 @@ struct Proposal {
     int order, pad;  // order = position in the reference's proposal list (level, row, column): the sort's tie-break
 };
 
-constexpr int kMaxLevels = 8, kClassBatch = 16;
+constexpr int kMaxLevels = 8, kClassBatch = 40, kBinBatch = 8;
 constexpr size_t kStagedBytes = 16u << 20;
 struct Levels {
     const float* pred[kMaxLevels];
@@ -48,31 +48,48 @@ nanodet_proposals_kernel(const __grid_constant__ Levels L, int num_class, int re
     const float* base = L.pred[l] + (long)img * (num_class + 4 * reg_bins) * plane + p;
     int label = -1;
     float score = -FLT_MAX;
-    int k = 0;
-    for (; k + kClassBatch <= num_class; k += kClassBatch) {
+    for (int k = 0; k < num_class; k += kClassBatch) {
         float v[kClassBatch];
 #pragma unroll
-        for (int j = 0; j < kClassBatch; ++j) v[j] = __ldg(base + (k + j) * plane);
+        for (int j = 0; j < kClassBatch; ++j) v[j] = k + j < num_class ? __ldg(base + (k + j) * plane) : -FLT_MAX;
 #pragma unroll
         for (int j = 0; j < kClassBatch; ++j)
             if (v[j] > score) { label = k + j; score = v[j]; }
     }
-    for (; k < num_class; ++k) {
-        const float v = __ldg(base + k * plane);
-        if (v > score) { label = k; score = v; }
-    }
     score = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-score)));
     if (!(score >= prob_threshold)) return;
     float ltrb[4];
-    for (int side = 0; side < 4; ++side) {
-        float v[kMaxRegBins], m = -FLT_MAX, sum = 0.f, dis = 0.f;
-        for (int b = 0; b < reg_bins; ++b) {
-            v[b] = __ldg(base + (num_class + side * reg_bins + b) * plane);
-            m = fmaxf(m, v[b]);
+    const float* bins = base + num_class * plane;
+    if (reg_bins <= kBinBatch) {  // all four sides' bins in flight at once
+        float v[4][kBinBatch];
+#pragma unroll
+        for (int side = 0; side < 4; ++side)
+#pragma unroll
+            for (int b = 0; b < kBinBatch; ++b) v[side][b] = b < reg_bins ? __ldg(bins + (side * reg_bins + b) * plane) : -FLT_MAX;
+#pragma unroll
+        for (int side = 0; side < 4; ++side) {
+            float m = -FLT_MAX, sum = 0.f, dis = 0.f;
+#pragma unroll
+            for (int b = 0; b < kBinBatch; ++b) m = fmaxf(m, v[side][b]);
+#pragma unroll
+            for (int b = 0; b < kBinBatch; ++b)
+                if (b < reg_bins) { v[side][b] = expf(__fsub_rn(v[side][b], m)); sum = __fadd_rn(sum, v[side][b]); }
+#pragma unroll
+            for (int b = 0; b < kBinBatch; ++b)
+                if (b < reg_bins) dis = __fadd_rn(dis, __fmul_rn((float)b, __fdiv_rn(v[side][b], sum)));
+            ltrb[side] = __fmul_rn(dis, (float)stride);
         }
-        for (int b = 0; b < reg_bins; ++b) { v[b] = expf(__fsub_rn(v[b], m)); sum = __fadd_rn(sum, v[b]); }
-        for (int b = 0; b < reg_bins; ++b) dis = __fadd_rn(dis, __fmul_rn((float)b, __fdiv_rn(v[b], sum)));
-        ltrb[side] = __fmul_rn(dis, (float)stride);
+    } else {
+        for (int side = 0; side < 4; ++side) {
+            float v[kMaxRegBins], m = -FLT_MAX, sum = 0.f, dis = 0.f;
+            for (int b = 0; b < reg_bins; ++b) {
+                v[b] = __ldg(bins + (side * reg_bins + b) * plane);
+                m = fmaxf(m, v[b]);
+            }
+            for (int b = 0; b < reg_bins; ++b) { v[b] = expf(__fsub_rn(v[b], m)); sum = __fadd_rn(sum, v[b]); }
+            for (int b = 0; b < reg_bins; ++b) dis = __fadd_rn(dis, __fmul_rn((float)b, __fdiv_rn(v[b], sum)));
+            ltrb[side] = __fmul_rn(dis, (float)stride);
+        }
     }
     const int i = p / gw, j = p - i * gw;
     const float cx = (float)(j * stride), cy = (float)(i * stride);

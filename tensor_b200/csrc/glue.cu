@@ -75,10 +75,11 @@ struct AxisTap {
     int i0, i1;
     float w0, w1;
 };
-__device__ __forceinline__ AxisTap axis_tap(int d, int in, int out, double user_scale, int rule) {
+// step: source positions per output position, see axis_step
+__device__ __forceinline__ AxisTap axis_tap(int d, int in, int out, double step, int rule) {
     AxisTap t;
     if (rule == 1) {
-        const double scale = (double)in / out;
+        const double scale = step;
         float f = (float)(((double)d + 0.5) * scale - 0.5);
         int s = (int)floorf(f);
         f -= (float)s;
@@ -88,8 +89,7 @@ __device__ __forceinline__ AxisTap axis_tap(int d, int in, int out, double user_
         t.w0 = __fsub_rn(1.f, f); t.w1 = f;
     } else {
         if (out == in) { t.i0 = t.i1 = d; t.w0 = 1.f; t.w1 = 0.f; return t; }
-        const float ratio = user_scale > 0. ? (float)(1.0 / user_scale) : (float)in / (float)out;
-        float real = (float)((double)ratio * ((double)d + 0.5) - 0.5);
+        float real = (float)(step * ((double)d + 0.5) - 0.5);
         if (real < 0.f) real = 0.f;
         t.i0 = (int)real;
         t.i1 = t.i0 + (t.i0 < in - 1 ? 1 : 0);
@@ -103,35 +103,32 @@ __device__ __forceinline__ AxisTap axis_tap(int d, int in, int out, double user_
 // rounding per product and one per fused multiply-add, in the operand order of the reference build:
 //   rule 1: fma(S1, w1, S0 * w0)      (Tensor/TensorInterpolation.cpp:199-207,251-259)
 //   rule 0: fma(S0, w0, S1 * w1)      (Tensor/UpSampleKernel.cpp:125-139 as compiled with -Ofast -mfma)
-// Thread = one output position (ox, oy) of kUpsamplePlanes consecutive planes. The taps depend on the position only and need
-// double-precision arithmetic, so one thread per row and per column of the block computes them once into shared memory.
+// Thread = one output position, counted through the plane so that no lane idles at the end of a narrow row, of `per` consecutive
+// planes. The taps depend on the position only; their double-precision arithmetic runs before the previous kernel has ended.
+// Bound by memory once enough blocks run (20x20 -> 40x40, 3072 planes: 25 MB); with few planes by the latency of one thread's loads,
+// eight planes of which are in flight.
 constexpr int kUpsamplePlanes = 32;
+double axis_step(int in, int out, double user_scale, int rule) {
+    if (rule == 1) return (double)in / out;
+    return (double)(user_scale > 0. ? (float)(1.0 / user_scale) : (float)in / (float)out);
+}
+
 __global__ void __launch_bounds__(256)
-upsample_bilinear_kernel(const float* __restrict__ x, float* __restrict__ y, int h, int w, int oh, int ow, double scale_h,
-                         double scale_w, int rule, long planes) {
-    __shared__ AxisTap taps_x[32], taps_y[8];
-    ottk::pdl_launch_dependents();  // the taps below depend on the sizes only; the previous kernel is awaited after them
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    if (tid < 32) {
-        const int ox = blockIdx.x * 32 + tid;
-        if (ox < ow) taps_x[tid] = axis_tap(ox, w, ow, scale_w, rule);
-    } else if (tid < 40) {
-        const int oy = blockIdx.y * 8 + (tid - 32);
-        if (oy < oh) taps_y[tid - 32] = axis_tap(oy, h, oh, scale_h, rule);
-    }
-    __syncthreads();
+upsample_bilinear_kernel(const float* __restrict__ x, float* __restrict__ y, int h, int w, int oh, int ow, double step_h, double step_w, int rule,
+                         int per, long planes) {
+    ottk::pdl_launch_dependents();
+    const long pos = (long)blockIdx.x * 256 + threadIdx.x, out_plane = (long)oh * ow;
+    if (pos >= out_plane) return;
+    const int oy = (int)(pos / ow), ox = (int)(pos - (long)oy * ow);
+    const AxisTap tx = axis_tap(ox, w, ow, step_w, rule), ty = axis_tap(oy, h, oh, step_h, rule);
     ottk::pdl_wait();
-    const int ox = blockIdx.x * 32 + threadIdx.x;
-    const int oy = blockIdx.y * 8 + threadIdx.y;
-    if (ox >= ow || oy >= oh) return;
-    const AxisTap tx = taps_x[threadIdx.x], ty = taps_y[threadIdx.y];
     const int o00 = ty.i0 * w + tx.i0, o01 = ty.i0 * w + tx.i1, o10 = ty.i1 * w + tx.i0, o11 = ty.i1 * w + tx.i1;
-    const long p0 = (long)blockIdx.z * kUpsamplePlanes;
-    const long p1 = p0 + kUpsamplePlanes < planes ? p0 + kUpsamplePlanes : planes;
-    const long in_plane = (long)h * w, out_plane = (long)oh * ow;
+    const long p0 = (long)blockIdx.y * per;
+    const long p1 = p0 + per < planes ? p0 + per : planes;
+    const long in_plane = (long)h * w;
     const float* xp = x + p0 * in_plane;
-    float* yp = y + p0 * out_plane + (long)oy * ow + ox;
-#pragma unroll 4
+    float* yp = y + p0 * out_plane + pos;
+#pragma unroll 8
     for (long p = p0; p < p1; ++p, xp += in_plane, yp += out_plane) {
         const float a00 = __ldg(xp + o00), a01 = __ldg(xp + o01), a10 = __ldg(xp + o10), a11 = __ldg(xp + o11);
         float v;
@@ -250,9 +247,14 @@ int ott_upsample_bilinear_f32_nchw(ott_ctx* ctx, const float* in, int n, int c, 
     const long zblocks = (planes + kUpsamplePlanes - 1) / kUpsamplePlanes;
     if (zblocks > 65535 || (oh + 7) / 8 > 65535) return ctx->fail(OTT_ERR_UNSUPPORTED, "Upsample: more than 2097120 planes or 524280 rows in one call");
     cudaSetDevice(ctx->device);
-    const dim3 block(32, 8), grid((unsigned)((ow + 31) / 32), (unsigned)((oh + 7) / 8), (unsigned)zblocks);
-    OTT_CUDA_CHECK(ctx, ottk::launch_overlapped(upsample_bilinear_kernel, grid, block, 0, ctx->stream, in, out, h, w, oh, ow, scale_h, scale_w,
-                                                packed_rule ? 1 : 0, planes));
+    // four blocks per SM, of at most 32 planes and at least four
+    const long xblocks = ((long)oh * ow + 255) / 256, wanted = 4l * ctx->sm_count;
+    const long per = std::max(4l, std::min((long)kUpsamplePlanes, planes * xblocks / wanted)), yblocks = (planes + per - 1) / per;
+    const bool few = yblocks <= 65535;  // (per < 32 only where there are few planes)
+    const int rule = packed_rule ? 1 : 0;
+    const dim3 grid((unsigned)xblocks, (unsigned)(few ? yblocks : zblocks));
+    OTT_CUDA_CHECK(ctx, ottk::launch_overlapped(upsample_bilinear_kernel, grid, dim3(256), 0, ctx->stream, in, out, h, w, oh, ow,
+                                                axis_step(h, oh, scale_h, rule), axis_step(w, ow, scale_w, rule), rule, few ? (int)per : kUpsamplePlanes, planes));
     ctx->launches += 1;
     return OTT_OK;
 }
