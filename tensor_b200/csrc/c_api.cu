@@ -855,7 +855,9 @@ namespace {
 // int8 NHWC input of a 3x3 depthwise layer: the multiply-adds can go to the tensor cores as the data lies, no byte transposes,
 // at one 128-row MMA per tap, 32 channels and 8 x 16 output pixels. That pays where the CUDA cores have the most transposing to
 // do per output - stride 2 (four input pixels per output) and fp32 output (whose stores the other kernel cannot coalesce) - on
-// launches long enough to amortise its longer pipeline (6 M outputs) and maps its tiles fit. Measured, tensor cores against
+// launches long enough to amortise its longer pipeline (6 M outputs) and maps its tiles fit. A gathered layer's channels come in
+// 32-channel blocks of which it may want a few each; they cost the tensor cores little more than the bytes, so its maps may fit half as
+// well (116 channels from 12 blocks, 20x20 outputs, 256 images: 34.5 / 37.2; 232 from 13, 10x10: 28.5 / 36.1). Measured, tensor cores against
 // CUDA cores: 256 channels 56x56 stride 2, 64 images 15.7 / 20.2 us; 58 channels 80x80 stride 2, 256 images 27.1 / 43.2; 512
 // channels 28x28, fp32 out 57.8 / 64.9; but 128 channels 28x28 stride 2, 64 images 5.9 / 5.0 (too short), 58 channels 40x40
 // stride 2, 256 images 12.6 / 11.6 (20x20 outputs fill 52 % of their tiles), 256 channels 56x56 stride 1 41.1 / 40.7.
@@ -864,7 +866,7 @@ bool depthwise_on_tensor_cores(const ott_ctx* ctx, const ott_conv* c, const Conv
     if (ctx->dw_tensor_cores == 2) return true;
     if (s.sh == 1 && out_dtype != OTT_F32_NCHW) return false;
     const long tiles = (long)((s.oh + 15) / 16) * ((s.ow + 7) / 8), pixels = (long)s.oh * s.ow;
-    return pixels * 10 >= tiles * 128 * 7 && (double)s.n * pixels * (c->dw_plan.ncb_total * 32) >= 6e6;
+    return pixels * 20 >= tiles * 128 * (c->block_x.empty() ? 14 : 7) && (double)s.n * pixels * (c->dw_plan.ncb_total * 32) >= 6e6;
 }
 }  // namespace
 
