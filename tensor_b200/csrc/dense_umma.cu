@@ -309,7 +309,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                         const uint64_t b0 = make_smem_desc(sB + kb * b_tile_bytes, P.bkc);
                         const uint32_t b_tap_step = ((uint32_t)P.ncb * b_tile_bytes) >> 4, a_px_step = (uint32_t)P.bkc >> 4;
                         uint32_t accumulate = kb != 0 ? 1u : 0u, a_row = 0, b_off = 0;
-                        if (!COMPACT && s.kh == 3 && s.kw == 3) {
+                        if ((!COMPACT || QUANT) && s.kh == 3 && s.kw == 3) {
                             // the common filter: all loops unrolled, every descriptor the base's low word plus a constant (the
                             // address field cannot carry), so that the one issuing thread spends its time issuing
                             const uint32_t a_lo = (uint32_t)a0, b_lo = (uint32_t)b0;
@@ -1016,7 +1016,9 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
     // room for it on the same SMs, so the plan takes no more than one tile needs: eight epilogue warps at 96 registers, the stages of
     // one tile, one accumulator (464 -> 1024 on 10x10, 128 CTAs: 4.6 -> 3.5 us).
     p.out_kind = out_dtype;
-    if ((long)p.m_tiles * p.n_tiles <= sm_count) {
+    // (A halo tile wants its MMA issue unrolled, rolled it costs 0.9 us: on fp32 input in the compact build, which few layers of a network
+    // run, on int8 input in the specialised ones.)
+    if ((long)p.m_tiles * p.n_tiles <= sm_count && (f32 || !p.halo)) {
         p.compact = 1;
         p.epi_warps = kMaxEpiWarps;
         const int loads = p.halo ? p.ncb : (p.gather && p.gather_whole ? 1 : p.nkb);
