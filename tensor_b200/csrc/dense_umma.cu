@@ -13,7 +13,8 @@
 //   tiles never straddle anything. k x k convolutions load, per pixel tile of 8 x 16 and channel block, ONE box
 //   that holds the tile and its halo; filter tap (ky, kx) is an MMA whose A descriptor starts (ky, kx) pixels
 //   into that box and steps one halo row per 8-row group (the swizzle is a function of the shared-memory
-//   address, so shifted views read what TMA wrote). Dilated layers load one shifted box per tap instead.
+//   address, so shifted views read what TMA wrote). At stride 2 there are two boxes, one per column parity; other
+//   strides and dilated layers load one shifted box per tap instead.
 // * B (the layer's weights for this CTA's BN output channels, all taps) is loaded once per CTA and stays in
 //   shared memory while the CTA walks over its pixel tiles (persistent, weight-stationary).
 // * tcgen05.mma.kind::i8 accumulates exact s32 in TMEM; two accumulators are double-buffered so the
@@ -118,6 +119,16 @@ __device__ __forceinline__ void quantize16(uint32_t addr, const float (&v)[16], 
     store_chunk(addr, w[0], w[1], w[2], w[3]);
 }
 
+// Stride-2 halo (UmmaPlan::halo == 2): the input columns under a pixel tile as two planes, one per parity, every row of each. The 8
+// pixels of a tile row are then 8 neighbours of the plane that a tap reads, and tile rows are two plane rows apart.
+struct ParityHalo {
+    int cols[2], rows;
+    __host__ __device__ __forceinline__ ParityHalo(int kh, int kw) : cols{kHaloTw + (kw - 1) / 2, kHaloTw + (kw - 2) / 2}, rows(2 * (kHaloTh - 1) + kh) {}
+    __host__ __device__ __forceinline__ uint32_t plane_bytes(int i, int bkc) const { return (uint32_t)(rows * cols[i] * bkc); }
+    __host__ __device__ __forceinline__ uint32_t second(int bkc) const { return (plane_bytes(0, bkc) + 1023u) & ~1023u; }  // offset of plane 1
+    __host__ __device__ __forceinline__ uint32_t stage_bytes(int bkc) const { return second(bkc) + ((plane_bytes(1, bkc) + 1023u) & ~1023u); }
+};
+
 // columns of an accumulator an epilogue warp takes at a time
 __host__ __device__ __forceinline__ int epi_chunk(const UmmaPlan& p) { return p.bn <= 32 || p.compact ? 16 : 32; }
 
@@ -181,6 +192,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
     const uint32_t a_stage_bytes = (uint32_t)P.a_stage_bytes, b_tile_bytes = (uint32_t)P.bn * P.bkc;
     // halo mode: the 8 pixels of one tile row are one 8-row operand group; groups (tile rows) are one halo row apart
     const int halo_w = kHaloTw + s.kw - 1, halo_h = kHaloTh + s.kh - 1;
+    const ParityHalo parity(s.kh, s.kw);
     // pipeline stages one pixel tile consumes (a gathered layer's stage holds all the K blocks of a tile: one barrier round
     // trip per tile instead of one per 32-channel block)
     const int loads_per_tile = P.halo ? P.ncb : (P.gather && P.gather_whole ? 1 : P.nkb);
@@ -241,6 +253,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
             uint32_t st = 0, phase = 1;  // stage, and the parity that says it is free (the first round finds every stage free)
             bool ok = true, waited = false;
             const uint32_t load_bytes = P.gather && P.gather_whole ? (uint32_t)(tile_rows * P.bkc * P.nkb)
+                                        : P.halo == 2               ? parity.plane_bytes(0, P.bkc) + parity.plane_bytes(1, P.bkc)
                                         : P.halo                    ? (uint32_t)(halo_w * halo_h * P.bkc)
                                                                     : (uint32_t)(tile_rows * P.bkc);
             for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
@@ -267,6 +280,9 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                     } else if (P.gather) {
                         // K block kb = 32 channels of one of the source tensors (channels past that tensor's end arrive as zeros)
                         tma_load_4d(&maps.tm[maps.block_src[kb]], full, dst, (int)maps.block_x[kb], x0, 0, 0);
+                    } else if (!COMPACT && P.halo == 2) {
+                        tma_load_4d(&maps.tm[0], full, dst, kb * P.bkc, x0, y0, img);
+                        tma_load_4d(&maps.tm[1], full, dst + parity.second(P.bkc), kb * P.bkc, x0 + 1, y0, img);
                     } else if (P.halo) {
                         // the (8 + kw - 1) x (16 + kh - 1) pixels under the tile, one channel block; out-of-image pixels arrive as zeros
                         tma_load_4d(&maps.tm[0], full, dst, kb * P.bkc, x0, y0, img);
@@ -301,7 +317,32 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                 for (int kb = 0; kb < loads_per_tile; ++kb) {
                     if (!mbar_wait(bar_full + 8u * st, phase, abort_flag, status, 2u, P.wait_ns)) { ok = false; break; }
                     tc_fence_after();
-                    if (P.halo) {
+                    if (!COMPACT && !QUANT && P.halo == 2) {
+                        // a tap of column kx reads plane kx & 1, from column kx >> 1 on
+                        const uint32_t tile = sA + st * a_stage_bytes, px_step = (uint32_t)P.bkc >> 4;
+                        const uint64_t a0 = make_smem_desc(tile, P.bkc, 2 * parity.cols[0] * P.bkc);
+                        const uint64_t a1 = make_smem_desc(tile + parity.second(P.bkc), P.bkc, 2 * parity.cols[1] * P.bkc);
+                        const uint64_t b0 = make_smem_desc(sB + kb * b_tile_bytes, P.bkc);
+                        const uint32_t b_tap_step = ((uint32_t)P.ncb * b_tile_bytes) >> 4;
+                        auto tap = [&](int ky, int kx, int J, uint32_t b_off) {
+                            const uint32_t a_off = (uint32_t)(ky * parity.cols[kx & 1] + (kx >> 1)) * px_step;
+                            const uint64_t a = ((kx & 1) ? a1 : a0) + a_off;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (j < J) umma_i8(d, a + 2u * j, b0 + b_off + 2u * j, P.idesc, (kb | ky | kx | j) != 0 ? 1u : 0u);
+                        };
+                        const int J = P.bkc / 32;
+                        if (s.kh == 3 && s.kw == 3) {
+#pragma unroll
+                            for (int i = 0; i < 9; ++i) tap(i / 3, i % 3, J, (uint32_t)i * b_tap_step);
+                        } else {
+#pragma unroll 1
+                            for (int i = 0, ky = 0, kx = 0; i < P.taps; ++i) {
+                                tap(ky, kx, J, (uint32_t)i * b_tap_step);
+                                if (++kx == s.kw) { kx = 0; ++ky; }
+                            }
+                        }
+                    } else if (P.halo) {
                         // every filter tap reads the same halo tile through a view shifted by (ky, kx) pixels
                         // (one thread issues all of these back to back, so the per-tap descriptors are the base descriptors plus
                         // an offset in their 16-byte address field, not rebuilt from scratch)
@@ -766,8 +807,8 @@ static bool plan_panel(UmmaPlan& p, int smem_budget) {
     return true;
 }
 
-bool umma_plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, int dw, int smem_budget, UmmaPlan* plan, int bkc_override,
-                     bool whole_tile_stages) {
+static bool plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, int dw, int smem_budget, UmmaPlan* plan, int bkc_override,
+                       bool whole_tile_stages, bool parity_halo) {
     UmmaPlan p{};
     const int cin_pad = nhwc_channels(cin), cout_pad = nhwc_channels(cout);
     if (sh < 1 || sw < 1 || sh > 4 || sw > 4) return false;
@@ -782,10 +823,11 @@ bool umma_plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, 
     // preferring a split of cout_pad into equal tiles
     // strided and dilated layers load one box per filter tap (a strided layer's box takes every sw-th / sh-th pixel: TMA
     // element strides); undilated stride-1 k x k layers load one halo tile per pixel tile
-    p.halo = (p.taps > 1 && dh == 1 && dw == 1 && sh == 1 && sw == 1) ? 1 : 0;
+    p.halo = parity_halo ? 2 : (p.taps > 1 && dh == 1 && dw == 1 && sh == 1 && sw == 1) ? 1 : 0;
     const bool whole = whole_tile_stages && !p.halo && p.taps == 1;
     p.gather_whole = whole ? 1 : 0;
-    const long a_stage = p.halo ? ((long)p.bkc * (kHaloTw + kw - 1) * (kHaloTh + kh - 1) + 1023) / 1024 * 1024
+    const long a_stage = p.halo == 2 ? (long)ParityHalo(kh, kw).stage_bytes(p.bkc)
+                         : p.halo ? ((long)p.bkc * (kHaloTw + kw - 1) * (kHaloTh + kh - 1) + 1023) / 1024 * 1024
                                 : (long)kTileM * p.bkc * (whole ? p.nkb : 1);
     p.a_stage_bytes = (int)a_stage;
     const long avail = (long)smem_budget - 1024 /*alignment slack*/ - 4096 /*barriers + epilogue parameters*/ - (whole ? 2 : 3) * a_stage;
@@ -803,6 +845,19 @@ bool umma_plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, 
     if (!plan_panel(p, smem_budget)) return false;
     *plan = p;
     return true;
+}
+
+bool umma_plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, int dw, int smem_budget, UmmaPlan* plan, int bkc_override,
+                     bool whole_tile_stages) {
+    const bool have = plan_layer(cin, cout, kh, kw, sh, sw, dh, dw, smem_budget, plan, bkc_override, whole_tile_stages, false);
+    // Stride 2: the two parity planes of a tile's halo are half the rows of one box per tap (3x3: 561 against 1152), where they
+    // leave room for as wide a weight panel (us: 64 -> 128 75x75 x32, fp32 out 14.1 -> 11.8, int8 out 13.5 -> 10.4; 173 -> 93 57x20 x44
+    // 22.1 -> 13.6; 40 -> 40 40x40 x64 12.3 -> 8.7; 64 -> 64 56x56 one image 4.6 -> 3.8).
+    UmmaPlan p{};
+    if (have && sh == 2 && sw == 2 && dh == 1 && dw == 1 && kh > 1 && kw > 1 && kh <= 7 && kw <= 7 && bkc_override == 0 &&
+        plan_layer(cin, cout, kh, kw, sh, sw, dh, dw, smem_budget, &p, plan->bkc > 64 ? 64 : 0, whole_tile_stages, true) && p.n_tiles <= plan->n_tiles)
+        *plan = p;
+    return have;
 }
 
 bool umma_narrow_plan(const UmmaPlan& base, int bn, int cout, int smem_budget, UmmaPlan* plan) {
@@ -870,7 +925,7 @@ bool umma_float_input(const float* x, const PlaneGather* table, int cin, long hw
 // 7.6 / 14.5).
 bool umma_quantizes_inside(const UmmaPlan& p, const ConvShape& s, int sm_count) {
     const bool flat = s.kh == 1 && s.kw == 1 && s.ph == 0 && s.pw == 0 && s.sh == 1 && s.sw == 1;
-    if ((!flat && !p.halo) || s.cin_pad <= 32 || (double)s.n * s.h * s.w > 2147483647.0) return false;
+    if ((!flat && p.halo != 1) || s.cin_pad <= 32 || (double)s.n * s.h * s.w > 2147483647.0) return false;
     const long tiles = flat ? ((long)s.n * s.oh * s.ow + kTileM - 1) / kTileM : (long)s.n * ((s.ow + kHaloTw - 1) / kHaloTw) * ((s.oh + kHaloTh - 1) / kHaloTh);
     const bool small = tiles * p.n_tiles <= sm_count;
     if (!flat) return small && p.ncb == 1;
@@ -962,13 +1017,20 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
         cuuint64_t dims[4] = {(cuuint64_t)s.cin_pad, (cuuint64_t)s.w, (cuuint64_t)s.h, (cuuint64_t)s.n};
         cuuint64_t strides[3] = {(cuuint64_t)s.cin_pad, (cuuint64_t)s.cin_pad * s.w, (cuuint64_t)s.cin_pad * s.w * s.h};
         // a strided layer's box spans (tw - 1) * sw + 1 columns of which the traversal takes every sw-th: tw land in shared memory
-        cuuint32_t box[4] = {(cuuint32_t)p.bkc, (cuuint32_t)(p.halo ? p.tw + s.kw - 1 : (p.tw - 1) * s.sw + 1),
-                             (cuuint32_t)(p.halo ? p.th + s.kh - 1 : (p.th - 1) * s.sh + 1), 1};
+        const ParityHalo parity(s.kh, s.kw);
+        const int cols = p.halo == 2 ? 2 * parity.cols[0] - 1 : p.halo ? p.tw + s.kw - 1 : (p.tw - 1) * s.sw + 1;
+        const int rows = p.halo == 2 ? parity.rows : p.halo ? p.th + s.kh - 1 : (p.th - 1) * s.sh + 1;
+        cuuint32_t box[4] = {(cuuint32_t)p.bkc, (cuuint32_t)cols, (cuuint32_t)rows, 1};
         estr[1] = (cuuint32_t)s.sw;
-        estr[2] = (cuuint32_t)s.sh;
+        estr[2] = (cuuint32_t)(p.halo == 2 ? 1 : s.sh);
         if (!f32)
             r = enc(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (p.halo == 2 && r == CUDA_SUCCESS) {
+            box[1] = (cuuint32_t)(2 * parity.cols[1] - 1);
+            r = enc(&km.tm[1], CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        }
     }
     if (r != CUDA_SUCCESS) return "cuTensorMapEncodeTiled(activations) failed";
     p.wait_ns = wait_limit_ns;

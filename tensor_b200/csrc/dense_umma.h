@@ -22,7 +22,8 @@ struct UmmaPlan {
     // per call
     int compact;     // the compact build runs it
     int out_kind;    // DT_ of the output
-    int halo;        // k x k layers: one TMA box per pixel tile and channel block holds the tile plus its halo; the taps read shifted views
+    int halo;        // k x k layers: one TMA box per pixel tile and channel block holds the tile plus its halo; the taps read shifted views.
+                     // 2: stride 2, one box per column parity
     int a_stage_bytes;  // bytes of one activation stage (a 128-pixel tile, or a halo tile rounded up to 1 KiB)
     int flat;                          // 1x1: activations viewed as one [pixels, channels] matrix
     int gather;                        // > 0: the K blocks come from this many int8 NHWC tensors (see UmmaSources)

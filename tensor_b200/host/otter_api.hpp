@@ -145,8 +145,8 @@ public:
     bool routing_active = false;
     // a depthwise 3x3 layer (pad 1, stride 1 / 2) whose int8 output only the 1x1 layer behind it reads runs inside that layer's
     // kernel (ott_dwpw): one launch instead of two, the tensor between them never leaves the SM. Asking for the depthwise
-    // layer's blob through Extractor::extract still delivers it (the pair then runs as two layers). Off by default: it pays
-    // for small batches only (fewer launches), large batches run faster as two kernels whose epilogues overlap.
+    // layer's blob through Extractor::extract still delivers it (the pair then runs as two layers). Off by default: two
+    // kernels in a chain, whose set-up and epilogues overlap, are faster.
     bool fuse_depthwise_pointwise = false;
     int host_chunk = 64;  // ott_net_forward from host memory: images per chunk of the upload / compute / download pipeline
     const std::vector<char>* keep_blobs = nullptr;  // set by Extractor::keep: blobs lightmode must not release

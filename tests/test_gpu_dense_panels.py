@@ -40,3 +40,15 @@ def test_few_pixels_per_tile(ctx, cin, cout, pixels):
         got, want = run_gpu(ctx, case, ROUND_ADD_HALF_TRUNC), run_port(case, ROUND_ADD_HALF_TRUNC)
         assert np.array_equal(got["acc"], want["acc"])
         assert np.array_equal(bits(got["y"]), bits(want["y"]))
+
+
+@pytest.mark.parametrize("k,pad", [(2, 0), (2, 1), (3, 0), (3, 1), (4, 1), (5, 2), (7, 3)])
+@pytest.mark.parametrize("cin,cout,h,w,n", [(33, 20, 7, 9, 1), (64, 64, 31, 15, 3), (70, 40, 33, 17, 2), (130, 100, 35, 34, 1), (40, 48, 64, 65, 40)])
+def test_stride_two_halo(ctx, cin, cout, h, w, n, k, pad):
+    from gpu_support import bits, run_gpu
+    for term, act in ((101, ACT_LRELU), (1, ACT_NONE)):
+        case = ConvCase(f"s2_{k}_{cin}", cin, cout, k, 2, pad, n=n, h=h, w=w, bias_term=1, int8_scale_term=term, act_type=act, act_param0=0.1, s8_input=True,
+                        seed=cin + k).make()
+        got, want = run_gpu(ctx, case, ROUND_ADD_HALF_TRUNC), run_port(case, ROUND_ADD_HALF_TRUNC)
+        assert np.array_equal(got["acc"], want["acc"])
+        assert np.array_equal(bits(got["y"]), bits(want["y"]))
