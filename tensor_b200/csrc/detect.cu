@@ -266,7 +266,7 @@ extern "C" int ott_nanodet_detect(ott_ctx* ctx, const float* const* heads_dev, c
                                                                           nms_threshold, max_det, static_cast<float*>(rows_dev.p), staged, staged_rows, const_cast<int*>(kept));
     OTT_CUDA_CHECK(ctx, cudaGetLastError());
     ctx->launches += 1;
-    OTT_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+    if (const int rc = ott_sync(ctx)) return rc;  // (a wait that ran out in front of the decode leaves heads that mean nothing)
     for (int img = 0; img < n; ++img) {
         counts_host[img] = kept[img];
         const int rows = std::min(kept[img], max_det), first = std::min(rows, staged_rows);
