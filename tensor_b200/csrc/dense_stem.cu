@@ -46,7 +46,7 @@ dense_stem_kernel(const float* __restrict__ x, const __grid_constant__ StemParam
 
     // ---- 1. quantize the halo tile ----
     const float* ximg = x + (long)img * 3 * s.h * s.w;
-    const bool vec_ok = s.w % 4 == 0;
+    const bool vec_ok = s.w % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;  // four pixels are one 16-byte load
     for (int i = threadIdx.x; i < 3 * IH * RP; i += ST_TX * ST_TY) {
         const int xw = i % RP, r = (i / RP) % IH, c = i / (RP * IH);
         const int iy = iy0 + r, ix = ix_al + xw * 4;
@@ -210,7 +210,7 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
     // quantized input halo tile, as int8 channel planes. All of a thread's loads are issued before the first is used: the CTA
     // runs its phases one after the other, so this phase's DRAM latency must be paid once, not once per loop trip.
     const float* ximg = x + (long)img * 3 * s.h * s.w;
-    const bool vec_ok = s.w % 4 == 0;
+    const bool vec_ok = s.w % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;  // four pixels are one 16-byte load
     constexpr int TIN_WORDS = 3 * IH * RP, TIN_TRIPS = (TIN_WORDS + 255) / 256;
     if (vec_ok) {
         float4 v[TIN_TRIPS];
