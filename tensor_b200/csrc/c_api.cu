@@ -489,6 +489,7 @@ int create_gathered_depthwise(ott_ctx* ctx, const ott_conv_desc* d, const int8_t
     // of the MMA per group; every source must then be at least 32 channels wide), else the CUDA-core kernel's 16.
     bool tensor = ctx->dw_tensor_cores != 0 && d->kh == 3 && d->kw == 3 && d->ph == 1 && d->pw == 1 && d->sh == d->sw && (d->sh == 1 || d->sh == 2) &&
                   d->rounding == OTT_ROUND_ADD_HALF_TRUNC;
+    for (int i = 0; tensor && out_scales && i < n_out_scales; ++i) tensor = !(out_scales[i] < 0.f);
     for (int i = 0; tensor && i < n_sources; ++i) tensor = nhwc_channels(source_channels[i]) >= 32;
     const int C = d->cin, G16 = tensor ? 32 : 16;
     std::vector<int> lo(n_sources, 1 << 30), hi(n_sources, -1), base(n_sources, 0);
@@ -616,6 +617,7 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
     c->scale_out_host = scale_out;
     c->in_scale0 = in_scales[0];
     if (requant) {
+        c->negative_scale = std::any_of(scale_out.begin(), scale_out.end(), [](float v) { return v < 0.f; }) ? 1 : 0;
         c->one_scale_out = std::all_of(scale_out.begin(), scale_out.begin() + d->cout, [&](float v) { return v == scale_out[0]; }) ? 1 : 0;
         // whether the clamp of the int8 output can stand for the activation (EpilogueParams::int8_pos): the largest sum the
         // weights allow bounds what is requantized, and ReLU6 must have nothing to cut that the clamp would not
@@ -724,7 +726,7 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
         rc = upload(ctx, wtiled.data(), wtiled.size() * 4, (void**)&c->w_tiled_dev);
     }
     if (rc == OTT_OK && depthwise && !gi && d->kh == 3 && d->kw == 3 && d->ph == 1 && d->pw == 1 && d->dh == 1 && d->dw == 1 && d->sh == d->sw &&
-        (d->sh == 1 || d->sh == 2) && d->rounding == OTT_ROUND_ADD_HALF_TRUNC) {
+        (d->sh == 1 || d->sh == 2) && d->rounding == OTT_ROUND_ADD_HALF_TRUNC && !c->negative_scale) {
         int smem_optin = 0;
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
         if (dw_umma_plan(d->cout, d->sh, smem_optin, &c->dw_plan)) {
@@ -1018,7 +1020,7 @@ int forward_maxpool_impl(ott_ctx* ctx, const ott_conv* c, const float* in_dev, i
     cudaSetDevice(ctx->device);
     EpilogueParams ep{};
     ep.scale_in = c->scale_in_dev; ep.bias = c->bias_dev; ep.scale_out = c->scale_out_dev;
-    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos;
+    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos; ep.negative_scale = c->negative_scale;
     ep.has_bias = d.bias_term ? 1 : 0;
     ep.act_type = d.act_type; ep.act_param0 = d.act_param0; ep.rounding = d.rounding;
     OTT_CUDA_CHECK(ctx, launch_dense_stem_pool(ctx->stream, s, in_dev, c->w_host.data(), c->scale_in_host.data(), c->bias_host.data(),
@@ -1102,10 +1104,16 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
 
     EpilogueParams ep{};
     ep.scale_in = c->scale_in_dev; ep.bias = c->bias_dev; ep.scale_out = c->scale_out_dev;
-    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos;
+    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos; ep.negative_scale = c->negative_scale;
     ep.has_bias = d.bias_term ? 1 : 0;
     ep.act_type = d.act_type; ep.act_param0 = d.act_param0; ep.rounding = d.rounding;
 
+    // The CUDA-core depthwise kernel rounds what ReLU left as a number that is not negative. Under a negative scale the layer runs as
+    // the LeakyReLU of slope 0, whose results are the same int8 values (ReLU6: see the kernel).
+    if (c->kind == OTT_KERNEL_DEPTHWISE && c->negative_scale && out_dtype == OTT_S8_NHWC && d.act_type == ACT_RELU) {
+        ep.act_type = ACT_LRELU;
+        ep.act_param0 = 0.f;
+    }
     uint32_t* status = status_word_dev ? status_word_dev : ctx->status_dev;
     PlaneGather groups8;  // depthwise over gathered int8 input: where each 16-channel group lies
     const bool dw_tensor = c->kind == OTT_KERNEL_DEPTHWISE && in_dtype == OTT_S8_NHWC && (!gathered || c->gather_group == 32) &&

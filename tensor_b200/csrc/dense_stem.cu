@@ -370,8 +370,10 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
                 int qv[4];
 #pragma unroll
                 for (int j = 0; j < 4; j += 2) {
-                    // after ReLU / ReLU6 nothing is negative (scales are positive); the saturating pack clamps at 127
-                    const int2 r = round2_act<ACT>(__fmul2_rn(make_float2(y[j], y[j + 1]), make_float2(soa[j], soa[j + 1])), half);
+                    // after ReLU / ReLU6 nothing is negative where the scales are positive (the host gives C24 no others); the saturating
+                    // pack clamps at 127
+                    const float2 t = __fmul2_rn(make_float2(y[j], y[j + 1]), make_float2(soa[j], soa[j + 1]));
+                    const int2 r = C24 ? round2_act<ACT>(t, half) : round2(t, half);
                     qv[j] = 4 * q4 + j >= s.cout ? 0 : r.x;
                     qv[j + 1] = 4 * q4 + j + 1 >= s.cout ? 0 : r.y;
                 }
@@ -440,7 +442,7 @@ static cudaError_t launch_pool_s(cudaStream_t stream, const float* x, const Stem
     const size_t front = (size_t)SPM_ROWS * 32 + 1024 + (size_t)3 * IH * RP * 4;
     const size_t tile = (size_t)SP_CY * SP_CX * (((s.cout + 3) / 4) * 4 + 4) * 4;
     const size_t smem = 1024 + (front > tile ? front : tile);
-    const bool c24 = s.cout == 24 && s.cout_pad == 32 && ep.has_bias && ep.rounding == ROUND_ADD_HALF_TRUNC;
+    const bool c24 = s.cout == 24 && s.cout_pad == 32 && ep.has_bias && ep.rounding == ROUND_ADD_HALF_TRUNC && (!OUT8 || !ep.negative_scale);
 #define OTT_STEMPOOL_LAUNCH(ACT)                                                                                          \
     {                                                                                                                     \
         auto kernel = c24 ? dense_stem_pool_mma_kernel<S, ACT, OUT8, true> : dense_stem_pool_mma_kernel<S, ACT, OUT8, false>;    \

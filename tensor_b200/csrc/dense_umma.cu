@@ -641,7 +641,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                         if constexpr (ACT == ACT_POS) {
                             wds[g] = requant4_pos(ta, tb, half);
                         } else {
-                            const int2 qa = round2_act<ACT>(ta, half), qb = round2_act<ACT>(tb, half);
+                            const int2 qa = round2(ta, half), qb = round2(tb, half);  // (signed: a scale may be negative)
                             wds[g] = pack_sat_s8x4(qa.x, qa.y, qb.x, qb.y);
                         }
                     }

@@ -37,6 +37,7 @@ struct EpilogueParams {
     // ReLU, or ReLU6 where f(6) is 127 in every channel, and |v * scale_out| + 1 stays below 2^15 in every channel whatever the int8
     // input is: float2int8(act(v) * scale_out) is trunc(v * scale_out + h) clamped to [0, 127], see requant4_pos
     int int8_pos;
+    int negative_scale;      // some channel's scale_out is below zero
 };
 
 __device__ __forceinline__ float dequant(int acc, float scale_in, float bias, int has_bias) {
@@ -117,7 +118,7 @@ __device__ __forceinline__ int2 round2(float2 v, uint32_t h) {
     return make_int2(__float2int_rz(fmaxf(r.x, -127.5f)), __float2int_rz(fmaxf(r.y, -127.5f)));
 }
 
-// the same for v >= 0 (after ReLU / ReLU6): copysign(h, v) is +h; v == -0 truncates to 0 either way
+// the same for v >= 0 (after ReLU / ReLU6, times a scale that is not negative): copysign(h, v) is +h; v == -0 truncates to 0 either way
 __device__ __forceinline__ int2 round2_nonneg(float2 v, uint32_t h) {
     const float2 r = __fadd2_rn(v, make_float2(__uint_as_float(h), __uint_as_float(h)));
     return make_int2(__float2int_rz(r.x), __float2int_rz(r.y));
