@@ -618,7 +618,7 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
     c->in_scale0 = in_scales[0];
     if (requant) {
         c->negative_scale = std::any_of(scale_out.begin(), scale_out.end(), [](float v) { return v < 0.f; }) ? 1 : 0;
-        c->one_scale_out = std::all_of(scale_out.begin(), scale_out.begin() + d->cout, [&](float v) { return v == scale_out[0]; }) ? 1 : 0;
+        c->one_scale_out = std::isfinite(scale_out[0]) && std::all_of(scale_out.begin(), scale_out.begin() + d->cout, [&](float v) { return v == scale_out[0]; }) ? 1 : 0;
         // whether the clamp of the int8 output can stand for the activation (EpilogueParams::int8_pos): the largest sum the
         // weights allow bounds what is requantized, and ReLU6 must have nothing to cut that the clamp would not
         bool pos = d->act_type == ACT_RELU || d->act_type == ACT_RELU6;

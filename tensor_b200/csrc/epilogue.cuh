@@ -32,7 +32,7 @@ struct EpilogueParams {
     int act_type;
     float act_param0;
     int rounding;
-    int one_scale_out;       // every channel's scale_out is scale_out0
+    int one_scale_out;       // every channel's scale_out is scale_out0, and finite (padding channels, which hold 0, take it too)
     float scale_out0;
     // ReLU, or ReLU6 where f(6) is 127 in every channel, and |v * scale_out| + 1 stays below 2^15 in every channel whatever the int8
     // input is: float2int8(act(v) * scale_out) is trunc(v * scale_out + h) clamped to [0, 127], see requant4_pos

@@ -1,5 +1,6 @@
 """GPU: requantizing layers with output scales of both signs behind ReLU and ReLU6 (what is rounded is then below zero), both rounding
-rules, bit for bit against the CPU checker: the dense kernel's one-tile and specialised builds and the depthwise kernels."""
+rules, bit for bit against the CPU checker: the dense kernel's one-tile and specialised builds and the depthwise kernels; and a scale
+that is infinite."""
 import ctypes as C
 
 import numpy as np
@@ -54,3 +55,19 @@ def test_first_layer_maxpool_with_negative_scales(ctx):
         ctx.free(p)
     f32_layer.close()
     s8_layer.close()
+
+
+def test_infinite_scale_leaves_the_padding_channels_zero(ctx):
+    """A launch large enough for the build that takes one scale as a scalar; every real output saturates."""
+    from tensor_b200 import S8_NHWC, ConvInt8
+    rng, cin, cout, h, w = np.random.default_rng(4), 32, 20, 1024, 1024
+    weight = rng.integers(-127, 128, size=(cout, cin, 1, 1), dtype=np.int8)
+    layer = ConvInt8(ctx, cin=cin, cout=cout, kh=1, kw=1, int8_scale_term=101, weight=weight, bias=np.full(cout, 0.123, np.float32),
+                     w_scales=np.full(cout, 50, np.float32), in_scales=np.full(1, 127, np.float32), out_scales=np.full(1, np.inf, np.float32))
+    x, y = ctx.to_device(rng.integers(-127, 128, size=(1, h, w, cin), dtype=np.int8)), ctx.malloc(h * w * 32)
+    layer.forward(x, S8_NHWC, 1, h, w, y, S8_NHWC)
+    got = ctx.to_host(y, (h, w, 32), np.int8)
+    assert not got[..., cout:].any() and (np.abs(got[..., :cout].astype(np.int32)) == 127).all()
+    for p in (x, y):
+        ctx.free(p)
+    layer.close()
