@@ -22,7 +22,10 @@
 class DeviceCachingAllocator {
 public:
     explicit DeviceCachingAllocator(int device) : device_(device) {}
-    ~DeviceCachingAllocator() { release_cached(); }
+    ~DeviceCachingAllocator() {
+        log_.clear();
+        release_cached();
+    }
 
     static size_t round_size(size_t bytes) {
         if (bytes == 0) bytes = 1;
@@ -164,17 +167,23 @@ public:
     }
 
 private:
+    // Blocks that the open log holds stay: the kernels captured so far address them.
     void release_cached_locked() {
         for (auto& kv : available_) {
+            std::vector<void*> stay;
             for (void* p : kv.second) {
+                if (log_.count(p)) {
+                    stay.push_back(p);
+                    continue;
+                }
                 auto gi = guards_.find(p);
                 cudaFree(gi == guards_.end() ? p : static_cast<void*>(static_cast<char*>(p) - gi->second));
                 if (gi != guards_.end()) guards_.erase(gi);
                 sizes_.erase(p);
+                bytes_cached_ -= kv.first;
             }
-            kv.second.clear();
+            kv.second.swap(stay);
         }
-        bytes_cached_ = 0;
     }
 
     int device_;
