@@ -26,15 +26,6 @@ int upload(ott_ctx* ctx, const void* host, size_t bytes, void** dev) {
     return OTT_OK;
 }
 
-bool is_pinned(const void* p) {
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeHost;
-}
-
 int check_status_word(ott_ctx* ctx, bool copied = false) {
     if (!copied) OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(ctx->status_host, ctx->status_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     OTT_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
@@ -61,12 +52,11 @@ size_t dtype_bytes(int dtype, int n, int c, int h, int w) {
 }  // namespace
 
 int ctx_upload(ott_ctx* ctx, const HostCopy& copy) {
-    if (is_pinned(copy.host)) {
+    HostStaging& ring = ctx->upload;
+    if (!ring.takes(copy.host)) {
         OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(copy.dev, copy.host, copy.bytes, cudaMemcpyHostToDevice, ctx->stream));
         return OTT_OK;
     }
-    HostStaging& ring = ctx->upload;
-    OTT_CUDA_CHECK(ctx, ring.ready());
     for (size_t at = 0; at < copy.bytes; at += HostStaging::kPiece) {
         const size_t len = std::min(HostStaging::kPiece, copy.bytes - at);
         const int slot = ring.next;
@@ -96,11 +86,10 @@ int ctx_download_and_sync(ott_ctx* ctx, const HostCopy* copies, int n) {
         return OTT_OK;
     };
     for (int i = 0; i < n; ++i) {
-        if (is_pinned(copies[i].host)) {
+        if (!ring.takes(copies[i].host)) {
             OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(copies[i].host, copies[i].dev, copies[i].bytes, cudaMemcpyDeviceToHost, ctx->stream));
             continue;
         }
-        OTT_CUDA_CHECK(ctx, ring.ready());
         for (size_t at = 0; at < copies[i].bytes; at += HostStaging::kPiece) {
             if (issued - first == HostStaging::kSlots)
                 if (const int rc = retire()) return rc;

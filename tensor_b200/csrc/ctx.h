@@ -215,6 +215,15 @@ struct HostStaging {
             }
         return cudaMallocHost(reinterpret_cast<void**>(&mem), kPiece * kSlots);
     }
+    // Whether a host buffer's copies go through the ring: pageable memory, and only that (what else a caller names, the driver copies
+    // or refuses), as long as there is pinned memory to be had.
+    bool takes(const void* host) {
+        cudaPointerAttributes a{};
+        const bool known = cudaPointerGetAttributes(&a, host) == cudaSuccess;
+        if (known && a.type == cudaMemoryTypeUnregistered && ready() == cudaSuccess) return true;
+        (void)cudaGetLastError();
+        return false;
+    }
     void release() {
         if (mem) cudaFreeHost(mem);
         mem = nullptr;
@@ -271,7 +280,7 @@ struct ott_event {
     cudaEvent_t ev = nullptr;
 };
 
-// One transfer between host and device memory. Pinned host memory is copied straight, pageable memory through the ring.
+// One transfer between host and device memory. Pageable host memory goes through the ring, any other is copied straight.
 struct HostCopy {
     void* host;
     void* dev;
