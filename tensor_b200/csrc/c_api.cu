@@ -52,7 +52,7 @@ size_t dtype_bytes(int dtype, int n, int c, int h, int w) {
 }  // namespace
 
 int ctx_upload(ott_ctx* ctx, const HostCopy& copy) {
-    HostStaging& ring = ctx->upload;
+    HostStaging& ring = ctx->staging;
     if (!ring.takes(copy.host)) {
         OTT_CUDA_CHECK(ctx, cudaMemcpyAsync(copy.dev, copy.host, copy.bytes, cudaMemcpyHostToDevice, ctx->stream));
         return OTT_OK;
@@ -71,7 +71,7 @@ int ctx_upload(ott_ctx* ctx, const HostCopy& copy) {
 }
 
 int ctx_download_and_sync(ott_ctx* ctx, const HostCopy* copies, int n) {
-    HostStaging& ring = ctx->download;
+    HostStaging& ring = ctx->staging;
     struct Piece {
         char* dst;
         size_t len;
@@ -168,8 +168,7 @@ int ott_ctx_destroy(ott_ctx* ctx) {
     delete ctx->alloc;
     if (ctx->status_dev) cudaFree(ctx->status_dev);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
-    ctx->upload.release();
-    ctx->download.release();
+    ctx->staging.release();
     if (ctx->detect_mem) cudaFreeHost(ctx->detect_mem);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;

@@ -199,10 +199,13 @@ private:
 };
 
 // Pinned ring through which copies from and to pageable host memory run piece by piece, so that the host's copy of one piece
-// overlaps the transfer of another (the driver's own pageable path: 90 / 106 us for 1.2 MB up / down, this one 62 / 66).
+// overlaps the transfer of another (the driver's own pageable path: 90 / 106 us for 1.2 MB up / down, this one 62 / 66). One ring
+// serves both directions: a download into a piece is behind the upload from it on the context's stream. Its 1.5 MB fit one block of the
+// driver's pinned pool, which costs 1 to 3 ms to extend (two rings of 2 MB extended it twice on the second call of a Net: 4.8 ms, now
+// 0.9). Pieces of 128 / 256 KB are slower on copies of several MB (6 images 224x288: 695 / 659 us a forward, 512 KB 635).
 struct HostStaging {
     static constexpr size_t kPiece = 512u << 10;
-    static constexpr int kSlots = 4;
+    static constexpr int kSlots = 3;
     char* mem = nullptr;  // kSlots pieces, allocated on first use
     cudaEvent_t done[kSlots] = {};
     int next = 0;
@@ -247,7 +250,7 @@ struct ott_ctx {
     unsigned long long wait_limit_ns = 2000000000ull;  // limit of every bounded wait inside the kernels (ott_set_wait_limit_ms)
     uint32_t* status_dev = nullptr;   // default status word the kernels report into
     uint32_t* status_host = nullptr;  // pinned mirror
-    HostStaging upload, download;
+    HostStaging staging;
     void* detect_mem = nullptr;  // pinned memory the detection decode writes its rows into; grows to the largest batch seen
     size_t detect_bytes = 0;
     void* detect_stage(size_t bytes) {
