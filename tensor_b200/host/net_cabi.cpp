@@ -87,6 +87,7 @@ ott_ctx* ott_net_context(ott_net* net) { return net ? net->net.context() : nullp
 int ott_net_load_model(ott_net* net, const char* otter_path, const char* weight_path, int weight_type) {
     if (!net || !otter_path || !weight_path || (weight_type != 0 && weight_type != 1)) return OTT_ERR_INVALID;
     net->error.clear();
+    net->drop_pipelines();
     int rc = net->net.load_otter(otter_path, otter::CompileMode::Inference);
     if (rc != 0) return rc;
     return net->net.load_weight(weight_path, weight_type == 1 ? otter::Net::WeightType::Ncnn : otter::Net::WeightType::Otter);
@@ -154,6 +155,7 @@ int ott_otter_parse_text(const char* text, char* out, int cap) {
 int ott_net_compile(ott_net* net) {
     if (!net) return OTT_ERR_INVALID;
     net->error.clear();
+    net->drop_pipelines();  // captured forwards are those of the layers compiled before
     return net->net.compile(otter::CompileMode::Initial);
 }
 

@@ -1,6 +1,6 @@
 """GPU: the host-buffer forward replays a captured graph from the second call of a shape on: every call must equal the checker, with
 changing inputs and batch sizes, more shapes than are kept, parameters replaced in between, an int8 output blob (which is not
-captured), copies longer than the staging ring, and pinned buffers."""
+captured), copies longer than the staging ring, pinned buffers, and a Net compiled again."""
 import ctypes as C
 
 import numpy as np
@@ -68,3 +68,21 @@ def test_pinned_buffers(small):
         assert np.array_equal(y.view(np.int32), want(x, "conv5").view(np.int32))
     for b in buf:
         net.lib.ott_host_free(b)
+
+
+def test_a_net_compiled_again_forgets_its_graphs():
+    from graph_support import build_net, oracle_conv_for_calibration
+    from graph_walk import calibrate
+    from tensor_b200 import graphs
+    L = graphs.shufflenetv2_layers(40, 48, batch=1, stage_repeats=(2, 2, 2))
+    params = graphs.make_params(L, seed=22)
+    x = np.random.default_rng(0).uniform(0, 1, size=(1, 3, 40, 48)).astype(np.float32)
+    calibrate(L, params, x, oracle_conv_for_calibration)
+    net, fresh = build_net(L, params), build_net(L, {})
+    for _ in range(3):
+        before = net.forward("data", x, ["conv5"])[0]
+    net.compile()  # the new layers have no parameters yet
+    after = net.forward("data", x, ["conv5"])[0]
+    assert np.array_equal(after, fresh.forward("data", x, ["conv5"])[0]) and not np.array_equal(after, before)
+    net.close()
+    fresh.close()
