@@ -85,8 +85,9 @@ int ott_net_set_conv_params_f32(ott_net* net, const char* layer, const float* w_
  * out_host[i]: NULL = only compute the blob; else a host buffer that receives the blob in the reference's plain
  * layout (fp32 NCHW, or int8 NCHW for int8 blobs) after the stream has been synchronised.
  * With every out_host NULL the call is asynchronous on the Net's stream.
- * From host memory to host memory the forward is replayed as a captured graph from the second call of a shape on (a few shapes are
- * kept; replaced parameters or options start over). */
+ * From host memory to host memory the forward is captured at the end of the second call of a shape and replayed from the third on
+ * (the graphs of the four shapes in most recent use are kept; replaced parameters, options or layers start over). A capture that
+ * fails, or gets no memory, changes no result: the shape goes on layer by layer. */
 int ott_net_forward(ott_net* net, const char* input_blob, const void* in, int in_on_device, int n, int c, int h, int w,
                     int n_out, const char* const* out_blobs, void* const* out_host);
 

@@ -14,12 +14,13 @@ struct ott_net_graph {
 };
 
 // What the host-buffer calls keep between calls of one shape: the device input buffer and one captured forward per chunk of the
-// batch (the chunks differ in where they read the input). A batch of less than two chunks is one graph, captured when its shape
-// comes for the second time: a program that runs a shape once does not pay for a capture it never replays.
+// batch (the chunks differ in where they read the input). A batch of less than two chunks is one graph, captured at the end of the
+// second call of its shape: a program that runs a shape once does not pay for a capture it never replays.
 struct HostPipeline {
     std::string key;
     void* dev_in = nullptr;
     std::vector<ott_net_graph*> graphs;
+    int calls = 0;       // calls of this shape so far
     bool plain = false;  // cannot be captured, or delivers a blob that has to be re-ordered on the host: runs layer by layer
 };
 constexpr size_t kMaxPipelines = 4;  // shapes kept; the oldest goes
@@ -30,8 +31,11 @@ struct ott_net {
     std::vector<HostPipeline> pipelines;
     void drop(HostPipeline& p);
     void drop_pipelines();
-    HostPipeline* pipeline(const std::string& key, bool* seen_before);
-    int build(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs);
+    HostPipeline* pipeline(const std::string& key);
+    bool may_capture(const HostPipeline& p);
+    int build(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs, bool warm);
+    int capture(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs, bool warm);
+    bool release_graphs();
     ~ott_net() { drop_pipelines(); }
 };
 
@@ -57,6 +61,33 @@ void copy_str(const std::string& s, char* dst, int cap) {
     if (!dst || cap <= 0) return;
     std::strncpy(dst, s.c_str(), (size_t)cap - 1);
     dst[cap - 1] = 0;
+}
+
+// Extractor::input + extract, layer by layer.
+int forward_layers(ott_net* net, const char* input_blob, const void* in, int in_on_device, int n, int c, int h, int w, int n_out,
+                   const char* const* out_blobs, void* const* out_host) {
+    otter::Extractor ex = net->net.create_extractor();
+    otter::Tensor x;
+    if (in_on_device)
+        x = otter::Tensor::wrap(const_cast<void*>(in), (size_t)n * c * h * w * 4, otter::Device::CUDA, nullptr, {n, c, h, w}, otter::ScalarType::Float);
+    else
+        x = otter::from_blob(const_cast<void*>(in), {n, c, h, w}, otter::ScalarType::Float);
+    int rc = ex.input(input_blob, x);
+    if (rc != 0) return fail(net, rc, "Extractor::input failed");
+    // outputs are pulled in order; a requested blob that is consumed on the way to another output must survive lightmode
+    for (int i = 0; i < n_out; ++i)
+        if (ex.keep(out_blobs[i]) != 0) return fail(net, OTT_ERR_INVALID, std::string("unknown blob ") + out_blobs[i]);
+    std::vector<otter::Tensor> dev((size_t)n_out);
+    for (int i = 0; i < n_out; ++i) {
+        rc = ex.extract(out_blobs[i], dev[(size_t)i], 1);
+        if (rc != 0) return rc;
+    }
+    for (int i = 0; i < n_out; ++i) {
+        if (!out_host || !out_host[i]) continue;
+        rc = ex.extract_into(out_blobs[i], out_host[i]);
+        if (rc != 0) return rc;
+    }
+    return OTT_OK;
 }
 
 }  // namespace
@@ -270,13 +301,13 @@ int ott_net_forward(ott_net* net, const char* input_blob, const void* in, int in
     for (int i = 0; all_host_out && i < n_out; ++i) all_host_out = out_host[i] != nullptr;
     const int chunk = net->net.option.host_chunk > 0 ? net->net.option.host_chunk : 64;
     ott_ctx* ctx = net->net.context();
+    HostPipeline* pipe = nullptr;
     if (!in_on_device && all_host_out && n > 0 && c > 0 && h > 0 && w > 0 && ctx) {
         const size_t img_bytes = (size_t)c * h * w * sizeof(float);
         const bool chunked = n >= 2 * chunk;
-        bool seen = false;
-        HostPipeline* pipe = net->pipeline(pipeline_key(net, "forward", input_blob, n, c, h, w, n_out, out_blobs), &seen);
-        if (pipe->graphs.empty() && !pipe->plain && (chunked || seen)) {
-            const int rc = net->build(*pipe, input_blob, n, c, h, w, chunked ? chunk : n, n_out, out_blobs);
+        pipe = net->pipeline(pipeline_key(net, "forward", input_blob, n, c, h, w, n_out, out_blobs));
+        if (chunked && pipe->graphs.empty() && !pipe->plain) {
+            const int rc = net->build(*pipe, input_blob, n, c, h, w, chunk, n_out, out_blobs, true);
             if (rc != OTT_OK) return rc;
         }
         if (!pipe->graphs.empty() && !chunked) {
@@ -308,33 +339,20 @@ int ott_net_forward(ott_net* net, const char* input_blob, const void* in, int in
             return rc != OTT_OK ? rc : rc_sync;
         }
     }
-    otter::Extractor ex = net->net.create_extractor();
-    otter::Tensor x;
-    if (in_on_device)
-        x = otter::Tensor::wrap(const_cast<void*>(in), (size_t)n * c * h * w * 4, otter::Device::CUDA, nullptr, {n, c, h, w}, otter::ScalarType::Float);
-    else
-        x = otter::from_blob(const_cast<void*>(in), {n, c, h, w}, otter::ScalarType::Float);
-    int rc = ex.input(input_blob, x);
-    if (rc != 0) return fail(net, rc, "Extractor::input failed");
-    // outputs are pulled in order; a requested blob that is consumed on the way to another output must survive lightmode
-    for (int i = 0; i < n_out; ++i)
-        if (ex.keep(out_blobs[i]) != 0) return fail(net, OTT_ERR_INVALID, std::string("unknown blob ") + out_blobs[i]);
-    std::vector<otter::Tensor> dev((size_t)n_out);
-    for (int i = 0; i < n_out; ++i) {
-        rc = ex.extract(out_blobs[i], dev[(size_t)i], 1);
-        if (rc != 0) return rc;
-    }
-    for (int i = 0; i < n_out; ++i) {
-        if (!out_host || !out_host[i]) continue;
-        rc = ex.extract_into(out_blobs[i], out_host[i]);
-        if (rc != 0) return rc;
-    }
-    return OTT_OK;
+    int rc = forward_layers(net, input_blob, in, in_on_device, n, c, h, w, n_out, out_blobs, out_host);
+    // memory that captured forwards of other shapes hold
+    if (rc == OTT_ERR_ALLOC && net->release_graphs()) rc = forward_layers(net, input_blob, in, in_on_device, n, c, h, w, n_out, out_blobs, out_host);
+    // A shape that has come before: captured for the calls to come. This call has run its kernels and left its temporaries in the
+    // cache, so nothing runs once more for it, and it has its answer whatever becomes of the capture.
+    if (rc == OTT_OK && pipe && !pipe->plain && net->may_capture(*pipe)) rc = net->build(*pipe, input_blob, n, c, h, w, n, n_out, out_blobs, false);
+    return rc;
 }
 
-int ott_net_capture(ott_net* net, const char* input_blob, const void* in_dev, int n, int c, int h, int w, int n_out,
-                    const char* const* out_blobs, ott_net_graph** out) {
-    if (!net || !input_blob || !in_dev || n_out < 1 || !out_blobs || !out) return OTT_ERR_INVALID;
+}  // extern "C"
+
+// warm: run the forward once before capturing it
+static int capture_forward(ott_net* net, const char* input_blob, const void* in_dev, int n, int c, int h, int w, int n_out, const char* const* out_blobs,
+                           bool warm, ott_net_graph** out) {
     net->error.clear();
     ott_ctx* ctx = net->net.context();
     if (!ctx) return fail(net, OTT_ERR_INVALID, "capture before compile");
@@ -353,10 +371,13 @@ int ott_net_capture(ott_net* net, const char* input_blob, const void* in_dev, in
         return rc;
     };
     std::vector<otter::Tensor> outs;
-    int rc = run(outs);  // warm-up: every buffer size is in the allocator's cache afterwards, one-time kernel set-up is done
-    if (rc == 0) rc = ott_sync(ctx);
-    outs.clear();
-    if (rc != 0) return rc;
+    int rc = 0;
+    if (warm) {  // every buffer size is in the allocator's cache afterwards, one-time kernel set-up is done
+        rc = run(outs);
+        if (rc == 0) rc = ott_sync(ctx);
+        outs.clear();
+        if (rc != 0) return rc;
+    }
     rc = ott_graph_capture_begin(ctx);
     if (rc != 0) return rc;
     rc = run(outs);
@@ -376,6 +397,14 @@ int ott_net_capture(ott_net* net, const char* input_blob, const void* in_dev, in
     ng->outputs = std::move(outs);
     *out = ng;
     return OTT_OK;
+}
+
+extern "C" {
+
+int ott_net_capture(ott_net* net, const char* input_blob, const void* in_dev, int n, int c, int h, int w, int n_out,
+                    const char* const* out_blobs, ott_net_graph** out) {
+    if (!net || !input_blob || !in_dev || n_out < 1 || !out_blobs || !out) return OTT_ERR_INVALID;
+    return capture_forward(net, input_blob, in_dev, n, c, h, w, n_out, out_blobs, true, out);
 }
 
 int ott_net_graph_launch(ott_net_graph* graph) {
@@ -414,45 +443,65 @@ void ott_net::drop_pipelines() {
     pipelines.clear();
 }
 
-HostPipeline* ott_net::pipeline(const std::string& key, bool* seen_before) {
-    for (HostPipeline& p : pipelines)
-        if (p.key == key) {
-            *seen_before = true;
-            return &p;
-        }
-    *seen_before = false;
-    if (pipelines.size() >= kMaxPipelines) {
-        drop(pipelines.front());
-        pipelines.erase(pipelines.begin());
+// Gives the memory of every captured forward back to the cache; false when there was none.
+bool ott_net::release_graphs() {
+    bool any = false;
+    for (HostPipeline& p : pipelines) {
+        if (p.graphs.empty()) continue;
+        any = true;
+        drop(p);
+        p.calls = 0;
     }
-    pipelines.emplace_back();
-    pipelines.back().key = key;
-    return &pipelines.back();
+    return any;
 }
 
-// Captures the pipeline's graphs. A failure to allocate is reported and may be tried again; any other failure to capture, or an
-// output that is not dense fp32 NCHW, makes the shape a plain one.
-int ott_net::build(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs) {
+// The entry of a shape; counts the call.
+HostPipeline* ott_net::pipeline(const std::string& key) {
+    size_t at = 0;
+    while (at < pipelines.size() && pipelines[at].key != key) ++at;
+    if (at == pipelines.size()) {
+        if (at >= kMaxPipelines) {
+            drop(pipelines.front());
+            pipelines.erase(pipelines.begin());
+        }
+        pipelines.emplace_back();
+        pipelines.back().key = key;
+        at = pipelines.size() - 1;
+    }
+    pipelines[at].calls += 1;
+    return &pipelines[at];
+}
+
+bool ott_net::may_capture(const HostPipeline& p) { return p.calls >= 2; }
+
+int ott_net::capture(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs, bool warm) {
     ott_ctx* ctx = net.context();
     const size_t img_bytes = (size_t)c * h * w * sizeof(float);
     if (ott_malloc(ctx, img_bytes * n, &p.dev_in) != OTT_OK) return fail(this, OTT_ERR_ALLOC, "device allocation for the input batch failed");
-    // the warm-up forward inside every capture reads the (not yet uploaded) buffer: give it defined contents
-    int rc = ott_memset(ctx, p.dev_in, 0, img_bytes * n);
+    // the warm-up forward inside a capture reads the (not yet uploaded) buffer: give it defined contents
+    int rc = warm ? ott_memset(ctx, p.dev_in, 0, img_bytes * n) : OTT_OK;
     for (int b0 = 0; b0 < n && rc == OTT_OK; b0 += chunk) {
         ott_net_graph* g = nullptr;
-        rc = ott_net_capture(this, input_blob, static_cast<char*>(p.dev_in) + img_bytes * b0, n - b0 < chunk ? n - b0 : chunk, c, h, w, n_out, out_blobs, &g);
+        rc = capture_forward(this, input_blob, static_cast<char*>(p.dev_in) + img_bytes * b0, n - b0 < chunk ? n - b0 : chunk, c, h, w, n_out, out_blobs, warm, &g);
         if (rc == OTT_OK) p.graphs.push_back(g);
     }
-    bool dense = rc == OTT_OK;
-    for (size_t gi = 0; dense && gi < p.graphs.size(); ++gi)
-        for (const otter::Tensor& t : p.graphs[gi]->outputs) dense = dense && t.layout() == otter::Layout::NCHW;
-    if (dense) return OTT_OK;
-    drop(p);
-    if (rc == OTT_OK || rc == OTT_ERR_UNSUPPORTED) {
-        p.plain = true;
-        error.clear();
-    }
-    return p.plain ? OTT_OK : rc;
+    for (size_t gi = 0; rc == OTT_OK && gi < p.graphs.size(); ++gi)
+        for (const otter::Tensor& t : p.graphs[gi]->outputs)
+            if (t.layout() != otter::Layout::NCHW) rc = OTT_ERR_UNSUPPORTED;
+    if (rc != OTT_OK) drop(p);
+    return rc;
+}
+
+// Captures the pipeline's graphs. A wait that ran out is reported (the next call tries again). Any other failure, or an output that
+// is not dense NCHW, makes the shape a plain one: it runs layer by layer, as its first calls did. Memory that other shapes' graphs
+// hold is given back before that.
+int ott_net::build(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs, bool warm) {
+    int rc = capture(p, input_blob, n, c, h, w, chunk, n_out, out_blobs, warm);
+    if (rc == OTT_ERR_ALLOC && release_graphs()) rc = capture(p, input_blob, n, c, h, w, chunk, n_out, out_blobs, warm);
+    if (rc == OTT_OK || rc == OTT_ERR_DEVICE_WAIT) return rc;
+    p.plain = true;
+    error.clear();
+    return OTT_OK;
 }
 
 extern "C" {
@@ -467,35 +516,39 @@ int ott_net_forward_rows(ott_net* net, const char* input_blob, const void* in, i
     // result has a size only it knows, runs behind the replay.
     const int blob = net->net.find_blob_index_by_name(out_blob);
     const otter::Layer* last = blob >= 0 && net->net.blob(blob).producer >= 0 ? net->net.layer(net->net.blob(blob).producer) : nullptr;
+    std::vector<std::string> names;
+    std::vector<const char*> outs;
+    HostPipeline* pipe = nullptr;
     if (!in_on_device && last && last->type() == "NanodetPlusDetectionOutput" && n > 0 && c > 0 && h > 0 && w > 0 && net->net.context()) {
-        std::vector<std::string> names;
-        std::vector<const char*> outs;
         for (int b : last->bottoms) names.push_back(net->net.blob(b).name);
         for (const std::string& nm : names) outs.push_back(nm.c_str());
-        bool seen = false;
-        HostPipeline* pipe = net->pipeline(pipeline_key(net, "rows", input_blob, n, c, h, w, (int)outs.size(), outs.data()), &seen);
-        if (pipe->graphs.empty() && !pipe->plain && seen) {
-            rc = net->build(*pipe, input_blob, n, c, h, w, n, (int)outs.size(), outs.data());
-            if (rc != OTT_OK) return rc;
-        }
+        pipe = net->pipeline(pipeline_key(net, "rows", input_blob, n, c, h, w, (int)outs.size(), outs.data()));
         if (!pipe->graphs.empty()) {
             rc = ctx_upload(net->net.context(), HostCopy{const_cast<void*>(in), pipe->dev_in, (size_t)n * c * h * w * sizeof(float)});
             if (rc == OTT_OK) rc = ott_net_graph_launch(pipe->graphs[0]);
             std::vector<otter::Tensor> tops(1);
             if (rc == OTT_OK) rc = last->forward(pipe->graphs[0]->outputs, tops, net->net.option);
-            if (rc != OTT_OK) return fail(net, rc, std::string("forward of layer ") + last->name + " failed: " + ott_last_error(net->net.context()));
-            feat = tops[0];
+            if (rc == OTT_OK) feat = tops[0];
+            else if (rc != OTT_ERR_ALLOC || !net->release_graphs())
+                return fail(net, rc, std::string("forward of layer ") + last->name + " failed: " + ott_last_error(net->net.context()));
         }
     }
-    if (!feat.defined()) {
+    auto layers = [&]() -> int {
         otter::Extractor ex = net->net.create_extractor();
         otter::Tensor x = in_on_device ? otter::Tensor::wrap(const_cast<void*>(in), (size_t)n * c * h * w * 4, otter::Device::CUDA, nullptr,
                                                               {n, c, h, w}, otter::ScalarType::Float)
                                        : otter::from_blob(const_cast<void*>(in), {n, c, h, w}, otter::ScalarType::Float);
-        rc = ex.input(input_blob, x);
-        if (rc != 0) return fail(net, rc, "Extractor::input failed");
-        rc = ex.extract(out_blob, feat, 0);
+        const int ret = ex.input(input_blob, x);
+        return ret != 0 ? fail(net, ret, "Extractor::input failed") : ex.extract(out_blob, feat, 0);
+    };
+    if (!feat.defined()) {
+        rc = layers();
+        if (rc == OTT_ERR_ALLOC && net->release_graphs()) rc = layers();
         if (rc != 0) return rc;
+        if (pipe && !pipe->plain && net->may_capture(*pipe)) {
+            rc = net->build(*pipe, input_blob, n, c, h, w, n, (int)outs.size(), outs.data(), false);
+            if (rc != OTT_OK) return rc;
+        }
     }
     if (feat.dim() != 2 || feat.scalar_type() != otter::ScalarType::Float) return fail(net, OTT_ERR_INVALID, std::string(out_blob) + " is not a 2-D fp32 blob");
     *rows = (int)feat.size(0);

@@ -1,6 +1,6 @@
-"""GPU: the host-buffer forward replays a captured graph from the second call of a shape on: every call must equal the checker, with
+"""GPU: the host-buffer forward replays a captured graph from the third call of a shape on: every call must equal the checker, with
 changing inputs and batch sizes, more shapes than are kept, parameters replaced in between, an int8 output blob (which is not
-captured), copies longer than the staging ring, pinned buffers, and a Net compiled again."""
+captured), copies longer than the staging ring, pinned buffers, memory refused to a capture, and a Net compiled again."""
 import ctypes as C
 
 import numpy as np
@@ -68,6 +68,32 @@ def test_pinned_buffers(small):
         assert np.array_equal(y.view(np.int32), want(x, "conv5").view(np.int32))
     for b in buf:
         net.lib.ott_host_free(b)
+
+
+def test_memory_refused_to_a_capture(small):
+    """The n-th allocation of a shape's second call fails (the first is the capture's input buffer, further ones its temporaries): the
+    forward is right all the same, and so is every later one."""
+    net, params, want = small
+    ctx = net.context()
+    rng = np.random.default_rng(5)
+    for i, nth in enumerate((1, 2, 5, 20, 40)):
+        n = 7 + i
+        x = rng.uniform(0, 1, size=(n, 3, 40, 48)).astype(np.float32)
+        expect = want(x, "conv5").view(np.int32)
+        assert np.array_equal(net.forward("data", x, ["conv5"])[0].view(np.int32), expect)
+        ctx.check(ctx.lib.ott_debug_fail_alloc_after(ctx.h, nth))
+        for _ in range(3):
+            assert np.array_equal(net.forward("data", x, ["conv5"])[0].view(np.int32), expect)
+        ctx.check(ctx.lib.ott_debug_fail_alloc_after(ctx.h, 0))
+
+
+def test_an_output_that_does_not_exist_is_refused_on_every_call(small):
+    net, params, want = small
+    x = np.zeros((1, 3, 40, 48), np.float32)
+    out = np.empty(1, np.float32)
+    for _ in range(3):
+        with pytest.raises(RuntimeError, match="unknown blob"):
+            net.forward_raw("data", x.ctypes.data_as(C.c_void_p), False, x.shape, ["conv99"], [out.ctypes.data])
 
 
 def test_a_net_compiled_again_forgets_its_graphs():
