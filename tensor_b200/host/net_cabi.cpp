@@ -1,4 +1,5 @@
 // C-ABI over the host-side graph runtime (include/otter_b200_net.h).
+#include <algorithm>
 #include <cstring>
 #include <sstream>
 
@@ -23,12 +24,16 @@ struct HostPipeline {
     int calls = 0;       // calls of this shape so far
     bool plain = false;  // cannot be captured, or delivers a blob that has to be re-ordered on the host: runs layer by layer
 };
-constexpr size_t kMaxPipelines = 4;  // shapes kept; the oldest goes
+// Shapes with captured graphs, and shapes remembered in all. The shape unused for longest goes: of those without graphs, or, when a
+// shape has come kCallsToReplace times and no graph is free for it, of those with (a capture costs about ten forwards of one image,
+// so a program that cycles through more shapes than are kept had better not capture one on every call).
+constexpr size_t kMaxCaptured = 4, kMaxPipelines = 12;
+constexpr int kCallsToReplace = 8;
 
 struct ott_net {
     otter::Net net;
     std::string error;
-    std::vector<HostPipeline> pipelines;
+    std::vector<HostPipeline> pipelines;  // least recently used first
     void drop(HostPipeline& p);
     void drop_pipelines();
     HostPipeline* pipeline(const std::string& key);
@@ -455,24 +460,31 @@ bool ott_net::release_graphs() {
     return any;
 }
 
-// The entry of a shape; counts the call.
+// The entry of a shape, now the last one; counts the call.
 HostPipeline* ott_net::pipeline(const std::string& key) {
     size_t at = 0;
     while (at < pipelines.size() && pipelines[at].key != key) ++at;
     if (at == pipelines.size()) {
-        if (at >= kMaxPipelines) {
-            drop(pipelines.front());
-            pipelines.erase(pipelines.begin());
-        }
+        if (pipelines.size() >= kMaxPipelines)  // (more entries than graphs: there is one without)
+            for (size_t i = 0; i < pipelines.size(); ++i)
+                if (pipelines[i].graphs.empty()) {
+                    pipelines.erase(pipelines.begin() + (long)i);
+                    break;
+                }
         pipelines.emplace_back();
         pipelines.back().key = key;
-        at = pipelines.size() - 1;
+    } else {
+        std::rotate(pipelines.begin() + (long)at, pipelines.begin() + (long)at + 1, pipelines.end());
     }
-    pipelines[at].calls += 1;
-    return &pipelines[at];
+    pipelines.back().calls += 1;
+    return &pipelines.back();
 }
 
-bool ott_net::may_capture(const HostPipeline& p) { return p.calls >= 2; }
+bool ott_net::may_capture(const HostPipeline& p) {
+    size_t captured = 0;
+    for (const HostPipeline& q : pipelines) captured += q.graphs.empty() ? 0 : 1;
+    return p.calls >= (captured < kMaxCaptured ? 2 : kCallsToReplace);
+}
 
 int ott_net::capture(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs, bool warm) {
     ott_ctx* ctx = net.context();
@@ -496,6 +508,14 @@ int ott_net::capture(HostPipeline& p, const char* input_blob, int n, int c, int 
 // is not dense NCHW, makes the shape a plain one: it runs layer by layer, as its first calls did. Memory that other shapes' graphs
 // hold is given back before that.
 int ott_net::build(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs, bool warm) {
+    size_t captured = 0;
+    for (const HostPipeline& q : pipelines) captured += q.graphs.empty() ? 0 : 1;
+    for (HostPipeline& q : pipelines)
+        if (captured >= kMaxCaptured && !q.graphs.empty()) {
+            drop(q);
+            q.calls = 0;
+            --captured;
+        }
     int rc = capture(p, input_blob, n, c, h, w, chunk, n_out, out_blobs, warm);
     if (rc == OTT_ERR_ALLOC && release_graphs()) rc = capture(p, input_blob, n, c, h, w, chunk, n_out, out_blobs, warm);
     if (rc == OTT_OK || rc == OTT_ERR_DEVICE_WAIT) return rc;

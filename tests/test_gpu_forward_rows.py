@@ -1,4 +1,4 @@
-"""GPU: the detector's row-returning forward call after call: with changing images (from the second call of a shape on the heads come
+"""GPU: the detector's row-returning forward call after call: with changing images (from the third call of a shape on the heads come
 from a replayed graph) against the CPU checker's decode, and with a bounded wait that ran out in front of the decode."""
 import numpy as np
 import pytest

@@ -96,6 +96,29 @@ def test_an_output_that_does_not_exist_is_refused_on_every_call(small):
             net.forward_raw("data", x.ctypes.data_as(C.c_void_p), False, x.shape, ["conv99"], [out.ctypes.data])
 
 
+def _allocations(net):
+    """Blocks the Net's context has handed out so far: a replayed forward takes none."""
+    ctx = net.context()
+    m, h, u, c = (C.c_uint64() for _ in range(4))
+    ctx.check(ctx.lib.ott_alloc_stats(ctx.h, C.byref(m), C.byref(h), C.byref(u), C.byref(c)))
+    return m.value + h.value
+
+
+def test_a_shape_in_use_stays_captured_among_many_others(small):
+    net, params, want = small
+    rng = np.random.default_rng(6)
+    hot = rng.uniform(0, 1, size=(1, 3, 40, 48)).astype(np.float32)
+    expect = want(hot, "conv5").view(np.int32)
+    net.set_option("host_chunk", 64)  # forgets all shapes
+    for _ in range(2):
+        net.forward("data", hot, ["conv5"])
+    for n in list(range(2, 20)) + [2, 3, 4, 5, 2, 3, 4, 5, 6, 6]:  # one-off shapes, then more shapes with graphs than are kept
+        net.forward("data", np.repeat(hot, n, axis=0), ["conv5"])
+        before = _allocations(net)
+        assert np.array_equal(net.forward("data", hot, ["conv5"])[0].view(np.int32), expect)
+        assert _allocations(net) == before, n
+
+
 def test_a_net_compiled_again_forgets_its_graphs():
     from graph_support import build_net, oracle_conv_for_calibration
     from graph_walk import calibrate
