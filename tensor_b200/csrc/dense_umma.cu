@@ -100,13 +100,14 @@ __device__ __forceinline__ void store_chunk(uint32_t addr, uint32_t a, uint32_t 
 }
 
 // The same position of 16 channels' planes: one load each, 4 bytes (V = float) or 16 (float4). A chunk that lies in one run walks its
-// planes; the address arithmetic of a run look-up per load costs more than the load.
+// planes, the last one of the layer too; the address arithmetic of a run look-up per load costs more than the load (58 -> 114 3x3 48x8
+// x15, whose last chunk has 10 channels: 8.0 -> 6.4 us, quantized inside).
 template <typename V>
 __device__ __forceinline__ void load16(V (&v)[16], const QuantSource& Q, int c0, int cin, int img, int hw, int p) {
-    if (c0 + 16 <= cin && (c0 >= Q.first[1] || c0 + 16 <= Q.first[1])) {
+    if (c0 >= Q.first[1] || min(c0 + 16, cin) <= Q.first[1]) {
         const float* ptr = Q.plane(c0, img, hw) + p;
 #pragma unroll
-        for (int j = 0; j < 16; ++j, ptr += hw) v[j] = __ldg(reinterpret_cast<const V*>(ptr));
+        for (int j = 0; j < 16; ++j, ptr += hw) v[j] = c0 + j < cin ? __ldg(reinterpret_cast<const V*>(ptr)) : V{};
     } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = c0 + j < cin ? __ldg(reinterpret_cast<const V*>(Q.plane(c0 + j, img, hw) + p)) : V{};
