@@ -119,13 +119,15 @@ constexpr int kNmsThreads = 256, kNmsMaxProposals = 4096;
 // behind each key, the sorted boxes, and one "struck" flag per box.
 __global__ void __launch_bounds__(kNmsThreads)
 nanodet_nms_kernel(const Proposal* __restrict__ props, const int* __restrict__ counts, int capacity, int slots, float nms_threshold, int max_det,
-                   float* __restrict__ out, float* __restrict__ staged, int staged_rows, int* __restrict__ out_counts) {
+                   float* __restrict__ out, float* __restrict__ staged, int staged_rows, int* __restrict__ out_counts, const uint32_t* __restrict__ status,
+                   uint32_t* __restrict__ status_out) {
     extern __shared__ unsigned long long nms_smem[];
     unsigned long long* key = nms_smem;
     int* idx = reinterpret_cast<int*>(key + slots);
     Proposal* box = reinterpret_cast<Proposal*>(idx + slots);
     unsigned char* struck = reinterpret_cast<unsigned char*>(box + slots);
     const int img = blockIdx.x;
+    if (img == 0 && threadIdx.x == 0) *status_out = *status;  // what the kernels in front of the decode report, without a copy of its own
     const int c = counts[img] < capacity ? counts[img] : capacity;
     if (c > slots) {  // more than this launch was sized for: the caller finishes this image on the host
         if (threadIdx.x == 0) out_counts[img] = -1;
@@ -214,12 +216,13 @@ extern "C" int ott_nanodet_detect(ott_ctx* ctx, const float* const* heads_dev, c
         (void)cudaGetLastError();
         return ctx->fail(OTT_ERR_ALLOC, "device allocation for the proposals failed");
     }
-    // per image: staged_rows rows, then (behind all images) the number of rows kept; written by the GPU, read here
+    // per image: staged_rows rows, then (behind all images) the number of rows kept, and the status word; written by the GPU, read here
     const int staged_rows = (int)std::min<size_t>((size_t)max_det, kStagedBytes / (6 * sizeof(float)) / (size_t)n);
-    const size_t staged_bytes = (size_t)n * (staged_rows * 6 * sizeof(float) + sizeof(int));
+    const size_t staged_bytes = (size_t)n * (staged_rows * 6 * sizeof(float) + sizeof(int)) + sizeof(uint32_t);
     float* staged = static_cast<float*>(ctx->detect_stage(staged_bytes));
     if (!staged) return ctx->fail(OTT_ERR_ALLOC, "pinned allocation for the detections failed");
     const int* kept = reinterpret_cast<const int*>(staged + (size_t)n * staged_rows * 6);
+    const uint32_t* status = reinterpret_cast<const uint32_t*>(kept + n);
     OTT_CUDA_CHECK(ctx, cudaMemsetAsync(counts.p, 0, (size_t)n * sizeof(int), ctx->stream));
     int order_base = 0;
     for (int l0 = 0; l0 < n_levels; l0 += kMaxLevels) {
@@ -263,10 +266,13 @@ extern "C" int ott_nanodet_detect(ott_ctx* ctx, const float* const* heads_dev, c
         }
     }
     nanodet_nms_kernel<<<(unsigned)n, kNmsThreads, nms_smem, ctx->stream>>>(static_cast<const Proposal*>(props.p), static_cast<const int*>(counts.p), capacity, slots,
-                                                                          nms_threshold, max_det, static_cast<float*>(rows_dev.p), staged, staged_rows, const_cast<int*>(kept));
+                                                                          nms_threshold, max_det, static_cast<float*>(rows_dev.p), staged, staged_rows, const_cast<int*>(kept),
+                                                                          ctx->status_dev, const_cast<uint32_t*>(status));
     OTT_CUDA_CHECK(ctx, cudaGetLastError());
     ctx->launches += 1;
-    if (const int rc = ott_sync(ctx)) return rc;  // (a wait that ran out in front of the decode leaves heads that mean nothing)
+    OTT_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+    if (*status != 0u)  // a wait ran out in front of the decode: the heads mean nothing
+        if (const int rc = ott_sync(ctx)) return rc;
     for (int img = 0; img < n; ++img) {
         counts_host[img] = kept[img];
         const int rows = std::min(kept[img], max_det), first = std::min(rows, staged_rows);
