@@ -92,6 +92,11 @@ int ott_set_depthwise_tensor_cores(ott_ctx* ctx, int mode);
  * (cudaErrorMemoryAllocation without calling cudaMalloc); n <= 0 switches the injection off. */
 int ott_debug_wait_probe(ott_ctx* ctx);
 int ott_debug_fail_alloc_after(ott_ctx* ctx, int n);
+/* What a dense k x k layer (padding k / 2) on the tensor cores would launch on a GPU of sm_count SMs; needs no GPU. plan: 128-pixel
+ * tiles, weight panels, columns of a panel, CTAs per SM of the plan, fp32 input quantized inside the kernel, the one-tile-per-CTA
+ * build, pixels per tile, halo form (0: one load per tap, 1: halo tiles, 2: one halo tile per column parity). OTT_ERR_UNSUPPORTED:
+ * the layer does not run there. */
+int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int w, int f32_input, int sm_count, int plan[8]);
 /* Guard bands, the tests' stand-in for a device memory checker: after ott_debug_guard_bands(ctx, bytes) every block the
  * context's allocator obtains from the driver carries `bytes` (rounded up to 512) of a fill pattern on both sides;
  * ott_debug_check_guards synchronizes the stream, reads every band of every block (in use or cached) back and returns

@@ -736,11 +736,7 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
     if (rc == OTT_OK && c->kind == OTT_KERNEL_DENSE_UMMA) {
         int smem_optin = 0;
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-        UmmaVariant v;
-        v.plan = c->plan;
-        c->umma.push_back(v);
-        for (int bn : kUmmaNarrow)
-            if (umma_narrow_plan(c->plan, bn, d->cout, smem_optin, &v.plan)) c->umma.push_back(v);
+        c->umma = umma_variants(c->plan, d->cout, smem_optin);
         for (UmmaVariant& u : c->umma) {
             const char* err = umma_encode_weight_map(u.plan, c->w_dev, u.weight_map);
             if (err) rc = ctx->fail(OTT_ERR_CUDA, "%s", err);
@@ -836,6 +832,25 @@ int ott_conv_f32_forward(ott_ctx* ctx, const ott_conv_f32* c, const float* in_de
     cudaSetDevice(ctx->device);
     OTT_CUDA_CHECK(ctx, launch_conv_f32(ctx->stream, s, c->depthwise ? 1 : 0, in_dev, c->w_dev, c->bias_dev, d.act_type, d.act_param0, out_dev));
     ctx->launches += 1;
+    return OTT_OK;
+}
+
+int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int w, int f32_input, int sm_count, int plan[8]) {
+    if (!plan || cin < 1 || cout < 1 || k < 1 || stride < 1 || n < 1 || h < 1 || w < 1 || sm_count < 1) return OTT_ERR_INVALID;
+    constexpr int kSmemOptin = 227 * 1024;
+    UmmaPlan widest{};
+    if (!umma_plan_layer(cin, cout, k, k, stride, stride, 1, 1, kSmemOptin, &widest)) return OTT_ERR_UNSUPPORTED;
+    const std::vector<UmmaVariant> all = umma_variants(widest, cout, kSmemOptin);
+    ConvShape s{};
+    s.n = n; s.h = h; s.w = w; s.cin = cin; s.cout = cout; s.cin_pad = nhwc_channels(cin); s.cout_pad = nhwc_channels(cout);
+    s.kh = s.kw = k; s.sh = s.sw = stride; s.ph = s.pw = k / 2; s.dh = s.dw = 1;
+    s.oh = out_dim(h, k, stride, k / 2, 1);
+    s.ow = out_dim(w, k, stride, k / 2, 1);
+    if (s.oh < 1 || s.ow < 1) return OTT_ERR_INVALID;
+    long tiles = 0;
+    const UmmaChoice c = umma_choose(all.data(), (int)all.size(), s, sm_count, f32_input != 0, &tiles);
+    const int out[8] = {(int)tiles, c.variant->plan.n_tiles, c.variant->plan.bn, c.variant->plan.ctas_per_sm, c.inside, c.compact, c.tile_rows, c.variant->plan.halo};
+    std::memcpy(plan, out, sizeof out);
     return OTT_OK;
 }
 
@@ -1162,9 +1177,11 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
     DeviceBlock xq;
     const int8_t* x = static_cast<const int8_t*>(in_dev);
     UmmaFloatInput f32;
-    const bool quant_inside = in_dtype == OTT_F32_NCHW && c->kind == OTT_KERNEL_DENSE_UMMA && c->n_in_scales == 1 &&
-                              umma_quantizes_inside(c->plan, s, ctx->sm_count) &&
-                              umma_float_input(static_cast<const float*>(in_dev), gather, d.cin, (long)h * w, c->in_scale0, &f32);
+    UmmaChoice choice{};
+    if (c->kind == OTT_KERNEL_DENSE_UMMA)
+        choice = umma_choose(c->umma.data(), (int)c->umma.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW && c->n_in_scales == 1 &&
+                             umma_float_input(static_cast<const float*>(in_dev), gather, d.cin, (long)h * w, c->in_scale0, &f32));
+    const bool quant_inside = choice.inside;
     if (in_dtype == OTT_F32_NCHW) {
         if (xq.alloc(ctx, (size_t)n * h * w * c->cin_pad) != cudaSuccess) {
             (void)cudaGetLastError();
@@ -1204,7 +1221,7 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
                     us.block_src[kb] = c->block_src[kb];
                 }
             }
-            const char* err = launch_dense_umma(ctx->stream, ctx->sm_count, c->umma.data(), (int)c->umma.size(), s, x, ep, out_dev, out_dtype, status,
+            const char* err = launch_dense_umma(ctx->stream, ctx->sm_count, choice, s, x, ep, out_dev, out_dtype, status,
                                                 gathered ? &us : nullptr, mixed, ctx->wait_limit_ns, quant_inside ? &f32 : nullptr);
             if (err) return ctx->fail(OTT_ERR_CUDA, "%s: %s", err, cudaGetErrorString(cudaGetLastError()));
             break;

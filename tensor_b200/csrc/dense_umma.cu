@@ -870,6 +870,15 @@ bool umma_narrow_plan(const UmmaPlan& base, int bn, int cout, int smem_budget, U
     return true;
 }
 
+std::vector<UmmaVariant> umma_variants(const UmmaPlan& widest, int cout, int smem_budget) {
+    std::vector<UmmaVariant> all(1);
+    all[0].plan = widest;
+    UmmaVariant v;
+    for (int bn : {128, 64, 32})
+        if (umma_narrow_plan(widest, bn, cout, smem_budget, &v.plan)) all.push_back(v);
+    return all;
+}
+
 void umma_pack_weights(const UmmaPlan& p, const int8_t* w_oihw, int cin, int cout, int kh, int kw, int8_t* dst) {
     // dst[cout_rows][k_total], k = (tap*ncb + cb)*bkc + (channel - cb*bkc); zero elsewhere
     const long kt = p.k_total;
@@ -917,36 +926,140 @@ bool umma_float_input(const float* x, const PlaneGather* table, int cin, long hw
     return true;
 }
 
-// The int8 copy of an fp32 input costs a kernel of its own (about 4 us of chain on a small launch) and an HBM round trip; inside the
-// convolution it costs every weight panel its own pass over the input, by eight warps, and leaves the epilogue eight. 1x1 layers
-// whose images are whole pixel quads win with one panel that does not want sixteen epilogue warps, or with one wave of CTAs (us,
-// copy / inside: 192 -> 48 20x20 one image 7.9 / 4.8, 717 -> 152 18x20 x36 16.0 / 13.5, 953 -> 160 16x60 x33 41 / 39, 116 -> 116
-// 20x20 x256 17.5 / 16.1; but 256 -> 512 28x28 x128 52 / 55). Pixel-by-pixel loads only pay on small launches (90 -> 77 31x33 x60:
-// 12.5 / 19.2), and for halo tiles only with one channel block (64 -> 64 56x56 one image 8.5 / 5.3; 100 -> 200 with two blocks
-// 7.6 / 14.5).
-bool umma_quantizes_inside(const UmmaPlan& p, const ConvShape& s, int sm_count) {
-    const bool flat = s.kh == 1 && s.kw == 1 && s.ph == 0 && s.pw == 0 && s.sh == 1 && s.sw == 1;
-    if ((!flat && p.halo != 1) || s.cin_pad <= 32 || (double)s.n * s.h * s.w > 2147483647.0) return false;
-    const long tiles = flat ? ((long)s.n * s.oh * s.ow + kTileM - 1) / kTileM : (long)s.n * ((s.ow + kHaloTw - 1) / kHaloTw) * ((s.oh + kHaloTh - 1) / kHaloTh);
-    const bool small = tiles * p.n_tiles <= sm_count;
-    if (!flat) return small && p.ncb == 1;
-    return small || (p.n_tiles == 1 && p.bn <= 192 && (long)s.h * s.w % 4 == 0);
+namespace {
+
+// How a plan tiles the output pixels of a call.
+struct PixelTiles {
+    int flat, tw, th, x, y;
+    long tiles;
+};
+PixelTiles tile_pixels(const UmmaPlan& p, const ConvShape& s) {
+    PixelTiles t{};
+    t.flat = s.kh == 1 && s.kw == 1 && s.ph == 0 && s.pw == 0 && s.sh == 1 && s.sw == 1 ? 1 : 0;
+    if (t.flat) {
+        t.tw = kTileM; t.th = 1; t.y = 1;
+        t.tiles = ((long)s.n * s.oh * s.ow + kTileM - 1) / kTileM;
+        t.x = (int)t.tiles;
+        return t;
+    }
+    // rectangle of 128 output pixels with the least padding waste (halo mode: always 8 x 16)
+    long best = -1;
+    for (int tw = 8; tw <= 128; tw *= 2) {
+        const int th = kTileM / tw;
+        if ((tw - 1) * s.sw + 1 > 256 || (th - 1) * s.sh + 1 > 256) continue;  // a TMA box spans at most 256 elements per dimension
+        const long cover = (long)((s.ow + tw - 1) / tw) * tw * ((s.oh + th - 1) / th) * th;
+        if (best < 0 || cover < best) { best = cover; t.tw = tw; t.th = th; }
+    }
+    if (p.halo) { t.tw = kHaloTw; t.th = kHaloTh; }
+    t.x = (s.ow + t.tw - 1) / t.tw;
+    t.y = (s.oh + t.th - 1) / t.th;
+    t.tiles = (long)s.n * t.x * t.y;
+    return t;
 }
 
-const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVariant* variants, int n_variants, const ConvShape& s,
+// Width of the weight panels. A launch with fewer CTAs than SMs is bound by the chain of one tile, most of which (MMAs, requantize,
+// stores) shrinks with the panel, so panels of 128 and 64 columns are taken as long as all the CTAs are resident at once. Panels of 32
+// halve little more than the fixed part of that chain and read the activations twice as often, which other streams pay for: only
+// where every CTA still has an SM to itself. A panel that is not a quarter narrower than the next wider one adds a pass and saves
+// little: not while half the SMs are free. 1x1, us with the panels the rule takes / wider ones / narrower ones: 96 -> 512, 40 tiles
+// 4.8 / 7.8 / 5.5; 196 -> 140, 60 tiles (3 panels) 4.1 / 4.9 / 4.7; 205 -> 56, 133 tiles (1) 4.3 / - / 4.4; over 500 layers of 24 to 1024
+// channels 1.1 % from the best of every layer. Three ShuffleNetV2 forwards at a time, 9 images each: 122 us a forward, with panels of
+// 32 wherever they are resident 141.
+// A k x k layer's panel holds all its taps. Where two CTAs do not fit an SM for it, the next launch's panels come in beside this
+// one's only if half the SMs are free (202 -> 130 3x3 10x15 x12: 72 CTAs 5.3, 120 narrower ones 6.8).
+constexpr int kNarrowPanel = 32;
+int pick_panels(const UmmaVariant* v, int n, long tiles, int sm_count) {
+    int pick = 0;
+    for (int i = 1; i < n && tiles * v[pick].plan.n_tiles < sm_count; ++i) {
+        const UmmaPlan& p = v[i].plan;
+        if (4 * p.bn > 3 * v[pick].plan.bn && 2 * tiles * v[pick].plan.n_tiles <= sm_count) continue;
+        const long room = p.halo && p.ctas_per_sm == 1 ? sm_count / 2 : (long)sm_count * (p.bn <= kNarrowPanel ? 1 : p.ctas_per_sm);
+        if (tiles * p.n_tiles <= room) pick = i;
+    }
+    return pick;
+}
+
+// Pixels per tile of a one-tile-per-CTA launch. SMs still idle: fewer. A tile's loads arrive a row at a time, and a gathered layer has a row of
+// 32 bytes per pixel and K block (232 channels gathered in 15 blocks: 1900 rows for 128 pixels). 128 / 64 / 32 / 16 pixels at most: 116 -> 116
+// 20x20 2.59 / 2.47 / 2.37 / 2.30 us, detector on one 416x416 image 450 / 433 / 429 / 427, backbone 169 / 164 / 160 / 159. A quantizing
+// launch, whose CTAs have an SM to themselves, keeps 32 (116 -> 116: 3.8, with 16 4.4).
+int small_tile_rows(long pixels, int n_tiles, bool inside, int sm_count) {
+    int rows = kTileM;
+    while (rows > (inside ? 32 : 16) && (pixels + rows / 2 - 1) / (rows / 2) * n_tiles <= sm_count) rows /= 2;
+    return rows;
+}
+
+// Whether a launch of one tile per CTA runs the compact build. A quantizing one always does; on int8 input a halo tile wants its MMA issue
+// unrolled (rolled it costs 0.9 us), and a wide panel the unrolled epilogue (compact / specialised, 130 layers alone: 32 columns 0.97,
+// 64 1.04, 128 1.11, 240 1.21; in a chain of layers the compact build gains what kAnyOut says).
+bool runs_compact(const UmmaPlan& p, long tiles, bool inside, int sm_count) {
+    return tiles * p.n_tiles <= sm_count && (inside || (!p.halo && p.bn <= 64));
+}
+
+// Costs (us) of a flat launch on fp32 input: quantized inside, one tile per CTA, and through an int8 copy. Fitted to 250 layers of 33 to 1024
+// channels (7 and 9 % from the measured times): the eight quantizing warps' items, the operand bytes of a tile, the panel's columns
+// and bytes; the quantize kernel and what the convolution behind it takes.
+double inside_us(const UmmaPlan& p, const ConvShape& s, int rows) {
+    const bool quads = (long)s.h * s.w % 4 == 0;
+    const double items = (quads ? (rows + 127) / 128 : (rows + 31) / 32) * (p.k_total / 16) / (double)kQuantWarps;
+    return 2.9 + (quads ? 0.79 : 0.42) * items + 3.5e-5 * rows * p.k_total + 0.012 * p.bn + 2.8e-6 * p.bn * p.k_total + 6.7e-4 * p.k_total;
+}
+double copy_us(const UmmaPlan& p, const ConvShape& s, long tiles, int sm_count) {
+    const double per_sm = (double)((tiles * p.n_tiles + sm_count - 1) / sm_count);
+    return 4.9 + 8.1e-7 * s.n * s.h * s.w * s.cin_pad + 2.1e-3 * p.k_total + 1.6e-3 * p.bn + per_sm * (9.6e-3 * p.bn + 6e-4 * p.k_total);
+}
+
+}  // namespace
+
+// fp32 input, 1x1: inside where that is estimated to be faster, over the panels for which it is fastest (every panel quantizes the input once
+// more, but a narrower one may leave the launch short tiles). 196 -> 140 48x31 x5: 59 tiles, one panel 7.3 us; three of 64 columns, two
+// tiles for some CTAs, 8.6; through a copy 8.3. With more tiles than SMs one panel that does not want sixteen
+// epilogue warps wins, where the images are whole pixel quads (116 -> 116 20x20 x256: copy / inside 17.5 / 16.1; but two panels,
+// 256 -> 512 28x28 x128: 52 / 55, and pixel by pixel, 90 -> 77 31x33 x60: 12.5 / 19.2). Halo tiles: up to 64 channels in one block and one
+// wave of CTAs, panels narrowed into half of one (64 -> 64 56x56 one image 8.5 / 5.3; 128 -> 128 28x28 x8 8.8 / 11.6).
+UmmaChoice umma_choose(const UmmaVariant* v, int n, const ConvShape& s, int sm_count, bool may_quantize, long* n_tiles) {
+    const PixelTiles t = tile_pixels(v[0].plan, s);
+    if (n_tiles) *n_tiles = t.tiles;
+    const long pixels = (long)s.n * s.oh * s.ow;
+    UmmaChoice c{v + pick_panels(v, n, t.tiles, sm_count), false, kTileM, false};
+    const bool can = may_quantize && (t.flat || v[0].plan.halo == 1) && s.cin_pad > 32 && (double)s.n * s.h * s.w <= 2147483647.0;
+    if (can && !t.flat && v[0].plan.ncb == 1 && s.cin_pad <= 64 && t.tiles * v[0].plan.n_tiles <= sm_count) {
+        c.variant = v;
+        c.inside = true;
+        for (int i = 1; i < n; ++i)
+            if (2 * t.tiles * v[i].plan.n_tiles <= sm_count) c.variant = v + i;
+    } else if (can && t.flat && t.tiles * v[0].plan.n_tiles <= sm_count) {
+        double best = copy_us(c.variant->plan, s, t.tiles, sm_count);
+        for (int i = 0; i < n && t.tiles * v[i].plan.n_tiles <= sm_count; ++i) {
+            const double us = inside_us(v[i].plan, s, small_tile_rows(pixels, v[i].plan.n_tiles, true, sm_count));
+            if (us >= best) continue;
+            best = us;
+            c.variant = v + i;
+            c.inside = true;
+        }
+    } else if (can && t.flat && v[0].plan.n_tiles == 1 && v[0].plan.bn <= 192 && (long)s.h * s.w % 4 == 0) {
+        c.variant = v;
+        c.inside = true;
+    }
+    c.compact = runs_compact(c.variant->plan, t.tiles, c.inside, sm_count);
+    if (c.compact && t.flat) c.tile_rows = small_tile_rows(pixels, c.variant->plan.n_tiles, c.inside, sm_count);
+    return c;
+}
+
+const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaChoice& choice, const ConvShape& s,
                               const int8_t* x, const EpilogueParams& ep, void* out, int out_dtype, uint32_t* status,
                               const UmmaSources* sources, const UmmaMixedOut* mixed_in, unsigned long long wait_limit_ns, const UmmaFloatInput* f32) {
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return "cuTensorMapEncodeTiled entry point not available";
-    // The tiling of the pixels is the same for every variant. A launch with fewer tiles than SMs is bound by the chain of one
-    // tile, most of which (MMAs, requantize, stores) shrinks with the panel: take the widest panels that put a CTA on every SM,
-    // or the narrowest, as long as all the CTAs are resident at once. Measured: 232 -> 232 on 10x10, one image 4.2 us with one
-    // panel of 240 columns, 2.9 with 32; but 717 -> 152 on 102 tiles 20.5 us with one panel and 23.4 with two that do not fit an
-    // SM together; with more tiles than SMs every extra panel only reads the activations once more.
-    UmmaPlan p = variants[0].plan;
-    const UmmaVariant* chosen = variants;
     const long pixels = (long)s.n * s.oh * s.ow;
     if (pixels == 0) return nullptr;
+    if ((f32 != nullptr) != choice.inside) return "fp32 input without a launch that quantizes it (or the reverse)";
+    UmmaPlan p = choice.variant->plan;
+    const PixelTiles tiles = tile_pixels(p, s);
+    p.flat = tiles.flat; p.tw = tiles.tw; p.th = tiles.th; p.tiles_x = tiles.x; p.tiles_y = tiles.y; p.m_tiles = (int)tiles.tiles;
+    p.tile_rows = choice.tile_rows;
+    if (p.tile_rows != kTileM) p.m_tiles = p.tiles_x = (int)((pixels + p.tile_rows - 1) / p.tile_rows);
+    const bool flat = p.flat != 0;
     KernelMaps km;  // only the entries the plan uses are filled in
     CUtensorMap& tmA = km.tm[0];
     UmmaMixedOut mixed{};
@@ -954,44 +1067,8 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
         if (out_dtype != DT_S8_NHWC || s.cout > 1024) return "fp32 side output needs an int8 launch with at most 1024 output channels";
         mixed = *mixed_in;
     }
-    const bool flat = s.kh == 1 && s.kw == 1 && s.ph == 0 && s.pw == 0 && s.sh == 1 && s.sw == 1;
-    p.flat = flat ? 1 : 0;
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = CUDA_SUCCESS;
-    if (flat) {
-        p.tw = p.tile_rows = kTileM; p.th = 1; p.tiles_x = (int)((pixels + kTileM - 1) / kTileM); p.tiles_y = 1;
-        p.m_tiles = p.tiles_x;
-    } else {
-        p.tile_rows = kTileM;
-        // rectangle of 128 output pixels with the least padding waste (halo mode: always 8 x 16)
-        long best = -1;
-        for (int tw = 8; tw <= 128; tw *= 2) {
-            const int th = kTileM / tw;
-            if ((tw - 1) * s.sw + 1 > 256 || (th - 1) * s.sh + 1 > 256) continue;  // a TMA box spans at most 256 elements per dimension
-            const long cover = (long)((s.ow + tw - 1) / tw) * tw * ((s.oh + th - 1) / th) * th;
-            if (best < 0 || cover < best) { best = cover; p.tw = tw; p.th = th; }
-        }
-        if (p.halo) { p.tw = kHaloTw; p.th = kHaloTh; }
-        p.tiles_x = (s.ow + p.tw - 1) / p.tw;
-        p.tiles_y = (s.oh + p.th - 1) / p.th;
-        p.m_tiles = s.n * p.tiles_x * p.tiles_y;
-    }
-    for (int i = 1; i < n_variants && (long)p.m_tiles * chosen->plan.n_tiles < sm_count; ++i)
-        if ((long)p.m_tiles * variants[i].plan.n_tiles <= (long)sm_count * variants[i].plan.ctas_per_sm) chosen = variants + i;
-    {
-        const UmmaPlan tiling = p;
-        p = chosen->plan;
-        p.flat = tiling.flat; p.tw = tiling.tw; p.th = tiling.th; p.tiles_x = tiling.tiles_x; p.tiles_y = tiling.tiles_y; p.m_tiles = tiling.m_tiles;
-        p.tile_rows = tiling.tile_rows;
-    }
-    // SMs still idle: fewer pixels per tile. A tile's loads arrive a row at a time, and a gathered layer has a row of 32 bytes per pixel
-    // and K block (232 channels gathered in 15 blocks: 1900 rows for 128 pixels). 128 / 64 / 32 / 16 pixels at most: 116 -> 116 20x20
-    // 2.59 / 2.47 / 2.37 / 2.30 us, detector on one 416x416 image 450 / 433 / 429 / 427, backbone 169 / 164 / 160 / 159. A quantizing
-    // launch, whose CTAs have an SM to themselves, keeps 32 (116 -> 116: 3.8, with 16 4.4).
-    while (flat && p.tile_rows > (f32 ? 32 : 16) && (pixels + p.tile_rows / 2 - 1) / (p.tile_rows / 2) * p.n_tiles <= sm_count) {
-        p.tile_rows /= 2;
-        p.m_tiles = p.tiles_x = (int)((pixels + p.tile_rows - 1) / p.tile_rows);
-    }
     if ((p.gather > 0) != (sources != nullptr)) return "gathered layer launched without its sources (or the reverse)";
     if (p.gather > 0) {
         if (!flat || sources->n_src != p.gather || p.nkb > kUmmaMaxGatherBlocks || p.bkc != kUmmaGatherBlock) return "bad gathered launch";
@@ -1039,7 +1116,7 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
     p.div_tx = make_fast_div((uint32_t)p.tiles_x);
     p.div_plane = make_fast_div((uint32_t)(s.oh * s.ow));
 
-    const CUtensorMap& tmB = *reinterpret_cast<const CUtensorMap*>(chosen->weight_map);
+    const CUtensorMap& tmB = *reinterpret_cast<const CUtensorMap*>(choice.variant->weight_map);
     const char* err = nullptr;
     QuantSource qs;
     if (f32) {
@@ -1079,9 +1156,7 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVaria
     // room for it on the same SMs, so the plan takes no more than one tile needs: eight epilogue warps at 96 registers, the stages of
     // one tile, one accumulator (464 -> 1024 on 10x10, 128 CTAs: 4.6 -> 3.5 us).
     p.out_kind = out_dtype;
-    // (A halo tile wants its MMA issue unrolled, rolled it costs 0.9 us: on fp32 input in the compact build, which few layers of a network
-    // run, on int8 input in the specialised ones.)
-    if ((long)p.m_tiles * p.n_tiles <= sm_count && (f32 || !p.halo)) {
+    if (choice.compact) {
         p.compact = 1;
         p.epi_warps = kMaxEpiWarps;
         const int loads = p.halo ? p.ncb : (p.gather && p.gather_whole ? 1 : p.nkb);

@@ -1,6 +1,8 @@
 // Host-visible plan of the tensor-core (tcgen05) dense convolution kernel.
 #pragma once
 
+#include <vector>
+
 #include "kernels.h"
 
 namespace ottk {
@@ -48,7 +50,7 @@ struct UmmaVariant {
     UmmaPlan plan{};
     alignas(128) unsigned char weight_map[128];
 };
-constexpr int kUmmaNarrow[] = {128, 64, 32};
+std::vector<UmmaVariant> umma_variants(const UmmaPlan& widest, int cout, int smem_budget);  // weight maps not filled in
 
 // A 1x1 layer whose input channels are spread over several int8 NHWC tensors (each written by one producer layer): K block
 // kb of the implicit GEMM is the 32 channels starting at block_x[kb] of tensor block_src[kb]. The layer's weights are laid
@@ -93,16 +95,23 @@ struct UmmaFloatInput {
 };
 bool umma_float_input(const float* x, const PlaneGather* table, int cin, long hw, float scale, UmmaFloatInput* in);
 
+// What a call runs: which of the layer's plans (widest panels first), whether it quantizes fp32 input itself, how many pixels a tile has,
+// and whether it is the compact build, one tile per CTA. may_quantize: the input is fp32 and umma_float_input can describe it.
+// tiles: NULL, or receives the number of 128-pixel tiles.
+struct UmmaChoice {
+    const UmmaVariant* variant;
+    bool inside;
+    int tile_rows;
+    bool compact;
+};
+UmmaChoice umma_choose(const UmmaVariant* variants, int n_variants, const ConvShape& s, int sm_count, bool may_quantize, long* tiles = nullptr);
+
 // Launch. Returns NULL or an error text.
 // sources: NULL, or where the K blocks of a plan with gather > 0 come from (x is then unused). mixed: NULL, or the fp32 side
-// output of an int8 launch.
-// variants: the layer's plans, widest panels first; which one runs depends on the number of pixel tiles.
-const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaVariant* variants, int n_variants, const ConvShape& s,
+// output of an int8 launch. f32: the input of a choice that quantizes inside.
+const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaChoice& choice, const ConvShape& s,
                               const int8_t* x, const EpilogueParams& ep, void* out, int out_dtype, uint32_t* status,
                               const UmmaSources* sources = nullptr, const UmmaMixedOut* mixed = nullptr,
                               unsigned long long wait_limit_ns = 2000000000ull, const UmmaFloatInput* f32 = nullptr);
-
-// whether a launch on fp32 input should quantize inside the kernel rather than read an int8 copy
-bool umma_quantizes_inside(const UmmaPlan& p, const ConvShape& s, int sm_count);
 
 }  // namespace ottk

@@ -1,0 +1,67 @@
+"""Which launch a dense layer takes, on the CPU over thousands of layers: narrow weight panels must not cost a launch what the wide ones
+would have had (one tile per CTA, one pass over fp32 input)."""
+import ctypes as C
+import random
+
+import pytest
+
+SMS = 148
+
+
+@pytest.fixture(scope="module")
+def plan():
+    from tensor_b200 import capi
+    lib = capi.library()
+
+    def ask(cin, cout, k, stride, n, h, w, f32):
+        out = (C.c_int * 8)()
+        assert lib.ott_debug_dense_plan(cin, cout, k, stride, n, h, w, f32, SMS, out) == 0
+        return dict(zip(("tiles", "panels", "columns", "per_sm", "inside", "compact", "rows", "halo"), out))
+
+    return ask
+
+
+def _layers(count, seed):
+    rng = random.Random(seed)
+    for _ in range(count):
+        k = rng.choice((1, 3))
+        top = 1024 if k == 1 else 256
+        yield (rng.randint(24, top), rng.randint(24, top), k, rng.choice((1, 1, 2)) if k == 3 else 1, rng.randint(1, 64), rng.randint(7, 80), rng.randint(7, 80))
+
+
+def test_launches_keep_to_the_wave_they_were_planned_for(plan):
+    seen = set()
+    for layer in _layers(4000, 1):
+        for f32 in (0, 1):
+            p = plan(*layer, f32)
+            ctas = p["tiles"] * p["panels"]
+            if p["inside"]:
+                # one CTA per SM: a second panel means one more pass over the input, and pays only for a launch of one tile per CTA
+                assert f32 and (p["panels"] == 1 or ctas <= SMS), (layer, p)
+            if p["compact"]:
+                assert ctas <= SMS and (p["inside"] or p["columns"] <= 64), (layer, p)
+            else:
+                assert p["rows"] == 128
+            seen.add((p["inside"], p["compact"], p["columns"] <= 32, p["panels"] > 1))
+    assert len(seen) >= 8
+
+
+@pytest.mark.parametrize("layer,f32,panels,inside", [
+    ((205, 56, 1, 1, 20, 47, 18), 0, 1, 0),   # 133 tiles: two panels of 32 would be 266 CTAs that read every activation twice
+    ((94, 192, 1, 1, 6, 31, 26), 0, 3, 0),    # 38 tiles: panels of 64, not 228 CTAs of 32
+    ((96, 512, 1, 1, 40, 8, 16), 0, 4, 0),    # 40 tiles
+    ((232, 232, 1, 1, 1, 10, 10), 0, 8, 0),   # 1 tile: as narrow as it gets
+    ((202, 130, 3, 1, 12, 10, 15), 0, 3, 0),  # 24 tiles of a weight-heavy layer: 72 CTAs, not 120
+    ((256, 512, 1, 1, 128, 28, 28), 1, 2, 0),
+    ((116, 116, 1, 1, 256, 20, 20), 1, 1, 1),
+    ((64, 64, 3, 1, 1, 56, 56), 1, 2, 1),
+    ((128, 128, 3, 1, 8, 28, 28), 1, 1, 0)])
+def test_named_launches(plan, layer, f32, panels, inside):
+    p = plan(*layer, f32)
+    assert (p["panels"], p["inside"]) == (panels, inside), p
+
+
+def test_fp32_input_is_not_quantized_once_per_narrow_panel(plan):
+    for layer, most in (((196, 140, 1, 1, 5, 48, 31), 2), ((113, 197, 1, 1, 11, 23, 12), 4)):
+        p = plan(*layer, 1)
+        assert p["panels"] <= most and p["tiles"] * p["panels"] <= SMS, p
