@@ -707,6 +707,7 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
         }
     }
     rc = upload(ctx, wpacked.data(), wpacked.size(), (void**)&c->w_dev);
+    std::vector<int8_t> wparity;
     std::vector<uint32_t> wtiled;
     if (rc == OTT_OK && depthwise && d->kh == d->kw && (d->kh == 3 || d->kh == 5)) {
         wtiled.resize((size_t)c->cout_pad * depthwise_tiled_weight_words(d->kh));
@@ -737,10 +738,18 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
         int smem_optin = 0;
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
         c->umma = umma_variants(c->plan, d->cout, smem_optin);
-        for (UmmaVariant& u : c->umma) {
-            const char* err = umma_encode_weight_map(u.plan, c->w_dev, u.weight_map);
-            if (err) rc = ctx->fail(OTT_ERR_CUDA, "%s", err);
+        UmmaPlan parity{};
+        if (!gi && umma_plan_parity(c->plan, d->cin, d->cout, d->kh, d->kw, d->sh, d->sw, d->dh, d->dw, smem_optin, &parity)) {
+            wparity.resize((size_t)parity.cout_rows * parity.k_total);
+            umma_pack_weights(parity, w_oihw, d->cin, d->cout, d->kh, d->kw, wparity.data());
+            rc = upload(ctx, wparity.data(), wparity.size(), (void**)&c->w_parity_dev);
+            c->umma_parity = umma_variants(parity, d->cout, smem_optin);
         }
+        for (auto* form : {&c->umma, &c->umma_parity})
+            for (UmmaVariant& u : *form) {
+                const char* err = rc == OTT_OK ? umma_encode_weight_map(u.plan, form == &c->umma ? c->w_dev : c->w_parity_dev, u.weight_map) : nullptr;
+                if (err) rc = ctx->fail(OTT_ERR_CUDA, "%s", err);
+            }
     }
     // host staging vectors die at return: make sure the uploads have consumed them
     if (rc == OTT_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = ctx->fail(OTT_ERR_CUDA, "upload failed");
@@ -757,6 +766,7 @@ int ott_conv_int8_destroy(ott_ctx* ctx, ott_conv* c) {
     if (!c) return OTT_OK;
     if (ctx) {
         ctx->alloc->free(c->w_dev);
+        ctx->alloc->free(c->w_parity_dev);
         ctx->alloc->free(c->w_tiled_dev);
         ctx->alloc->free(c->w_dwu_dev);
         ctx->alloc->free(c->scale_in_dev);
@@ -848,7 +858,12 @@ int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int
     s.ow = out_dim(w, k, stride, k / 2, 1);
     if (s.oh < 1 || s.ow < 1) return OTT_ERR_INVALID;
     long tiles = 0;
-    const UmmaChoice c = umma_choose(all.data(), (int)all.size(), s, sm_count, f32_input != 0, &tiles);
+    UmmaPlan other{};
+    const bool has_parity = umma_plan_parity(widest, cin, cout, k, k, stride, stride, 1, 1, kSmemOptin, &other);
+    const std::vector<UmmaVariant> parity = has_parity ? umma_variants(other, cout, kSmemOptin) : std::vector<UmmaVariant>();
+    const bool by_parity = has_parity && umma_prefers_parity(parity.data(), (int)parity.size(), all.data(), s, sm_count);
+    const std::vector<UmmaVariant>& form = by_parity ? parity : all;
+    const UmmaChoice c = umma_choose(form.data(), (int)form.size(), s, sm_count, f32_input != 0, &tiles);
     const int out[8] = {(int)tiles, c.variant->plan.n_tiles, c.variant->plan.bn, c.variant->plan.ctas_per_sm, c.inside, c.compact, c.tile_rows, c.variant->plan.halo};
     std::memcpy(plan, out, sizeof out);
     return OTT_OK;
@@ -1178,9 +1193,12 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
     const int8_t* x = static_cast<const int8_t*>(in_dev);
     UmmaFloatInput f32;
     UmmaChoice choice{};
-    if (c->kind == OTT_KERNEL_DENSE_UMMA)
-        choice = umma_choose(c->umma.data(), (int)c->umma.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW && c->n_in_scales == 1 &&
+    if (c->kind == OTT_KERNEL_DENSE_UMMA) {
+        const bool parity = !c->umma_parity.empty() && umma_prefers_parity(c->umma_parity.data(), (int)c->umma_parity.size(), c->umma.data(), s, ctx->sm_count);
+        const std::vector<UmmaVariant>& form = parity ? c->umma_parity : c->umma;
+        choice = umma_choose(form.data(), (int)form.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW && c->n_in_scales == 1 &&
                              umma_float_input(static_cast<const float*>(in_dev), gather, d.cin, (long)h * w, c->in_scale0, &f32));
+    }
     const bool quant_inside = choice.inside;
     if (in_dtype == OTT_F32_NCHW) {
         if (xq.alloc(ctx, (size_t)n * h * w * c->cin_pad) != cudaSuccess) {

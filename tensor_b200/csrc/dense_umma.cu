@@ -850,15 +850,12 @@ static bool plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh
 
 bool umma_plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, int dw, int smem_budget, UmmaPlan* plan, int bkc_override,
                      bool whole_tile_stages) {
-    const bool have = plan_layer(cin, cout, kh, kw, sh, sw, dh, dw, smem_budget, plan, bkc_override, whole_tile_stages, false);
-    // Stride 2: the two parity planes of a tile's halo are half the rows of one box per tap (3x3: 561 against 1152), where they
-    // leave room for as wide a weight panel (us: 64 -> 128 75x75 x32, fp32 out 14.1 -> 11.8, int8 out 13.5 -> 10.4; 173 -> 93 57x20 x44
-    // 22.1 -> 13.6; 40 -> 40 40x40 x64 12.3 -> 8.7; 64 -> 64 56x56 one image 4.6 -> 3.8).
-    UmmaPlan p{};
-    if (have && sh == 2 && sw == 2 && dh == 1 && dw == 1 && kh > 1 && kw > 1 && kh <= 7 && kw <= 7 && bkc_override == 0 &&
-        plan_layer(cin, cout, kh, kw, sh, sw, dh, dw, smem_budget, &p, plan->bkc > 64 ? 64 : 0, whole_tile_stages, true) && p.n_tiles <= plan->n_tiles)
-        *plan = p;
-    return have;
+    return plan_layer(cin, cout, kh, kw, sh, sw, dh, dw, smem_budget, plan, bkc_override, whole_tile_stages, false);
+}
+
+bool umma_plan_parity(const UmmaPlan& taps, int cin, int cout, int kh, int kw, int sh, int sw, int dh, int dw, int smem_budget, UmmaPlan* plan) {
+    return sh == 2 && sw == 2 && dh == 1 && dw == 1 && kh > 1 && kw > 1 && kh <= 7 && kw <= 7 &&
+           plan_layer(cin, cout, kh, kw, sh, sw, dh, dw, smem_budget, plan, taps.bkc > 64 ? 64 : 0, false, true) && plan->n_tiles <= taps.n_tiles;
 }
 
 bool umma_narrow_plan(const UmmaPlan& base, int bn, int cout, int smem_budget, UmmaPlan* plan) {
@@ -1010,6 +1007,17 @@ double copy_us(const UmmaPlan& p, const ConvShape& s, long tiles, int sm_count) 
 }
 
 }  // namespace
+
+// Stride 2: the two parity planes of a tile's halo are half the rows of one box per tap (3x3: 561 against 1152; us: 64 -> 128 75x75 x32,
+// fp32 out 14.1 -> 11.8, int8 out 13.5 -> 10.4; 173 -> 93 57x20 x44 22.1 -> 13.6; 40 -> 40 40x40 x64 12.3 -> 8.7; 64 -> 64 56x56 one image
+// 4.6 -> 3.8), but its tiles are 8 x 16 whatever the map is, while the other form takes the rectangle that covers it best. Where
+// that makes half as many tiles again, and not all of them run at once, the advantage is gone: 53 -> 44 9x59 x101, 404 tiles against
+// 202, 8.1 / 6.0; 32 -> 32 8x40 x128, 384 against 128, 6.2 / 4.7; 154 -> 140 13x32 x78, 156 against 78, 16.9 / 14.2 (250 layers: 0.5 %
+// from the better form of each on average; always by parity 0.9 %, always by tap 22 %).
+bool umma_prefers_parity(const UmmaVariant* parity, int n_parity, const UmmaVariant* taps, const ConvShape& s, int sm_count) {
+    const long by_parity = tile_pixels(parity[0].plan, s).tiles, by_tap = tile_pixels(taps[0].plan, s).tiles;
+    return 2 * by_parity <= 3 * by_tap || by_parity * parity[pick_panels(parity, n_parity, by_parity, sm_count)].plan.n_tiles <= sm_count;
+}
 
 // fp32 input, 1x1: inside where that is estimated to be faster, over the panels for which it is fastest (every panel quantizes the input once
 // more, but a narrower one may leave the launch short tiles). 196 -> 140 48x31 x5: 59 tiles, one panel 7.3 us; three of 64 columns, two

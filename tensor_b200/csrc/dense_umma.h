@@ -42,6 +42,10 @@ struct UmmaPlan {
 bool umma_plan_layer(int cin, int cout, int kh, int kw, int sh, int sw, int dh, int dw, int smem_budget, UmmaPlan* plan,
                      int bkc_override = 0, bool whole_tile_stages = false);
 
+// The other form of a stride-2 layer, see umma_prefers_parity; false where there is none or it has less room for weights than `taps`.
+// It reads the weights packed for its own plan.
+bool umma_plan_parity(const UmmaPlan& taps, int cin, int cout, int kh, int kw, int sh, int sw, int dh, int dw, int smem_budget, UmmaPlan* plan);
+
 // The same layer over narrower weight panels of bn columns, for launches with few pixel tiles; false where it makes no difference.
 bool umma_narrow_plan(const UmmaPlan& base, int bn, int cout, int smem_budget, UmmaPlan* plan);
 
@@ -94,6 +98,9 @@ struct UmmaFloatInput {
     float scale;
 };
 bool umma_float_input(const float* x, const PlaneGather* table, int cin, long hw, float scale, UmmaFloatInput* in);
+
+// Which form a call of such a layer takes.
+bool umma_prefers_parity(const UmmaVariant* parity, int n_parity, const UmmaVariant* taps, const ConvShape& s, int sm_count);
 
 // What a call runs: which of the layer's plans (widest panels first), whether it quantizes fp32 input itself, how many pixels a tile has,
 // and whether it is the compact build, one tile per CTA. may_quantize: the input is fp32 and umma_float_input can describe it.

@@ -1,5 +1,5 @@
 """Which launch a dense layer takes, on the CPU over thousands of layers: narrow weight panels must not cost a launch what the wide ones
-would have had (one tile per CTA, one pass over fp32 input)."""
+would have had (one tile per CTA, one pass over fp32 input), and a stride-2 layer takes the form that suits its map."""
 import ctypes as C
 import random
 
@@ -65,3 +65,11 @@ def test_fp32_input_is_not_quantized_once_per_narrow_panel(plan):
     for layer, most in (((196, 140, 1, 1, 5, 48, 31), 2), ((113, 197, 1, 1, 11, 23, 12), 4)):
         p = plan(*layer, 1)
         assert p["panels"] <= most and p["tiles"] * p["panels"] <= SMS, p
+
+
+def test_stride_two_form_follows_the_map(plan):
+    assert plan(64, 128, 3, 2, 32, 75, 75, 0)["halo"] == 2
+    assert plan(64, 64, 3, 2, 1, 56, 56, 0)["halo"] == 2
+    for flat, tiles in (((53, 44, 3, 2, 101, 9, 59), 202), ((32, 32, 3, 2, 128, 8, 40), 128), ((154, 140, 3, 2, 78, 13, 32), 78)):
+        p = plan(*flat, 0)  # twice to three times the tiles as halo tiles of 8 x 16
+        assert (p["halo"], p["tiles"]) == (0, tiles), p
