@@ -361,19 +361,26 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
 // issued), or the latency of one CTA (memory round trip, then one warp's dependent instructions at six cycles each) times the
 // waves. The instruction counts are those of the inner loops: 26 per fp32 word loaded and quantized, 7 per 32 int8 quads
 // loaded and transposed, 46 / 75 per warp and output row of a 3x3 / 5x5 filter, 12 per row that only fills the ring.
-constexpr int kPlaneWords = 384, kSms = 148;
-template <int K, int S, bool IN_F32>
+// fp32 output from int8, stride 1: a lane stores 16 bytes of its own channel's plane, half a sector (single pixels where the rows are not
+// aligned), and the rest of the sector and of the line comes from the next warps. An output that does not fit L2, or one of single
+// pixels, wants that to happen soon: low bands (planes of 128 words), eight warps side by side on the same rows. us, high bands / low:
+// 5x5 256 channels 56x56 x64 194 / 114, 116 30x73 x110 182 / 110, 288 15x9 x71 20.1 / 15.4; 3x3 251 67x33 x52 195 / 117. But 5x5 199
+// 25x56 x69, 77 MB of aligned rows, 34.7 / 38.7.
+constexpr int kPlaneWords = 384, kLowPlaneWords = 128, kSms = 148;
+constexpr long kBeyondL2 = 96l << 20, kMuchOutput = 8l << 20;
+template <int K, int S, bool IN_F32, int EPI>
 inline Tile plan_tile(const ConvShape& s) {
     Tile T{};
+    const bool low = !IN_F32 && EPI == EPI_F32 && S == 1 && 4l * s.n * s.cout * s.oh * s.ow >= (s.ow % 4 == 0 ? kBeyondL2 : kMuchOutput);
     const int ow4 = (s.ow + 3) / 4, max_nxq = S == 1 ? 16 : 10;
     T.tiles_x = (ow4 + max_nxq - 1) / max_nxq;
     T.nxq = (ow4 + T.tiles_x - 1) / T.tiles_x;
     T.rp = (T.nxq - 1) * S + Geo<K, S>::NRAW;
     T.cgroups = (s.cout_pad + CG - 1) / CG;
-    const int ty_max = (kPlaneWords / T.rp - K) / S + 1;
+    const int ty_max = ((low ? kLowPlaneWords : kPlaneWords) / T.rp - K) / S + 1;
     const long per_band = (long)s.n * T.tiles_x * T.cgroups;
     // a throughput-bound launch wants every warp to have the same work, a latency-bound one as many warps as there are
-    const int widths[2] = {T.nxq > 8 ? (T.nxq + 1) / 2 : T.nxq > 2 ? T.nxq : 2, THREADS / 32};
+    const int widths[2] = {low ? THREADS / 32 : T.nxq > 8 ? (T.nxq + 1) / 2 : T.nxq > 2 ? T.nxq : 2, THREADS / 32};
     double best = 0;
     for (int bands = (s.oh + ty_max - 1) / ty_max; bands <= s.oh; ++bands) {
         const int ty = (s.oh + bands - 1) / bands, tiles_y = (s.oh + ty - 1) / ty;
@@ -382,7 +389,7 @@ inline Tile plan_tile(const ConvShape& s) {
         const int npos = ((ty - 1) * S + K) * T.rp;
         for (int w : widths) {
             int nrg = 1;
-            while (T.nxq * nrg < w && ty > 2 * nrg) ++nrg;
+            while ((!low || T.nxq <= 2) && T.nxq * nrg < w && ty > 2 * nrg) ++nrg;
             const int rpt = (ty + nrg - 1) / nrg;
             nrg = (ty + rpt - 1) / rpt;
             const int passes = (T.nxq * nrg + w - 1) / w;
@@ -411,7 +418,7 @@ inline Tile plan_tile(const ConvShape& s) {
 template <int K, int S, bool IN_F32, int EPI, int ACT>
 cudaError_t launch_t(cudaStream_t stream, const ConvShape& s, const void* x, const PlaneGather& G, const uint32_t* wq, const float* in_scales,
                      int n_in_scales, const EpilogueParams& ep, void* out) {
-    const Tile T = plan_tile<K, S, IN_F32>(s);
+    const Tile T = plan_tile<K, S, IN_F32, EPI>(s);
     const size_t smem = (size_t)CG * T.ps * 4;
     // fp32 rows whose 16-byte words never cross a row's end: a width that is a multiple of 4 and 16-byte aligned planes
     int aligned = s.w % 4 == 0 ? 1 : 0;

@@ -34,6 +34,23 @@ def test_tile_edges(ctx, c, n, h, w, k, stride, s8_input):
         assert np.array_equal(bits(got), bits(run_port(case, rounding, want_acc=False)["y"]))
 
 
+@pytest.mark.parametrize("k,c,n,h,w", [(3, 40, 31, 41, 45), (5, 40, 31, 41, 45), (5, 33, 100, 66, 10), (3, 64, 110, 60, 64)])
+def test_large_fp32_outputs(ctx, k, c, n, h, w):
+    """8 MB of rows that are not 16-byte aligned and 100 MB of aligned ones: the low bands, with and without row groups; four images each."""
+    from gpu_support import bits, make_layer
+    from support import nchw_to_nhwc_padded
+    from tensor_b200 import F32_NCHW, S8_NHWC, nhwc_channels
+    case = ConvCase(f"dwt_low_{k}_{w}", c, c, k, 1, k // 2, groups=c, n=n, h=h, w=w, int8_scale_term=1, act_type=ACT_RELU, w_std=0.1, s8_input=True, seed=c + w).make()
+    layer = make_layer(ctx, case, ROUND_ADD_HALF_TRUNC)
+    ctx.check(ctx.lib.ott_set_depthwise_tensor_cores(ctx.h, 0))
+    got = layer.forward_host(nchw_to_nhwc_padded(case.x_s8, nhwc_channels(c)), S8_NHWC, F32_NCHW)
+    ctx.check(ctx.lib.ott_set_depthwise_tensor_cores(ctx.h, 1))
+    layer.close()
+    some = [0, 1, n // 2, n - 1]
+    case.n, case.x_s8 = len(some), np.ascontiguousarray(case.x_s8[some])
+    assert np.array_equal(bits(got[some]), bits(run_port(case, ROUND_ADD_HALF_TRUNC, want_acc=False)["y"]))
+
+
 @pytest.mark.parametrize("first,total", [(1, 7), (2, 6), (3, 6)])
 def test_channel_range_on_every_alignment(ctx, first, total):
     """Planes of an odd size inside a wider tensor: every plane starts at another offset from a 16-byte boundary."""
