@@ -873,20 +873,28 @@ int ott_conv_int8_kernel_kind(const ott_conv* c) { return c ? c->kind : OTT_ERR_
 
 namespace {
 // int8 NHWC input of a 3x3 depthwise layer: the multiply-adds can go to the tensor cores as the data lies, no byte transposes,
-// at one 128-row MMA per tap, 32 channels and 8 x 16 output pixels. That pays where the CUDA cores have the most transposing to
-// do per output - stride 2 (four input pixels per output) and fp32 output (whose stores the other kernel cannot coalesce) - on
-// launches long enough to amortise its longer pipeline (6 M outputs) and maps its tiles fit. A gathered layer's channels come in
-// 32-channel blocks of which it may want a few each; they cost the tensor cores little more than the bytes, so its maps may fit half as
-// well (116 channels from 12 blocks, 20x20 outputs, 256 images: 34.5 / 37.2; 232 from 13, 10x10: 28.5 / 36.1). Measured, tensor cores against
-// CUDA cores: 256 channels 56x56 stride 2, 64 images 15.7 / 20.2 us; 58 channels 80x80 stride 2, 256 images 27.1 / 43.2; 512
-// channels 28x28, fp32 out 57.8 / 64.9; but 128 channels 28x28 stride 2, 64 images 5.9 / 5.0 (too short), 58 channels 40x40
-// stride 2, 256 images 12.6 / 11.6 (20x20 outputs fill 52 % of their tiles), 256 channels 56x56 stride 1 41.1 / 40.7.
+// at one 128-row MMA per tap, 32 channels and 8 x 16 output pixels. That pays where the CUDA cores have the most to do per output, on
+// launches long enough to amortise its longer pipeline and maps its tiles fit. Measured (us, tensor cores / CUDA cores):
+// int8 output, stride 2 (four input pixels to transpose per output), from 4.5 M outputs on: 256 channels 56x56 x64 15.8 / 20.7, 233
+// 77x76 x13 11.6 / 13.1, 459 63x31 x41 16.7 / 16.3; but 256 56x56 x16 7.3 / 6.6, 407 48x39 x38 (tiles 62 % full) 14.5 / 13.3. Stride 1: 256
+// 56x56 x64 41.2 / 40.8, 114 71x38 x74 24.3 / 27.9, 343 23x60 x57 33.2 / 26.7: the CUDA cores.
+// fp32 output, whose stores the other kernel cannot coalesce: 256 56x56 x64 55 / 100, 58 40x40 x64 9.9 / 12.7, 256 56x56 x4 10.2 / 11.5; but
+// 141 11x56 x34 (69 % full) 9.2 / 7.2, 58 40x40 x16 5.7 / 6.1, x4 4.5 / 3.5. Rows that are not 16-byte aligned leave it pixel by pixel: 345 37x63
+// x6 12.8 / 25.3, 186 72x11 x85 (62 %) 24.6 / 58.0, 328 30x11 x12 (1.4 M outputs) 8.5 / 9.5, of one channel block 31 37x79 x16 5.8 / 10.6, 30
+// 13x67 x23 4.4 / 6.1; but 121 17x37 x16 (49 %) 9.4 / 7.3, 139 63x13 x4 (0.5 M) 7.0 / 4.2.
+// A gathered layer's channels come in 32-channel blocks of which it may want a few each; they cost the tensor cores little more than the
+// bytes, so its maps may fit half as well (116 channels from 12 blocks, 20x20 outputs, 256 images: 34.5 / 37.2; 232 from 13, 10x10: 28.5 /
+// 36.1), from 6 M outputs on: ShuffleNetV2 with these two layers on the tensor cores from 6 M / 1.5 M / 0 on, us a forward: 47 images, three
+// at a time 299 / 308 / 308, 64 images 351 / 358 / 358, one image alone 160 / 160 / 166.
 bool depthwise_on_tensor_cores(const ott_ctx* ctx, const ott_conv* c, const ConvShape& s, int out_dtype) {
     if (!c->dw_umma || out_dtype == OTT_S32_NHWC || ctx->dw_tensor_cores == 0) return false;
     if (ctx->dw_tensor_cores == 2) return true;
-    if (s.sh == 1 && out_dtype != OTT_F32_NCHW) return false;
-    const long tiles = (long)((s.oh + 15) / 16) * ((s.ow + 7) / 8), pixels = (long)s.oh * s.ow;
-    return pixels * 20 >= tiles * 128 * (c->block_x.empty() ? 14 : 7) && (double)s.n * pixels * (c->dw_plan.ncb_total * 32) >= 6e6;
+    const double tiles = (double)((s.oh + 15) / 16) * ((s.ow + 7) / 8), pixels = (double)s.oh * s.ow, fill = pixels / (128 * tiles);
+    const double outputs = s.n * pixels * (c->dw_plan.ncb_total * 32);
+    if (!c->block_x.empty()) return s.sh == 2 && fill >= 0.35 && outputs >= 6e6;
+    if (out_dtype != OTT_F32_NCHW) return s.sh == 2 && fill >= 0.7 && outputs >= 4.5e6;
+    if (s.sh == 1 && s.ow % 4 != 0) return fill >= 0.6 && outputs >= (c->dw_plan.ncb_total == 1 ? 4e5 : 1.4e6);
+    return fill >= 0.7 && outputs >= 3e6;
 }
 }  // namespace
 
