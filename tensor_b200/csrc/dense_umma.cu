@@ -13,18 +13,18 @@
 //   tiles never straddle anything. k x k convolutions load, per pixel tile of 8 x 16 and channel block, ONE box
 //   that holds the tile and its halo; filter tap (ky, kx) is an MMA whose A descriptor starts (ky, kx) pixels
 //   into that box and steps one halo row per 8-row group (the swizzle is a function of the shared-memory
-//   address, so shifted views read what TMA wrote). At stride 2 there are two boxes, one per column parity; other
-//   strides and dilated layers load one shifted box per tap instead.
+//   address, so shifted views read what TMA wrote). At stride 2 there are two boxes, one per column parity, where the
+//   map suits them (umma_prefers_parity); other strides and dilated layers load one shifted box per tap instead.
 // * B (the layer's weights for this CTA's BN output channels, all taps) is loaded once per CTA and stays in
 //   shared memory while the CTA walks over its pixel tiles (persistent, weight-stationary).
-// * tcgen05.mma.kind::i8 accumulates exact s32 in TMEM; two accumulators are double-buffered so the
-//   epilogue of tile i overlaps the loads and MMAs of tile i+1.
+// * tcgen05.mma.kind::i8 accumulates exact s32 in TMEM; two accumulators (four of at most 64 columns; one in a
+//   compact launch) let the epilogue of tile i overlap the loads and MMAs of the tiles behind it.
 // * The epilogue warps read TMEM (tcgen05.ld), apply fma(acc, scale_in, bias) -> activation -> requantize
 //   (epilogue.cuh) and store int8 NHWC / fp32 NCHW / s32 NHWC.
 //
 // Warp roles (320 threads): warp 0 = TMA producer (one lane), warp 1 = TMEM owner + MMA issuer (one lane),
 // warps 2..9 = epilogue: warp w reads TMEM lanes 32*(w%4)..+31 (the hardware's lane window of a warp) and
-// takes every other 32-column chunk, so two warps share each lane quarter.
+// shares that quarter's column chunks with the other warps of the same window, dealt out over all the CTA's tiles.
 // Every mbarrier wait is bounded in time: on expiry the waiter raises a CTA-wide abort flag, ORs a code
 // into the status word, and all roles fall through to the common teardown, which frees TMEM.
 #include <cuda.h>
@@ -57,8 +57,7 @@ struct KernelMaps {
     uint8_t block_src[kUmmaMaxGatherBlocks];
 };
 
-// BUILD of the kernel, see dense_umma_kernel
-// added to the activation of an int8 build: scale_out is one scalar. The parameters are what the epilogue waits for (a float4 from
+// Added to the activation of an int8 build: scale_out is one scalar. The parameters are what the epilogue waits for (a float4 from
 // shared memory, the same for all lanes, takes two passes of the data pipe that the output stores need too): a third fewer of
 // them, 64 -> 256 56x56 x128 without activation 51.9 -> 48.1 us. A test inside one build costs as much as it saves.
 constexpr int kOneScale = 8;
@@ -779,7 +778,7 @@ static bool plan_panel(UmmaPlan& p, int smem_budget) {
     // a halo stage feeds all the taps of a whole pixel tile and channel block: three are a deep enough pipeline
     if (p.halo && p.stages > 3) p.stages = 3;
     if (p.stages < 2) return false;
-    // two accumulators of bn columns each; TMEM allocations are powers of two >= 32 columns
+    // accumulators of bn columns each; TMEM allocations are powers of two >= 32 columns
     p.acc_stride = p.bn <= 32 ? 32 : (p.bn <= 64 ? 64 : (p.bn <= 128 ? 128 : 256));
     // narrow tiles finish quickly; four accumulators let the MMA issuer run three tiles ahead of the epilogue
     p.acc_bufs = p.acc_stride <= 64 ? 4 : 2;

@@ -13,7 +13,8 @@ __host__ __device__ inline int nhwc_channels(int c) { return (c + 15) & ~15; }
 
 enum : int { DT_F32_NCHW = 0, DT_S8_NHWC = 1, DT_S32_NHWC = 2 };
 
-// Quotients by a divisor known at launch: n / d = (umulhi(n, mul) + n) >> shift for n < 2^31.
+// Quotients by a divisor known at launch, by multiply and shift (Granlund and Montgomery, 1994): n / d = (umulhi(n, mul) + n) >> shift for
+// n < 2^31.
 struct FastDiv {
     uint32_t mul, shift;
 };
