@@ -95,7 +95,8 @@ def test_batched_equals_single_images(ctx):
     ("four_n_tiles", dict(cin=512, cout=1024, k=1, n=2, h=14, w=14, int8_scale_term=101, act_type=ACT_RELU6)),
 ])
 def test_medium_case_bit_exact(ctx, name, kw):
-    """More pixel tiles than SMs, several weight panels: exercises the persistent loop and the pipelines."""
+    """About as many pixel tiles as SMs, several weight panels, tiles ragged in both directions (launches of several tiles per CTA:
+    test_gpu_dense_builds.py)."""
     from gpu_support import bits, run_gpu
     case = ConvCase(name, kw.pop("cin"), kw.pop("cout"), kw.pop("k"), kw.pop("stride", 1), kw.pop("pad", 0), seed=91, **kw).make()
     got = run_gpu(ctx, case, 0)

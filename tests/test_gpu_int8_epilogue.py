@@ -1,4 +1,5 @@
-"""GPU: the requantizing epilogue's builds, bit for bit against the CPU checker: activations that the int8 clamp carries out and ones
+"""GPU: the requantizing epilogue on launches of one tile per CTA, bit for bit against the
+CPU checker: activations that the int8 clamp carries out and ones
 that it cannot (a ReLU6 whose 6 is not 127, sums that may leave 16 bits, a scale that saturates everything), one output scale and one
 per channel, both roundings, with and without bias, sums of both signs."""
 import numpy as np
