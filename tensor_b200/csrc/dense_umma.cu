@@ -248,7 +248,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
 
     if (warp == 0) {
         if constexpr (!QUANT)
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- TMA producer (activations; the weights were requested during set-up) ----
             uint32_t st = 0, phase = 1;  // stage, and the parity that says it is free (the first round finds every stage free)
             bool ok = true, waited = false;
@@ -303,7 +303,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- MMA issuer ----
             bool ok = mbar_wait(bar_b, 0, abort_flag, status, 16u, P.wait_ns);
             tc_fence_after();

@@ -66,6 +66,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// One thread of a converged warp. Unlike a test of the lane number it tells the compiler that what follows runs on one thread, so that
+// operand descriptors and addresses stay in uniform registers instead of being moved there for every instruction: back-to-back MMAs
+// (M 128, N 32, K 32) 40 cycles apart, the tensor pipe's rate, against 50. Dense layers, time with a lane test / with this, geometric
+// mean over a few hundred of 24 to 1024 channels: 3x3 1.11 to 1.22, 1x1 on int8 1.05 to 1.09.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(r));
+    return r != 0;
+}
+
 // Brings a TMA descriptor (kernel parameter or global memory) into the descriptor cache ahead of its first use, so that the
 // first load through it does not wait for the fetch.
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
