@@ -745,9 +745,10 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
             rc = upload(ctx, wparity.data(), wparity.size(), (void**)&c->w_parity_dev);
             c->umma_parity = umma_variants(parity, d->cout, smem_optin);
         }
-        for (auto* form : {&c->umma, &c->umma_parity})
+        if (d->int8_scale_term > 100) c->umma_rows = umma_row_variants(c->plan, d->cout, smem_optin);
+        for (auto* form : {&c->umma, &c->umma_rows, &c->umma_parity})
             for (UmmaVariant& u : *form) {
-                const char* err = rc == OTT_OK ? umma_encode_weight_map(u.plan, form == &c->umma ? c->w_dev : c->w_parity_dev, u.weight_map) : nullptr;
+                const char* err = rc == OTT_OK ? umma_encode_weight_map(u.plan, form == &c->umma_parity ? c->w_parity_dev : c->w_dev, u.weight_map) : nullptr;
                 if (err) rc = ctx->fail(OTT_ERR_CUDA, "%s", err);
             }
     }
@@ -867,6 +868,19 @@ int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int
     const int out[8] = {(int)tiles, c.variant->plan.n_tiles, c.variant->plan.bn, c.variant->plan.ctas_per_sm, c.inside, c.compact, c.tile_rows, c.variant->plan.halo};
     std::memcpy(plan, out, sizeof out);
     return OTT_OK;
+}
+
+int ott_debug_dense_rows(int cin, int cout, int n, int h, int w, int sm_count) {
+    if (cin < 1 || cout < 1 || n < 1 || h < 1 || w < 1 || sm_count < 1) return OTT_ERR_INVALID;
+    constexpr int kSmemOptin = 227 * 1024;
+    UmmaPlan widest{};
+    if (!umma_plan_layer(cin, cout, 1, 1, 1, 1, 1, 1, kSmemOptin, &widest)) return OTT_ERR_UNSUPPORTED;
+    const std::vector<UmmaVariant> all = umma_variants(widest, cout, kSmemOptin), rows = umma_row_variants(widest, cout, kSmemOptin);
+    ConvShape s{};
+    s.n = n; s.h = s.oh = h; s.w = s.ow = w; s.cin = cin; s.cout = cout; s.cin_pad = nhwc_channels(cin); s.cout_pad = nhwc_channels(cout);
+    s.kh = s.kw = s.sh = s.sw = s.dh = s.dw = 1;
+    const UmmaChoice c = umma_choose_rows(umma_choose(all.data(), (int)all.size(), s, sm_count, false), rows.data(), (int)rows.size(), s, sm_count);
+    return c.variant->plan.rows ? c.variant->plan.bn : 0;
 }
 
 int ott_conv_int8_kernel_kind(const ott_conv* c) { return c ? c->kind : OTT_ERR_INVALID; }
@@ -1206,6 +1220,7 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
         const std::vector<UmmaVariant>& form = parity ? c->umma_parity : c->umma;
         choice = umma_choose(form.data(), (int)form.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW && c->n_in_scales == 1 &&
                              umma_float_input(static_cast<const float*>(in_dev), gather, d.cin, (long)h * w, c->in_scale0, &f32));
+        if (in_dtype == OTT_S8_NHWC && out_dtype == OTT_S8_NHWC && !mixed) choice = umma_choose_rows(choice, c->umma_rows.data(), (int)c->umma_rows.size(), s, ctx->sm_count);
     }
     const bool quant_inside = choice.inside;
     if (in_dtype == OTT_F32_NCHW) {

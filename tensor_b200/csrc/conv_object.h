@@ -31,6 +31,7 @@ struct ott_conv {
     ottk::UmmaPlan plan{};
     std::vector<ottk::UmmaVariant> umma;  // tensor-core layers: `plan` and the narrower ones, each with its weight map
     std::vector<ottk::UmmaVariant> umma_parity;  // stride-2 layers: the other form, over weights packed for it
+    std::vector<ottk::UmmaVariant> umma_rows;  // requantizing 1x1 layers: over the same weights, with channels as accumulator rows
     int8_t* w_parity_dev = nullptr;
     // a layer whose input channels are gathered from several int8 tensors (ott_conv_int8_create_gathered): which K block is
     // which 32 channels of which source, and the channel count every source tensor must have

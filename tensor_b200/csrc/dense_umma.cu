@@ -29,9 +29,9 @@
 // into the status word, and all roles fall through to the common teardown, which frees TMEM.
 #include <cuda.h>
 
-#include <type_traits>
-
+#include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "dense_umma.h"
 #include "launch.cuh"
@@ -69,6 +69,14 @@ constexpr int kAnyOut = 7, kAnyAct = 7;
 constexpr int kCompactBuild = 4, kCompactQuantBuild = 5;
 constexpr __host__ __device__ bool build_quantizes(int build) { return build == 3 || build == kCompactQuantBuild; }
 constexpr int kQuantBuild = 3, kQuantWarps = 8, kQuantRuns = 2;
+// Builds whose accumulator rows are output channels (int8 output): see UmmaPlan::rows. Two CTAs per SM, or one with sixteen epilogue warps.
+constexpr int kRowsBuild = 6, kRowsWideBuild = 7;
+constexpr __host__ __device__ bool build_rows(int build) { return build == kRowsBuild || build == kRowsWideBuild; }
+constexpr int kRowsPixels = 128, kOutSlots = 4;  // pixels (accumulator columns) of a tile; finished tiles on their way out, at most
+constexpr uint32_t kTeamWarps = 8;               // epilogue warps that share an accumulator
+constexpr __host__ __device__ int build_threads(int build) {
+    return build == 2 || build_quantizes(build) ? 64 + 32 * 16 : build == kRowsWideBuild ? 96 + 32 * 16 : build == kRowsBuild ? 96 + 32 * 8 : kMaxThreads;
+}
 
 // fp32 input of a launch that quantizes on the way in (kQuantBuild)
 struct QuantSource {
@@ -133,16 +141,23 @@ struct ParityHalo {
 __host__ __device__ __forceinline__ int epi_chunk(const UmmaPlan& p) { return p.bn <= 32 || p.compact ? 16 : 32; }
 
 struct SmemLayout {
-    uint32_t b_panel, a_stages, bars, tmem_slot, abort_flag, params, total;
+    uint32_t b_panel, a_stages, out_slots, bars, tmem_slot, abort_flag, params, total;
 };
+
+// ROWS: where finished accumulators of 128 and of 64 channels go.
+struct RowsOut {
+    CUtensorMap full, half;
+};
+__host__ __device__ __forceinline__ uint32_t out_slot_bytes(const UmmaPlan& p) { return kRowsPixels * (p.bn <= 64 ? 64u : 128u); }
 
 __host__ __device__ inline SmemLayout smem_layout(const UmmaPlan& p) {
     SmemLayout L;
     L.b_panel = 0;
     L.a_stages = (uint32_t)p.nkb * p.bn * p.bkc;
-    L.bars = L.a_stages + (uint32_t)p.stages * (uint32_t)p.a_stage_bytes;
-    // barriers: full[stages], empty[stages], b_full, tmem_full[kMaxAccBufs], tmem_empty[kMaxAccBufs]
-    L.tmem_slot = L.bars + 8u * (2u * p.stages + 1u + 2u * kMaxAccBufs);
+    L.out_slots = L.a_stages + (uint32_t)p.stages * (uint32_t)p.a_stage_bytes;
+    L.bars = L.out_slots + (p.rows ? (uint32_t)p.out_slots * out_slot_bytes(p) : 0u);
+    // barriers: full[stages], empty[stages], b_full, tmem_full[kMaxAccBufs], tmem_empty[kMaxAccBufs], out_full[kOutSlots], out_free[kOutSlots]
+    L.tmem_slot = L.bars + 8u * (2u * p.stages + 1u + 2u * kMaxAccBufs + (p.rows ? 2u * kOutSlots : 0u));
     L.abort_flag = L.tmem_slot + 8;
     L.params = (L.abort_flag + 8 + 15u) & ~15u;  // scale_in[bn], bias[bn], scale_out[bn]; read as float4
     L.total = L.params + 3u * 4u * p.bn;
@@ -162,15 +177,23 @@ __host__ __device__ inline SmemLayout smem_layout(const UmmaPlan& p) {
 //
 // BUILDs 4 and 5: see kAnyOut.
 //
+// BUILDs 6 and 7: the operands change places, D[channels, pixels] = W x A^T. Written with pixels as rows, a thread's accumulators belong
+// to 16 or 32 channels, whose three parameters each it has to fetch from shared memory for every pixel, and its results are 32 bytes
+// of a row of their own, of which a warp's store touches 32: TMEM -> int8 reached 18.9 values per ns and SM that way (ReLU; without
+// the stores 31). With channels as rows a thread has the same two channels of every 16 (tcgen05.ld.16x256b) and keeps their parameters in
+// registers; stmatrix turns four pixels' bytes into rows of 16 channels in shared memory, and a warp of its own sends a finished tile of
+// 128 pixels x 128 channels off as one TMA store: 32.5 values per ns and SM (24 against 18.3 with the general rounding).
+//
 // BUILD 3: fp32 NCHW input, quantized inside the kernel: warps 10..17 take the TMA producer's place, load the planes, quantize and
 // write the operand tiles (with TMA's swizzle) themselves. No int8 copy of the input crosses HBM and no second kernel runs.
 template <int OUT, int ACT_BUILD, int BUILD>
-__global__ void __launch_bounds__(BUILD == 2 || build_quantizes(BUILD) ? 64 + 32 * 16 : kMaxThreads, BUILD == 1 || BUILD == kCompactBuild ? 2 : 1)
+__global__ void __launch_bounds__(build_threads(BUILD), BUILD == 1 || BUILD == kCompactBuild || BUILD == kRowsBuild ? 2 : 1)
 dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUILD), QuantSource, KernelMaps> maps, const __grid_constant__ CUtensorMap tmB, const UmmaPlan P,
                   const ConvShape s, const EpilogueParams ep, void* __restrict__ out, uint32_t* __restrict__ status,
-                  const __grid_constant__ UmmaMixedOut mixed) {
+                  const __grid_constant__ std::conditional_t<build_rows(BUILD), RowsOut, UmmaMixedOut> mixed) {
     constexpr int ACT = ACT_BUILD & ~kOneScale;
-    constexpr bool ONE_SCALE = (ACT_BUILD & kOneScale) != 0, COMPACT = BUILD >= kCompactBuild, QUANT = build_quantizes(BUILD);
+    constexpr bool ONE_SCALE = (ACT_BUILD & kOneScale) != 0, COMPACT = BUILD == kCompactBuild || BUILD == kCompactQuantBuild, QUANT = build_quantizes(BUILD),
+                   ROWS = build_rows(BUILD);
     // Pixels of a tile that are loaded and written: 128, or in a compact launch of a 1x1 layer fewer (the MMA's other rows read what
     // the stage happens to hold and nobody reads their sums).
     const int tile_rows = COMPACT ? P.tile_rows : kTileM;
@@ -182,6 +205,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
     const uint32_t sB = base + L.b_panel, sA = base + L.a_stages;
     const uint32_t bar_full = base + L.bars, bar_empty = bar_full + 8u * P.stages, bar_b = bar_empty + 8u * P.stages;
     const uint32_t bar_tfull = bar_b + 8, bar_tempty = bar_tfull + 8u * kMaxAccBufs;
+    const uint32_t bar_ofull = bar_tempty + 8u * kMaxAccBufs, bar_ofree = bar_ofull + 8u * kOutSlots;  // (ROWS)
     const uint32_t acc_mask = (uint32_t)P.acc_bufs - 1u, acc_shift = P.acc_bufs == 4 ? 2u : 1u;  // 2 or 4 accumulators in TMEM
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + L.tmem_slot);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + L.abort_flag);
@@ -189,6 +213,9 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tile = blockIdx.x % P.n_tiles;
     const int m_first = blockIdx.x / P.n_tiles, m_step = gridDim.x / P.n_tiles;
+    // ROWS: accumulators of a pixel tile, 128 channels each, the last one of the layer 64 where that holds what is left
+    const int cols_left = s.cout_pad - n_tile * P.bn, my_cols = cols_left < P.bn ? cols_left : P.bn;
+    const int blocks = ROWS ? (my_cols + kTileM - 1) / kTileM : 1;
     const uint32_t a_stage_bytes = (uint32_t)P.a_stage_bytes, b_tile_bytes = (uint32_t)P.bn * P.bkc;
     // halo mode: the 8 pixels of one tile row are one 8-row operand group; groups (tile rows) are one halo row apart
     const int halo_w = kHaloTw + s.kw - 1, halo_h = kHaloTh + s.kh - 1;
@@ -220,7 +247,17 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
 #pragma unroll 1
         for (int i = 0; i < P.acc_bufs; ++i) {
             mbar_init(bar_tfull + 8u * i, 1);
-            mbar_init(bar_tempty + 8u * i, (uint32_t)(tile_rows + 31) / 32u * (uint32_t)((P.bn + epi_chunk(P) - 1) / epi_chunk(P)));  // one arrival per lane quarter and column chunk
+            mbar_init(bar_tempty + 8u * i, ROWS ? kTeamWarps
+                                                : (uint32_t)(tile_rows + 31) / 32u * (uint32_t)((P.bn + epi_chunk(P) - 1) / epi_chunk(P)));  // one arrival per lane quarter and column chunk
+        }
+        if constexpr (ROWS) {
+            prefetch_tensormap(&mixed.full);
+            prefetch_tensormap(&mixed.half);
+#pragma unroll 1
+            for (int i = 0; i < P.out_slots; ++i) {
+                mbar_init(bar_ofull + 8u * i, kTeamWarps);
+                mbar_init(bar_ofree + 8u * i, 1);
+            }
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -308,12 +345,28 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
             bool ok = mbar_wait(bar_b, 0, abort_flag, status, 16u, P.wait_ns);
             tc_fence_after();
             pdl_wait();  // (no wait below is counted against its limit while the previous kernel still runs)
-            uint32_t st = 0, phase = 0, tile_i = 0;
-            for (int m = m_first; ok && m < P.m_tiles; m += m_step, ++tile_i) {
+            uint32_t st = 0, phase = 0, tile_i = 0;  // (tile_i counts accumulators: ROWS has several per tile)
+            const uint32_t idesc_half = P.idesc - ((uint32_t)(kTileM >> 5) << 24);  // ROWS, 64 rows
+            for (int m = m_first; ok && m < P.m_tiles; m += m_step, tile_i += (uint32_t)blocks) {
                 const uint32_t buf = tile_i & acc_mask, use = tile_i >> acc_shift;
                 if (!mbar_wait(bar_tempty + 8u * buf, (use & 1u) ^ 1u, abort_flag, status, 4u, P.wait_ns)) { ok = false; break; }
-                tc_fence_after();
                 const uint32_t d = tmem_base + buf * (uint32_t)P.acc_stride;
+                uint32_t d1 = 0;
+                if (ROWS && blocks > 1) {
+                    const uint32_t buf1 = (tile_i + 1) & acc_mask, use1 = (tile_i + 1) >> acc_shift;
+                    if (!mbar_wait(bar_tempty + 8u * buf1, (use1 & 1u) ^ 1u, abort_flag, status, 4u, P.wait_ns)) { ok = false; break; }
+                    d1 = tmem_base + buf1 * (uint32_t)P.acc_stride;
+                }
+                tc_fence_after();
+                // pixels: the operand with the tile's pixels as rows; weights: the one with channels as rows
+                auto mma = [&](uint64_t pixels, uint64_t weights, uint32_t accumulate) {
+                    if constexpr (ROWS) {
+                        umma_i8(d, weights, pixels, blocks > 1 || my_cols > 64 ? P.idesc : idesc_half, accumulate);
+                        if (blocks > 1) umma_i8(d1, weights + ((uint32_t)(kTileM * P.bkc) >> 4), pixels, my_cols > kTileM + 64 ? P.idesc : idesc_half, accumulate);
+                    } else {
+                        umma_i8(d, pixels, weights, P.idesc, accumulate);
+                    }
+                };
                 for (int kb = 0; kb < loads_per_tile; ++kb) {
                     if (!mbar_wait(bar_full + 8u * st, phase, abort_flag, status, 2u, P.wait_ns)) { ok = false; break; }
                     tc_fence_after();
@@ -329,7 +382,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                             const uint64_t a = ((kx & 1) ? a1 : a0) + a_off;
 #pragma unroll
                             for (int j = 0; j < 4; ++j)
-                                if (j < J) umma_i8(d, a + 2u * j, b0 + b_off + 2u * j, P.idesc, (kb | ky | kx | j) != 0 ? 1u : 0u);
+                                if (j < J) mma(a + 2u * j, b0 + b_off + 2u * j, (kb | ky | kx | j) != 0 ? 1u : 0u);
                         };
                         const int J = P.bkc / 32;
                         if (s.kh == 3 && s.kw == 3) {
@@ -363,7 +416,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                                     const uint32_t ao = (uint32_t)(tap / 3) * row_step + (uint32_t)(tap % 3) * a_px_step, bo = (uint32_t)tap * b_tap_step;
 #pragma unroll
                                     for (int j = 0; j < J; ++j) {
-                                        umma_i8(d, a_hi | (uint64_t)(a_lo + ao + 2u * j), b_hi | (uint64_t)(b_lo + bo + 2u * j), P.idesc, accumulate);
+                                        mma(a_hi | (uint64_t)(a_lo + ao + 2u * j), b_hi | (uint64_t)(b_lo + bo + 2u * j), accumulate);
                                         accumulate = 1u;
                                     }
                                 }
@@ -377,7 +430,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                             for (int kx = 0; kx < s.kw; ++kx, a_off += a_px_step, b_off += b_tap_step) {
 #pragma unroll (COMPACT ? 1 : 4)
                                 for (int j = 0; j < P.bkc / 32; ++j) {
-                                    umma_i8(d, a0 + a_off + 2u * j, b0 + b_off + 2u * j, P.idesc, accumulate);
+                                    mma(a0 + a_off + 2u * j, b0 + b_off + 2u * j, accumulate);
                                     accumulate = 1u;
                                 }
                             }
@@ -393,7 +446,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                         for (int g = 0; g < P.nkb; ++g, ao += a_step, bo += b_step)
 #pragma unroll 1
                             for (int j = 0; j < P.bkc / 32; ++j)
-                                umma_i8(d, a_hi | (uint64_t)(a_lo + ao + 2u * j), b_hi | (uint64_t)(b_lo + bo + 2u * j), P.idesc, (g | j) != 0 ? 1u : 0u);
+                                mma(a_hi | (uint64_t)(a_lo + ao + 2u * j), b_hi | (uint64_t)(b_lo + bo + 2u * j), (g | j) != 0 ? 1u : 0u);
                     } else {
                         const uint64_t adesc = make_smem_desc(sA + st * a_stage_bytes, P.bkc);
                         const uint64_t bdesc = make_smem_desc(sB + kb * b_tile_bytes, P.bkc);
@@ -402,11 +455,11 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                         auto steps = [&](auto n) {
                             constexpr int J = decltype(n)::value;
 #pragma unroll
-                            for (int j = 0; j < J; ++j) umma_i8(d, a_hi | (uint64_t)(a_lo + 2u * j), b_hi | (uint64_t)(b_lo + 2u * j), P.idesc, (kb | j) != 0 ? 1u : 0u);
+                            for (int j = 0; j < J; ++j) mma(a_hi | (uint64_t)(a_lo + 2u * j), b_hi | (uint64_t)(b_lo + 2u * j), (kb | j) != 0 ? 1u : 0u);
                         };
                         if (COMPACT) {
 #pragma unroll 1
-                            for (int j = 0; j < P.bkc / 32; ++j) umma_i8(d, a_hi | (uint64_t)(a_lo + 2u * j), b_hi | (uint64_t)(b_lo + 2u * j), P.idesc, (kb | j) != 0 ? 1u : 0u);
+                            for (int j = 0; j < P.bkc / 32; ++j) mma(a_hi | (uint64_t)(a_lo + 2u * j), b_hi | (uint64_t)(b_lo + 2u * j), (kb | j) != 0 ? 1u : 0u);
                         } else if (P.bkc == 128) steps(std::integral_constant<int, 4>{});
                         else if (P.bkc == 64) steps(std::integral_constant<int, 2>{});
                         else steps(std::integral_constant<int, 1>{});
@@ -416,6 +469,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                 }
                 if (!ok) break;
                 umma_commit(bar_tfull + 8u * buf);  // accumulator complete
+                if (ROWS && blocks > 1) umma_commit(bar_tfull + 8u * ((tile_i + 1) & acc_mask));
             }
             // every accumulator read for the last time: the tensor memory can go back
             for (uint32_t b = 0; ok && b <= acc_mask && b < tile_i; ++b)
@@ -512,7 +566,121 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                 }
             }
         }
-    } else {
+    } else if (ROWS && warp == 2 + P.epi_warps) {
+        if constexpr (ROWS) {
+            if (elect_one()) {
+                // ---- finished tiles: one TMA store each (what lies outside the tensor is clipped) ----
+                pdl_wait();  // the outputs may still be read by the previous kernel
+                uint32_t unit = 0;
+                bool ok = true;
+                for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
+                    for (int blk = 0; blk < blocks; ++blk, ++unit) {
+                        const uint32_t slot = unit & ((uint32_t)P.out_slots - 1u), use = unit / (uint32_t)P.out_slots;
+                        if (!mbar_wait(bar_ofull + 8u * slot, use & 1u, abort_flag, status, 64u, P.wait_ns)) { ok = false; break; }
+                        tma_store_2d(my_cols - blk * kTileM > 64 ? &mixed.full : &mixed.half, base + L.out_slots + slot * out_slot_bytes(P),
+                                     n_tile * P.bn + blk * kTileM, m * kRowsPixels);
+                        bulk_commit();
+                        // A slot is free when its store has been read, 0.5 us after it was issued. With two slots a team waits for that; with
+                        // four the next tile's store is issued first (64 -> 256 56x56 x128: one at a time 35.4 us, two 27.7).
+                        if (P.out_slots == kOutSlots) {
+                            bulk_wait_read<1>();
+                            if (unit > 0) mbar_arrive(bar_ofree + 8u * ((unit - 1u) & (kOutSlots - 1)));
+                        } else {
+                            bulk_wait_read<0>();
+                            mbar_arrive(bar_ofree + 8u * slot);
+                        }
+                    }
+                }
+                bulk_wait_all();
+            }
+        }
+    } else if (ROWS) {
+        if constexpr (ROWS) {
+            // ---- epilogue warps, channels as rows. A team of eight (two per lane quarter) takes an accumulator; two teams take them in turn,
+            // so that a warp has one block's channels for good, and one team's arithmetic fills the other's waits ----
+            constexpr uint32_t teams = BUILD == kRowsWideBuild ? 2 : 1;
+            const int q = warp & 3, sub = ((warp - 2) >> 2) & 1;
+            const uint32_t team = teams == 2 ? (uint32_t)(warp - 2) >> 3 : 0u;
+            const int blk = blocks > 1 ? (int)team : 0;
+            const int left = my_cols - blk * kTileM;                  // channels from the block's first on
+            const int per_q = left > 64 ? 32 : 16, c0 = q * per_q;    // rows of a quarter (64-row accumulators: its first 16 lanes)
+            const bool hi = per_q == 32 && c0 + 16 < left;            // 16 channels at a time: the quarter's first, and its second
+            const uint32_t half = half_bits(ep.rounding);
+            float2 si[2][2], bi[2][2], so[2][2];  // [first / second 16][channel lane / 4, + 8], each twice: for two pixels
+            {
+                const float* sp = reinterpret_cast<const float*>(base_ptr + L.params);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int c = blk * kTileM + c0 + (per_q == 32 ? h * 16 : 0) + j * 8 + (lane >> 2);
+                        si[h][j] = make_float2(sp[c], sp[c]);
+                        bi[h][j] = make_float2(sp[P.bn + c], sp[P.bn + c]);
+                        so[h][j] = make_float2(sp[2 * P.bn + c], sp[2 * P.bn + c]);
+                    }
+            }
+            // one byte per channel and row; the 16-byte chunks of a row trade places by the row's number, as the store's swizzle has it
+            const uint32_t row_bytes = 4u * (uint32_t)per_q, swz = per_q == 32 ? (uint32_t)lane & 7u : ((uint32_t)lane >> 1) & 3u, chunk = (uint32_t)c0 >> 4;
+            const uint32_t row0 = base + L.out_slots + ((uint32_t)(sub * 64) + (uint32_t)lane) * row_bytes;
+            const uint32_t at_lo = row0 + ((chunk ^ swz) << 4), at_hi = row0 + (((chunk + 1u) ^ swz) << 4);
+            const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(sub * 64);
+            const uint32_t slot_bytes = out_slot_bytes(P), slot_mask = (uint32_t)P.out_slots - 1u, slot_shift = P.out_slots == 4 ? 2u : 1u;
+            auto emit = [&](const int (&a)[16], int h, uint32_t at) {
+                uint32_t w[4];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    float2 y[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const float2 t = __ffma2_rn(make_float2(__int2float_rn(a[4 * g + 2 * j]), __int2float_rn(a[4 * g + 2 * j + 1])), si[h][j], bi[h][j]);
+                        y[j] = __fmul2_rn(make_float2(activate_t<ACT>(t.x, ep.act_param0), activate_t<ACT>(t.y, ep.act_param0)), so[h][j]);
+                    }
+                    if constexpr (ACT == ACT_POS) {
+                        w[g] = requant4_pos(y[0], y[1], half);
+                    } else {
+                        const int2 qa = round2(y[0], half), qb = round2(y[1], half);
+                        w[g] = pack_sat_s8x4(qa.x, qa.y, qb.x, qb.y);
+                    }
+                }
+                stmatrix_t8(at, w);
+            };
+            const uint32_t units = m_first < P.m_tiles ? (uint32_t)((P.m_tiles - 1 - m_first) / m_step + 1) * (uint32_t)blocks : 0u;
+            for (uint32_t unit = team; unit < units; unit += teams) {
+                const uint32_t buf = unit & acc_mask, use = unit >> acc_shift, slot = unit & slot_mask;
+                const uint32_t taddr = t_lane + buf * (uint32_t)P.acc_stride, out_at = slot * slot_bytes;
+                if (!mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) break;
+                tc_fence_after();
+                // 32 pixels x 16 channels at a time, the next ones on their way while these are computed
+                int v[2][16];
+                if (c0 < left) tmem_ld16x256(taddr, v[0]);
+                if (!mbar_wait(bar_ofree + 8u * slot, ((unit >> slot_shift) & 1u) ^ 1u, abort_flag, status, 128u, P.wait_ns)) break;
+                tmem_wait_ld16(v[0]);
+                if (hi) {
+                    tmem_ld16x256(taddr + (16u << 16), v[1]);
+                    emit(v[0], 0, at_lo + out_at);
+                    tmem_wait_ld16(v[1]);
+                    tmem_ld16x256(taddr + 32u, v[0]);
+                    emit(v[1], 1, at_hi + out_at);
+                    tmem_wait_ld16(v[0]);
+                    tmem_ld16x256(taddr + (16u << 16) + 32u, v[1]);
+                    emit(v[0], 0, at_lo + out_at + 32u * row_bytes);
+                    tmem_wait_ld16(v[1]);
+                } else if (c0 < left) {
+                    tmem_ld16x256(taddr + 32u, v[1]);
+                    emit(v[0], 0, at_lo + out_at);
+                    tmem_wait_ld16(v[1]);
+                }
+                tc_fence_before();  // the accumulator is read
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_tempty + 8u * buf);
+                if (hi) emit(v[1], 1, at_hi + out_at + 32u * row_bytes);
+                else if (c0 < left) emit(v[1], 0, at_lo + out_at + 32u * row_bytes);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // these writes -> the TMA store's reads
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_ofull + 8u * slot);
+            }
+        }
+    } else if constexpr (!ROWS) {
         // ---- epilogue warps ----
         const int q = warp & 3;            // TMEM lane quarter this warp may read
         const int sub = (warp - 2) >> 2;   // which of the epi_warps/4 warps sharing that quarter
@@ -719,9 +887,9 @@ CUtensorMapSwizzle swizzle_for(int bkc) {
     return bkc == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (bkc == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
-template <int OUT, int ACT, int BUILD, typename Source>
+template <int OUT, int ACT, int BUILD, typename Source, typename Dest>
 const char* launch_variant(cudaStream_t stream, int sm_count, const Source& maps, const CUtensorMap& tmB, const UmmaPlan& p,
-                           const ConvShape& s, const EpilogueParams& ep, void* out, uint32_t* status, const UmmaMixedOut& mixed) {
+                           const ConvShape& s, const EpilogueParams& ep, void* out, uint32_t* status, const Dest& mixed) {
     // per-device, per-instantiation set-up; several host threads may drive different GPUs through this function at once
     static std::mutex mu;
     static bool attr_set[64] = {};
@@ -743,7 +911,7 @@ const char* launch_variant(cudaStream_t stream, int sm_count, const Source& maps
     }
     // Tiles are dealt statically to the CTAs of the grid, so a grid larger than what is resident at once runs in waves.
     // The plan bounds residency by shared memory and TMEM; registers and threads are bounded here.
-    const int threads = 64 + 32 * (p.epi_warps + (build_quantizes(BUILD) ? kQuantWarps : 0));
+    const int threads = 64 + 32 * (p.epi_warps + (build_quantizes(BUILD) ? kQuantWarps : 0) + (build_rows(BUILD) ? 1 : 0));
     const int regs_per_warp = (regs * 32 + 255) / 256 * 256;
     int resident = 65536 / (regs_per_warp * (threads / 32));
     if (resident > 2048 / threads) resident = 2048 / threads;
@@ -872,6 +1040,50 @@ std::vector<UmmaVariant> umma_variants(const UmmaPlan& widest, int cout, int sme
     UmmaVariant v;
     for (int bn : {128, 64, 32})
         if (umma_narrow_plan(widest, bn, cout, smem_budget, &v.plan)) all.push_back(v);
+    return all;
+}
+
+std::vector<UmmaVariant> umma_row_variants(const UmmaPlan& base, int cout, int smem_budget) {
+    std::vector<UmmaVariant> all;
+    const int cout_pad = nhwc_channels(cout);
+    if (base.taps != 1) return all;
+    for (int bn : {256, 192, 128, 64}) {
+        if (bn >= cout_pad + 64 || (bn == 64 && cout_pad > 64)) continue;
+        UmmaVariant v;
+        UmmaPlan& p = v.plan;
+        p = base;
+        p.rows = 1;
+        p.bn = bn;
+        p.n_tiles = (cout_pad + bn - 1) / bn;
+        p.acc_stride = kRowsPixels;
+        p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kRowsPixels >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+        // Two CTAs per SM of eight epilogue warps and two accumulators each, or one of sixteen and four: the same warps and tensor memory,
+        // but two panels, and while one CTA's warps wait for an accumulator the other's have one.
+        p.epi_warps = 8;
+        p.stages = 1;
+        p.out_slots = 2;
+        int fixed = (int)smem_layout(p).total - p.a_stage_bytes + 1024;
+        auto stages_in = [&](int budget) { return budget > fixed ? (budget - fixed - 192 /*barriers of further stages*/) / p.a_stage_bytes : 0; };
+        const int most = p.gather_whole ? 2 : p.halo ? 3 : p.nkb <= 2 ? 4 : 8;
+        const bool pair = bn <= kTileM && stages_in(smem_budget / 2) >= 2;
+        p.ctas_per_sm = pair ? 2 : 1;
+        p.stages = stages_in(smem_budget / p.ctas_per_sm);
+        // two finished tiles per team, if three (of a tile in several loads: four) stages remain
+        if (!pair && stages_in(smem_budget - 2 * (int)out_slot_bytes(p)) >= (p.nkb > 1 && !p.gather_whole ? 4 : 3)) {
+            p.out_slots = 4;
+            fixed += 2 * (int)out_slot_bytes(p);
+            p.stages = stages_in(smem_budget);
+        }
+        if (p.stages > most) p.stages = most;
+        if (p.stages < 2) continue;
+        p.acc_bufs = pair ? 2 : 4;
+        p.tmem_cols = p.acc_bufs * p.acc_stride;
+        p.epi_warps = pair ? 8 : 16;
+        p.smem_bytes = (int)smem_layout(p).total + 1024;
+        const int min_smem = smem_budget / (p.ctas_per_sm + 1) + 1;  // (no more CTAs than tensor memory serves, see plan_panel)
+        if (p.smem_bytes < min_smem) p.smem_bytes = min_smem;
+        all.push_back(v);
+    }
     return all;
 }
 
@@ -1053,6 +1265,37 @@ UmmaChoice umma_choose(const UmmaVariant* v, int n, const ConvShape& s, int sm_c
     return c;
 }
 
+// Channels as accumulator rows (the two builds at the end of the comment in front of the kernel). What they gain is the epilogue; an
+// MMA of 128 channels x 128 pixels reads as many bytes of shared memory as its port delivers in the time it takes, one of 128 pixels x
+// 256 channels three quarters of them, so with more input channels the order of the operands that keeps the port free is the better one.
+// us, pixels as rows / channels as rows: 64 -> 256 56x56 x128 41.8 / 26.0, 256 -> 512 28x28 x128 23.9 / 18.5, 116 -> 116 20x20 x256 9.3 / 6.5,
+// 58 -> 58 40x40 x256 14.2 / 11.0, 512 -> 1024 28x28 x32 17.3 / 15.4; 110 layers of 24 to 1024 channels: up to 256 input channels 1.0 to 1.45
+// times as fast, 512 and 64 or whole panels of 256 output channels 1.05 to 1.15, else slower (323 -> 387, 369 tiles 14.2 / 21.9; 587 -> 86, 556
+// tiles 9.8 / 11.6). An accumulator is 128 or 64 channels, and what a layer does not fill is computed all the same: up to two fifths
+// more (73 -> 87, 1608 tiles 13.6 / 12.2; but 43 -> 25, 916 tiles 6.3 / 6.8). The panel that wastes least; among equals the widest, which fetches
+// the pixels fewest times (256 -> 512: 256 channels 18.4, 128 21.1), but up to four rounds of CTAs two small CTAs per SM (112 -> 250, 542
+// tiles 8.6 / 8.0; 232 -> 232, 200 tiles 6.5 / 5.9). Small launches keep their narrow panels of pixels. k x k layers read every pixel
+// once per tap and are bound by the MMAs: 192 of them 0.77 times as fast.
+UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count) {
+    const PixelTiles t = tile_pixels(choice.variant->plan, s);
+    if (choice.inside || choice.compact || !t.flat || (choice.variant->plan.bn <= 64 && t.tiles <= sm_count)) return choice;
+    const UmmaVariant* pick = nullptr;
+    int pick_work = 0;
+    for (int i = 0; i < n_rows; ++i) {
+        const UmmaPlan& p = rows[i].plan;
+        const int widest = s.cout_pad < p.bn ? s.cout_pad : p.bn, work = p.n_tiles * ((widest + 63) / 64);
+        const bool light = p.k_total <= 256;
+        if (64 * work * (light ? 5 : 7) > s.cout_pad * (light ? 7 : 8)) continue;
+        if (p.k_total > 512 || (!light && p.bn % 256 != 0 && p.bn != 64)) continue;
+        if (pick && work >= pick_work && !(work == pick_work && light && p.bn == kTileM && t.tiles * pick->plan.n_tiles < 4l * sm_count)) continue;
+        pick = &rows[i];
+        pick_work = work;
+    }
+    UmmaChoice c = choice;
+    if (pick) c.variant = pick;
+    return c;
+}
+
 const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaChoice& choice, const ConvShape& s,
                               const int8_t* x, const EpilogueParams& ep, void* out, int out_dtype, uint32_t* status,
                               const UmmaSources* sources, const UmmaMixedOut* mixed_in, unsigned long long wait_limit_ns, const UmmaFloatInput* f32) {
@@ -1174,6 +1417,23 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaChoic
         p.tmem_cols = p.acc_stride;
         err = f32 ? launch_variant<kAnyOut, kAnyAct, kCompactQuantBuild>(stream, sm_count, qs, tmB, p, s, ep, out, status, mixed)
                   : launch_variant<kAnyOut, kAnyAct, kCompactBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed);
+    } else if (p.rows) {
+        if (mixed_in || out_dtype != DT_S8_NHWC || !flat) return "a launch with channels as accumulator rows is a 1x1 layer with one int8 output";
+        RowsOut to;
+        cuuint64_t dims[2] = {(cuuint64_t)s.cout_pad, (cuuint64_t)pixels}, strides[1] = {(cuuint64_t)s.cout_pad};
+        for (int width : {128, 64}) {
+            cuuint32_t box[2] = {(cuuint32_t)width, (cuuint32_t)kRowsPixels}, one[2] = {1, 1};
+            if (enc(width == 128 ? &to.full : &to.half, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, out, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    swizzle_for(width), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                return "cuTensorMapEncodeTiled(output) failed";
+        }
+#define OTT_ROWS_LAUNCH(ACT)                                                                                                                 err = p.ctas_per_sm > 1 ? launch_variant<DT_S8_NHWC, ACT, kRowsBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, to)                             : launch_variant<DT_S8_NHWC, ACT, kRowsWideBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, to)
+        if (ep.int8_pos) OTT_ROWS_LAUNCH(ACT_POS);
+        else if (ep.act_type == ACT_RELU) OTT_ROWS_LAUNCH(ACT_RELU);
+        else if (ep.act_type == ACT_LRELU) OTT_ROWS_LAUNCH(ACT_LRELU);
+        else if (ep.act_type == ACT_RELU6) OTT_ROWS_LAUNCH(ACT_RELU6);
+        else OTT_ROWS_LAUNCH(ACT_NONE);
+#undef OTT_ROWS_LAUNCH
     } else if (out_dtype == DT_S32_NHWC) {
         OTT_UMMA_LAUNCH(DT_S32_NHWC, ACT_NONE);
     } else if (out_dtype == DT_F32_NCHW) {

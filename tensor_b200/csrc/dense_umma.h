@@ -21,6 +21,9 @@ struct UmmaPlan {
     int smem_bytes;  // dynamic shared memory of the launch
     int epi_warps;   // epilogue warps per CTA: 8 or 16
     int ctas_per_sm; // resident CTAs per SM the launch is sized for (limited by TMEM columns and shared memory)
+    int rows;        // int8 output with channels as accumulator rows: bn channels in accumulators of 128 (the last one 64 where that is enough)
+                     // x 128 pixels, see dense_umma.cu
+    int out_slots;   // rows: finished tiles on their way out, 2 or 4
     // per call
     int compact;     // the compact build runs it
     int out_kind;    // DT_ of the output
@@ -55,6 +58,8 @@ struct UmmaVariant {
     alignas(128) unsigned char weight_map[128];
 };
 std::vector<UmmaVariant> umma_variants(const UmmaPlan& widest, int cout, int smem_budget);  // weight maps not filled in
+// The same layer with channels as accumulator rows, the panels for long launches first; empty where nothing fits.
+std::vector<UmmaVariant> umma_row_variants(const UmmaPlan& base, int cout, int smem_budget);
 
 // A 1x1 layer whose input channels are spread over several int8 NHWC tensors (each written by one producer layer): K block
 // kb of the implicit GEMM is the 32 channels starting at block_x[kb] of tensor block_src[kb]. The layer's weights are laid
@@ -112,6 +117,8 @@ struct UmmaChoice {
     bool compact;
 };
 UmmaChoice umma_choose(const UmmaVariant* variants, int n_variants, const ConvShape& s, int sm_count, bool may_quantize, long* tiles = nullptr);
+// For an int8 launch without side outputs: the choice, or the same call with channels as accumulator rows.
+UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count);
 
 // Launch. Returns NULL or an error text.
 // sources: NULL, or where the K blocks of a plan with gather > 0 come from (x is then unused). mixed: NULL, or the fp32 side

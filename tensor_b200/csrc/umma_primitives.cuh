@@ -148,5 +148,31 @@ __device__ __forceinline__ void tmem_wait_ld16(int v[16]) {
                  : "memory");
 }
 
+// 16 lanes x 32 consecutive TMEM columns: thread t gets lanes t / 4 and t / 4 + 8, of every 8 columns 2 (t % 4) and the next:
+// v[4 g + 2 j + i] = lane t / 4 + 8 j, column 8 g + 2 (t % 4) + i.
+__device__ __forceinline__ void tmem_ld16x256(uint32_t taddr, int v[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+// Four 16 x 8 byte matrices, transposed on their way: word g of thread t holds (from byte 0) rows t / 4, t / 4 and t / 4 + 8, t / 4 + 8 of matrix g,
+// columns 2 (t % 4) and the next of each; column c of matrix g becomes the 16 bytes at the address that lane 8 g + c names.
+__device__ __forceinline__ void stmatrix_t8(uint32_t row_addr, const uint32_t (&w)[4]) {
+    asm volatile("stmatrix.sync.aligned.m16n8.x4.trans.shared.b8 [%0], {%1, %2, %3, %4};" ::"r"(row_addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+}
+
+// TMA store of a tile in shared memory, and the thread's own groups of such stores.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(src), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 }  // namespace umma
 }  // namespace ottk

@@ -1,0 +1,49 @@
+"""GPU: int8 launches of the dense tensor-core kernel with output channels as accumulator rows, bit for bit against the CPU checker: one
+and several accumulators per panel, 64-row ones, several panels, ragged last tiles, and every epilogue."""
+import numpy as np
+import pytest
+
+from support import ACT_LRELU, ACT_NONE, ACT_RELU, ACT_RELU6, ROUND_ADD_HALF_TRUNC, ROUND_HALF_AWAY, ConvCase, run_port
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from tensor_b200 import Context
+    with Context(0) as c:
+        yield c
+
+
+def _check(ctx, case, rounding=ROUND_ADD_HALF_TRUNC, scale=None):
+    from gpu_support import bits, run_gpu
+    case.make()
+    if scale is not None:
+        case.out_scales = scale
+    got, want = run_gpu(ctx, case, rounding, want_acc=False), run_port(case, rounding, want_acc=False)
+    assert np.array_equal(bits(got["y"]), bits(want["y"]))
+    assert not got["y_pad"].any()
+
+
+def _case(cin, cout, n, h, w, act):
+    return ConvCase(f"rows_{cin}_{cout}", cin, cout, 1, 1, 0, n=n, h=h, w=w, bias_term=1, int8_scale_term=101, act_type=act, act_param0=0.1, s8_input=True,
+                    w_std=0.5, seed=cin + cout)
+
+
+@pytest.mark.parametrize("cin,cout,panels", [(58, 58, (64, 64)), (340, 64, (64, 64)), (64, 96, (128, 128)), (116, 116, (128, 128)), (96, 176, (192, 192)),
+                                             (128, 192, (192, 192)), (232, 232, (128, 256)), (40, 352, (128, 192)), (200, 464, (128, 256)), (512, 480, (256, 256)),
+                                             (130, 992, (256, 256))])
+def test_pointwise(ctx, cin, cout, panels):
+    for n, panel in zip((7, 41), panels):  # 177 and 1036 tiles, the last one ragged: about one and seven per CTA
+        assert ctx.lib.ott_debug_dense_rows(cin, cout, n, 61, 53, 148) == panel
+        _check(ctx, _case(cin, cout, n, 61, 53, ACT_RELU))
+
+
+@pytest.mark.parametrize("act", [ACT_NONE, ACT_RELU, ACT_LRELU, ACT_RELU6])
+@pytest.mark.parametrize("scale", [0.2, 21.25, 3e6, -0.3])  # the third leaves 16 bits
+def test_epilogues(ctx, act, scale):
+    for rounding, per_channel in ((ROUND_ADD_HALF_TRUNC, False), (ROUND_HALF_AWAY, True)):
+        cout = 180
+        assert ctx.lib.ott_debug_dense_rows(64, cout, 7, 61, 53, 148) == 192
+        s = (scale * np.linspace(0.97, 1.03, cout)).astype(np.float32) if per_channel else np.full(1, scale, np.float32)
+        _check(ctx, _case(64, cout, 7, 61, 53, act), rounding, s)
