@@ -879,7 +879,7 @@ int ott_debug_dense_rows(int cin, int cout, int n, int h, int w, int sm_count) {
     ConvShape s{};
     s.n = n; s.h = s.oh = h; s.w = s.ow = w; s.cin = cin; s.cout = cout; s.cin_pad = nhwc_channels(cin); s.cout_pad = nhwc_channels(cout);
     s.kh = s.kw = s.sh = s.sw = s.dh = s.dw = 1;
-    const UmmaChoice c = umma_choose_rows(umma_choose(all.data(), (int)all.size(), s, sm_count, false), rows.data(), (int)rows.size(), s, sm_count);
+    const UmmaChoice c = umma_choose_rows(umma_choose(all.data(), (int)all.size(), s, sm_count, false), rows.data(), (int)rows.size(), s, sm_count, false);
     return c.variant->plan.rows ? c.variant->plan.bn : 0;
 }
 
@@ -1220,7 +1220,8 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
         const std::vector<UmmaVariant>& form = parity ? c->umma_parity : c->umma;
         choice = umma_choose(form.data(), (int)form.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW && c->n_in_scales == 1 &&
                              umma_float_input(static_cast<const float*>(in_dev), gather, d.cin, (long)h * w, c->in_scale0, &f32));
-        if (in_dtype == OTT_S8_NHWC && out_dtype == OTT_S8_NHWC && !mixed) choice = umma_choose_rows(choice, c->umma_rows.data(), (int)c->umma_rows.size(), s, ctx->sm_count);
+        if (out_dtype == OTT_S8_NHWC && !mixed)
+            choice = umma_choose_rows(choice, c->umma_rows.data(), (int)c->umma_rows.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW);
     }
     const bool quant_inside = choice.inside;
     if (in_dtype == OTT_F32_NCHW) {

@@ -215,7 +215,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
     const int m_first = blockIdx.x / P.n_tiles, m_step = gridDim.x / P.n_tiles;
     // ROWS: accumulators of a pixel tile, 128 channels each, the last one of the layer 64 where that holds what is left
     const int cols_left = s.cout_pad - n_tile * P.bn, my_cols = cols_left < P.bn ? cols_left : P.bn;
-    const int blocks = ROWS ? (my_cols + kTileM - 1) / kTileM : 1;
+    const int blocks = BUILD == kRowsWideBuild ? (my_cols + kTileM - 1) / kTileM : 1;
     const uint32_t a_stage_bytes = (uint32_t)P.a_stage_bytes, b_tile_bytes = (uint32_t)P.bn * P.bkc;
     // halo mode: the 8 pixels of one tile row are one 8-row operand group; groups (tile rows) are one halo row apart
     const int halo_w = kHaloTw + s.kw - 1, halo_h = kHaloTh + s.kh - 1;
@@ -231,7 +231,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                      "r"((uint32_t)P.tmem_cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        pdl_launch_dependents();
+        if (!ROWS || !P.late) pdl_launch_dependents();
     }
     if (threadIdx.x == 0) {
         prefetch_tensormap(&tmB);
@@ -251,8 +251,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                                                 : (uint32_t)(tile_rows + 31) / 32u * (uint32_t)((P.bn + epi_chunk(P) - 1) / epi_chunk(P)));  // one arrival per lane quarter and column chunk
         }
         if constexpr (ROWS) {
-            prefetch_tensormap(&mixed.full);
-            prefetch_tensormap(&mixed.half);
+            prefetch_tensormap(my_cols > 64 ? &mixed.full : &mixed.half);
 #pragma unroll 1
             for (int i = 0; i < P.out_slots; ++i) {
                 mbar_init(bar_ofull + 8u * i, kTeamWarps);
@@ -317,10 +316,10 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                     } else if (P.gather) {
                         // K block kb = 32 channels of one of the source tensors (channels past that tensor's end arrive as zeros)
                         tma_load_4d(&maps.tm[maps.block_src[kb]], full, dst, (int)maps.block_x[kb], x0, 0, 0);
-                    } else if (!COMPACT && P.halo == 2) {
+                    } else if (!COMPACT && !ROWS && P.halo == 2) {
                         tma_load_4d(&maps.tm[0], full, dst, kb * P.bkc, x0, y0, img);
                         tma_load_4d(&maps.tm[1], full, dst + parity.second(P.bkc), kb * P.bkc, x0 + 1, y0, img);
-                    } else if (P.halo) {
+                    } else if (!ROWS && P.halo) {
                         // the (8 + kw - 1) x (16 + kh - 1) pixels under the tile, one channel block; out-of-image pixels arrive as zeros
                         tma_load_4d(&maps.tm[0], full, dst, kb * P.bkc, x0, y0, img);
                     } else {
@@ -370,7 +369,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                 for (int kb = 0; kb < loads_per_tile; ++kb) {
                     if (!mbar_wait(bar_full + 8u * st, phase, abort_flag, status, 2u, P.wait_ns)) { ok = false; break; }
                     tc_fence_after();
-                    if (!COMPACT && !QUANT && P.halo == 2) {
+                    if (!COMPACT && !QUANT && !ROWS && P.halo == 2) {
                         // a tap of column kx reads plane kx & 1, from column kx >> 1 on
                         const uint32_t tile = sA + st * a_stage_bytes, px_step = (uint32_t)P.bkc >> 4;
                         const uint64_t a0 = make_smem_desc(tile, P.bkc, 2 * parity.cols[0] * P.bkc);
@@ -395,7 +394,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                                 if (++kx == s.kw) { kx = 0; ++ky; }
                             }
                         }
-                    } else if (P.halo) {
+                    } else if (!ROWS && P.halo) {
                         // every filter tap reads the same halo tile through a view shifted by (ky, kx) pixels
                         // (one thread issues all of these back to back, so the per-tap descriptors are the base descriptors plus
                         // an offset in their 16-byte address field, not rebuilt from scratch)
@@ -1240,7 +1239,7 @@ UmmaChoice umma_choose(const UmmaVariant* v, int n, const ConvShape& s, int sm_c
     const PixelTiles t = tile_pixels(v[0].plan, s);
     if (n_tiles) *n_tiles = t.tiles;
     const long pixels = (long)s.n * s.oh * s.ow;
-    UmmaChoice c{v + pick_panels(v, n, t.tiles, sm_count), false, kTileM, false};
+    UmmaChoice c{v + pick_panels(v, n, t.tiles, sm_count), false, kTileM, false, false};
     const bool can = may_quantize && (t.flat || v[0].plan.halo == 1) && s.cin_pad > 32 && (double)s.n * s.h * s.w <= 2147483647.0;
     if (can && !t.flat && v[0].plan.ncb == 1 && s.cin_pad <= 64 && t.tiles * v[0].plan.n_tiles <= sm_count) {
         c.variant = v;
@@ -1274,9 +1273,13 @@ UmmaChoice umma_choose(const UmmaVariant* v, int n, const ConvShape& s, int sm_c
 // tiles 9.8 / 11.6). An accumulator is 128 or 64 channels, and what a layer does not fill is computed all the same: up to two fifths
 // more (73 -> 87, 1608 tiles 13.6 / 12.2; but 43 -> 25, 916 tiles 6.3 / 6.8). The panel that wastes least; among equals the widest, which fetches
 // the pixels fewest times (256 -> 512: 256 channels 18.4, 128 21.1), but up to four rounds of CTAs two small CTAs per SM (112 -> 250, 542
-// tiles 8.6 / 8.0; 232 -> 232, 200 tiles 6.5 / 5.9). Small launches keep their narrow panels of pixels. k x k layers read every pixel
-// once per tap and are bound by the MMAs: 192 of them 0.77 times as fast.
-UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count) {
+// tiles 8.6 / 8.0; 232 -> 232, 200 tiles 6.5 / 5.9). Small launches keep their narrow panels of pixels. k x k layers read every pixel once per
+// tap and are bound by the MMAs: 192 of them 0.77 times as fast.
+// fp32 input that a quantize kernel brings: the kernel behind this one is likely another of its kind, and then starts better when this one
+// ends than as soon as there is room beside it (us, beside / at the end: 256 -> 512 28x28 x128 54.9 / 44.1, 307 -> 490 102648 pixels 65.9 /
+// 54.1, 473 -> 903 29520 pixels 35.1 / 30.9, 116 -> 974 6831 pixels 9.2 / 7.9; of up to 64 channels 45 -> 330 10260 pixels 6.7 / 7.5, 34 -> 473
+// 16640 pixels 8.7 / 9.4).
+UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count, bool f32_input) {
     const PixelTiles t = tile_pixels(choice.variant->plan, s);
     if (choice.inside || choice.compact || !t.flat || (choice.variant->plan.bn <= 64 && t.tiles <= sm_count)) return choice;
     const UmmaVariant* pick = nullptr;
@@ -1292,7 +1295,10 @@ UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, i
         pick_work = work;
     }
     UmmaChoice c = choice;
-    if (pick) c.variant = pick;
+    if (pick) {
+        c.variant = pick;
+        c.late = f32_input && pick->plan.k_total > 64;
+    }
     return c;
 }
 
@@ -1308,6 +1314,7 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaChoic
     const PixelTiles tiles = tile_pixels(p, s);
     p.flat = tiles.flat; p.tw = tiles.tw; p.th = tiles.th; p.tiles_x = tiles.x; p.tiles_y = tiles.y; p.m_tiles = (int)tiles.tiles;
     p.tile_rows = choice.tile_rows;
+    p.late = choice.late ? 1 : 0;
     if (p.tile_rows != kTileM) p.m_tiles = p.tiles_x = (int)((pixels + p.tile_rows - 1) / p.tile_rows);
     const bool flat = p.flat != 0;
     KernelMaps km;  // only the entries the plan uses are filled in
@@ -1419,9 +1426,14 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaChoic
                   : launch_variant<kAnyOut, kAnyAct, kCompactBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, mixed);
     } else if (p.rows) {
         if (mixed_in || out_dtype != DT_S8_NHWC || !flat) return "a launch with channels as accumulator rows is a 1x1 layer with one int8 output";
-        RowsOut to;
+        RowsOut to{};
+        // which of the two some panel's accumulators want (a map costs the host 0.2 us)
+        const int last = s.cout_pad - (p.n_tiles - 1) * p.bn;
+        auto ends_in_64 = [](int cols) { return (cols - 1) % kTileM < 64; };
+        const bool want_64 = ends_in_64(last) || (p.n_tiles > 1 && ends_in_64(p.bn)), want_128 = last > 64 || (p.n_tiles > 1 && p.bn > 64);
         cuuint64_t dims[2] = {(cuuint64_t)s.cout_pad, (cuuint64_t)pixels}, strides[1] = {(cuuint64_t)s.cout_pad};
         for (int width : {128, 64}) {
+            if (!(width == 64 ? want_64 : want_128)) continue;
             cuuint32_t box[2] = {(cuuint32_t)width, (cuuint32_t)kRowsPixels}, one[2] = {1, 1};
             if (enc(width == 128 ? &to.full : &to.half, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, out, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle_for(width), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)

@@ -26,6 +26,7 @@ struct UmmaPlan {
     int out_slots;   // rows: finished tiles on their way out, 2 or 4
     // per call
     int compact;     // the compact build runs it
+    int late;        // the next kernel is not to start beside this one
     int out_kind;    // DT_ of the output
     int halo;        // k x k layers: one TMA box per pixel tile and channel block holds the tile plus its halo; the taps read shifted views.
                      // 2: stride 2, one box per column parity
@@ -115,10 +116,11 @@ struct UmmaChoice {
     bool inside;
     int tile_rows;
     bool compact;
+    bool late;  // see umma_choose_rows
 };
 UmmaChoice umma_choose(const UmmaVariant* variants, int n_variants, const ConvShape& s, int sm_count, bool may_quantize, long* tiles = nullptr);
 // For an int8 launch without side outputs: the choice, or the same call with channels as accumulator rows.
-UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count);
+UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count, bool f32_input);
 
 // Launch. Returns NULL or an error text.
 // sources: NULL, or where the K blocks of a plan with gather > 0 come from (x is then unused). mixed: NULL, or the fp32 side
