@@ -97,9 +97,9 @@ int ott_debug_fail_alloc_after(ott_ctx* ctx, int n);
  * build, pixels per tile, halo form (0: one load per tap, 1: halo tiles, 2: one halo tile per column parity). OTT_ERR_UNSUPPORTED:
  * the layer does not run there. */
 int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int w, int f32_input, int sm_count, int plan[8]);
-/* The same question for an int8 to int8 1x1 layer: the output channels of a weight panel if the launch has channels as accumulator rows,
- * 0 if it has pixels as rows. */
-int ott_debug_dense_rows(int cin, int cout, int n, int h, int w, int sm_count);
+/* The same question for a 1x1 layer with int8 output: the output channels of a weight panel if the launch has channels as accumulator
+ * rows, 0 if it has pixels as rows. */
+int ott_debug_dense_rows(int cin, int cout, int n, int h, int w, int f32_input, int sm_count);
 /* Guard bands, the tests' stand-in for a device memory checker: after ott_debug_guard_bands(ctx, bytes) every block the
  * context's allocator obtains from the driver carries `bytes` (rounded up to 512) of a fill pattern on both sides;
  * ott_debug_check_guards synchronizes the stream, reads every band of every block (in use or cached) back and returns

@@ -42,7 +42,7 @@ SIGNATURES = {
     "ott_set_depthwise_tensor_cores": (i32, [vp, i32]),
     "ott_debug_fail_alloc_after": (i32, [vp, i32]),
     "ott_debug_dense_plan": (i32, [i32, i32, i32, i32, i32, i32, i32, i32, i32, vp]),
-    "ott_debug_dense_rows": (i32, [i32, i32, i32, i32, i32, i32]),
+    "ott_debug_dense_rows": (i32, [i32, i32, i32, i32, i32, i32, i32]),
     "ott_debug_guard_bands": (i32, [vp, C.c_size_t]),
     "ott_debug_check_guards": (i32, [vp, C.POINTER(C.c_long)]),
     "ott_malloc": (i32, [vp, sz, C.POINTER(vp)]),

@@ -870,7 +870,7 @@ int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int
     return OTT_OK;
 }
 
-int ott_debug_dense_rows(int cin, int cout, int n, int h, int w, int sm_count) {
+int ott_debug_dense_rows(int cin, int cout, int n, int h, int w, int f32_input, int sm_count) {
     if (cin < 1 || cout < 1 || n < 1 || h < 1 || w < 1 || sm_count < 1) return OTT_ERR_INVALID;
     constexpr int kSmemOptin = 227 * 1024;
     UmmaPlan widest{};
@@ -879,7 +879,8 @@ int ott_debug_dense_rows(int cin, int cout, int n, int h, int w, int sm_count) {
     ConvShape s{};
     s.n = n; s.h = s.oh = h; s.w = s.ow = w; s.cin = cin; s.cout = cout; s.cin_pad = nhwc_channels(cin); s.cout_pad = nhwc_channels(cout);
     s.kh = s.kw = s.sh = s.sw = s.dh = s.dw = 1;
-    const UmmaChoice c = umma_choose_rows(umma_choose(all.data(), (int)all.size(), s, sm_count, false), rows.data(), (int)rows.size(), s, sm_count, false);
+    const bool f32 = f32_input != 0;
+    const UmmaChoice c = umma_choose_rows(umma_choose(all.data(), (int)all.size(), s, sm_count, f32), rows.data(), (int)rows.size(), s, sm_count, f32, f32 && (long)h * w % 4 == 0);
     return c.variant->plan.rows ? c.variant->plan.bn : 0;
 }
 
@@ -1218,10 +1219,12 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
     if (c->kind == OTT_KERNEL_DENSE_UMMA) {
         const bool parity = !c->umma_parity.empty() && umma_prefers_parity(c->umma_parity.data(), (int)c->umma_parity.size(), c->umma.data(), s, ctx->sm_count);
         const std::vector<UmmaVariant>& form = parity ? c->umma_parity : c->umma;
-        choice = umma_choose(form.data(), (int)form.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW && c->n_in_scales == 1 &&
-                             umma_float_input(static_cast<const float*>(in_dev), gather, d.cin, (long)h * w, c->in_scale0, &f32));
+        const bool may_quantize = in_dtype == OTT_F32_NCHW && c->n_in_scales == 1 &&
+                                  umma_float_input(static_cast<const float*>(in_dev), gather, d.cin, (long)h * w, c->in_scale0, &f32);
+        choice = umma_choose(form.data(), (int)form.size(), s, ctx->sm_count, may_quantize);
         if (out_dtype == OTT_S8_NHWC && !mixed)
-            choice = umma_choose_rows(choice, c->umma_rows.data(), (int)c->umma_rows.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW);
+            choice = umma_choose_rows(choice, c->umma_rows.data(), (int)c->umma_rows.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW,
+                                      may_quantize && umma_box_input(f32, (long)h * w));
     }
     const bool quant_inside = choice.inside;
     if (in_dtype == OTT_F32_NCHW) {

@@ -44,7 +44,7 @@ namespace {
 constexpr int kMaxEpiWarps = 8;                     // 2 per TMEM lane quarter
 constexpr int kMaxThreads = 64 + 32 * kMaxEpiWarps;  // UmmaPlan::epi_warps is 4 or 8 (16 in the wide-tile build)
 constexpr int kTileM = 128;
-constexpr int kMaxAccBufs = 4;
+constexpr int kMaxAccBufs = 8;
 constexpr uint32_t kHalfSm = 113 * 1024;  // shared memory of a CTA that leaves room for another like it
 constexpr int kHaloTw = 8, kHaloTh = 16;  // pixel tile of the halo mode: 8 wide so that a tile row is one 8-row operand group
 using namespace umma;
@@ -67,15 +67,22 @@ constexpr int kOneScale = 8;
 // compact: the same layer over and over 2.57 / 2.65, two activations in turn 3.20 / 2.63, five builds in turn 4.07 / 2.63.
 constexpr int kAnyOut = 7, kAnyAct = 7;
 constexpr int kCompactBuild = 4, kCompactQuantBuild = 5;
-constexpr __host__ __device__ bool build_quantizes(int build) { return build == 3 || build == kCompactQuantBuild; }
+// Builds whose accumulator rows are output channels (int8 output): see UmmaPlan::rows. Two CTAs per SM, one with sixteen epilogue warps, or
+// one that quantizes fp32 input.
+constexpr int kRowsBuild = 6, kRowsWideBuild = 7, kRowsQuantBuild = 8;
+constexpr __host__ __device__ bool build_rows(int build) { return build == kRowsBuild || build == kRowsWideBuild || build == kRowsQuantBuild; }
+constexpr __host__ __device__ bool build_quantizes(int build) { return build == 3 || build == kCompactQuantBuild || build == kRowsQuantBuild; }
 constexpr int kQuantBuild = 3, kQuantWarps = 8, kQuantRuns = 2;
-// Builds whose accumulator rows are output channels (int8 output): see UmmaPlan::rows. Two CTAs per SM, or one with sixteen epilogue warps.
-constexpr int kRowsBuild = 6, kRowsWideBuild = 7;
-constexpr __host__ __device__ bool build_rows(int build) { return build == kRowsBuild || build == kRowsWideBuild; }
-constexpr int kRowsPixels = 128, kOutSlots = 4;  // pixels (accumulator columns) of a tile; finished tiles on their way out, at most
-constexpr uint32_t kTeamWarps = 8;               // epilogue warps that share an accumulator
+constexpr int kOutSlots = 4;  // finished tiles on their way out, at most
+// pixels (accumulator columns) of a tile, and epilogue warps that share an accumulator: 64 of either's results per thread
+constexpr __host__ __device__ int rows_pixels(int build) { return build == kRowsQuantBuild ? 64 : 128; }
+constexpr __host__ __device__ int team_warps(int build) { return rows_pixels(build) / 16; }
+constexpr int kRowsMaxBlocks = 4;
+// kRowsQuantBuild: quantizing warps, and the boxes of fp32 planes that they read, 16 channels x 64 pixels each
+constexpr int kBoxWarps = 10, kBoxChannels = 16;
+constexpr uint32_t kBoxBytes = 4096;
 constexpr __host__ __device__ int build_threads(int build) {
-    return build == 2 || build_quantizes(build) ? 64 + 32 * 16 : build == kRowsWideBuild ? 96 + 32 * 16 : build == kRowsBuild ? 96 + 32 * 8 : kMaxThreads;
+    return build == kRowsQuantBuild ? 96 + 32 * (8 + kBoxWarps) : build == kRowsWideBuild ? 96 + 32 * 16 : build == kRowsBuild ? 96 + 32 * 8 : build == 2 || build_quantizes(build) ? 64 + 32 * 16 : kMaxThreads;
 }
 
 // fp32 input of a launch that quantizes on the way in (kQuantBuild)
@@ -127,6 +134,32 @@ __device__ __forceinline__ void quantize16(uint32_t addr, const float (&v)[16], 
     store_chunk(addr, w[0], w[1], w[2], w[3]);
 }
 
+// kRowsQuantBuild: the fp32 planes as a tensor [image][channel][pixel]
+struct BoxSource {
+    CUtensorMap x;
+    float scale;
+    uint32_t half;
+};
+template <int BUILD>
+using InputOf = std::conditional_t<BUILD == kRowsQuantBuild, BoxSource, std::conditional_t<build_quantizes(BUILD), QuantSource, KernelMaps>>;
+
+// Four pixels of 16 channels -> chunk `chunk` of rows row .. row + 3 of an operand tile.
+__device__ __forceinline__ void quantize_quad(const float4 (&v)[16], uint32_t tile, int bkc, int row, int chunk, const QuantSource& Q) {
+    uint32_t w[4][4];  // [group of four channels][pixel]
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        uint32_t cw[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 f = v[4 * g + j];
+            cw[j] = quantize4_pack(f.x, f.y, f.z, f.w, Q.scale, Q.half);
+        }
+        transpose4x4(cw[0], cw[1], cw[2], cw[3], w[g]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) store_chunk(operand_chunk(tile, bkc, row + j, chunk), w[0][j], w[1][j], w[2][j], w[3][j]);
+}
+
 // Stride-2 halo (UmmaPlan::halo == 2): the input columns under a pixel tile as two planes, one per parity, every row of each. The 8
 // pixels of a tile row are then 8 neighbours of the plane that a tap reads, and tile rows are two plane rows apart.
 struct ParityHalo {
@@ -141,23 +174,24 @@ struct ParityHalo {
 __host__ __device__ __forceinline__ int epi_chunk(const UmmaPlan& p) { return p.bn <= 32 || p.compact ? 16 : 32; }
 
 struct SmemLayout {
-    uint32_t b_panel, a_stages, out_slots, bars, tmem_slot, abort_flag, params, total;
+    uint32_t b_panel, a_stages, out_slots, floats, bars, tmem_slot, abort_flag, params, total;
 };
 
 // ROWS: where finished accumulators of 128 and of 64 channels go.
 struct RowsOut {
     CUtensorMap full, half;
 };
-__host__ __device__ __forceinline__ uint32_t out_slot_bytes(const UmmaPlan& p) { return kRowsPixels * (p.bn <= 64 ? 64u : 128u); }
+__host__ __device__ __forceinline__ uint32_t out_slot_bytes(const UmmaPlan& p) { return (uint32_t)p.rows * (p.bn <= 64 ? 64u : 128u); }
 
 __host__ __device__ inline SmemLayout smem_layout(const UmmaPlan& p) {
     SmemLayout L;
     L.b_panel = 0;
     L.a_stages = (uint32_t)p.nkb * p.bn * p.bkc;
     L.out_slots = L.a_stages + (uint32_t)p.stages * (uint32_t)p.a_stage_bytes;
-    L.bars = L.out_slots + (p.rows ? (uint32_t)p.out_slots * out_slot_bytes(p) : 0u);
-    // barriers: full[stages], empty[stages], b_full, tmem_full[kMaxAccBufs], tmem_empty[kMaxAccBufs], out_full[kOutSlots], out_free[kOutSlots]
-    L.tmem_slot = L.bars + 8u * (2u * p.stages + 1u + 2u * kMaxAccBufs + (p.rows ? 2u * kOutSlots : 0u));
+    L.floats = L.out_slots + (p.rows ? (uint32_t)p.out_slots * out_slot_bytes(p) : 0u);
+    L.bars = L.floats + (uint32_t)p.boxes * kBoxBytes;
+    // barriers: full[stages], empty[stages], b_full, tmem_full[kMaxAccBufs], tmem_empty[kMaxAccBufs], out_full[kOutSlots], out_free[kOutSlots], box_full[boxes], box_free[boxes]
+    L.tmem_slot = L.bars + 8u * (2u * p.stages + 1u + 2u * kMaxAccBufs + (p.rows ? 2u * kOutSlots + 2u * p.boxes : 0u));
     L.abort_flag = L.tmem_slot + 8;
     L.params = (L.abort_flag + 8 + 15u) & ~15u;  // scale_in[bn], bias[bn], scale_out[bn]; read as float4
     L.total = L.params + 3u * 4u * p.bn;
@@ -177,18 +211,22 @@ __host__ __device__ inline SmemLayout smem_layout(const UmmaPlan& p) {
 //
 // BUILDs 4 and 5: see kAnyOut.
 //
-// BUILDs 6 and 7: the operands change places, D[channels, pixels] = W x A^T. Written with pixels as rows, a thread's accumulators belong
+// BUILDs 6, 7 and 8: the operands change places, D[channels, pixels] = W x A^T. Written with pixels as rows, a thread's accumulators belong
 // to 16 or 32 channels, whose three parameters each it has to fetch from shared memory for every pixel, and its results are 32 bytes
 // of a row of their own, of which a warp's store touches 32: TMEM -> int8 reached 18.9 values per ns and SM that way (ReLU; without
 // the stores 31). With channels as rows a thread has the same two channels of every 16 (tcgen05.ld.16x256b) and keeps their parameters in
 // registers; stmatrix turns four pixels' bytes into rows of 16 channels in shared memory, and a warp of its own sends a finished tile of
 // 128 pixels x 128 channels off as one TMA store: 32.5 values per ns and SM (24 against 18.3 with the general rounding).
+// BUILD 8 takes fp32 planes: TMA brings boxes of 16 channels x 64 pixels, ten warps quantize one box each at a time into the tile's operand
+// (so that every channel of the layer is computed from one quantized tile, four accumulators of 64 columns at most), and the shared
+// memory that up to 128 KB of weights leave is spent on boxes under way: six of them 50.8 us for 256 -> 512 28x28 x128, ten 38.7; by loads into
+// registers, which share what is left of L1, 43.3.
 //
 // BUILD 3: fp32 NCHW input, quantized inside the kernel: warps 10..17 take the TMA producer's place, load the planes, quantize and
 // write the operand tiles (with TMA's swizzle) themselves. No int8 copy of the input crosses HBM and no second kernel runs.
 template <int OUT, int ACT_BUILD, int BUILD>
 __global__ void __launch_bounds__(build_threads(BUILD), BUILD == 1 || BUILD == kCompactBuild || BUILD == kRowsBuild ? 2 : 1)
-dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUILD), QuantSource, KernelMaps> maps, const __grid_constant__ CUtensorMap tmB, const UmmaPlan P,
+dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_constant__ CUtensorMap tmB, const UmmaPlan P,
                   const ConvShape s, const EpilogueParams ep, void* __restrict__ out, uint32_t* __restrict__ status,
                   const __grid_constant__ std::conditional_t<build_rows(BUILD), RowsOut, UmmaMixedOut> mixed) {
     constexpr int ACT = ACT_BUILD & ~kOneScale;
@@ -196,7 +234,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                    ROWS = build_rows(BUILD);
     // Pixels of a tile that are loaded and written: 128, or in a compact launch of a 1x1 layer fewer (the MMA's other rows read what
     // the stage happens to hold and nobody reads their sums).
-    const int tile_rows = COMPACT ? P.tile_rows : kTileM;
+    const int tile_rows = COMPACT ? P.tile_rows : ROWS ? rows_pixels(BUILD) : kTileM;
     const auto writes = [&](int kind) { return OUT == kAnyOut ? P.out_kind == kind : OUT == kind; };
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -205,8 +243,10 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
     const uint32_t sB = base + L.b_panel, sA = base + L.a_stages;
     const uint32_t bar_full = base + L.bars, bar_empty = bar_full + 8u * P.stages, bar_b = bar_empty + 8u * P.stages;
     const uint32_t bar_tfull = bar_b + 8, bar_tempty = bar_tfull + 8u * kMaxAccBufs;
-    const uint32_t bar_ofull = bar_tempty + 8u * kMaxAccBufs, bar_ofree = bar_ofull + 8u * kOutSlots;  // (ROWS)
-    const uint32_t acc_mask = (uint32_t)P.acc_bufs - 1u, acc_shift = P.acc_bufs == 4 ? 2u : 1u;  // 2 or 4 accumulators in TMEM
+    const uint32_t bar_ofull = bar_tempty + 8u * kMaxAccBufs, bar_ofree = bar_ofull + 8u * kOutSlots, bar_xfull = bar_ofree + 8u * kOutSlots,
+                   bar_xfree = bar_xfull + 8u * P.boxes;  // (ROWS)
+    const int boxes_per_tile = (s.cin + kBoxChannels - 1) / kBoxChannels;  // (ROWS, QUANT)
+    const uint32_t acc_mask = (uint32_t)P.acc_bufs - 1u, acc_shift = P.acc_bufs == 8 ? 3u : P.acc_bufs == 4 ? 2u : 1u;  // 2, 4 or 8 accumulators in TMEM
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + L.tmem_slot);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + L.abort_flag);
 
@@ -215,14 +255,14 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
     const int m_first = blockIdx.x / P.n_tiles, m_step = gridDim.x / P.n_tiles;
     // ROWS: accumulators of a pixel tile, 128 channels each, the last one of the layer 64 where that holds what is left
     const int cols_left = s.cout_pad - n_tile * P.bn, my_cols = cols_left < P.bn ? cols_left : P.bn;
-    const int blocks = BUILD == kRowsWideBuild ? (my_cols + kTileM - 1) / kTileM : 1;
+    const int blocks = ROWS && BUILD != kRowsBuild ? (my_cols + kTileM - 1) / kTileM : 1;
     const uint32_t a_stage_bytes = (uint32_t)P.a_stage_bytes, b_tile_bytes = (uint32_t)P.bn * P.bkc;
     // halo mode: the 8 pixels of one tile row are one 8-row operand group; groups (tile rows) are one halo row apart
     const int halo_w = kHaloTw + s.kw - 1, halo_h = kHaloTh + s.kh - 1;
     const ParityHalo parity(s.kh, s.kw);
     // pipeline stages one pixel tile consumes (a gathered layer's stage holds all the K blocks of a tile: one barrier round
     // trip per tile instead of one per 32-channel block)
-    const int loads_per_tile = P.halo ? P.ncb : (P.gather && P.gather_whole ? 1 : P.nkb);
+    const int loads_per_tile = ROWS && QUANT ? 1 : P.halo ? P.ncb : (P.gather && P.gather_whole ? 1 : P.nkb);
 
     // Tensor memory first, and only then may the next kernel start: a CTA of it that shared this SM and allocated before this one
     // would hold the columns this one waits for while it waits for this kernel to end.
@@ -240,22 +280,27 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
             for (int i = 0; i < (P.gather > 0 ? P.gather : 1); ++i) prefetch_tensormap(&maps.tm[i]);
 #pragma unroll 1
         for (int i = 0; i < P.stages; ++i) {
-            mbar_init(bar_full + 8u * i, QUANT ? kQuantWarps : 1);
+            mbar_init(bar_full + 8u * i, ROWS && QUANT ? (uint32_t)boxes_per_tile : QUANT ? kQuantWarps : 1);
             mbar_init(bar_empty + 8u * i, 1);
         }
         mbar_init(bar_b, 1);
 #pragma unroll 1
         for (int i = 0; i < P.acc_bufs; ++i) {
             mbar_init(bar_tfull + 8u * i, 1);
-            mbar_init(bar_tempty + 8u * i, ROWS ? kTeamWarps
+            mbar_init(bar_tempty + 8u * i, ROWS ? (uint32_t)team_warps(BUILD)
                                                 : (uint32_t)(tile_rows + 31) / 32u * (uint32_t)((P.bn + epi_chunk(P) - 1) / epi_chunk(P)));  // one arrival per lane quarter and column chunk
         }
         if constexpr (ROWS) {
             prefetch_tensormap(my_cols > 64 ? &mixed.full : &mixed.half);
 #pragma unroll 1
             for (int i = 0; i < P.out_slots; ++i) {
-                mbar_init(bar_ofull + 8u * i, kTeamWarps);
+                mbar_init(bar_ofull + 8u * i, (uint32_t)team_warps(BUILD));
                 mbar_init(bar_ofree + 8u * i, 1);
+            }
+#pragma unroll 1
+            for (int i = 0; i < P.boxes; ++i) {
+                mbar_init(bar_xfull + 8u * i, 1);
+                mbar_init(bar_xfree + 8u * i, 1);
             }
         }
         *abort_flag = 0;
@@ -264,7 +309,13 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
         // the weight panel does not depend on the previous kernel: start loading it before waiting for that kernel
         mbar_expect_tx(bar_b, (uint32_t)P.nkb * b_tile_bytes);
 #pragma unroll 1
-        for (int kb = 0; kb < P.nkb; ++kb) tma_load_2d(&tmB, bar_b, sB + kb * b_tile_bytes, kb * P.bkc, n_tile * P.bn);
+        for (int kb = 0; kb < P.nkb; ++kb)
+            if constexpr (ROWS && QUANT) {  // (a panel of up to 512 channels: 64 at a time)
+#pragma unroll 1
+                for (int c = 0; c < P.bn; c += 64) tma_load_2d(&tmB, bar_b, sB + kb * b_tile_bytes + (uint32_t)(c * P.bkc), kb * P.bkc, n_tile * P.bn + c);
+            } else {
+                tma_load_2d(&tmB, bar_b, sB + kb * b_tile_bytes, kb * P.bkc, n_tile * P.bn);
+            }
     }
     {
         float* sp = reinterpret_cast<float*>(base_ptr + L.params);
@@ -283,6 +334,27 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
+        if constexpr (ROWS && QUANT) {
+            if (elect_one()) {
+                // ---- TMA producer (fp32 planes): box b of the CTA goes to quantizing warp b % kBoxWarps, whose boxes have places of their own ----
+                pdl_wait();
+                uint32_t at = 0, phase = 1;
+                bool ok = true;
+                for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
+                    const int img = (int)fast_div((uint32_t)m, P.div_img), p0 = (m - img * P.tiles_x) * rows_pixels(BUILD);
+                    for (int c = 0; c < s.cin; c += kBoxChannels) {
+                        if (!mbar_wait(bar_xfree + 8u * at, phase, abort_flag, status, 256u, P.wait_ns)) { ok = false; break; }
+                        mbar_expect_tx(bar_xfull + 8u * at, kBoxBytes);
+                        tma_load_3d(&maps.x, bar_xfull + 8u * at, base + L.floats + at * kBoxBytes, p0, c, img);
+                        if (++at == (uint32_t)P.boxes) { at = 0; phase ^= 1u; }
+                    }
+                }
+                if (!ok) {
+                    const unsigned long long t0 = globaltimer_ns();  // (as below)
+                    while (globaltimer_ns() - t0 < 1000000ull) {}
+                }
+            }
+        }
         if constexpr (!QUANT)
         if (elect_one()) {
             // ---- TMA producer (activations; the weights were requested during set-up) ----
@@ -350,18 +422,27 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                 const uint32_t buf = tile_i & acc_mask, use = tile_i >> acc_shift;
                 if (!mbar_wait(bar_tempty + 8u * buf, (use & 1u) ^ 1u, abort_flag, status, 4u, P.wait_ns)) { ok = false; break; }
                 const uint32_t d = tmem_base + buf * (uint32_t)P.acc_stride;
-                uint32_t d1 = 0;
-                if (ROWS && blocks > 1) {
-                    const uint32_t buf1 = (tile_i + 1) & acc_mask, use1 = (tile_i + 1) >> acc_shift;
-                    if (!mbar_wait(bar_tempty + 8u * buf1, (use1 & 1u) ^ 1u, abort_flag, status, 4u, P.wait_ns)) { ok = false; break; }
-                    d1 = tmem_base + buf1 * (uint32_t)P.acc_stride;
+                // ROWS: the tile's other accumulators
+                constexpr int kMore = BUILD == kRowsQuantBuild ? kRowsMaxBlocks - 1 : BUILD == kRowsWideBuild ? 1 : 0;
+                uint32_t more[kMore + 1];
+#pragma unroll
+                for (int b = 0; b < kMore; ++b) {
+                    if (b + 1 >= blocks) break;
+                    const uint32_t unit = tile_i + 1u + (uint32_t)b, bb = unit & acc_mask;
+                    if (ok && !mbar_wait(bar_tempty + 8u * bb, ((unit >> acc_shift) & 1u) ^ 1u, abort_flag, status, 4u, P.wait_ns)) ok = false;
+                    more[b] = tmem_base + bb * (uint32_t)P.acc_stride;
                 }
+                if (!ok) break;
                 tc_fence_after();
                 // pixels: the operand with the tile's pixels as rows; weights: the one with channels as rows
                 auto mma = [&](uint64_t pixels, uint64_t weights, uint32_t accumulate) {
                     if constexpr (ROWS) {
                         umma_i8(d, weights, pixels, blocks > 1 || my_cols > 64 ? P.idesc : idesc_half, accumulate);
-                        if (blocks > 1) umma_i8(d1, weights + ((uint32_t)(kTileM * P.bkc) >> 4), pixels, my_cols > kTileM + 64 ? P.idesc : idesc_half, accumulate);
+#pragma unroll
+                        for (int b = 0; b < kMore; ++b)
+                            if (b + 1 < blocks)
+                                umma_i8(more[b], weights + (uint32_t)(b + 1) * ((uint32_t)(kTileM * P.bkc) >> 4), pixels,
+                                        my_cols > (b + 1) * kTileM + 64 ? P.idesc : idesc_half, accumulate);
                     } else {
                         umma_i8(d, pixels, weights, P.idesc, accumulate);
                     }
@@ -434,6 +515,15 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                                 }
                             }
                         }
+                    } else if constexpr (ROWS && QUANT) {
+                        // one stage holds all the K blocks of the tile, 64 pixels each
+                        const uint64_t a0 = make_smem_desc(sA + st * a_stage_bytes, P.bkc), b0 = make_smem_desc(sB, P.bkc);
+                        const uint32_t a_step = (uint32_t)(rows_pixels(BUILD) * P.bkc) >> 4, b_step = b_tile_bytes >> 4;
+#pragma unroll 1
+                        for (int g = 0; g < P.nkb; ++g)
+#pragma unroll 1
+                            for (int j = 0; j < P.bkc / 32; ++j)
+                                mma(a0 + (uint32_t)g * a_step + 2u * j, b0 + (uint32_t)g * b_step + 2u * j, (g | j) != 0 ? 1u : 0u);
                     } else if (P.gather && P.gather_whole) {
                         // one stage holds all the K blocks of the tile; per block only the low words of the two descriptors move
                         const uint64_t a0 = make_smem_desc(sA + st * a_stage_bytes, P.bkc), b0 = make_smem_desc(sB, P.bkc);
@@ -468,7 +558,10 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                 }
                 if (!ok) break;
                 umma_commit(bar_tfull + 8u * buf);  // accumulator complete
-                if (ROWS && blocks > 1) umma_commit(bar_tfull + 8u * ((tile_i + 1) & acc_mask));
+                if (ROWS && !QUANT && blocks > 1) umma_commit(bar_tfull + 8u * ((tile_i + 1) & acc_mask));
+                if constexpr (ROWS && QUANT)
+#pragma unroll 1
+                    for (int b = 1; b < blocks; ++b) umma_commit(bar_tfull + 8u * ((tile_i + (uint32_t)b) & acc_mask));
             }
             // every accumulator read for the last time: the tensor memory can go back
             for (uint32_t b = 0; ok && b <= acc_mask && b < tile_i; ++b)
@@ -480,8 +573,57 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
         if (*abort_flag) __syncthreads();
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)P.tmem_cols) : "memory");
-    } else if (QUANT && warp >= 2 + kMaxEpiWarps) {
-        if constexpr (QUANT) {
+    } else if (ROWS && QUANT && warp > 2 + kMaxEpiWarps) {
+        if constexpr (ROWS && QUANT) {
+            // ---- quantizers: four pixels of eight channels per thread. A warp passes every tile, in order, whether it has a box of it or
+            // not, so that no phase of a barrier that it waits for goes by unseen ----
+            const int qw = warp - (3 + kMaxEpiWarps), quad = lane & 15, upper = lane >> 4, per_block = 31 - __clz(P.bkc >> 4);
+            const uint32_t words_at = base + L.floats + (uint32_t)(upper * 8 * rows_pixels(BUILD) * 4 + quad * 16);
+            uint32_t st = 0, phase = 1, at = (uint32_t)qw, xphase = 0;
+            int c = qw;  // this warp's next box, counted from the tile's first
+            bool ok = true;
+            for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
+                bool waited = false;
+                for (;; c += kBoxWarps) {
+                    float4 v[8];
+                    const bool mine = c < boxes_per_tile;
+                    if (mine) {
+                        if (!mbar_wait(bar_xfull + 8u * at, xphase, abort_flag, status, 512u, P.wait_ns)) { ok = false; break; }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w)
+                                         : "r"(words_at + at * kBoxBytes + (uint32_t)(j * rows_pixels(BUILD) * 4)) : "memory");
+                    }
+                    if (!waited && !mbar_wait(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
+                    waited = true;
+                    if (!mine) break;
+                    uint32_t w[2][4];  // [group of four channels][pixel]
+#pragma unroll
+                    for (int g = 0; g < 2; ++g) {
+                        uint32_t cw[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) cw[j] = quantize4_pack(v[4 * g + j].x, v[4 * g + j].y, v[4 * g + j].z, v[4 * g + j].w, maps.scale, maps.half);
+                        transpose4x4(cw[0], cw[1], cw[2], cw[3], w[g]);
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_xfree + 8u * at);  // the box is read
+                    at += kBoxWarps;
+                    if (at >= (uint32_t)P.boxes) { at = (uint32_t)qw; xphase ^= 1u; }
+                    const uint32_t block = sA + st * a_stage_bytes + (uint32_t)((c >> per_block) * rows_pixels(BUILD) * P.bkc);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(operand_chunk(block, P.bkc, quad * 4 + j, c & ((1 << per_block) - 1)) + (uint32_t)(upper * 8)),
+                                     "r"(w[0][j]), "r"(w[1][j]) : "memory");
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // these writes -> the MMA's reads
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_full + 8u * st);
+                }
+                c -= boxes_per_tile;
+                if (++st == (uint32_t)P.stages) { st = 0; phase ^= 1u; }
+            }
+        }
+    } else if (QUANT && !ROWS && warp >= 2 + kMaxEpiWarps) {
+        if constexpr (QUANT && !ROWS) {
             // ---- quantizers: warp q takes every eighth (16 channels, 32 pixels or pixel quads) item of a stage ----
             const int qw = warp - (2 + kMaxEpiWarps), chunks = P.bkc >> 4, hw = s.h * s.w;
             const long total_pix = (long)s.n * hw;
@@ -507,19 +649,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                             const int im = (int)fast_div((uint32_t)gp, P.div_plane), p = (int)(gp - (long)im * hw);
                             float4 v[16];
                             load16(v, maps, c0, s.cin, im, hw, p);
-                            uint32_t w[4][4];  // [group of four channels][pixel]
-#pragma unroll
-                            for (int g = 0; g < 4; ++g) {
-                                uint32_t cw[4];
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const float4 f = v[4 * g + j];
-                                    cw[j] = quantize4_pack(f.x, f.y, f.z, f.w, maps.scale, maps.half);
-                                }
-                                transpose4x4(cw[0], cw[1], cw[2], cw[3], w[g]);
-                            }
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) store_chunk(operand_chunk(tile, P.bkc, lane * 4 + j, ch), w[0][j], w[1][j], w[2][j], w[3][j]);
+                            quantize_quad(v, tile, P.bkc, lane * 4, ch, maps);
                         }
                     } else {
                         // pixel by pixel: flat tiles of any alignment, and halo tiles (out-of-image pixels are zeros)
@@ -573,11 +703,12 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                 uint32_t unit = 0;
                 bool ok = true;
                 for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
+                    const int img = QUANT ? (int)fast_div((uint32_t)m, P.div_img) : 0, p0 = (m - (QUANT ? img * P.tiles_x : 0)) * rows_pixels(BUILD);
                     for (int blk = 0; blk < blocks; ++blk, ++unit) {
                         const uint32_t slot = unit & ((uint32_t)P.out_slots - 1u), use = unit / (uint32_t)P.out_slots;
                         if (!mbar_wait(bar_ofull + 8u * slot, use & 1u, abort_flag, status, 64u, P.wait_ns)) { ok = false; break; }
-                        tma_store_2d(my_cols - blk * kTileM > 64 ? &mixed.full : &mixed.half, base + L.out_slots + slot * out_slot_bytes(P),
-                                     n_tile * P.bn + blk * kTileM, m * kRowsPixels);
+                        tma_store_3d(my_cols - blk * kTileM > 64 ? &mixed.full : &mixed.half, base + L.out_slots + slot * out_slot_bytes(P),
+                                     n_tile * P.bn + blk * kTileM, p0, img);
                         bulk_commit();
                         // A slot is free when its store has been read, 0.5 us after it was issued. With two slots a team waits for that; with
                         // four the next tile's store is issued first (64 -> 256 56x56 x128: one at a time 35.4 us, two 27.7).
@@ -595,18 +726,23 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
         }
     } else if (ROWS) {
         if constexpr (ROWS) {
-            // ---- epilogue warps, channels as rows. A team of eight (two per lane quarter) takes an accumulator; two teams take them in turn,
-            // so that a warp has one block's channels for good, and one team's arithmetic fills the other's waits ----
-            constexpr uint32_t teams = BUILD == kRowsWideBuild ? 2 : 1;
-            const int q = warp & 3, sub = ((warp - 2) >> 2) & 1;
-            const uint32_t team = teams == 2 ? (uint32_t)(warp - 2) >> 3 : 0u;
-            const int blk = blocks > 1 ? (int)team : 0;
-            const int left = my_cols - blk * kTileM;                  // channels from the block's first on
-            const int per_q = left > 64 ? 32 : 16, c0 = q * per_q;    // rows of a quarter (64-row accumulators: its first 16 lanes)
-            const bool hi = per_q == 32 && c0 + 16 < left;            // 16 channels at a time: the quarter's first, and its second
+            // ---- epilogue warps, channels as rows. A team of eight (two per lane quarter; of four where tiles are 64 pixels) takes an
+            // accumulator; two teams take them in turn, so that a warp has one block's channels for good (with more than two blocks per
+            // tile it changes them), and one team's arithmetic fills the other's waits ----
+            constexpr uint32_t teams = BUILD == kRowsBuild ? 1 : 2;
+            const int q = warp & 3, sub = team_warps(BUILD) == 8 ? ((warp - 2) >> 2) & 1 : 0;
+            const uint32_t team = teams == 2 ? (uint32_t)(warp - 2) / (uint32_t)team_warps(BUILD) : 0u;
+            int blk = 0, left, c0;  // accumulator block; channels from its first one on, this quarter's first
+            bool hi;                // 16 channels at a time: the quarter's first, and its second
+            uint32_t row_bytes, at_lo, at_hi;
             const uint32_t half = half_bits(ep.rounding);
             float2 si[2][2], bi[2][2], so[2][2];  // [first / second 16][channel lane / 4, + 8], each twice: for two pixels
-            {
+            auto take_block = [&](int b) {
+                blk = b;
+                left = my_cols - blk * kTileM;
+                const int per_q = left > 64 ? 32 : 16;  // rows of a quarter (64-row accumulators: its first 16 lanes)
+                c0 = q * per_q;
+                hi = per_q == 32 && c0 + 16 < left;
                 const float* sp = reinterpret_cast<const float*>(base_ptr + L.params);
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
@@ -617,11 +753,14 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
                         bi[h][j] = make_float2(sp[P.bn + c], sp[P.bn + c]);
                         so[h][j] = make_float2(sp[2 * P.bn + c], sp[2 * P.bn + c]);
                     }
-            }
-            // one byte per channel and row; the 16-byte chunks of a row trade places by the row's number, as the store's swizzle has it
-            const uint32_t row_bytes = 4u * (uint32_t)per_q, swz = per_q == 32 ? (uint32_t)lane & 7u : ((uint32_t)lane >> 1) & 3u, chunk = (uint32_t)c0 >> 4;
-            const uint32_t row0 = base + L.out_slots + ((uint32_t)(sub * 64) + (uint32_t)lane) * row_bytes;
-            const uint32_t at_lo = row0 + ((chunk ^ swz) << 4), at_hi = row0 + (((chunk + 1u) ^ swz) << 4);
+                // one byte per channel and row; the 16-byte chunks of a row trade places by the row's number, as the store's swizzle has it
+                row_bytes = 4u * (uint32_t)per_q;
+                const uint32_t swz = per_q == 32 ? (uint32_t)lane & 7u : ((uint32_t)lane >> 1) & 3u, chunk = (uint32_t)c0 >> 4;
+                const uint32_t row0 = base + L.out_slots + ((uint32_t)(sub * 64) + (uint32_t)lane) * row_bytes;
+                at_lo = row0 + ((chunk ^ swz) << 4);
+                at_hi = row0 + (((chunk + 1u) ^ swz) << 4);
+            };
+            take_block(blocks > 1 ? (int)team : 0);
             const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(sub * 64);
             const uint32_t slot_bytes = out_slot_bytes(P), slot_mask = (uint32_t)P.out_slots - 1u, slot_shift = P.out_slots == 4 ? 2u : 1u;
             auto emit = [&](const int (&a)[16], int h, uint32_t at) {
@@ -645,6 +784,7 @@ dense_umma_kernel(const __grid_constant__ std::conditional_t<build_quantizes(BUI
             };
             const uint32_t units = m_first < P.m_tiles ? (uint32_t)((P.m_tiles - 1 - m_first) / m_step + 1) * (uint32_t)blocks : 0u;
             for (uint32_t unit = team; unit < units; unit += teams) {
+                if (QUANT && blocks > 2 && unit != team) take_block(blk + 2 < blocks ? blk + 2 : blk + 2 - blocks);
                 const uint32_t buf = unit & acc_mask, use = unit >> acc_shift, slot = unit & slot_mask;
                 const uint32_t taddr = t_lane + buf * (uint32_t)P.acc_stride, out_at = slot * slot_bytes;
                 if (!mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) break;
@@ -910,7 +1050,7 @@ const char* launch_variant(cudaStream_t stream, int sm_count, const Source& maps
     }
     // Tiles are dealt statically to the CTAs of the grid, so a grid larger than what is resident at once runs in waves.
     // The plan bounds residency by shared memory and TMEM; registers and threads are bounded here.
-    const int threads = 64 + 32 * (p.epi_warps + (build_quantizes(BUILD) ? kQuantWarps : 0) + (build_rows(BUILD) ? 1 : 0));
+    const int threads = BUILD == kRowsQuantBuild ? build_threads(BUILD) : 64 + 32 * (p.epi_warps + (build_quantizes(BUILD) ? kQuantWarps : 0) + (build_rows(BUILD) ? 1 : 0));
     const int regs_per_warp = (regs * 32 + 255) / 256 * 256;
     int resident = 65536 / (regs_per_warp * (threads / 32));
     if (resident > 2048 / threads) resident = 2048 / threads;
@@ -1042,6 +1182,52 @@ std::vector<UmmaVariant> umma_variants(const UmmaPlan& widest, int cout, int sme
     return all;
 }
 
+// What follows from a plan's panel, tile and team shape with channels as accumulator rows: pipeline, tensor memory, CTAs per SM.
+static bool plan_rows(UmmaPlan& p, int cout_pad, int smem_budget) {
+    const bool quant = p.rows == rows_pixels(kRowsQuantBuild);
+    p.n_tiles = (cout_pad + p.bn - 1) / p.bn;
+    p.acc_stride = p.rows;
+    p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.rows >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+    // Two CTAs per SM of eight epilogue warps and two accumulators each, or one of sixteen and four: the same warps and tensor memory,
+    // but two panels, and while one CTA's warps wait for an accumulator the other's have one.
+    p.epi_warps = 8;
+    p.stages = 1;
+    p.out_slots = 2;
+    p.boxes = quant ? kBoxWarps : 0;
+    int fixed = (int)smem_layout(p).total - p.a_stage_bytes + 1024;
+    auto stages_in = [&](int budget) { return budget > fixed ? (budget - fixed - 512 /*barriers of further stages and boxes*/) / p.a_stage_bytes : 0; };
+    const int most = quant ? 8 : p.gather_whole ? 2 : p.nkb <= 2 ? 4 : 8;
+    const bool pair = !quant && p.bn <= kTileM && stages_in(smem_budget / 2) >= 2;
+    p.ctas_per_sm = pair ? 2 : 1;
+    p.stages = stages_in(smem_budget / p.ctas_per_sm);
+    // two finished tiles per team, if three (of a tile in several loads: four) stages remain
+    if (!quant && !pair && stages_in(smem_budget - 2 * (int)out_slot_bytes(p)) >= (p.nkb > 1 && !p.gather_whole ? 4 : 3)) {
+        p.out_slots = kOutSlots;
+        fixed += 2 * (int)out_slot_bytes(p);
+        p.stages = stages_in(smem_budget);
+    }
+    // twice as many boxes and finished tiles, if stages for as many tiles as the warps have boxes of, and one more, remain
+    const int want = quant ? kBoxWarps / (p.k_total / kBoxChannels) + 2 : 0;
+    if (quant && stages_in(smem_budget - kBoxWarps * (int)kBoxBytes) >= want) {
+        p.boxes = 2 * kBoxWarps;
+        fixed += kBoxWarps * (int)kBoxBytes;
+    }
+    if (quant && stages_in(smem_budget - 2 * (int)out_slot_bytes(p)) >= want) {
+        p.out_slots = kOutSlots;
+        fixed += 2 * (int)out_slot_bytes(p);
+    }
+    if (quant) p.stages = stages_in(smem_budget);
+    if (p.stages > most) p.stages = most;
+    if (p.stages < 2) return false;
+    p.acc_bufs = quant ? 8 : pair ? 2 : 4;
+    p.tmem_cols = p.acc_bufs * p.acc_stride;
+    if (!quant && !pair) p.epi_warps = 16;
+    p.smem_bytes = (int)smem_layout(p).total + 1024;
+    const int min_smem = smem_budget / (p.ctas_per_sm + 1) + 1;  // (no more CTAs than tensor memory serves, see plan_panel)
+    if (p.smem_bytes < min_smem) p.smem_bytes = min_smem;
+    return true;
+}
+
 std::vector<UmmaVariant> umma_row_variants(const UmmaPlan& base, int cout, int smem_budget) {
     std::vector<UmmaVariant> all;
     const int cout_pad = nhwc_channels(cout);
@@ -1049,40 +1235,19 @@ std::vector<UmmaVariant> umma_row_variants(const UmmaPlan& base, int cout, int s
     for (int bn : {256, 192, 128, 64}) {
         if (bn >= cout_pad + 64 || (bn == 64 && cout_pad > 64)) continue;
         UmmaVariant v;
-        UmmaPlan& p = v.plan;
-        p = base;
-        p.rows = 1;
-        p.bn = bn;
-        p.n_tiles = (cout_pad + bn - 1) / bn;
-        p.acc_stride = kRowsPixels;
-        p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kRowsPixels >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
-        // Two CTAs per SM of eight epilogue warps and two accumulators each, or one of sixteen and four: the same warps and tensor memory,
-        // but two panels, and while one CTA's warps wait for an accumulator the other's have one.
-        p.epi_warps = 8;
-        p.stages = 1;
-        p.out_slots = 2;
-        int fixed = (int)smem_layout(p).total - p.a_stage_bytes + 1024;
-        auto stages_in = [&](int budget) { return budget > fixed ? (budget - fixed - 192 /*barriers of further stages*/) / p.a_stage_bytes : 0; };
-        const int most = p.gather_whole ? 2 : p.halo ? 3 : p.nkb <= 2 ? 4 : 8;
-        const bool pair = bn <= kTileM && stages_in(smem_budget / 2) >= 2;
-        p.ctas_per_sm = pair ? 2 : 1;
-        p.stages = stages_in(smem_budget / p.ctas_per_sm);
-        // two finished tiles per team, if three (of a tile in several loads: four) stages remain
-        if (!pair && stages_in(smem_budget - 2 * (int)out_slot_bytes(p)) >= (p.nkb > 1 && !p.gather_whole ? 4 : 3)) {
-            p.out_slots = 4;
-            fixed += 2 * (int)out_slot_bytes(p);
-            p.stages = stages_in(smem_budget);
-        }
-        if (p.stages > most) p.stages = most;
-        if (p.stages < 2) continue;
-        p.acc_bufs = pair ? 2 : 4;
-        p.tmem_cols = p.acc_bufs * p.acc_stride;
-        p.epi_warps = pair ? 8 : 16;
-        p.smem_bytes = (int)smem_layout(p).total + 1024;
-        const int min_smem = smem_budget / (p.ctas_per_sm + 1) + 1;  // (no more CTAs than tensor memory serves, see plan_panel)
-        if (p.smem_bytes < min_smem) p.smem_bytes = min_smem;
-        all.push_back(v);
+        v.plan = base;
+        v.plan.rows = rows_pixels(kRowsBuild);
+        v.plan.bn = v.plan.panel_box = bn;
+        if (plan_rows(v.plan, cout_pad, smem_budget)) all.push_back(v);
     }
+    // fp32 input, quantized inside: one panel of all the channels, so that the input is quantized once; a stage holds a whole tile
+    UmmaVariant v;
+    v.plan = base;
+    v.plan.rows = rows_pixels(kRowsQuantBuild);
+    v.plan.bn = round_up(cout_pad, 64);
+    v.plan.panel_box = 64;
+    v.plan.a_stage_bytes = v.plan.rows * base.k_total;
+    if (!base.gather && v.plan.bn <= kRowsMaxBlocks * kTileM && plan_rows(v.plan, cout_pad, smem_budget)) all.push_back(v);
     return all;
 }
 
@@ -1103,12 +1268,16 @@ const char* umma_encode_weight_map(const UmmaPlan& p, const int8_t* w_dev, void*
     if (!enc) return "cuTensorMapEncodeTiled entry point not available";
     cuuint64_t dims[2] = {(cuuint64_t)p.k_total, (cuuint64_t)p.cout_rows};
     cuuint64_t strides[1] = {(cuuint64_t)p.k_total};
-    cuuint32_t box[2] = {(cuuint32_t)p.bkc, (cuuint32_t)p.bn};
+    cuuint32_t box[2] = {(cuuint32_t)p.bkc, (cuuint32_t)(p.rows ? p.panel_box : p.bn)};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(reinterpret_cast<CUtensorMap*>(map_out), CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)w_dev, dims, strides, box,
                      estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(p.bkc), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? nullptr : "cuTensorMapEncodeTiled(weights) failed";
+}
+
+bool umma_box_input(const UmmaFloatInput& in, long hw) {
+    return in.n_runs == 1 && hw % 4 == 0 && (reinterpret_cast<uintptr_t>(in.base[0]) & 15) == 0 && in.img_stride[0] % 4 == 0;
 }
 
 // Describes an fp32 input for quantization inside the kernel; false when its planes are scattered over more runs than that takes.
@@ -1279,13 +1448,27 @@ UmmaChoice umma_choose(const UmmaVariant* v, int n, const ConvShape& s, int sm_c
 // ends than as soon as there is room beside it (us, beside / at the end: 256 -> 512 28x28 x128 54.9 / 44.1, 307 -> 490 102648 pixels 65.9 /
 // 54.1, 473 -> 903 29520 pixels 35.1 / 30.9, 116 -> 974 6831 pixels 9.2 / 7.9; of up to 64 channels 45 -> 330 10260 pixels 6.7 / 7.5, 34 -> 473
 // 16640 pixels 8.7 / 9.4).
-UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count, bool f32_input) {
+// An fp32 input that fills L2 by itself is quantized inside, where one panel holds all the channels: the int8 copy then goes to HBM and
+// back, and the planes can be fetched while other tiles are multiplied. us, other forms / this one: 256 -> 512 28x28 x128 (103 MB) 44.1 /
+// 38.7, 249 -> 61 192660 pixels 47.9 / 42.2, 620 -> 37 109800 pixels 59.7 / 54.0; but 105 -> 453 55200 pixels (23 MB) 16.6 / 18.8, 178 -> 58 54880
+// pixels (39 MB) 11.6 / 13.5, 120 -> 46 143000 pixels (69 MB) 18.3 / 20.7.
+constexpr double kFillsL2 = 96.0 * (1 << 20);
+UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count, bool f32_input, bool may_box) {
     const PixelTiles t = tile_pixels(choice.variant->plan, s);
+    if (may_box && !choice.compact && t.flat && 4.0 * s.cin * s.n * s.h * s.w >= kFillsL2 && (double)s.n * s.h * s.w <= 2147483647.0 && n_rows > 0 &&
+        rows[n_rows - 1].plan.rows == rows_pixels(kRowsQuantBuild)) {
+        UmmaChoice c = choice;
+        c.variant = &rows[n_rows - 1];
+        c.inside = true;
+        c.tile_rows = c.variant->plan.rows;
+        return c;
+    }
     if (choice.inside || choice.compact || !t.flat || (choice.variant->plan.bn <= 64 && t.tiles <= sm_count)) return choice;
     const UmmaVariant* pick = nullptr;
     int pick_work = 0;
     for (int i = 0; i < n_rows; ++i) {
         const UmmaPlan& p = rows[i].plan;
+        if (p.rows != rows_pixels(kRowsBuild)) continue;
         const int widest = s.cout_pad < p.bn ? s.cout_pad : p.bn, work = p.n_tiles * ((widest + 63) / 64);
         const bool light = p.k_total <= 256;
         if (64 * work * (light ? 5 : 7) > s.cout_pad * (light ? 7 : 8)) continue;
@@ -1316,6 +1499,10 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaChoic
     p.tile_rows = choice.tile_rows;
     p.late = choice.late ? 1 : 0;
     if (p.tile_rows != kTileM) p.m_tiles = p.tiles_x = (int)((pixels + p.tile_rows - 1) / p.tile_rows);
+    if (f32 && p.rows) {  // tiles of one image each
+        p.tiles_x = (int)(((long)s.h * s.w + p.rows - 1) / p.rows);
+        p.m_tiles = s.n * p.tiles_x;
+    }
     const bool flat = p.flat != 0;
     KernelMaps km;  // only the entries the plan uses are filled in
     CUtensorMap& tmA = km.tm[0];
@@ -1431,15 +1618,29 @@ const char* launch_dense_umma(cudaStream_t stream, int sm_count, const UmmaChoic
         const int last = s.cout_pad - (p.n_tiles - 1) * p.bn;
         auto ends_in_64 = [](int cols) { return (cols - 1) % kTileM < 64; };
         const bool want_64 = ends_in_64(last) || (p.n_tiles > 1 && ends_in_64(p.bn)), want_128 = last > 64 || (p.n_tiles > 1 && p.bn > 64);
-        cuuint64_t dims[2] = {(cuuint64_t)s.cout_pad, (cuuint64_t)pixels}, strides[1] = {(cuuint64_t)s.cout_pad};
+        const cuuint64_t cp = (cuuint64_t)s.cout_pad, hw = (cuuint64_t)s.h * s.w;
+        cuuint64_t dims[3] = {cp, f32 ? hw : (cuuint64_t)pixels, f32 ? (cuuint64_t)s.n : 1}, strides[2] = {cp, cp * dims[1]};
         for (int width : {128, 64}) {
             if (!(width == 64 ? want_64 : want_128)) continue;
-            cuuint32_t box[2] = {(cuuint32_t)width, (cuuint32_t)kRowsPixels}, one[2] = {1, 1};
-            if (enc(width == 128 ? &to.full : &to.half, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, out, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            cuuint32_t box[3] = {(cuuint32_t)width, (cuuint32_t)p.rows, 1}, one[3] = {1, 1, 1};
+            if (enc(width == 128 ? &to.full : &to.half, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, out, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle_for(width), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return "cuTensorMapEncodeTiled(output) failed";
         }
-#define OTT_ROWS_LAUNCH(ACT)                                                                                                                 err = p.ctas_per_sm > 1 ? launch_variant<DT_S8_NHWC, ACT, kRowsBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, to)                             : launch_variant<DT_S8_NHWC, ACT, kRowsWideBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, to)
+        BoxSource planes;
+        if (f32) {
+            planes.scale = f32->scale;
+            planes.half = half_bits(ep.rounding);
+            cuuint64_t xd[3] = {hw, (cuuint64_t)s.cin, (cuuint64_t)s.n}, xs[2] = {hw * 4, (cuuint64_t)f32->img_stride[0] * 4};
+            cuuint32_t box[3] = {(cuuint32_t)p.rows, (cuuint32_t)kBoxChannels, 1}, one[3] = {1, 1, 1};
+            if (f32->n_runs != 1 || enc(&planes.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(f32->base[0]), xd, xs, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                return "cuTensorMapEncodeTiled(planes) failed";
+        }
+#define OTT_ROWS_LAUNCH(ACT)                                                                                                             \
+    err = f32                 ? launch_variant<DT_S8_NHWC, ACT, kRowsQuantBuild>(stream, sm_count, planes, tmB, p, s, ep, out, status, to)  \
+          : p.ctas_per_sm > 1 ? launch_variant<DT_S8_NHWC, ACT, kRowsBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, to)       \
+                              : launch_variant<DT_S8_NHWC, ACT, kRowsWideBuild>(stream, sm_count, km, tmB, p, s, ep, out, status, to)
         if (ep.int8_pos) OTT_ROWS_LAUNCH(ACT_POS);
         else if (ep.act_type == ACT_RELU) OTT_ROWS_LAUNCH(ACT_RELU);
         else if (ep.act_type == ACT_LRELU) OTT_ROWS_LAUNCH(ACT_LRELU);

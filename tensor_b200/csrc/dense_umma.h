@@ -22,8 +22,10 @@ struct UmmaPlan {
     int epi_warps;   // epilogue warps per CTA: 8 or 16
     int ctas_per_sm; // resident CTAs per SM the launch is sized for (limited by TMEM columns and shared memory)
     int rows;        // int8 output with channels as accumulator rows: bn channels in accumulators of 128 (the last one 64 where that is enough)
-                     // x 128 pixels, see dense_umma.cu
+                     // times this many pixels, see dense_umma.cu; 0: pixels as rows
+    int panel_box;   // rows: channels of the weight panel that one load brings
     int out_slots;   // rows: finished tiles on their way out, 2 or 4
+    int boxes;       // rows, fp32 input quantized inside: boxes of fp32 planes in shared memory
     // per call
     int compact;     // the compact build runs it
     int late;        // the next kernel is not to start beside this one
@@ -104,6 +106,8 @@ struct UmmaFloatInput {
     float scale;
 };
 bool umma_float_input(const float* x, const PlaneGather* table, int cin, long hw, float scale, UmmaFloatInput* in);
+// Whether TMA can bring it: one run of planes whose rows of four pixels are whole and 16-byte aligned.
+bool umma_box_input(const UmmaFloatInput& in, long hw);
 
 // Which form a call of such a layer takes.
 bool umma_prefers_parity(const UmmaVariant* parity, int n_parity, const UmmaVariant* taps, const ConvShape& s, int sm_count);
@@ -120,7 +124,7 @@ struct UmmaChoice {
 };
 UmmaChoice umma_choose(const UmmaVariant* variants, int n_variants, const ConvShape& s, int sm_count, bool may_quantize, long* tiles = nullptr);
 // For an int8 launch without side outputs: the choice, or the same call with channels as accumulator rows.
-UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count, bool f32_input);
+UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count, bool f32_input, bool may_box);
 
 // Launch. Returns NULL or an error text.
 // sources: NULL, or where the K blocks of a plan with gather > 0 come from (x is then unused). mixed: NULL, or the fp32 side

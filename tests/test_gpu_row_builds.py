@@ -35,7 +35,7 @@ def _case(cin, cout, n, h, w, act):
                                              (130, 992, (256, 256))])
 def test_pointwise(ctx, cin, cout, panels):
     for n, panel in zip((7, 41), panels):  # 177 and 1036 tiles, the last one ragged: about one and seven per CTA
-        assert ctx.lib.ott_debug_dense_rows(cin, cout, n, 61, 53, 148) == panel
+        assert ctx.lib.ott_debug_dense_rows(cin, cout, n, 61, 53, 0, 148) == panel
         _check(ctx, _case(cin, cout, n, 61, 53, ACT_RELU))
 
 
@@ -44,6 +44,34 @@ def test_pointwise(ctx, cin, cout, panels):
 def test_epilogues(ctx, act, scale):
     for rounding, per_channel in ((ROUND_ADD_HALF_TRUNC, False), (ROUND_HALF_AWAY, True)):
         cout = 180
-        assert ctx.lib.ott_debug_dense_rows(64, cout, 7, 61, 53, 148) == 192
+        assert ctx.lib.ott_debug_dense_rows(64, cout, 7, 61, 53, 0, 148) == 192
         s = (scale * np.linspace(0.97, 1.03, cout)).astype(np.float32) if per_channel else np.full(1, scale, np.float32)
         _check(ctx, _case(64, cout, 7, 61, 53, act), rounding, s)
+
+
+@pytest.mark.parametrize("cin,cout,h,w", [(256, 512, 44, 20), (40, 330, 44, 21), (130, 240, 20, 44), (33, 64, 44, 20), (64, 100, 46, 22), (100, 16, 44, 20)])
+@pytest.mark.parametrize("act", [ACT_RELU6, ACT_NONE])
+def test_quantized_inside(ctx, cin, cout, h, w, act):
+    """fp32 input of 100 MB: one to four accumulators per tile of 64 pixels, the last tile of an image ragged; the first, the middle and
+    the last image against the checker."""
+    from gpu_support import make_layer
+    from tensor_b200 import F32_NCHW, S8_NHWC, nhwc_channels
+    from support import nhwc_padded_to_nchw
+    n = (100 << 20) // (4 * cin * h * w) + 1
+    assert ctx.lib.ott_debug_dense_rows(cin, cout, n, h, w, 1, 148) == (cout + 63) // 64 * 64
+    case = _case(cin, cout, 3, h, w, act)
+    case.s8_input = False
+    case.make()
+    x = np.tile(np.random.default_rng(cin).uniform(-1, 1, size=(7, cin, h, w)).astype(np.float32), (n // 7 + 1, 1, 1, 1))[:n]
+    at = [0, n // 2, n - 1]
+    x[at] = case.x_f32
+    layer = make_layer(ctx, case, ROUND_ADD_HALF_TRUNC)
+    dx, shape = ctx.to_device(x), (n, h, w, nhwc_channels(cout))
+    y = ctx.malloc(int(np.prod(shape)))
+    layer.forward(dx, F32_NCHW, n, h, w, y, S8_NHWC)
+    got = ctx.to_host(y, shape, np.int8)
+    assert np.array_equal(nhwc_padded_to_nchw(got[at], cout), run_port(case, ROUND_ADD_HALF_TRUNC, want_acc=False)["y"])
+    assert np.array_equal(got[1:8], got[8:15]) and not got[..., cout:].any()
+    layer.close()
+    ctx.free(dx)
+    ctx.free(y)
