@@ -19,6 +19,20 @@ namespace ottk {
 
 namespace {
 
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_tiled() {
+    static const EncodeTiledFn fn = []() -> EncodeTiledFn {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<EncodeTiledFn>(p);
+        return nullptr;
+    }();
+    return fn;
+}
+
 constexpr int ST_TX = 32, ST_TY = 8;  // output tile
 constexpr int ST_COUT_MAX = 32;
 
@@ -121,73 +135,88 @@ dense_stem_kernel(const float* __restrict__ x, const __grid_constant__ StemParam
 
 // ---- stem convolution followed by a 3x3 stride-2 pad-1 max-pool, in one kernel ----
 // The pool is the only consumer of the first layer's output in the benchmark graphs (conv1 -> pool1), and that output is
-// the largest tensor of the whole network; here it never leaves the SM. One CTA produces a 16x7 tile of POOLED pixels for
-// all channels: it computes the 33x15 convolution outputs under that tile into shared memory (fp32, after the
-// dequantize epilogue and activation, exactly the values the separate layer would have stored) and max-reduces them.
+// the largest tensor of the whole network; here it never leaves the SM. One CTA produces a tile of 16 x 6 POOLED pixels for all
+// channels, as eight patches of 4 x 3: warp w has patch (w % 4, w / 4), i.e. the 9 x 7 convolution outputs under it.
 // pad_zero selects the reference's packed max-pool rule (padding counts as 0, Tensor/Pool.cpp:972-975) or its plain
 // rule (padding never wins).
-constexpr int SP_PX = 16, SP_PY = 7;                       // pooled tile: 33x15 = 495 convolution outputs ~ 2 x 256 threads
+constexpr int SP_PX = 16, SP_PY = 6;                         // pooled tile
 constexpr int SP_CX = 2 * SP_PX + 1, SP_CY = 2 * SP_PY + 1;  // convolution outputs under it
+constexpr int SP_PW = 9, SP_PH = 7, SP_ROWS = 64;            // convolution outputs of a patch, 63 and a row nobody reads
 
-// The multiply-adds run on the tensor cores: the 27 taps of a convolution pixel, gathered into 7 registers with funnel shifts
-// and byte permutes exactly as in the kernel above, are written out as one 32-byte row of an im2col tile in shared memory,
-// and four tcgen05 MMAs (M = 128 pixels, N = 32 channels, K = 32) produce the exact s32 accumulators of the CTA's 495
-// convolution pixels in TMEM. (A dp4a version of this kernel was measured first: 0.333 ms for 256 images of 320x320 against
-// 0.323 ms here; both are bound by the instruction count of the quantize, epilogue and pooling phases, not by the
-// multiply-adds.) One CTA = one pooled tile, no pipeline: build, fence, issue, wait (bounded), read, pool.
-// Shared memory per CTA is above a third of the SM's, so at most three CTAs (3 x 128 TMEM columns) are ever resident.
-constexpr int SPM_ROWS = 512;                 // im2col rows: 495 convolution pixels rounded up to 4 MMA tiles
-constexpr uint32_t SPM_TMEM_COLS = 128;       // 4 accumulators of 32 columns
-
+// The multiply-adds run on the tensor cores with channels as accumulator rows. A convolution pixel's 27 taps, gathered into 7 registers
+// with funnel shifts and byte permutes exactly as in the kernel above, are 32 bytes of a shared-memory row; a row has those of the same
+// pixel of four patches side by side (K = 128), and the filters stand four times on the diagonal of a 128 x 128 matrix, so that
+// D[32 g + channel, pixel] = filter(channel) * taps(patch g, pixel): three quarters of the products are with zeros, which the tensor pipe has
+// to spare (four MMAs, 256 cycles per CTA). Warp g of a lane quarter then holds one channel per lane and the pixels of ONE patch as
+// columns: the pool is 40 three-way maxima of its own registers, the epilogue's parameters are three registers, and nothing of the 495
+// accumulators goes through shared memory (which it did, 16 bytes at a time, at two thirds of what that pipe delivers). The fp32 halo
+// tile comes as one TMA box, zeros outside the image included, and is quantized word by word in the order it lies. The CTAs stay (four per
+// SM) and set the filter matrix and tensor memory up once; the next tile's box comes while this one is pooled. 24 channels, 320x320 x256, int8
+// out: 212 us with pixels as rows, an index calculation per loaded word and a CTA per tile; 174 with channels as rows and boxes, 151 with CTAs
+// that stay (48 at the copy rate). What is left is issue slots (half of them), spread over the phases.
+//
 // OUT8: the pooled values leave quantized, float2int8(v * scale_out[channel]), as an int8 NHWC tensor (what the quantize pass of
-// the layers reading the pooled blob would compute from the fp32 values) instead of fp32 NCHW planes.
-// C24: the instance for the usual first layer (24 output channels, a bias, the add-half-truncate rounding rule): channel-group
-// counts, the accumulator tile's pitch, the bias switch and the rounding rule are compile-time constants there, so the
-// channel loops unroll and their addresses are immediates (a fifth fewer instructions in a kernel bound by instruction issue).
-template <int S, int ACT, bool OUT8, bool C24>
-__global__ void __launch_bounds__(256)
-dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ StemParams P, float in_scale, int has_bias_arg, float act_p0,
-                           uint32_t half_arg, void* __restrict__ out_any, ConvShape s_arg, int ph_out, int pw_out, int tiles_x, int tiles_y, int pad_zero,
-                           uint32_t* __restrict__ status) {
+// the layers reading the pooled blob would compute from the fp32 values) instead of fp32 NCHW planes. A warp's four neighbouring
+// pooled pixels of 32 channels leave as 128 consecutive bytes.
+template <int S>
+struct StemTile {
+    static constexpr int IH = (SP_CY - 1) * S + 3;                  // input rows
+    static constexpr int RP = ((SP_CX - 1) * S + 3 + 3) / 4 + 1;    // words of four pixels in a row (tile origin rounded down to 4)
+    static constexpr int WORDS = 3 * IH * RP;
+    // filter matrix, then the fp32 words and later, over them, the rows of taps, then the quantized words
+    static constexpr int TAPS = 16384, REGION = TAPS + (WORDS * 16 > 16384 ? (WORDS * 16 + 1023) / 1024 * 1024 : 16384), BYTES = REGION + WORDS * 4;
+};
+
+template <int S, int ACT, bool OUT8>
+__global__ void __launch_bounds__(256, 4)
+dense_stem_pool_mma_kernel(const __grid_constant__ CUtensorMap image, const float* __restrict__ x, const __grid_constant__ StemParams P, float in_scale, float act_p0,
+                           uint32_t half, void* __restrict__ out_any, ConvShape s, int ph_out, int pw_out, int tiles_x, int tiles_y, int tiles, FastDiv div_x, FastDiv div_y,
+                           int by_box, int pad_zero, uint32_t* __restrict__ status) {
     using namespace umma;
-    const int has_bias = C24 ? 1 : has_bias_arg;
-    const uint32_t half = C24 ? kHalfTrunc : half_arg;
-    ConvShape s = s_arg;
-    if (C24) { s.cout = 24; s.cout_pad = 32; }
-    constexpr int IW = (SP_CX - 1) * S + 3, IH = (SP_CY - 1) * S + 3;
-    constexpr int RP = (IW + 3 + 3) / 4 + 1;
+    using Tile = StemTile<S>;
+    constexpr int IH = Tile::IH, RP = Tile::RP, WORDS = Tile::WORDS;
     extern __shared__ uint8_t smem_spm[];
     const uint32_t base = (smem_u32(smem_spm) + 1023u) & ~1023u;
     uint8_t* bp = smem_spm + (base - smem_u32(smem_spm));
-    uint8_t* sA = bp;                                   // [512 rows][32 B], 32-byte swizzle
-    uint8_t* sB = bp + SPM_ROWS * 32;                   // [32 output channels][32 B]
-    uint32_t(*tin)[IH][RP] = reinterpret_cast<uint32_t(*)[IH][RP]>(bp + SPM_ROWS * 32 + 1024);  // [3][IH][RP]
-    // The s32 accumulators of the convolution tile, [pixel][pitch]: written once the MMAs have completed, over the im2col
-    // rows, the filter rows and the input planes, which are all dead by then.
-    int* cacc = reinterpret_cast<int*>(bp);
-    const int cout4 = (s.cout + 3) >> 2;   // 4-channel groups
-    const int pitch = cout4 * 4 + 4;       // s32 per pixel row: 4 mod 8 words, so the 16-byte accesses of both phases spread over the banks
+    uint8_t* sW = bp;               // [128][128 B]: the filters on the diagonal, 128-byte swizzle
+    uint8_t* sT = bp + Tile::TAPS;  // [128][128 B]: pixel 64 (patch / 4) + i of patches 0..3 or 4..7, 128-byte swizzle
+    uint32_t* tin = reinterpret_cast<uint32_t*>(bp + Tile::REGION);  // [3][IH][RP] int8 channel planes
     __shared__ __align__(16) float sprm[3][ST_COUT_MAX];  // scale_in, bias, scale_out
-    __shared__ __align__(8) unsigned long long bar_storage;
+    __shared__ __align__(8) unsigned long long bar_storage[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    const uint32_t bar = smem_u32(&bar_storage);
+    const uint32_t bar_x = smem_u32(&bar_storage[0]), bar_d = smem_u32(&bar_storage[1]);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    int b = blockIdx.x;
-    const int tx = b % tiles_x; b /= tiles_x;
-    const int ty = b % tiles_y;
-    const int img = b / tiles_y;
-    const int px0 = tx * SP_PX, py0 = ty * SP_PY;     // first pooled pixel of the tile
-    const int cx0 = px0 * 2 - 1, cy0 = py0 * 2 - 1;   // first convolution output under it (pool pad 1)
-    const int iy0 = cy0 * S - s.ph, ix_first = cx0 * S - s.pw;
-    const int ix_al = (ix_first >= 0 ? ix_first : ix_first - 3) / 4 * 4;
-    const int sh = ix_first - ix_al;
+    // where a tile lies: its image, first pooled pixel, and the word its first input column lies in
+    struct Place {
+        int img, px0, py0, ix_al;
+    };
+    const auto locate = [&](int t) {
+        const int row = (int)fast_div((uint32_t)t, div_x), img = (int)fast_div((uint32_t)row, div_y), px0 = (t - row * tiles_x) * SP_PX;
+        const int ix = (2 * px0 - 1) * S - s.pw;  // (pool pad 1)
+        return Place{img, px0, (row - img * tiles_y) * SP_PY, (ix >= 0 ? ix : ix - 3) / 4 * 4};
+    };
+    const auto fetch = [&](int t) {
+        const Place a = locate(t);
+        mbar_expect_tx(bar_x, (uint32_t)WORDS * 16u);
+        tma_load_4d(&image, bar_x, base + Tile::TAPS, a.ix_al, (2 * a.py0 - 1) * S - s.ph, 0, a.img);
+    };
 
+    if (warp == 7) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(128u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        pdl_launch_dependents();  // not before this CTA has its tensor memory: see dense_umma.cu
+    }
     if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
+        mbar_init(bar_x, 1);
+        mbar_init(bar_d, 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (by_box) {
+            pdl_wait();
+            fetch((int)blockIdx.x);
+        }
     }
     if (threadIdx.x >= 64 && threadIdx.x < 64 + ST_COUT_MAX) {
         const int o = threadIdx.x - 64;
@@ -195,42 +224,44 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
         sprm[1][o] = P.bias[o];
         sprm[2][o] = P.scale_out[o];
     }
-    if (warp == 7) {  // the warp that pools nothing (224 of the 256 threads do): its de-allocation below delays nobody
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(SPM_TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        pdl_launch_dependents();  // not before this CTA has its tensor memory: see dense_umma.cu
-    }
-    // filters: row = output channel, 28 bytes of taps + 4 zero bytes, swizzled like the im2col rows
-    if (threadIdx.x < 64) {
-        const int o = threadIdx.x >> 1, j = threadIdx.x & 1;
-        const uint4 w4 = j == 0 ? make_uint4(P.w[o][0], P.w[o][1], P.w[o][2], P.w[o][3]) : make_uint4(P.w[o][4], P.w[o][5], P.w[o][6], 0u);
-        *reinterpret_cast<uint4*>(sB + o * 32 + ((j ^ ((o >> 2) & 1)) << 4)) = w4;
-    }
-    pdl_wait();  // set-up above overlaps the previous kernel; the image is read and the output written after it
-    // quantized input halo tile, as int8 channel planes. All of a thread's loads are issued before the first is used: the CTA
-    // runs its phases one after the other, so this phase's DRAM latency must be paid once, not once per loop trip.
-    const float* ximg = x + (long)img * 3 * s.h * s.w;
-    const bool vec_ok = s.w % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;  // four pixels are one 16-byte load
-    constexpr int TIN_WORDS = 3 * IH * RP, TIN_TRIPS = (TIN_WORDS + 255) / 256;
-    if (vec_ok) {
-        float4 v[TIN_TRIPS];
+    // filter matrix: row 32 g + channel, 28 bytes of taps and 4 of zeros at byte 32 g
+    {
+        const int row = threadIdx.x >> 1, j = threadIdx.x & 1;
 #pragma unroll
-        for (int u = 0; u < TIN_TRIPS; ++u) {
-            const int i = threadIdx.x + 256 * u;
-            const int xw = i % RP, r = (i / RP) % IH, c = i / (RP * IH);
-            const int iy = iy0 + r, ix = ix_al + xw * 4;
-            // w % 4 == 0 and ix % 4 == 0: an aligned float4 is wholly inside the row or wholly outside
-            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < TIN_WORDS && iy >= 0 && iy < s.h && ix >= 0 && ix < s.w)
-                v[u] = __ldg(reinterpret_cast<const float4*>(ximg + ((long)c * s.h + iy) * s.w + ix));
+        for (int d = 1; d < 4; ++d) {
+            const int chunk = 2 * (((row >> 5) + d) & 3) + j;
+            *reinterpret_cast<uint4*>(sW + row * 128 + ((chunk ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
         }
+        if (threadIdx.x < 64) {
+            const uint4 w4 = j == 0 ? make_uint4(P.w[row][0], P.w[row][1], P.w[row][2], P.w[row][3]) : make_uint4(P.w[row][4], P.w[row][5], P.w[row][6], 0u);
 #pragma unroll
-        for (int u = 0; u < TIN_TRIPS; ++u) {
-            const int i = threadIdx.x + 256 * u;
-            if (i < TIN_WORDS) (&tin[0][0][0])[i] = quantize4_pack(v[u].x, v[u].y, v[u].z, v[u].w, in_scale, half);
+            for (int g = 0; g < 4; ++g) *reinterpret_cast<uint4*>(sW + (32 * g + row) * 128 + (((2 * g + j) ^ (row & 7)) << 4)) = w4;
+        }
+    }
+    __syncthreads();
+    pdl_wait();  // set-up above overlaps the previous kernel; the image is read and the output written after it
+    const uint32_t tmem_base = tmem_slot;
+    const int c = lane, g = warp & 3, row3 = 3 * (warp >> 2);  // this thread's channel, its warp's patch: pooled columns 4 g .. 4 g + 3, rows row3 .. row3 + 2
+    const float p_si = sprm[0][c], p_bi = sprm[1][c], p_so = sprm[2][c];
+    bool ok = true;
+    uint32_t phase = 0;
+    for (int t = (int)blockIdx.x; t < tiles; t += (int)gridDim.x, phase ^= 1u) {
+    if (by_box) {
+        if (!mbar_wait(bar_x, phase, &abort_flag, status, 32u)) {
+            ok = false;
+            const unsigned long long t0 = globaltimer_ns();
+            while (globaltimer_ns() - t0 < 1000000ull) {}  // let the copy in flight land before its place is written
+        }
+#pragma unroll 2
+        for (int i = threadIdx.x; i < WORDS; i += 256) {
+            const float4 v = reinterpret_cast<const float4*>(sT)[i];
+            tin[i] = quantize4_pack(v.x, v.y, v.z, v.w, in_scale, half);
         }
     } else {
-        for (int i = threadIdx.x; i < TIN_WORDS; i += 256) {
+        const Place a = locate(t);
+        const float* ximg = x + (long)a.img * 3 * s.h * s.w;
+        const int iy0 = (2 * a.py0 - 1) * S - s.ph, ix_al = a.ix_al;
+        for (int i = threadIdx.x; i < WORDS; i += 256) {
             const int xw = i % RP, r = (i / RP) % IH, c = i / (RP * IH);
             const int iy = iy0 + r, ix = ix_al + xw * 4;
             uint32_t word = 0;
@@ -242,26 +273,30 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
                     if (ix + j >= 0 && ix + j < s.w) q[j] = quantize1(__ldg(row + ix + j), in_scale, half);
                 word = pack4(q[0], q[1], q[2], q[3]);
             }
-            (&tin[0][0][0])[i] = word;
+            tin[i] = word;
         }
     }
     __syncthreads();
 
-    // im2col rows: pixel p of the 33x15 convolution tile -> row p (byte k = tap (c, ky, kx), k = c*9 + ky*3 + kx)
-    for (int p = threadIdx.x; p < SPM_ROWS; p += 256) {
-        uint4 c0 = make_uint4(0, 0, 0, 0), c1 = make_uint4(0, 0, 0, 0);
-        if (p < SP_CX * SP_CY) {
-            const int lx = p % SP_CX, ly = p / SP_CX;
-            const int boff = sh + lx * S;
+    const Place at = locate(t);
+    // rows of taps (byte k = tap (c, ky, kx), k = c*9 + ky*3 + kx)
+#pragma unroll
+    for (int rep = 0; rep < 2; ++rep) {
+        const int p = threadIdx.x + 256 * rep, patch = p / SP_ROWS, i = p % SP_ROWS, g = patch & 3, n = (patch >> 2) * SP_ROWS + i;
+        if (i < SP_PW * SP_PH) {
+            const int lx = 8 * g + i % SP_PW, ly = 6 * (patch >> 2) + i / SP_PW;
+            const int boff = (2 * at.px0 - 1 + lx) * S - s.pw - at.ix_al;
             const int wi = boff >> 2, bs = (boff & 3) * 8;
+            const uint32_t* t0 = tin + ly * S * RP + wi;
             uint32_t win[9];
 #pragma unroll
             for (int c = 0; c < 3; ++c)
 #pragma unroll
                 for (int ky = 0; ky < 3; ++ky) {
-                    const uint32_t* q = &tin[c][ly * S + ky][wi];
+                    const uint32_t* q = t0 + (c * IH + ky) * RP;
                     win[c * 3 + ky] = __funnelshift_r(q[0], q[1], bs);
                 }
+            uint4 c0, c1;
             c0.x = __byte_perm(win[0], win[1], 0x4210);
             c0.y = __byte_perm(win[1], win[2], 0x5421);
             c0.z = __byte_perm(win[2], win[3], 0x6542);
@@ -269,126 +304,122 @@ dense_stem_pool_mma_kernel(const float* __restrict__ x, const __grid_constant__ 
             c1.x = __byte_perm(win[5], win[6], 0x5421);
             c1.y = __byte_perm(win[6], win[7], 0x6542);
             c1.z = __byte_perm(win[8], 0u, 0x4210);
+            c1.w = 0u;
+            *reinterpret_cast<uint4*>(sT + n * 128 + (((2 * g) ^ (n & 7)) << 4)) = c0;
+            *reinterpret_cast<uint4*>(sT + n * 128 + (((2 * g + 1) ^ (n & 7)) << 4)) = c1;
         }
-        const int swz = (p >> 2) & 1;
-        *reinterpret_cast<uint4*>(sA + p * 32 + ((0 ^ swz) << 4)) = c0;
-        *reinterpret_cast<uint4*>(sA + p * 32 + ((1 ^ swz) << 4)) = c1;
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the MMA's reads
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tmem_slot;
 
-    if (threadIdx.x == 32) {
-        // D = s32, A = B = signed int8, both K-major, N = 32, M = 128
-        const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((32u >> 3) << 17) | ((128u >> 4) << 24);
-        const uint64_t bdesc = make_smem_desc(smem_u32(sB), 32);
+    if (warp == 1) {
+        if (elect_one()) {
+            // D = s32, A = B = signed int8, both K-major, N = 128, M = 128
+            const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+            const uint64_t wdesc = make_smem_desc(smem_u32(sW), 128), tdesc = make_smem_desc(smem_u32(sT), 128);
 #pragma unroll
-        for (int t = 0; t < SPM_ROWS / 128; ++t) umma_i8(tmem_base + 32u * t, make_smem_desc(smem_u32(sA) + 4096u * t, 32), bdesc, idesc, 0u);
-        umma_commit(bar);
+            for (int k = 0; k < 4; ++k) umma_i8(tmem_base, wdesc + 2u * k, tdesc + 2u * k, idesc, k != 0 ? 1u : 0u);
+            umma_commit(bar_d);
+        }
+        __syncwarp();
     }
-    const bool ok = mbar_wait(bar, 0, &abort_flag, status, 32u);
+    if (!mbar_wait(bar_d, phase, &abort_flag, status, 32u)) ok = false;
     tc_fence_after();
+    // the next tile's box takes the place of the taps, which the MMAs have read, while this tile is pooled
+    if (by_box && threadIdx.x == 0 && ok && t + (int)gridDim.x < tiles) fetch(t + (int)gridDim.x);
 
     if (ok) {
-        // Accumulators -> shared memory as they are (one 16-byte store per four channels). Max-pooling happens on these exact
-        // s32 sums: dequantize + activation is non-decreasing in the sum for the non-negative scales the layer is prepared with,
-        // so the maximum of the window's outputs is the output of the window's maximum, bit for bit, and the float epilogue
-        // runs once per pooled value instead of once per convolution output. Pixels outside the image never win.
-        const int q = warp & 3;  // TMEM lane quarter this warp may read
-#pragma unroll
-        for (int rep = 0; rep < 2; ++rep) {
-            const int t = (warp >> 2) + 2 * rep;
-            const int p = t * 128 + q * 32 + lane;
-            const int lx = p % SP_CX, ly = p / SP_CX;
-            const int ox = cx0 + lx, oy = cy0 + ly;
-            const bool inside = ox >= 0 && ox < s.ow && oy >= 0 && oy < s.oh;
-            const uint32_t taddr = tmem_base + 32u * t + ((uint32_t)(q * 32) << 16);
+        // Max-pooling happens on the exact s32 sums: dequantize + activation is non-decreasing in the sum for the non-negative scales the
+        // layer is prepared with, so the maximum of the window's outputs is the output of the window's maximum, bit for bit, and the
+        // float epilogue runs once per pooled value instead of once per convolution output. Pixels outside the image never win.
+        const int ox0 = 2 * at.px0 - 1 + 8 * g, oy0 = 2 * at.py0 - 1 + 2 * row3;  // the patch's first convolution output
+        const bool edge = ox0 < 0 || oy0 < 0 || ox0 + SP_PW > s.ow || oy0 + SP_PH > s.oh;  // (uniform)
+        const uint32_t taddr = tmem_base + ((uint32_t)(g * 32) << 16) + (uint32_t)((warp >> 2) * SP_ROWS);
+        int h[SP_PH][4], rest[5];  // maxima of three neighbours in a row; the start of a row that the first 32 columns cut
+        auto inside = [&](int i) { return (unsigned)(ox0 + i % SP_PW) < (unsigned)s.ow && (unsigned)(oy0 + i / SP_PW) < (unsigned)s.oh; };
+        {
             int v[32];
-            __syncwarp();
             tmem_ld16(taddr, *reinterpret_cast<int(*)[16]>(&v[0]));
-            if (s.cout > 16) tmem_ld16(taddr + 16u, *reinterpret_cast<int(*)[16]>(&v[16]));  // warp-uniform
+            tmem_ld16(taddr + 16u, *reinterpret_cast<int(*)[16]>(&v[16]));
             tmem_wait_ld16(*reinterpret_cast<int(*)[16]>(&v[0]));
             tmem_wait_ld16(*reinterpret_cast<int(*)[16]>(&v[16]));
-            if (p >= SP_CX * SP_CY) continue;
-            int4* dst = reinterpret_cast<int4*>(cacc + p * pitch);
-            if (inside) {
+            if (edge)
 #pragma unroll
-                for (int g = 0; g < ST_COUT_MAX / 4; ++g)
-                    if (g < cout4) dst[g] = make_int4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-            } else {
+                for (int i = 0; i < 32; ++i)
+                    if (!inside(i)) v[i] = INT_MIN;
 #pragma unroll
-                for (int g = 0; g < ST_COUT_MAX / 4; ++g)
-                    if (g < cout4) dst[g] = make_int4(INT_MIN, INT_MIN, INT_MIN, INT_MIN);
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) h[r][k] = __vimax3_s32(v[r * 9 + 2 * k], v[r * 9 + 2 * k + 1], v[r * 9 + 2 * k + 2]);
+#pragma unroll
+            for (int j = 0; j < 5; ++j) rest[j] = v[27 + j];
+        }
+        {
+            int v[32];
+            tmem_ld16(taddr + 32u, *reinterpret_cast<int(*)[16]>(&v[0]));
+            tmem_ld16(taddr + 48u, *reinterpret_cast<int(*)[16]>(&v[16]));
+            tmem_wait_ld16(*reinterpret_cast<int(*)[16]>(&v[0]));
+            tmem_wait_ld16(*reinterpret_cast<int(*)[16]>(&v[16]));
+            if (edge)
+#pragma unroll
+                for (int i = 0; i < 31; ++i)
+                    if (!inside(32 + i)) v[i] = INT_MIN;
+            h[3][0] = __vimax3_s32(rest[0], rest[1], rest[2]);
+            h[3][1] = __vimax3_s32(rest[2], rest[3], rest[4]);
+            h[3][2] = __vimax3_s32(rest[4], v[0], v[1]);
+            h[3][3] = __vimax3_s32(v[1], v[2], v[3]);
+#pragma unroll
+            for (int r = 4; r < SP_PH; ++r)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) h[r][k] = __vimax3_s32(v[r * 9 - 32 + 2 * k], v[r * 9 - 31 + 2 * k], v[r * 9 - 30 + 2 * k]);
+        }
+        const int px = at.px0 + 4 * g;
+        const long pplane = (long)ph_out * pw_out;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            const int py = at.py0 + row3 + r;
+            float y[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int m = __vimax3_s32(h[2 * r][k], h[2 * r + 1][k], h[2 * r + 2][k]);
+                y[k] = activate_t<ACT>(__fmaf_rn(__int2float_rn(m), p_si, p_bi), act_p0);
+                if (ACT != ACT_RELU && ACT != ACT_RELU6) {  // (after a ReLU nothing is below the padding's 0)
+                    // the reference's packed max-pool lets the padding take part as 0 (Tensor/Pool.cpp:972-975); its plain one never lets it win
+                    const int cx = 2 * (px + k) - 1, cy = 2 * py - 1;
+                    if (pad_zero && (cx < 0 || cx + 2 >= s.ow || cy < 0 || cy + 2 >= s.oh)) y[k] = fmaxf(y[k], 0.f);
+                }
+            }
+            if (OUT8) {
+                const int2 a = round2(__fmul2_rn(make_float2(y[0], y[1]), make_float2(p_so, p_so)), half);
+                const int2 e = round2(__fmul2_rn(make_float2(y[2], y[3]), make_float2(p_so, p_so)), half);
+                uint32_t w = c < s.cout ? pack_sat_s8x4(a.x, a.y, e.x, e.y) : 0u;
+                // 4x4 byte transpose across four lanes: lane 4 k + p then holds pixel p's channels 4 k .. 4 k + 3
+                const int p = lane & 3;
+                w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 2), p < 2 ? 0x5410u : 0x3276u);
+                w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 1), (p & 1) == 0 ? 0x6240u : 0x3715u);
+                const int cq = lane & ~3;
+                if (py < ph_out && px + p < pw_out && cq < s.cout_pad)
+                    *reinterpret_cast<uint32_t*>(static_cast<int8_t*>(out_any) + (((long)at.img * ph_out + py) * pw_out + px + p) * s.cout_pad + cq) = w;
+            } else if (py < ph_out && c < s.cout) {
+                float* o = static_cast<float*>(out_any) + ((long)at.img * s.cout + c) * pplane + (long)py * pw_out + px;
+                if (px + 3 < pw_out && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+                    *reinterpret_cast<float4*>(o) = make_float4(y[0], y[1], y[2], y[3]);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (px + k < pw_out) o[k] = y[k];
+                }
             }
         }
     }
-    tc_fence_before();
+    tc_fence_before();  // (the next tile's MMAs come after the barriers below its loads)
+    }
     __syncthreads();
     if (warp == 7) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(SPM_TMEM_COLS) : "memory");
-    }
-    if (!ok) return;
-
-    // thread = (pooled pixel, half of the channels): the two threads of a pixel are neighbours, so its channels leave together
-    const int half_groups = (cout4 + 1) >> 1;
-    const long pplane = (long)ph_out * pw_out;
-    for (int i = threadIdx.x; i < 2 * SP_PY * SP_PX; i += 256) {
-        const int g = i & 1, lx = (i >> 1) % SP_PX, ly = (i >> 1) / SP_PX;
-        const int px = px0 + lx, py = py0 + ly;
-        if (px >= pw_out || py >= ph_out) continue;
-        // the reference's packed max-pool lets the padding take part as 0 (Tensor/Pool.cpp:972-975); its plain one never lets it win
-        const bool pad_counts = pad_zero && (2 * py - 1 < 0 || 2 * py + 1 >= s.oh || 2 * px - 1 < 0 || 2 * px + 1 >= s.ow);
-        const int* cp = cacc + ((2 * ly) * SP_CX + 2 * lx) * pitch;
-        const int q_end = g == 0 ? half_groups : cout4;
-        for (int q4 = g == 0 ? 0 : half_groups; q4 < q_end; ++q4) {
-            const int4* w0 = reinterpret_cast<const int4*>(cp + 4 * q4);
-            int4 v[9];
-#pragma unroll
-            for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-                for (int dx = 0; dx < 3; ++dx) v[dy * 3 + dx] = *reinterpret_cast<const int4*>(reinterpret_cast<const int*>(w0) + (dy * SP_CX + dx) * pitch);
-            int m[4];
-#define OTT_MAX9(F) __vimax3_s32(__vimax3_s32(v[0].F, v[1].F, v[2].F), __vimax3_s32(v[3].F, v[4].F, v[5].F), __vimax3_s32(v[6].F, v[7].F, v[8].F))
-            m[0] = OTT_MAX9(x); m[1] = OTT_MAX9(y); m[2] = OTT_MAX9(z); m[3] = OTT_MAX9(w);
-#undef OTT_MAX9
-            const float4 si = *reinterpret_cast<const float4*>(&sprm[0][4 * q4]);
-            const float4 bi = *reinterpret_cast<const float4*>(&sprm[1][4 * q4]);
-            const float sia[4] = {si.x, si.y, si.z, si.w}, bia[4] = {bi.x, bi.y, bi.z, bi.w};
-            float y[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float a = __int2float_rn(m[j]);
-                y[j] = activate_t<ACT>(has_bias ? __fmaf_rn(a, sia[j], bia[j]) : __fmul_rn(a, sia[j]), act_p0);
-                if (ACT != ACT_RELU && ACT != ACT_RELU6 && pad_counts) y[j] = fmaxf(y[j], 0.f);  // (after a ReLU nothing is below the padding's 0)
-            }
-            if (OUT8) {
-                const float4 so = *reinterpret_cast<const float4*>(&sprm[2][4 * q4]);
-                const float soa[4] = {so.x, so.y, so.z, so.w};
-                int qv[4];
-#pragma unroll
-                for (int j = 0; j < 4; j += 2) {
-                    // after ReLU / ReLU6 nothing is negative where the scales are positive (the host gives C24 no others); the saturating
-                    // pack clamps at 127
-                    const float2 t = __fmul2_rn(make_float2(y[j], y[j + 1]), make_float2(soa[j], soa[j + 1]));
-                    const int2 r = C24 ? round2_act<ACT>(t, half) : round2(t, half);
-                    qv[j] = 4 * q4 + j >= s.cout ? 0 : r.x;
-                    qv[j + 1] = 4 * q4 + j + 1 >= s.cout ? 0 : r.y;
-                }
-                *reinterpret_cast<uint32_t*>(static_cast<int8_t*>(out_any) + (((long)img * ph_out + py) * pw_out + px) * s.cout_pad + 4 * q4) =
-                    pack_sat_s8x4(qv[0], qv[1], qv[2], qv[3]);
-            } else {
-                float* o = static_cast<float*>(out_any) + ((long)img * s.cout + 4 * q4) * pplane + (long)py * pw_out + px;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (4 * q4 + j < s.cout) o[j * pplane] = y[j];
-            }
-        }
-        if (OUT8 && g == 1)  // padding channels of the int8 row (the stride is a multiple of 16 channels): zeros
-            for (int c4 = cout4; c4 < s.cout_pad / 4; ++c4)
-                *reinterpret_cast<uint32_t*>(static_cast<int8_t*>(out_any) + (((long)img * ph_out + py) * pw_out + px) * s.cout_pad + 4 * c4) = 0u;
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(128u) : "memory");
     }
 }
 
@@ -433,23 +464,35 @@ static void fill_stem_params(StemParams& P, const ConvShape& s, const int8_t* w,
 template <int S, bool OUT8>
 static cudaError_t launch_pool_s(cudaStream_t stream, const float* x, const StemParams& P, float in_scale, const EpilogueParams& ep, void* out,
                                  const ConvShape& s, int pad_zero, uint32_t* status) {
+    using Tile = StemTile<S>;
     const int ph_out = (s.oh + 2 - 3) / 2 + 1, pw_out = (s.ow + 2 - 3) / 2 + 1;
     const int tiles_x = (pw_out + SP_PX - 1) / SP_PX, tiles_y = (ph_out + SP_PY - 1) / SP_PY;
     const long blocks = (long)s.n * tiles_x * tiles_y;
     if (blocks <= 0) return cudaSuccess;
-    constexpr int IW = (SP_CX - 1) * S + 3, IH = (SP_CY - 1) * S + 3, RP = (IW + 3 + 3) / 4 + 1;
-    // alignment slack + the larger of (im2col rows + filter rows + input tile) and the s32 convolution tile that later overlays them
-    const size_t front = (size_t)SPM_ROWS * 32 + 1024 + (size_t)3 * IH * RP * 4;
-    const size_t tile = (size_t)SP_CY * SP_CX * (((s.cout + 3) / 4) * 4 + 4) * 4;
-    const size_t smem = 1024 + (front > tile ? front : tile);
-    const bool c24 = s.cout == 24 && s.cout_pad == 32 && ep.has_bias && ep.rounding == ROUND_ADD_HALF_TRUNC && (!OUT8 || !ep.negative_scale);
+    if (blocks > 0x7FFFFFFFl) return cudaErrorInvalidValue;
+    constexpr long kResident = 148 * 4;  // CTAs of the whole GPU at once; each walks over its tiles
+    // the halo tile as one box: rows of whole 16-byte words from a 16-byte boundary; any other image pixel by pixel
+    CUtensorMap image{};
+    const int by_box = s.w % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? 1 : 0;
+    if (by_box) {
+        const EncodeTiledFn enc = encode_tiled();
+        if (!enc) return cudaErrorNotSupported;
+        cuuint64_t dims[4] = {(cuuint64_t)s.w, (cuuint64_t)s.h, 3, (cuuint64_t)s.n};
+        cuuint64_t strides[3] = {(cuuint64_t)s.w * 4, (cuuint64_t)s.w * s.h * 4, (cuuint64_t)s.w * s.h * 12};
+        cuuint32_t box[4] = {Tile::RP * 4, Tile::IH, 3, 1}, one[4] = {1, 1, 1, 1};
+        if (enc(&image, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(x), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    const size_t smem = 1024 + Tile::BYTES;
 #define OTT_STEMPOOL_LAUNCH(ACT)                                                                                          \
     {                                                                                                                     \
-        auto kernel = c24 ? dense_stem_pool_mma_kernel<S, ACT, OUT8, true> : dense_stem_pool_mma_kernel<S, ACT, OUT8, false>;    \
+        auto kernel = dense_stem_pool_mma_kernel<S, ACT, OUT8>;                                                           \
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);            \
         if (e != cudaSuccess) return e;                                                                                   \
-        e = launch_overlapped(kernel, dim3((unsigned)blocks), dim3(256), smem, stream, x, P, in_scale, ep.has_bias, ep.act_param0,        \
-                              half_bits(ep.rounding), out, s, ph_out, pw_out, tiles_x, tiles_y, pad_zero, status);                    \
+        e = launch_overlapped(kernel, dim3((unsigned)(blocks < kResident ? blocks : kResident)), dim3(256), smem, stream, image, x, P, in_scale,  \
+                              ep.act_param0, half_bits(ep.rounding), out, s, ph_out, pw_out, tiles_x, tiles_y, (int)blocks,             \
+                              make_fast_div((uint32_t)tiles_x), make_fast_div((uint32_t)tiles_y), by_box, pad_zero, status);            \
         if (e != cudaSuccess) return e;                                                                                   \
     }
     switch (ep.act_type) {
@@ -468,6 +511,7 @@ cudaError_t launch_dense_stem_pool(cudaStream_t stream, const ConvShape& s, cons
                                    int out_dtype, int pad_zero, uint32_t* status) {
     StemParams P{};
     fill_stem_params(P, s, w_oihw_host, scale_in_host, bias_host, out_dtype == DT_S8_NHWC ? scale_out_host : nullptr);
+    for (int o = 0; o < ST_COUT_MAX && !ep.has_bias; ++o) P.bias[o] = -0.f;  // (see epilogue.cuh)
     if (out_dtype == DT_S8_NHWC)
         return s.sh == 1 ? launch_pool_s<1, true>(stream, x, P, in_scale, ep, out, s, pad_zero, status)
                          : launch_pool_s<2, true>(stream, x, P, in_scale, ep, out, s, pad_zero, status);
