@@ -74,16 +74,17 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
     const int cb0 = grp * P.ncb;
     const int nb = P.ncb_total - cb0 < P.ncb ? P.ncb_total - cb0 : P.ncb;
     const int c_base = cb0 * kBlock;
+    const int issuers = nb < kIssueWarps ? nb : kIssueWarps;
     if (threadIdx.x == 0) {
         prefetch_tensormap(&tmW);
         for (int cb = 0; cb < nb; ++cb) prefetch_tensormap(&maps.tm[maps.block_src[cb0 + cb]]);
         mbar_init(bar_w, 1);
         for (int i = 0; i < P.stages; ++i) {
             mbar_init(bar_full + 8u * i, 1);
-            mbar_init(bar_empty + 8u * i, (uint32_t)nb);  // one commit per issuing lane
+            mbar_init(bar_empty + 8u * i, (uint32_t)issuers);  // one commit per issuing warp
         }
         for (int i = 0; i < P.acc_bufs; ++i) {
-            mbar_init(bar_afull + 8u * i, (uint32_t)nb);
+            mbar_init(bar_afull + 8u * i, (uint32_t)issuers);
             mbar_init(bar_aempty + 8u * i, kEpiWarps);
         }
         *abort_flag = 0;
@@ -115,20 +116,20 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
     const uint32_t acc_mask = (uint32_t)P.acc_bufs - 1u;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- TMA producer ----
-            uint32_t it = 0;
+            uint32_t st = 0, ph = 0;
             bool ok = true;
-            for (int m = m_first; ok && m < P.m_tiles; m += m_step, ++it) {
-                const int img = m / per_img, r = m - img * per_img;
-                const int y0 = (r / P.tiles_x) * kTh * P.stride - 1, x0 = (r % P.tiles_x) * kTw * P.stride - 1;
-                const uint32_t st = it % P.stages, ph = (it / P.stages) & 1u;
+            for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
+                const int img = (int)fast_div((uint32_t)m, P.div_img), r = m - img * per_img, ty = (int)fast_div((uint32_t)r, P.div_x);
+                const int y0 = ty * kTh * P.stride - 1, x0 = (r - ty * P.tiles_x) * kTw * P.stride - 1;
                 if (!mbar_wait(bar_empty + 8u * st, ph ^ 1u, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
                 mbar_expect_tx(bar_full + 8u * st, (uint32_t)(nb * P.sets * P.set_load_bytes));
                 for (int cb = 0; cb < nb; ++cb)
                     for (int s = 0; s < P.sets; ++s)
                         tma_load_4d(&maps.tm[maps.block_src[cb0 + cb]], bar_full + 8u * st,
                                     sX + st * (uint32_t)P.stage_bytes + (uint32_t)(cb * P.block_bytes + s * P.set_bytes), (int)maps.block_x[cb0 + cb], x0 + s, y0, img);
+                if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1u; }
             }
             if (!ok) {
                 const unsigned long long t0 = globaltimer_ns();
@@ -136,44 +137,42 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
             }
         }
     } else if (warp <= kIssueWarps) {
-        // lane l of issuing warp w takes channel block w + l * (issuing warps)
-        const int cb = (warp - 1) + lane * kIssueWarps;
-        if (cb < nb) {
-            // ---- MMA issuers: lane cb issues the nine taps of channel block cb (an MMA is started by one thread; the lanes of
-            // the warp execute the instruction together, so a tile costs nine issue slots however many channel blocks it has),
-            // and commits its own MMAs to the barriers, whose arrival counts are the number of issuing lanes ----
+        if (warp <= issuers && elect_one()) {
+            // ---- MMA issuers: one thread per issuing warp, which takes every kIssueWarps-th channel block, nine taps each ----
             bool ok = mbar_wait(bar_w, 0, abort_flag, status, 16u, P.wait_ns);
             tc_fence_after();
-            // Per tap: the filter matrix's descriptor and the offset of the shifted input view inside a block (16-byte units;
-            // stride 2: the taps kx = 1 read the second column set, kx = 2 one column on). Worked out once: between two MMAs the
-            // issuing thread then only adds a constant to the low word of the block's descriptor (the address field cannot carry).
-            uint64_t bdesc[9];
+            // The offset of a tap's shifted input view inside a block (16-byte units; stride 2: the taps kx = 1 read the second column set,
+            // kx = 2 one column on). Worked out once: between two MMAs the issuing thread only adds to the low words of the block's
+            // descriptors (the address field cannot carry).
             uint32_t aoff[9];
 #pragma unroll
             for (int tap = 0; tap < 9; ++tap) {
                 const int ky = tap / 3, kx = tap % 3;
-                bdesc[tap] = make_smem_desc(sW + (uint32_t)(cb * 9 + tap) * 1024u, kBlock);
                 const int col = P.stride == 1 ? kx : (kx >> 1);
                 aoff[tap] = (uint32_t)((ky * P.set_w + col) * (kBlock >> 4)) + ((P.stride == 2 && kx == 1) ? (uint32_t)(P.set_bytes >> 4) : 0u);
             }
             const uint32_t sbo = (uint32_t)(P.stride * P.set_w * kBlock);
-            uint32_t it = 0;
+            uint32_t it = 0, st = 0, ph = 0;
             for (int m = m_first; ok && m < P.m_tiles; m += m_step, ++it) {
-                const uint32_t buf = it & acc_mask, use = it / (uint32_t)P.acc_bufs;
-                const uint32_t st = it % P.stages, ph = (it / P.stages) & 1u;
+                const uint32_t buf = it & acc_mask, use = it / kMaxAcc;
                 if (!mbar_wait(bar_aempty + 8u * buf, (use & 1u) ^ 1u, abort_flag, status, 4u, P.wait_ns)) { ok = false; break; }
                 if (!mbar_wait(bar_full + 8u * st, ph, abort_flag, status, 2u, P.wait_ns)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t d = tmem_base + buf * (uint32_t)P.cols + (uint32_t)(cb * kBlock);
-                const uint32_t blk = sX + st * (uint32_t)P.stage_bytes + (uint32_t)(cb * P.block_bytes);
-                // 8-row groups (one tile row of 8 pixels each) are `stride` input rows apart
-                const uint64_t a_base = make_smem_desc(blk, kBlock, (int)sbo);
-                const uint32_t a_lo = (uint32_t)a_base;
-                const uint64_t a_hi = a_base & 0xFFFFFFFF00000000ull;
+#pragma unroll 1
+                for (int cb = warp - 1; cb < nb; cb += kIssueWarps) {
+                    const uint32_t d = tmem_base + buf * (uint32_t)P.cols + (uint32_t)(cb * kBlock);
+                    // 8-row groups (one tile row of 8 pixels each) are `stride` input rows apart
+                    const uint64_t a0 = make_smem_desc(sX + st * (uint32_t)P.stage_bytes + (uint32_t)(cb * P.block_bytes), kBlock, (int)sbo);
+                    const uint64_t b0 = make_smem_desc(sW + (uint32_t)(cb * 9) * 1024u, kBlock);
+                    const uint32_t a_lo = (uint32_t)a0, b_lo = (uint32_t)b0;
+                    const uint64_t a_hi = a0 & 0xFFFFFFFF00000000ull, b_hi = b0 & 0xFFFFFFFF00000000ull;
 #pragma unroll
-                for (int tap = 0; tap < 9; ++tap) umma_i8(d, a_hi | (uint64_t)(a_lo + aoff[tap]), bdesc[tap], P.idesc, tap != 0 ? 1u : 0u);
+                    for (int tap = 0; tap < 9; ++tap)
+                        umma_i8(d, a_hi | (uint64_t)(a_lo + aoff[tap]), b_hi | (uint64_t)(b_lo + 64u * tap), P.idesc, tap != 0 ? 1u : 0u);
+                }
                 umma_commit(bar_empty + 8u * st);
                 umma_commit(bar_afull + 8u * buf);
+                if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1u; }
             }
         }
     } else {
@@ -186,11 +185,11 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
         bool ok = true;
         uint32_t it = 0;
         for (int m = m_first; ok && m < P.m_tiles; m += m_step, ++it) {
-            const uint32_t buf = it & acc_mask, use = it / (uint32_t)P.acc_bufs;
+            const uint32_t buf = it & acc_mask, use = it / kMaxAcc;  // (acc_bufs is kMaxAcc)
             if (!mbar_wait(bar_afull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
             tc_fence_after();
-            const int img = m / per_img, r = m - img * per_img;
-            const int oy = (r / P.tiles_x) * kTh + (row >> 3), ox = (r % P.tiles_x) * kTw + (row & 7);
+            const int img = (int)fast_div((uint32_t)m, P.div_img), r = m - img * per_img, ty = (int)fast_div((uint32_t)r, P.div_x);
+            const int oy = ty * kTh + (row >> 3), ox = (r - ty * P.tiles_x) * kTw + (row & 7);
             store_accumulator_row<ACT, OUT>(tmem_base + buf * (uint32_t)P.cols + lane_sel, nb * kBlock, sub, nsub, oy < G.oh && ox < G.ow, img,
                                             (long)oy * G.ow + ox, plane, sp, sp + P.cols, sp + 2 * P.cols, ep.act_param0, G.cpad, G.cout, out, no_side, c_base);
             tc_fence_before();
@@ -336,6 +335,8 @@ const char* launch_dw_umma(cudaStream_t stream, int sm_count, const DwPlan& plan
     p.tiles_x = (s.ow + kTw - 1) / kTw;
     p.tiles_y = (s.oh + kTh - 1) / kTh;
     p.m_tiles = s.n * p.tiles_x * p.tiles_y;
+    p.div_img = make_fast_div((uint32_t)(p.tiles_x * p.tiles_y));
+    p.div_x = make_fast_div((uint32_t)p.tiles_x);
     DwMaps km;
     const int n_src = sources ? sources->n_src : 1;
     if (n_src < 1 || n_src > kUmmaMaxSources) return "bad source count";

@@ -21,6 +21,7 @@ struct DwPlan {
     int smem_bytes;
     // per call
     int tiles_x, tiles_y, m_tiles;
+    FastDiv div_img, div_x;  // by the tiles of an image, of a row of tiles
     unsigned long long wait_ns;
 };
 
