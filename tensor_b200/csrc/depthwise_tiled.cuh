@@ -360,7 +360,9 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
 // best depends on how the CTAs fall on the SMs, so each is rated by the larger of what bounds it: the instructions of the SM with most CTAs (about 2.5 per cycle are
 // issued), or the latency of one CTA (memory round trip, then one warp's dependent instructions at six cycles each) times the
 // waves. The instruction counts are those of the inner loops: 26 per fp32 word loaded and quantized, 7 per 32 int8 quads
-// loaded and transposed, 46 / 75 per warp and output row of a 3x3 / 5x5 filter, 12 per row that only fills the ring.
+// loaded and transposed, 46 / 75 per warp and output row of a 3x3 / 5x5 filter, 12 per row that only fills the ring. Counting the warps that
+// have no item in the last pass as if they issued kept eight-warp CTAs from launches that want them: 3x3 256 channels fp32 -> int8 56x56
+// x64 68.6 -> 65.7 us; fp32 -> fp32 from 15 us on 1.09 times as fast, the rest of 360 layers 0.99 to 1.03.
 // fp32 output from int8, stride 1: a lane stores 16 bytes of its own channel's plane, half a sector (single pixels where the rows are not
 // aligned), and the rest of the sector and of the line comes from the next warps. An output that does not fit L2, or one of single
 // pixels, wants that to happen soon: low bands (planes of 128 words), eight warps side by side on the same rows. us, high bands / low:
@@ -380,7 +382,9 @@ inline Tile plan_tile(const ConvShape& s) {
     const int ty_max = ((low ? kLowPlaneWords : kPlaneWords) / T.rp - K) / S + 1;
     const long per_band = (long)s.n * T.tiles_x * T.cgroups;
     // a throughput-bound launch wants every warp to have the same work, a latency-bound one as many warps as there are
-    const int widths[2] = {low ? THREADS / 32 : T.nxq > 8 ? (T.nxq + 1) / 2 : T.nxq > 2 ? T.nxq : 2, THREADS / 32};
+    // (fp32 input: of two that are rated alike the wider one, which has more loads under way)
+    const int few = low ? THREADS / 32 : T.nxq > 8 ? (T.nxq + 1) / 2 : T.nxq > 2 ? T.nxq : 2;
+    const int widths[2] = {IN_F32 ? THREADS / 32 : few, IN_F32 ? few : THREADS / 32};
     double best = 0;
     for (int bands = (s.oh + ty_max - 1) / ty_max; bands <= s.oh; ++bands) {
         const int ty = (s.oh + bands - 1) / bands, tiles_y = (s.oh + ty - 1) / ty;
@@ -393,12 +397,13 @@ inline Tile plan_tile(const ConvShape& s) {
             const int rpt = (ty + nrg - 1) / nrg;
             nrg = (ty + rpt - 1) / rpt;
             const int passes = (T.nxq * nrg + w - 1) / w;
-            const double instr = npos * (IN_F32 ? 26.0 : 7.0) + passes * w * (rpt * (K == 3 ? 46.0 : 75.0) + (K - S) * 12.0);
+            const double load = npos * (IN_F32 ? 26.0 : 7.0), item = rpt * (K == 3 ? 46.0 : 75.0) + (K - S) * 12.0;
+            const double issued = load + T.nxq * nrg * item, instr = load + passes * w * item;  // (a warp without an item in the last pass issues nothing)
             int resident = 65536 / ((K == 3 ? 64 : 80) * 32 * w);
             const int by_smem = 224 * 1024 / (CG * 4 * npos + 2048);
             if (by_smem < resident) resident = by_smem;
             const double waves = (double)ctas / ((double)kSms * resident);
-            const double busy = (double)((ctas + kSms - 1) / kSms) * instr / 2.5;
+            const double busy = (double)((ctas + kSms - 1) / kSms) * issued / 2.5;
             const double chain = (waves <= 1.0 ? 1.0 : waves + 0.5) * (1800.0 + 6.0 * instr / w);
             const double score = busy > chain ? busy : chain;
             if (T.ty != 0 && score >= best) continue;
