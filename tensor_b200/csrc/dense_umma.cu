@@ -21,8 +21,9 @@
 //   compact launch) let the epilogue of tile i overlap the loads and MMAs of the tiles behind it.
 // * The epilogue warps read TMEM (tcgen05.ld), apply fma(acc, scale_in, bias) -> activation -> requantize
 //   (epilogue.cuh) and store int8 NHWC / fp32 NCHW / s32 NHWC.
+// * Long 1x1 launches with int8 output exchange the operands, D[128 channels, pixels], see the comment on the builds in front of the kernel.
 //
-// Warp roles (320 threads): warp 0 = TMA producer (one lane), warp 1 = TMEM owner + MMA issuer (one lane),
+// Warp roles (320 threads): warp 0 = TMA producer (one elected thread), warp 1 = TMEM owner + MMA issuer (one elected thread),
 // warps 2..9 = epilogue: warp w reads TMEM lanes 32*(w%4)..+31 (the hardware's lane window of a warp) and
 // shares that quarter's column chunks with the other warps of the same window, dealt out over all the CTA's tiles.
 // Every mbarrier wait is bounded in time: on expiry the waiter raises a CTA-wide abort flag, ORs a code
