@@ -55,10 +55,12 @@ struct DwPwGeom {
 enum : uint32_t { B_W = 0, B_FULL = 1, B_EMPTY = B_FULL + kDwPwStagesMax, B_DFULL = B_EMPTY + kDwPwStagesMax, B_DEMPTY = B_DFULL + 2, B_YFULL = B_DEMPTY + 2,
                   B_YEMPTY = B_YFULL + 2, B_PFULL = B_YEMPTY + 2, B_PEMPTY = B_PFULL + 2, B_COUNT = B_PEMPTY + 2 };
 
-template <int ACT, int OUT, bool MULTI>
+template <int ACT_BUILD, int OUT, bool MULTI>
 __global__ void __launch_bounds__(kThreads, MULTI ? 2 : 1)
 dwpw_umma_kernel(const __grid_constant__ DwPwMaps maps, const __grid_constant__ CUtensorMap tmWdw, const __grid_constant__ CUtensorMap tmWpw, const DwPwPlan P,
                  const DwPwGeom G, const DwPwEpilogues ep, void* __restrict__ out, uint32_t* __restrict__ status, const __grid_constant__ UmmaMixedOut mixed) {
+    constexpr int ACT = ACT_BUILD & ~kSignedScale;
+    constexpr bool SIGNED = (ACT_BUILD & kSignedScale) != 0;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -265,7 +267,7 @@ dwpw_umma_kernel(const __grid_constant__ DwPwMaps maps, const __grid_constant__ 
             const int m = m_first + (int)t * m_step;
             const int img = m / per_img, r = m - img * per_img;
             const int oy = (r / P.tiles_x) * kTh + (row >> 3), ox = (r % P.tiles_x) * kTw + (row & 7);
-            store_accumulator_row<ACT, OUT>(t_pw + pb * (uint32_t)P.c2 + lane_sel, P.c2, sub, nsub, oy < G.oh && ox < G.ow, img, (long)oy * G.ow + ox, plane, s2,
+            store_accumulator_row<ACT, OUT, SIGNED>(t_pw + pb * (uint32_t)P.c2 + lane_sel, P.c2, sub, nsub, oy < G.oh && ox < G.ow, img, (long)oy * G.ow + ox, plane, s2,
                                             s2 + P.c2, s2 + 2 * P.c2, ep.pw.act_param0, G.c2pad, G.cout2, out, mixed);
             tc_fence_before();
             __syncwarp();
@@ -471,13 +473,17 @@ const char* launch_dwpw_umma(cudaStream_t stream, int sm_count, const DwPwPlan& 
     err = p.ctas_per_sm > 1 ? launch_variant<ACT, OUT, true>(stream, grid, km, wts, p, g, ep, out, status, mixed)            \
                             : launch_variant<ACT, OUT, false>(stream, grid, km, wts, p, g, ep, out, status, mixed)
 #define OTT_DWPW_ACT(OUT)                                       \
-    switch (ep.pw.act_type) {                                   \
+    switch (act) {                                              \
         case ACT_RELU: OTT_DWPW_LAUNCH(ACT_RELU, OUT); break;   \
         case ACT_LRELU: OTT_DWPW_LAUNCH(ACT_LRELU, OUT); break; \
         case ACT_RELU6: OTT_DWPW_LAUNCH(ACT_RELU6, OUT); break; \
         default: OTT_DWPW_LAUNCH(ACT_NONE, OUT); break;         \
     }
-    if (out_dtype == DT_F32_NCHW) { OTT_DWPW_ACT(DT_F32_NCHW) } else { OTT_DWPW_ACT(DT_S8_NHWC) }
+    const int act = ep.pw.act_type;
+    if (out_dtype == DT_F32_NCHW) { OTT_DWPW_ACT(DT_F32_NCHW) }
+    else if (ep.pw.negative_scale && act == ACT_RELU) OTT_DWPW_LAUNCH((ACT_RELU | kSignedScale), DT_S8_NHWC);
+    else if (ep.pw.negative_scale && act == ACT_RELU6) OTT_DWPW_LAUNCH((ACT_RELU6 | kSignedScale), DT_S8_NHWC);
+    else { OTT_DWPW_ACT(DT_S8_NHWC) }
 #undef OTT_DWPW_ACT
 #undef OTT_DWPW_LAUNCH
     if (err) return err;

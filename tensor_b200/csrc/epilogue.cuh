@@ -124,9 +124,10 @@ __device__ __forceinline__ int2 round2_nonneg(float2 v, uint32_t h) {
     return make_int2(__float2int_rz(r.x), __float2int_rz(r.y));
 }
 
-template <int ACT>
+// SIGNED: some output scale is below zero, so that what follows ReLU / ReLU6 may be too
+template <int ACT, bool SIGNED = false>
 __device__ __forceinline__ int2 round2_act(float2 v, uint32_t h) {
-    return ACT == ACT_RELU || ACT == ACT_RELU6 ? round2_nonneg(v, h) : round2(v, h);
+    return !SIGNED && (ACT == ACT_RELU || ACT == ACT_RELU6) ? round2_nonneg(v, h) : round2(v, h);
 }
 
 // Four v * scale_out of an int8_pos layer -> four int8 of the activated values, a.x in byte 0. Adding 1.5 * 2^23 with rounding toward

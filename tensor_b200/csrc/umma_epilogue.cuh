@@ -8,8 +8,11 @@
 
 namespace ottk {
 
+// Added to the activation of a build of the fused kernels: some layer of it has an output scale below zero behind ReLU or ReLU6.
+constexpr int kSignedScale = 8;
+
 // 16 accumulators -> 16 int8 (rounding rule: add half, truncate), packed into four words
-template <int ACT>
+template <int ACT, bool SIGNED = false>
 __device__ __forceinline__ void requant16(const int (&v)[16], const float* __restrict__ s_si, const float* __restrict__ s_bi,
                                           const float* __restrict__ s_so, float p0, uint32_t (&wds)[4]) {
 #pragma unroll
@@ -24,7 +27,7 @@ __device__ __forceinline__ void requant16(const int (&v)[16], const float* __res
             const float2 t = __ffma2_rn(a, h ? make_float2(si.z, si.w) : make_float2(si.x, si.y), h ? make_float2(bi.z, bi.w) : make_float2(bi.x, bi.y));
             const float2 y = make_float2(activate_t<ACT>(t.x, p0), activate_t<ACT>(t.y, p0));
             const float2 u = __fmul2_rn(y, h ? make_float2(so.z, so.w) : make_float2(so.x, so.y));
-            const int2 r = round2_act<ACT>(u, kHalfTrunc);
+            const int2 r = round2_act<ACT, SIGNED>(u, kHalfTrunc);
             qv[2 * h] = r.x;
             qv[2 * h + 1] = r.y;
         }
@@ -49,7 +52,7 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 // ncols = accumulator columns (a multiple of 32); warps sharing a lane quarter take every nsub-th 32-column chunk, starting
 // at chunk sub. s_si / s_bi / s_so: the per-channel parameters of these columns in shared memory. inimg = oy * w + ox.
 // c_base: the layer's channel that accumulator column 0 holds (a CTA may own a slice of the layer's channels).
-template <int ACT, int OUT>
+template <int ACT, int OUT, bool SIGNED = false>
 __device__ __forceinline__ void store_accumulator_row(uint32_t taddr, int ncols, int sub, int nsub, bool valid, int img, long inimg, long plane,
                                                       const float* __restrict__ s_si, const float* __restrict__ s_bi, const float* __restrict__ s_so,
                                                       float p0, int cpad, int cout, void* __restrict__ out, const UmmaMixedOut& mixed, int c_base = 0) {
@@ -123,7 +126,7 @@ __device__ __forceinline__ void store_accumulator_row(uint32_t taddr, int ncols,
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const float2 u = __fmul2_rn(make_float2(y[g * 4 + 2 * h], y[g * 4 + 2 * h + 1]), h ? make_float2(o4.z, o4.w) : make_float2(o4.x, o4.y));
-                    const int2 r = round2_act<ACT>(u, kHalfTrunc);
+                    const int2 r = round2_act<ACT, SIGNED>(u, kHalfTrunc);
                     qv[2 * h] = r.x;
                     qv[2 * h + 1] = r.y;
                 }

@@ -55,11 +55,13 @@ struct UnitGeom {
 
 enum : uint32_t { B_W = 0, B_XFULL = 1, B_XEMPTY = 3, B_ACC1 = 5, B_Y1 = 6, B_ACC2 = 7, B_Y2 = 8, B_ACC3 = 9, B_COUNT = 10 };
 
-template <int ACT, int OUT, bool MULTI>
+template <int ACT_BUILD, int OUT, bool MULTI>
 __global__ void __launch_bounds__(kMaxThreads, MULTI ? 2 : 1)
 unit_umma_kernel(const __grid_constant__ UnitMaps maps, const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmWdw,
                  const __grid_constant__ CUtensorMap tmW2, const UnitPlan P, const UnitGeom G, const UnitEpilogues ep, void* __restrict__ out,
                  uint32_t* __restrict__ status, const __grid_constant__ UmmaMixedOut mixed) {
+    constexpr int ACT = ACT_BUILD & ~kSignedScale;
+    constexpr bool SIGNED = (ACT_BUILD & kSignedScale) != 0;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -231,8 +233,8 @@ unit_umma_kernel(const __grid_constant__ UnitMaps maps, const __grid_constant__ 
                     if (!store) continue;
                     uint32_t wa[4] = {0u, 0u, 0u, 0u}, wb[4] = {0u, 0u, 0u, 0u};
                     if (inside) {
-                        requant16<ACT>(va, s1 + c0, s1 + P.cm + c0, s1 + 2 * P.cm + c0, ep.e1.act_param0, wa);
-                        requant16<ACT>(vb, s1 + c0 + 16, s1 + P.cm + c0 + 16, s1 + 2 * P.cm + c0 + 16, ep.e1.act_param0, wb);
+                        requant16<ACT, SIGNED>(va, s1 + c0, s1 + P.cm + c0, s1 + 2 * P.cm + c0, ep.e1.act_param0, wa);
+                        requant16<ACT, SIGNED>(vb, s1 + c0 + 16, s1 + P.cm + c0 + 16, s1 + 2 * P.cm + c0 + 16, ep.e1.act_param0, wb);
                     }
                     const uint32_t blk = sY1 + (uint32_t)(c0 >> 5) * kUnitHaloBlockBytes;
                     st_shared_v4(swz32(blk, p, 0), wa[0], wa[1], wa[2], wa[3]);
@@ -268,7 +270,7 @@ unit_umma_kernel(const __grid_constant__ UnitMaps maps, const __grid_constant__ 
             if (!mbar_wait(bar(B_ACC3), ph, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
             tc_fence_after();
             const int oy = ty0 + (row >> 3), ox = tx0 + (row & 7);
-            store_accumulator_row<ACT, OUT>(t_acc3 + lane_sel, P.c2, sub, nsub, oy < G.h && ox < G.w, img, (long)oy * G.w + ox, plane, s2, s2 + P.c2,
+            store_accumulator_row<ACT, OUT, SIGNED>(t_acc3 + lane_sel, P.c2, sub, nsub, oy < G.h && ox < G.w, img, (long)oy * G.w + ox, plane, s2, s2 + P.c2,
                                             s2 + 2 * P.c2, ep.e2.act_param0, G.c2pad, G.cout2, out, mixed);
             tc_fence_before();
         }
@@ -460,7 +462,16 @@ const char* launch_unit_umma(cudaStream_t stream, int sm_count, const UnitPlan& 
         case ACT_RELU6: OTT_UNIT_LAUNCH(ACT_RELU6, OUT); break; \
         default: OTT_UNIT_LAUNCH(ACT_NONE, OUT); break;         \
     }
-    if (out_dtype == DT_F32_NCHW) { OTT_UNIT_ACT(DT_F32_NCHW) } else { OTT_UNIT_ACT(DT_S8_NHWC) }
+#define OTT_UNIT_SIGNED(ACT)                                                                                 \
+    {                                                                                                        \
+        if (out_dtype == DT_F32_NCHW) OTT_UNIT_LAUNCH((ACT | kSignedScale), DT_F32_NCHW);                    \
+        else OTT_UNIT_LAUNCH((ACT | kSignedScale), DT_S8_NHWC);                                              \
+    }
+    const bool negative = ep.e1.negative_scale || ep.e2.negative_scale;
+    if (negative && act == ACT_RELU) OTT_UNIT_SIGNED(ACT_RELU)
+    else if (negative && act == ACT_RELU6) OTT_UNIT_SIGNED(ACT_RELU6)
+    else if (out_dtype == DT_F32_NCHW) { OTT_UNIT_ACT(DT_F32_NCHW) } else { OTT_UNIT_ACT(DT_S8_NHWC) }
+#undef OTT_UNIT_SIGNED
 #undef OTT_UNIT_ACT
 #undef OTT_UNIT_LAUNCH
     if (err) return err;

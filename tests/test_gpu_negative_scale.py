@@ -1,12 +1,12 @@
 """GPU: requantizing layers with output scales of both signs behind ReLU and ReLU6 (what is rounded is then below zero), both rounding
-rules, bit for bit against the CPU checker: the dense kernel's one-tile and specialised builds and the depthwise kernels; and a scale
-that is infinite."""
+rules, bit for bit against the CPU checker: the dense kernel's one-tile and specialised builds, the depthwise kernels and the fused pair
+and unit; and a scale that is infinite."""
 import ctypes as C
 
 import numpy as np
 import pytest
 
-from support import ACT_RELU, ACT_RELU6, ROUND_ADD_HALF_TRUNC, ROUND_HALF_AWAY, ConvCase, nhwc_padded_to_nchw, run_port
+from support import ACT_NONE, ACT_RELU, ACT_RELU6, ROUND_ADD_HALF_TRUNC, ROUND_HALF_AWAY, ConvCase, nchw_to_nhwc_padded, nhwc_padded_to_nchw, run_port
 
 pytestmark = pytest.mark.gpu
 
@@ -31,6 +31,41 @@ def test_scales_of_both_signs(ctx, rounding, act, cin, k, stride, n, h, depthwis
     got, want = run_gpu(ctx, case, rounding, want_acc=False)["y"], run_port(case, rounding, want_acc=False)["y"]
     assert want.min() == -127 and want.max() == 127 and np.unique(want).size > 100
     assert np.array_equal(bits(got), bits(want))
+
+
+@pytest.mark.parametrize("act", [ACT_RELU, ACT_RELU6])
+@pytest.mark.parametrize("unit,f32_out", [(False, False), (True, False), (True, True)])
+def test_fused_layers(ctx, act, unit, f32_out):
+    """1x1 layers with scales of both signs before and behind a depthwise layer, in the fused kernels."""
+    from gpu_support import bits, make_layer
+    from tensor_b200 import F32_NCHW, S8_NHWC, DwPwInt8, UnitInt8, nhwc_channels
+    c, n, h, w = 40, 2, 17, 20
+    signs = np.where(np.arange(c) % 3 == 0, 1, -1) * np.geomspace(0.5, 300.0, c)
+    common = dict(n=n, h=h, w=w, bias_term=1, s8_input=True)
+    pw1 = ConvCase("neg_pw1", c, c, 1, 1, 0, int8_scale_term=101, act_type=act, w_std=0.1, seed=1, **common).make()
+    dw = ConvCase("neg_dw", c, c, 3, 1, 1, groups=c, int8_scale_term=101, act_type=ACT_NONE, w_std=0.5, seed=2, **common).make()
+    pw2 = ConvCase("neg_pw2", c, c, 1, 1, 0, int8_scale_term=1 if f32_out else 101, act_type=act, w_std=0.1, seed=3, **common).make()
+    pw1.out_scales = signs.astype(np.float32)
+    if not f32_out:
+        pw2.out_scales = signs[::-1].astype(np.float32)
+    if unit:
+        dw.x_s8 = run_port(pw1, ROUND_ADD_HALF_TRUNC, want_acc=False)["y"]
+        assert dw.x_s8.min() == -127 and dw.x_s8.max() == 127
+    pw2.x_s8 = run_port(dw, ROUND_ADD_HALF_TRUNC, want_acc=False)["y"]
+    want = run_port(pw2, ROUND_ADD_HALF_TRUNC, want_acc=False)["y"]
+    assert f32_out or (want.min() == -127 and want.max() == 127 and np.unique(want).size > 100)
+    layers = [make_layer(ctx, x, ROUND_ADD_HALF_TRUNC) for x in ((pw1, dw, pw2) if unit else (dw, pw2))]
+    fused = (UnitInt8 if unit else DwPwInt8)(ctx, *layers)
+    dtype = F32_NCHW if f32_out else S8_NHWC
+    out = layers[-1].out_array(n, h, w, dtype)
+    x, y = ctx.to_device(nchw_to_nhwc_padded((pw1 if unit else dw).x_s8, nhwc_channels(c))), ctx.malloc(out.nbytes)
+    fused.forward_io(n, h, w, y, dtype, in_dev=x)
+    got = ctx.to_host(y, out.shape, out.dtype)
+    assert np.array_equal(bits(got if f32_out else nhwc_padded_to_nchw(got, c)), bits(want))
+    for p in (x, y):
+        ctx.free(p)
+    for o in (fused, *layers):
+        o.close()
 
 
 def test_first_layer_maxpool_with_negative_scales(ctx):
