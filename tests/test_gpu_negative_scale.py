@@ -40,7 +40,7 @@ def test_fused_layers(ctx, act, unit, f32_out):
     from gpu_support import bits, make_layer
     from tensor_b200 import F32_NCHW, S8_NHWC, DwPwInt8, UnitInt8, nhwc_channels
     c, n, h, w = 40, 2, 17, 20
-    signs = np.where(np.arange(c) % 3 == 0, 1, -1) * np.geomspace(0.5, 300.0, c)
+    signs = np.where(np.arange(c) % 3 == 0, 1, -1) * np.geomspace(2.0, 1200.0, c)
     common = dict(n=n, h=h, w=w, bias_term=1, s8_input=True)
     pw1 = ConvCase("neg_pw1", c, c, 1, 1, 0, int8_scale_term=101, act_type=act, w_std=0.1, seed=1, **common).make()
     dw = ConvCase("neg_dw", c, c, 3, 1, 1, groups=c, int8_scale_term=101, act_type=ACT_NONE, w_std=0.5, seed=2, **common).make()
