@@ -168,6 +168,7 @@ int ott_net_add_layer(ott_net* net, const char* options) {
 int ott_net_load_otter(ott_net* net, const char* path) {
     if (!net || !path) return OTT_ERR_INVALID;
     net->error.clear();
+    net->drop_pipelines();  // the layers are made anew
     return net->net.load_otter(path, otter::CompileMode::Initial);
 }
 

@@ -135,3 +135,24 @@ def test_a_net_compiled_again_forgets_its_graphs():
     assert np.array_equal(after, fresh.forward("data", x, ["conv5"])[0]) and not np.array_equal(after, before)
     net.close()
     fresh.close()
+
+
+def test_a_graph_file_loaded_into_a_net_forgets_its_graphs(tmp_path):
+    """Loading appends the file's layers and makes every layer anew, the ones that have been captured before included."""
+    from graph_support import build_net, oracle_conv_for_calibration
+    from graph_walk import calibrate
+    from tensor_b200 import graphs
+    L = graphs.shufflenetv2_layers(40, 48, batch=1, stage_repeats=(2, 2, 2))
+    params = graphs.make_params(L, seed=23)
+    x = np.random.default_rng(0).uniform(0, 1, size=(1, 3, 40, 48)).astype(np.float32)
+    calibrate(L, params, x, oracle_conv_for_calibration)
+    path = tmp_path / "more.otter"
+    path.write_text(graphs.to_otter_text([dict(type="Input", name="more", output="more", batchsize=1, channel=3, height=8, width=8)]))
+    net, fresh = build_net(L, params), build_net(L, {})
+    for _ in range(3):
+        before = net.forward("data", x, ["conv5"])[0]
+    net.load_otter(path)
+    after = net.forward("data", x, ["conv5"])[0]
+    assert np.array_equal(after, fresh.forward("data", x, ["conv5"])[0]) and not np.array_equal(after, before)
+    net.close()
+    fresh.close()
