@@ -281,7 +281,7 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
             for (int i = 0; i < (P.gather > 0 ? P.gather : 1); ++i) prefetch_tensormap(&maps.tm[i]);
 #pragma unroll 1
         for (int i = 0; i < P.stages; ++i) {
-            mbar_init(bar_full + 8u * i, ROWS && QUANT ? (uint32_t)boxes_per_tile : QUANT ? kQuantWarps : 1);
+            mbar_init(bar_full + 8u * i, ROWS && QUANT ? kBoxWarps : QUANT ? kQuantWarps : 1);
             mbar_init(bar_empty + 8u * i, 1);
         }
         mbar_init(bar_b, 1);
@@ -576,8 +576,9 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)P.tmem_cols) : "memory");
     } else if (ROWS && QUANT && warp > 2 + kMaxEpiWarps) {
         if constexpr (ROWS && QUANT) {
-            // ---- quantizers: four pixels of eight channels per thread. A warp passes every tile, in order, whether it has a box of it or
-            // not, so that no phase of a barrier that it waits for goes by unseen ----
+            // ---- quantizers: four pixels of eight channels per thread. Every warp waits for every tile's stage and arrives on its barrier
+            // once, after its last box of the tile or without one (fewer than kBoxWarps boxes): the tile is multiplied, and its stage
+            // freed again, only when all of them have seen the stage free, so that none misses a phase of bar_empty ----
             const int qw = warp - (3 + kMaxEpiWarps), quad = lane & 15, upper = lane >> 4, per_block = 31 - __clz(P.bkc >> 4);
             const uint32_t words_at = base + L.floats + (uint32_t)(upper * 8 * rows_pixels(BUILD) * 4 + quad * 16);
             uint32_t st = 0, phase = 1, at = (uint32_t)qw, xphase = 0;
@@ -585,19 +586,15 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
             bool ok = true;
             for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
                 bool waited = false;
-                for (;; c += kBoxWarps) {
+                for (; c < boxes_per_tile; c += kBoxWarps) {
                     float4 v[8];
-                    const bool mine = c < boxes_per_tile;
-                    if (mine) {
-                        if (!mbar_wait(bar_xfull + 8u * at, xphase, abort_flag, status, 512u, P.wait_ns)) { ok = false; break; }
+                    if (!mbar_wait(bar_xfull + 8u * at, xphase, abort_flag, status, 512u, P.wait_ns)) { ok = false; break; }
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w)
-                                         : "r"(words_at + at * kBoxBytes + (uint32_t)(j * rows_pixels(BUILD) * 4)) : "memory");
-                    }
+                    for (int j = 0; j < 8; ++j)
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w)
+                                     : "r"(words_at + at * kBoxBytes + (uint32_t)(j * rows_pixels(BUILD) * 4)) : "memory");
                     if (!waited && !mbar_wait(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
                     waited = true;
-                    if (!mine) break;
                     uint32_t w[2][4];  // [group of four channels][pixel]
 #pragma unroll
                     for (int g = 0; g < 2; ++g) {
@@ -615,10 +612,12 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
                     for (int j = 0; j < 4; ++j)
                         asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(operand_chunk(block, P.bkc, quad * 4 + j, c & ((1 << per_block) - 1)) + (uint32_t)(upper * 8)),
                                      "r"(w[0][j]), "r"(w[1][j]) : "memory");
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // these writes -> the MMA's reads
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_full + 8u * st);
                 }
+                if (ok && !waited && !mbar_wait(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) ok = false;
+                if (!ok) break;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tile's writes -> the MMA's reads
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full + 8u * st);
                 c -= boxes_per_tile;
                 if (++st == (uint32_t)P.stages) { st = 0; phase ^= 1u; }
             }

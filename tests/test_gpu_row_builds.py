@@ -49,11 +49,12 @@ def test_epilogues(ctx, act, scale):
         _check(ctx, _case(64, cout, 7, 61, 53, act), rounding, s)
 
 
-@pytest.mark.parametrize("cin,cout,h,w", [(256, 512, 44, 20), (40, 330, 44, 21), (130, 240, 20, 44), (33, 64, 44, 20), (64, 100, 46, 22), (100, 16, 44, 20)])
+@pytest.mark.parametrize("cin,cout,h,w", [(256, 512, 44, 20), (40, 330, 44, 21), (130, 240, 20, 44), (33, 64, 44, 20), (64, 100, 46, 22), (100, 16, 44, 20), (17, 40, 44, 20), (24, 24, 12, 10),
+                                          (32, 512, 20, 18)])
 @pytest.mark.parametrize("act", [ACT_RELU6, ACT_NONE])
 def test_quantized_inside(ctx, cin, cout, h, w, act):
     """fp32 input of 100 MB: one to four accumulators per tile of 64 pixels, the last tile of an image ragged; the first, the middle and
-    the last image against the checker."""
+    the last image against the checker. From two boxes of 16 channels per tile on, so that most of the warps that quantize have none."""
     from gpu_support import make_layer
     from tensor_b200 import F32_NCHW, S8_NHWC, nhwc_channels
     from support import nhwc_padded_to_nchw
