@@ -247,7 +247,7 @@ dense_stem_pool_mma_kernel(const __grid_constant__ CUtensorMap image, const floa
     uint32_t phase = 0;
     for (int t = (int)blockIdx.x; t < tiles; t += (int)gridDim.x, phase ^= 1u) {
     if (by_box) {
-        if (!mbar_wait(bar_x, phase, &abort_flag, status, 32u)) {
+        if (!mbar_wait_warp(bar_x, phase, &abort_flag, status, 32u)) {
             ok = false;
             const unsigned long long t0 = globaltimer_ns();
             while (globaltimer_ns() - t0 < 1000000ull) {}  // let the copy in flight land before its place is written
@@ -325,10 +325,11 @@ dense_stem_pool_mma_kernel(const __grid_constant__ CUtensorMap image, const floa
         }
         __syncwarp();
     }
-    if (!mbar_wait(bar_d, phase, &abort_flag, status, 32u)) ok = false;
+    if (!mbar_wait_warp(bar_d, phase, &abort_flag, status, 32u)) ok = false;
     tc_fence_after();
     // the next tile's box takes the place of the taps, which the MMAs have read, while this tile is pooled
     if (by_box && threadIdx.x == 0 && ok && t + (int)gridDim.x < tiles) fetch(t + (int)gridDim.x);
+    __syncwarp();
 
     if (ok) {
         // Max-pooling happens on the exact s32 sums: dequantize + activation is non-decreasing in the sum for the non-negative scales the

@@ -588,12 +588,12 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
                 bool waited = false;
                 for (; c < boxes_per_tile; c += kBoxWarps) {
                     float4 v[8];
-                    if (!mbar_wait(bar_xfull + 8u * at, xphase, abort_flag, status, 512u, P.wait_ns)) { ok = false; break; }
+                    if (!mbar_wait_warp(bar_xfull + 8u * at, xphase, abort_flag, status, 512u, P.wait_ns)) { ok = false; break; }
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w)
                                      : "r"(words_at + at * kBoxBytes + (uint32_t)(j * rows_pixels(BUILD) * 4)) : "memory");
-                    if (!waited && !mbar_wait(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
+                    if (!waited && !mbar_wait_warp(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
                     waited = true;
                     uint32_t w[2][4];  // [group of four channels][pixel]
 #pragma unroll
@@ -613,7 +613,7 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
                         asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(operand_chunk(block, P.bkc, quad * 4 + j, c & ((1 << per_block) - 1)) + (uint32_t)(upper * 8)),
                                      "r"(w[0][j]), "r"(w[1][j]) : "memory");
                 }
-                if (ok && !waited && !mbar_wait(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) ok = false;
+                if (ok && !waited && !mbar_wait_warp(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) ok = false;
                 if (!ok) break;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tile's writes -> the MMA's reads
                 __syncwarp();
@@ -640,7 +640,7 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
                     x0 = (r - ty * P.tiles_x) * P.tw - s.pw;
                 }
                 for (int kb = 0; kb < loads_per_tile; ++kb) {
-                    if (!mbar_wait(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
+                    if (!mbar_wait_warp(bar_empty + 8u * st, phase, abort_flag, status, 1u, P.wait_ns)) { ok = false; break; }
                     const uint32_t tile = sA + st * a_stage_bytes;
                     if (P.flat && maps.vec) {
                         const int ch = turn & 7, c0 = kb * P.bkc + ch * 16;
@@ -787,12 +787,15 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
                 if (QUANT && blocks > 2 && unit != team) take_block(blk + 2 < blocks ? blk + 2 : blk + 2 - blocks);
                 const uint32_t buf = unit & acc_mask, use = unit >> acc_shift, slot = unit & slot_mask;
                 const uint32_t taddr = t_lane + buf * (uint32_t)P.acc_stride, out_at = slot * slot_bytes;
-                if (!mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) break;
+                // A lane whose wait has run out goes on with the others, over sums that mean nothing, to the warp's last unit (the abort flag is
+                // up, so that no further wait lasts, and the call reports it): what follows wants all 32 lanes. Leaving the loop by a vote costs
+                // 58 -> 58 40x40 x256 0.45 us, this way, which joins the lanes behind each wait, 0.2 of 10.4.
+                (void)mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns);
                 tc_fence_after();
                 // 32 pixels x 16 channels at a time, the next ones on their way while these are computed
                 int v[2][16];
                 if (c0 < left) tmem_ld16x256(taddr, v[0]);
-                if (!mbar_wait(bar_ofree + 8u * slot, ((unit >> slot_shift) & 1u) ^ 1u, abort_flag, status, 128u, P.wait_ns)) break;
+                (void)mbar_wait(bar_ofree + 8u * slot, ((unit >> slot_shift) & 1u) ^ 1u, abort_flag, status, 128u, P.wait_ns);
                 tmem_wait_ld16(v[0]);
                 if (hi) {
                     tmem_ld16x256(taddr + (16u << 16), v[1]);
@@ -957,7 +960,7 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
             // Chunks of 32 columns: two TMEM loads in flight, and int8 rows leave as one 32-byte store per thread, a whole
             // DRAM sector (two 16-byte stores from different warps would each touch half of it).
             const bool wide_ok = writes(DT_S8_NHWC) && ((s.cout_pad | (c_base)) & 31) == 0;
-            if (!mbar_wait(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) break;
+            if (!mbar_wait_warp(bar_tfull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) break;
             tc_fence_after();
             for (; ci < n_chunks; ci += nsub) {
                 const int col0 = ci * chunk;

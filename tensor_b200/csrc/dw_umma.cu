@@ -186,7 +186,7 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
         uint32_t it = 0;
         for (int m = m_first; ok && m < P.m_tiles; m += m_step, ++it) {
             const uint32_t buf = it & acc_mask, use = it / kMaxAcc;  // (acc_bufs is kMaxAcc)
-            if (!mbar_wait(bar_afull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
+            if (!mbar_wait_warp(bar_afull + 8u * buf, use & 1u, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
             tc_fence_after();
             const int img = (int)fast_div((uint32_t)m, P.div_img), r = m - img * per_img, ty = (int)fast_div((uint32_t)r, P.div_x);
             const int oy = ty * kTh + (row >> 3), ox = (r - ty * P.tiles_x) * kTw + (row & 7);

@@ -231,8 +231,8 @@ dwpw_umma_kernel(const __grid_constant__ DwPwMaps maps, const __grid_constant__ 
         // A: depthwise accumulators of tile t -> requantized operand tile Y
         auto epi_a = [&](uint32_t t) -> bool {
             const uint32_t buf = t & dmask, yb = t & ymask;
-            if (!mbar_wait(bar(B_DFULL + buf), (t >> dsh) & 1u, abort_flag, status, 8u, P.wait_ns)) return false;
-            if (!mbar_wait(bar(B_YEMPTY + yb), ((t >> ysh) & 1u) ^ 1u, abort_flag, status, 128u, P.wait_ns)) return false;
+            if (!mbar_wait_warp(bar(B_DFULL + buf), (t >> dsh) & 1u, abort_flag, status, 8u, P.wait_ns)) return false;
+            if (!mbar_wait_warp(bar(B_YEMPTY + yb), ((t >> ysh) & 1u) ^ 1u, abort_flag, status, 128u, P.wait_ns)) return false;
             tc_fence_after();
             const uint32_t acc = t_dw + buf * (uint32_t)P.dwcols + lane_sel;
             const uint32_t yt = sY + yb * (uint32_t)P.ncb * kYBlockBytes;
@@ -262,7 +262,7 @@ dwpw_umma_kernel(const __grid_constant__ DwPwMaps maps, const __grid_constant__ 
         // B: the 1x1 layer's accumulators of tile t -> its output
         auto epi_b = [&](uint32_t t) -> bool {
             const uint32_t pb = t & pmask;
-            if (!mbar_wait(bar(B_PFULL + pb), (t >> psh) & 1u, abort_flag, status, 256u, P.wait_ns)) return false;
+            if (!mbar_wait_warp(bar(B_PFULL + pb), (t >> psh) & 1u, abort_flag, status, 256u, P.wait_ns)) return false;
             tc_fence_after();
             const int m = m_first + (int)t * m_step;
             const int img = m / per_img, r = m - img * per_img;

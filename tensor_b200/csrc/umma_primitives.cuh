@@ -66,6 +66,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// The same wait by every lane of a warp that executes warp-wide instructions behind it (tcgen05.ld, stmatrix, shuffles): one answer for
+// all of them, and they go on together. Each lane has its own clock and looks at the abort flag by itself, so that without the vote a
+// limit that runs out could take some lanes away and leave the others in front of an instruction that wants all 32.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code,
+                                               unsigned long long limit_ns = kWaitLimitNs) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag, status, code, limit_ns)) != 0;
+}
+
 // One thread of a converged warp. Unlike a test of the lane number it tells the compiler that what follows runs on one thread, so that
 // operand descriptors and addresses stay in uniform registers instead of being moved there for every instruction: back-to-back MMAs
 // (M 128, N 32, K 32) 40 cycles apart, the tensor pipe's rate, against 50. Dense layers, time with a lane test / with this, geometric

@@ -213,7 +213,7 @@ unit_umma_kernel(const __grid_constant__ UnitMaps maps, const __grid_constant__ 
             const int img = m / per_img, r = m - img * per_img;
             const int ty0 = (r / P.tiles_x) * kUnitTh, tx0 = (r % P.tiles_x) * kUnitTw;
             // ---- epilogue 1: acc1 (two blocks of 128 halo pixels) -> Y1 ----
-            if (!mbar_wait(bar(B_ACC1), ph, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
+            if (!mbar_wait_warp(bar(B_ACC1), ph, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
             tc_fence_after();
 #pragma unroll 1
             for (int mb = 0; mb < 2; ++mb) {
@@ -246,7 +246,7 @@ unit_umma_kernel(const __grid_constant__ UnitMaps maps, const __grid_constant__ 
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(B_Y1));
             // ---- epilogue 2: acc2 (depthwise sums of the 128 output pixels) -> Y2 ----
-            if (!mbar_wait(bar(B_ACC2), ph, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
+            if (!mbar_wait_warp(bar(B_ACC2), ph, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
             tc_fence_after();
             for (int c0 = sub * 32; c0 < P.cm; c0 += nsub * 32) {
                 int va[16], vb[16];
@@ -267,7 +267,7 @@ unit_umma_kernel(const __grid_constant__ UnitMaps maps, const __grid_constant__ 
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(B_Y2));
             // ---- epilogue 3: acc3 -> the second 1x1 layer's output ----
-            if (!mbar_wait(bar(B_ACC3), ph, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
+            if (!mbar_wait_warp(bar(B_ACC3), ph, abort_flag, status, 8u, P.wait_ns)) { ok = false; break; }
             tc_fence_after();
             const int oy = ty0 + (row >> 3), ox = tx0 + (row & 7);
             store_accumulator_row<ACT, OUT, SIGNED>(t_acc3 + lane_sel, P.c2, sub, nsub, oy < G.h && ox < G.w, img, (long)oy * G.w + ox, plane, s2, s2 + P.c2,

@@ -16,14 +16,24 @@ __global__ void wait_probe_kernel(uint32_t* status, unsigned long long limit_ns)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    // phase 0 of a freshly initialised barrier with one pending arrival never completes: nobody arrives
-    if (threadIdx.x == 0) (void)umma::mbar_wait(umma::smem_u32(&bar), 0, &abort_flag, status, 0x100u, limit_ns);
+    // Phase 0 of a freshly initialised barrier with one pending arrival: nobody arrives before lane 0 of the waiting warp has given up
+    // (the other lanes have more time). What the others then see, the arrival or the abort flag, must not matter: 0x200 reports a lane
+    // that was told to go on.
+    volatile int* flag = &abort_flag;
+    if (threadIdx.x < 32) {
+        const bool ok = umma::mbar_wait_warp(umma::smem_u32(&bar), 0, flag, status, 0x100u, threadIdx.x == 0 ? limit_ns : 4 * limit_ns);
+        if (ok) atomicOr(status, 0x200u);
+    } else if (threadIdx.x == 32) {
+        const unsigned long long t0 = umma::globaltimer_ns();
+        while (*flag == 0 && umma::globaltimer_ns() - t0 < 8 * limit_ns) {}
+        umma::mbar_arrive(umma::smem_u32(&bar));
+    }
     __syncthreads();
 }
 }  // namespace
 
 cudaError_t launch_wait_probe(cudaStream_t stream, uint32_t* status, unsigned long long limit_ns) {
-    wait_probe_kernel<<<1, 32, 0, stream>>>(status, limit_ns);
+    wait_probe_kernel<<<1, 64, 0, stream>>>(status, limit_ns);
     return cudaGetLastError();
 }
 
