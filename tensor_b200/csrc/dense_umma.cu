@@ -584,6 +584,7 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
             uint32_t st = 0, phase = 1, at = (uint32_t)qw, xphase = 0;
             int c = qw;  // this warp's next box, counted from the tile's first
             bool ok = true;
+            pdl_wait();  // (as the issuer: the previous kernel's time does not count against the limits of the waits below)
             for (int m = m_first; ok && m < P.m_tiles; m += m_step) {
                 bool waited = false;
                 for (; c < boxes_per_tile; c += kBoxWarps) {
@@ -782,6 +783,7 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
                 }
                 stmatrix_t8(at, w);
             };
+            pdl_wait();  // (as the issuer)
             const uint32_t units = m_first < P.m_tiles ? (uint32_t)((P.m_tiles - 1 - m_first) / m_step + 1) * (uint32_t)blocks : 0u;
             for (uint32_t unit = team; unit < units; unit += teams) {
                 if (QUANT && blocks > 2 && unit != team) take_block(blk + 2 < blocks ? blk + 2 : blk + 2 - blocks);

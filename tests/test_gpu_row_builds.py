@@ -1,5 +1,6 @@
 """GPU: int8 launches of the dense tensor-core kernel with output channels as accumulator rows, bit for bit against the CPU checker: one
-and several accumulators per panel, 64-row ones, several panels, ragged last tiles, and every epilogue."""
+and several accumulators per panel, 64-row ones, several panels, ragged last tiles, every epilogue, and a start long before the previous
+kernel ends."""
 import numpy as np
 import pytest
 
@@ -76,3 +77,43 @@ def test_quantized_inside(ctx, cin, cout, h, w, act):
     layer.close()
     ctx.free(dx)
     ctx.free(y)
+
+
+@pytest.mark.parametrize("f32", [False, True])
+def test_waits_do_not_count_the_previous_kernel(ctx, f32):
+    """A launch of several milliseconds that leaves SMs idle (eight panels: 144 of 148 CTAs), the next one's first CTAs beside it, and
+    waits limited to one millisecond. The long launch's output is not looked at."""
+    from gpu_support import make_layer
+    from tensor_b200 import F32_NCHW, S8_NHWC, ConvInt8, nhwc_channels
+    from support import nchw_to_nhwc_padded, nhwc_padded_to_nchw
+    assert ctx.lib.ott_debug_dense_rows(512, 2048, 1, 1600, 1600, 0, 148) == 256
+    rng = np.random.default_rng(2)
+    before = ConvInt8(ctx, cin=512, cout=2048, kh=1, kw=1, int8_scale_term=101, act_type=ACT_RELU, weight=rng.integers(-127, 128, (2048, 512, 1, 1), dtype=np.int8),
+                      bias=np.zeros(2048, np.float32), w_scales=np.full(2048, 50, np.float32), in_scales=np.full(1, 127, np.float32),
+                      out_scales=np.full(1, 0.1, np.float32))
+    n, h, w, cout = (320, 44, 20, 100) if f32 else (16, 52, 52, 100)
+    cin = 96 if f32 else 64
+    case = _case(cin, cout, 2, h, w, ACT_RELU)
+    case.s8_input = not f32
+    case.make()
+    want = run_port(case, ROUND_ADD_HALF_TRUNC, want_acc=False)["y"]
+    assert ctx.lib.ott_debug_dense_rows(cin, cout, n, h, w, int(f32), 148) == 128
+    layer = make_layer(ctx, case, ROUND_ADD_HALF_TRUNC)
+    one = case.x_f32 if f32 else nchw_to_nhwc_padded(case.x_s8, nhwc_channels(cin))
+    x, shape = ctx.to_device(np.tile(one, (n // 2, 1, 1, 1))), (n, h, w, nhwc_channels(cout))
+    y, big_x, big_y = ctx.malloc(int(np.prod(shape))), ctx.malloc(1600 * 1600 * 512), ctx.malloc(1600 * 1600 * 2048)
+    ctx.memset(big_x, 1, 1600 * 1600 * 512)
+    ctx.sync()
+    ctx.check(ctx.lib.ott_set_wait_limit_ms(ctx.h, 1))
+    for _ in range(3):
+        before.forward(big_x, S8_NHWC, 1, 1600, 1600, big_y, S8_NHWC)
+        layer.forward(x, F32_NCHW if f32 else S8_NHWC, n, h, w, y, S8_NHWC)
+    ctx.sync()
+    ctx.check(ctx.lib.ott_set_wait_limit_ms(ctx.h, 2000))
+    got = ctx.to_host(y, shape, np.int8)
+    for i in (0, n // 2, n - 2):
+        assert np.array_equal(nhwc_padded_to_nchw(got[i:i + 2], cout), want)
+    for p in (x, y, big_x, big_y):
+        ctx.free(p)
+    before.close()
+    layer.close()
