@@ -92,13 +92,14 @@ int ott_set_depthwise_tensor_cores(ott_ctx* ctx, int mode);
  * (cudaErrorMemoryAllocation without calling cudaMalloc); n <= 0 switches the injection off. */
 int ott_debug_wait_probe(ott_ctx* ctx);
 int ott_debug_fail_alloc_after(ott_ctx* ctx, int n);
-/* What a dense k x k layer (padding k / 2) on the tensor cores would launch on a GPU of sm_count SMs; needs no GPU. plan: 128-pixel
- * tiles, weight panels, columns of a panel, CTAs per SM of the plan, fp32 input quantized inside the kernel, the one-tile-per-CTA
- * build, pixels per tile, halo form (0: one load per tap, 1: halo tiles, 2: one halo tile per column parity). OTT_ERR_UNSUPPORTED:
- * the layer does not run there. */
+/* What a dense k x k layer (padding k / 2) on the tensor cores would launch on a GPU of sm_count SMs; needs no GPU. int8_output: one
+ * int8 tensor and nothing else; 0: fp32 output, side outputs or scattered chunks. plan: 128-pixel tiles, weight panels, columns of a
+ * panel, CTAs per SM of the plan, fp32 input quantized inside the kernel, the one-tile-per-CTA build, pixels per tile, halo form (0: one
+ * load per tap, 1: halo tiles, 2: one halo tile per column parity), and the pixels of an accumulator that has output channels as rows
+ * (0: pixels are the rows). OTT_ERR_UNSUPPORTED: the layer does not run there. */
+int ott_debug_dense_launch(int cin, int cout, int k, int stride, int n, int h, int w, int f32_input, int int8_output, int sm_count, int plan[9]);
+/* The first eight of these without int8_output; and of a 1x1 layer with it the columns of a panel if channels are rows, else 0. */
 int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int w, int f32_input, int sm_count, int plan[8]);
-/* The same question for a 1x1 layer with int8 output: the output channels of a weight panel if the launch has channels as accumulator
- * rows, 0 if it has pixels as rows. */
 int ott_debug_dense_rows(int cin, int cout, int n, int h, int w, int f32_input, int sm_count);
 /* Guard bands, the tests' stand-in for a device memory checker: after ott_debug_guard_bands(ctx, bytes) every block the
  * context's allocator obtains from the driver carries `bytes` (rounded up to 512) of a fill pattern on both sides;

@@ -41,6 +41,7 @@ SIGNATURES = {
     "ott_debug_mma_rate": (i32, [vp, i32, i32, i32, i32, i32, C.POINTER(C.c_float)]),
     "ott_set_depthwise_tensor_cores": (i32, [vp, i32]),
     "ott_debug_fail_alloc_after": (i32, [vp, i32]),
+    "ott_debug_dense_launch": (i32, [i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp]),
     "ott_debug_dense_plan": (i32, [i32, i32, i32, i32, i32, i32, i32, i32, i32, vp]),
     "ott_debug_dense_rows": (i32, [i32, i32, i32, i32, i32, i32, i32]),
     "ott_debug_guard_bands": (i32, [vp, C.c_size_t]),

@@ -39,6 +39,16 @@ int check_status_word(ott_ctx* ctx, bool copied = false) {
     return OTT_OK;
 }
 
+// The launch of a dense layer on the tensor cores: the form of a stride-2 layer by its map, panels, tile and build for pixels as rows, and
+// for one int8 output channels as rows where that is faster.
+UmmaChoice choose_dense(const std::vector<UmmaVariant>& taps, const std::vector<UmmaVariant>& parity, const std::vector<UmmaVariant>& rows, const ConvShape& s,
+                        int sm_count, bool f32_input, bool may_quantize, bool may_box, bool one_int8_output, long* tiles = nullptr) {
+    const bool by_parity = !parity.empty() && umma_prefers_parity(parity.data(), (int)parity.size(), taps.data(), s, sm_count);
+    const std::vector<UmmaVariant>& form = by_parity ? parity : taps;
+    const UmmaChoice c = umma_choose(form.data(), (int)form.size(), s, sm_count, may_quantize, tiles);
+    return one_int8_output ? umma_choose_rows(c, rows.data(), (int)rows.size(), s, sm_count, f32_input, may_box) : c;
+}
+
 size_t dtype_bytes(int dtype, int n, int c, int h, int w) {
     const size_t pix = (size_t)n * h * w;
     switch (dtype) {
@@ -846,12 +856,14 @@ int ott_conv_f32_forward(ott_ctx* ctx, const ott_conv_f32* c, const float* in_de
     return OTT_OK;
 }
 
-int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int w, int f32_input, int sm_count, int plan[8]) {
+int ott_debug_dense_launch(int cin, int cout, int k, int stride, int n, int h, int w, int f32_input, int int8_output, int sm_count, int plan[9]) {
     if (!plan || cin < 1 || cout < 1 || k < 1 || stride < 1 || n < 1 || h < 1 || w < 1 || sm_count < 1) return OTT_ERR_INVALID;
     constexpr int kSmemOptin = 227 * 1024;
-    UmmaPlan widest{};
+    UmmaPlan widest{}, other{};
     if (!umma_plan_layer(cin, cout, k, k, stride, stride, 1, 1, kSmemOptin, &widest)) return OTT_ERR_UNSUPPORTED;
-    const std::vector<UmmaVariant> all = umma_variants(widest, cout, kSmemOptin);
+    std::vector<UmmaVariant> parity, rows;
+    if (umma_plan_parity(widest, cin, cout, k, k, stride, stride, 1, 1, kSmemOptin, &other)) parity = umma_variants(other, cout, kSmemOptin);
+    if (int8_output) rows = umma_row_variants(widest, cout, kSmemOptin);
     ConvShape s{};
     s.n = n; s.h = h; s.w = w; s.cin = cin; s.cout = cout; s.cin_pad = nhwc_channels(cin); s.cout_pad = nhwc_channels(cout);
     s.kh = s.kw = k; s.sh = s.sw = stride; s.ph = s.pw = k / 2; s.dh = s.dw = 1;
@@ -859,29 +871,25 @@ int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int
     s.ow = out_dim(w, k, stride, k / 2, 1);
     if (s.oh < 1 || s.ow < 1) return OTT_ERR_INVALID;
     long tiles = 0;
-    UmmaPlan other{};
-    const bool has_parity = umma_plan_parity(widest, cin, cout, k, k, stride, stride, 1, 1, kSmemOptin, &other);
-    const std::vector<UmmaVariant> parity = has_parity ? umma_variants(other, cout, kSmemOptin) : std::vector<UmmaVariant>();
-    const bool by_parity = has_parity && umma_prefers_parity(parity.data(), (int)parity.size(), all.data(), s, sm_count);
-    const std::vector<UmmaVariant>& form = by_parity ? parity : all;
-    const UmmaChoice c = umma_choose(form.data(), (int)form.size(), s, sm_count, f32_input != 0, &tiles);
-    const int out[8] = {(int)tiles, c.variant->plan.n_tiles, c.variant->plan.bn, c.variant->plan.ctas_per_sm, c.inside, c.compact, c.tile_rows, c.variant->plan.halo};
+    const UmmaChoice c = choose_dense(umma_variants(widest, cout, kSmemOptin), parity, rows, s, sm_count, f32_input != 0, f32_input != 0,
+                                      f32_input && (long)h * w % 4 == 0, int8_output != 0, &tiles);
+    const UmmaPlan& p = c.variant->plan;
+    const int out[9] = {(int)tiles, p.n_tiles, p.bn, p.ctas_per_sm, c.inside, c.compact, c.tile_rows, p.halo, p.rows};
     std::memcpy(plan, out, sizeof out);
     return OTT_OK;
 }
 
+int ott_debug_dense_plan(int cin, int cout, int k, int stride, int n, int h, int w, int f32_input, int sm_count, int plan[8]) {
+    int all[9];
+    const int rc = plan ? ott_debug_dense_launch(cin, cout, k, stride, n, h, w, f32_input, 0, sm_count, all) : OTT_ERR_INVALID;
+    if (rc == OTT_OK) std::memcpy(plan, all, 8 * sizeof(int));
+    return rc;
+}
+
 int ott_debug_dense_rows(int cin, int cout, int n, int h, int w, int f32_input, int sm_count) {
-    if (cin < 1 || cout < 1 || n < 1 || h < 1 || w < 1 || sm_count < 1) return OTT_ERR_INVALID;
-    constexpr int kSmemOptin = 227 * 1024;
-    UmmaPlan widest{};
-    if (!umma_plan_layer(cin, cout, 1, 1, 1, 1, 1, 1, kSmemOptin, &widest)) return OTT_ERR_UNSUPPORTED;
-    const std::vector<UmmaVariant> all = umma_variants(widest, cout, kSmemOptin), rows = umma_row_variants(widest, cout, kSmemOptin);
-    ConvShape s{};
-    s.n = n; s.h = s.oh = h; s.w = s.ow = w; s.cin = cin; s.cout = cout; s.cin_pad = nhwc_channels(cin); s.cout_pad = nhwc_channels(cout);
-    s.kh = s.kw = s.sh = s.sw = s.dh = s.dw = 1;
-    const bool f32 = f32_input != 0;
-    const UmmaChoice c = umma_choose_rows(umma_choose(all.data(), (int)all.size(), s, sm_count, f32), rows.data(), (int)rows.size(), s, sm_count, f32, f32 && (long)h * w % 4 == 0);
-    return c.variant->plan.rows ? c.variant->plan.bn : 0;
+    int all[9];
+    const int rc = ott_debug_dense_launch(cin, cout, 1, 1, n, h, w, f32_input, 1, sm_count, all);
+    return rc != OTT_OK ? rc : all[8] ? all[2] : 0;
 }
 
 int ott_conv_int8_kernel_kind(const ott_conv* c) { return c ? c->kind : OTT_ERR_INVALID; }
@@ -1217,14 +1225,10 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
     UmmaFloatInput f32;
     UmmaChoice choice{};
     if (c->kind == OTT_KERNEL_DENSE_UMMA) {
-        const bool parity = !c->umma_parity.empty() && umma_prefers_parity(c->umma_parity.data(), (int)c->umma_parity.size(), c->umma.data(), s, ctx->sm_count);
-        const std::vector<UmmaVariant>& form = parity ? c->umma_parity : c->umma;
         const bool may_quantize = in_dtype == OTT_F32_NCHW && c->n_in_scales == 1 &&
                                   umma_float_input(static_cast<const float*>(in_dev), gather, d.cin, (long)h * w, c->in_scale0, &f32);
-        choice = umma_choose(form.data(), (int)form.size(), s, ctx->sm_count, may_quantize);
-        if (out_dtype == OTT_S8_NHWC && !mixed)
-            choice = umma_choose_rows(choice, c->umma_rows.data(), (int)c->umma_rows.size(), s, ctx->sm_count, in_dtype == OTT_F32_NCHW,
-                                      may_quantize && umma_box_input(f32, (long)h * w));
+        choice = choose_dense(c->umma, c->umma_parity, c->umma_rows, s, ctx->sm_count, in_dtype == OTT_F32_NCHW, may_quantize,
+                              may_quantize && umma_box_input(f32, (long)h * w), out_dtype == OTT_S8_NHWC && !mixed);
     }
     const bool quant_inside = choice.inside;
     if (in_dtype == OTT_F32_NCHW) {

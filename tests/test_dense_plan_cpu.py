@@ -1,5 +1,6 @@
 """Which launch a dense layer takes, on the CPU over thousands of layers: narrow weight panels must not cost a launch what the wide ones
-would have had (one tile per CTA, one pass over fp32 input), and a stride-2 layer takes the form that suits its map."""
+would have had (one tile per CTA, one pass over fp32 input), a stride-2 layer takes the form that suits its map, and of the layers with one int8
+output only those whose panels waste little have channels as rows."""
 import ctypes as C
 import random
 
@@ -73,3 +74,54 @@ def test_stride_two_form_follows_the_map(plan):
     for flat, tiles in (((53, 44, 3, 2, 101, 9, 59), 202), ((32, 32, 3, 2, 128, 8, 40), 128), ((154, 140, 3, 2, 78, 13, 32), 78)):
         p = plan(*flat, 0)  # twice to three times the tiles as halo tiles of 8 x 16
         assert (p["halo"], p["tiles"]) == (0, tiles), p
+
+
+@pytest.fixture(scope="module")
+def launch():
+    from tensor_b200 import capi
+    lib = capi.library()
+
+    def ask(cin, cout, k, stride, n, h, w, f32, int8):
+        out = (C.c_int * 9)()
+        assert lib.ott_debug_dense_launch(cin, cout, k, stride, n, h, w, f32, int8, SMS, out) == 0
+        return dict(zip(("tiles", "panels", "columns", "per_sm", "inside", "compact", "rows", "halo", "channel_rows"), out))
+
+    return ask
+
+
+def test_int8_launches(plan, launch):
+    seen = set()
+    for layer in _layers(4000, 2):
+        cin, cout, k, stride, n, h, w = layer
+        for f32 in (0, 1):
+            base, p = plan(*layer, f32), launch(*layer, f32, 1)
+            without = launch(*layer, f32, 0)
+            assert without.pop("channel_rows") == 0 and without == base
+            if not p["channel_rows"]:
+                assert {key: p[key] for key in base} == base
+                continue
+            cout_pad, k_total = (cout + 15) // 16 * 16, (cin + 31) // 32 * 32
+            assert k == 1 and not p["compact"] and p["halo"] == 0, (layer, p)
+            if p["inside"]:  # the input quantized once, in front of all the channels
+                assert f32 and p["channel_rows"] == p["rows"] == 64 and p["panels"] == 1 and 4 * cin * n * h * w >= 96 << 20 and h * w % 4 == 0, (layer, p)
+                assert cout_pad <= p["columns"] <= 512, (layer, p)
+            else:
+                assert p["channel_rows"] == 128 and p["columns"] in (64, 128, 192, 256) and k_total <= 512 + 128, (layer, p)
+                last = cout_pad - (p["panels"] - 1) * p["columns"]
+                computed = sum((min(p["columns"], c) + 63) // 64 * 64 for c in [p["columns"]] * (p["panels"] - 1) + [last])
+                assert computed <= 1.4 * cout_pad, (layer, p)
+            seen.add((p["inside"], p["columns"] if not p["inside"] else 0, p["panels"] > 1, p["per_sm"]))
+    assert len(seen) >= 8, seen
+
+
+@pytest.mark.parametrize("layer,f32,panels,columns,inside,rows", [
+    ((256, 512, 1, 1, 128, 28, 28), 1, 1, 512, 1, 64),
+    ((256, 512, 1, 1, 128, 28, 27), 1, 2, 256, 0, 128),  # 99.1 MB of input
+    ((256, 512, 1, 1, 128, 28, 28), 0, 2, 256, 0, 128),
+    ((64, 256, 1, 1, 128, 56, 56), 0, 1, 256, 0, 128),
+    ((58, 58, 1, 1, 64, 40, 40), 0, 1, 64, 0, 128),
+    ((600, 256, 1, 1, 128, 28, 28), 0, 1, 256, 0, 0),    # the MMAs are the longer half
+    ((64, 64, 3, 1, 256, 56, 56), 0, 1, 64, 0, 0)])
+def test_named_int8_launches(launch, layer, f32, panels, columns, inside, rows):
+    p = launch(*layer, f32, 1)
+    assert (p["panels"], p["columns"], p["inside"], p["channel_rows"]) == (panels, columns, inside, rows), p
