@@ -871,7 +871,8 @@ int ott_debug_dense_launch(int cin, int cout, int k, int stride, int n, int h, i
     s.ow = out_dim(w, k, stride, k / 2, 1);
     if (s.oh < 1 || s.ow < 1) return OTT_ERR_INVALID;
     long tiles = 0;
-    const UmmaChoice c = choose_dense(umma_variants(widest, cout, kSmemOptin), parity, rows, s, sm_count, f32_input != 0, f32_input != 0,
+    const std::vector<UmmaVariant> taps = umma_variants(widest, cout, kSmemOptin);  // (the choice points into one of these)
+    const UmmaChoice c = choose_dense(taps, parity, rows, s, sm_count, f32_input != 0, f32_input != 0,
                                       f32_input && (long)h * w % 4 == 0, int8_output != 0, &tiles);
     const UmmaPlan& p = c.variant->plan;
     const int out[9] = {(int)tiles, p.n_tiles, p.bn, p.ctas_per_sm, c.inside, c.compact, c.tile_rows, p.halo, p.rows};
