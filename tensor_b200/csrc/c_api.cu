@@ -1074,7 +1074,8 @@ int forward_maxpool_impl(ott_ctx* ctx, const ott_conv* c, const float* in_dev, i
     ep.has_bias = d.bias_term ? 1 : 0;
     ep.act_type = d.act_type; ep.act_param0 = d.act_param0; ep.rounding = d.rounding;
     OTT_CUDA_CHECK(ctx, launch_dense_stem_pool(ctx->stream, s, in_dev, c->w_host.data(), c->scale_in_host.data(), c->bias_host.data(),
-                                                c->scale_out_host.data(), c->in_scale0, ep, out_dev, out_dtype, pad_with_zero, ctx->status_dev));
+                                                c->scale_out_host.data(), c->in_scale0, ep, out_dev, out_dtype, pad_with_zero, ctx->status_dev, ctx->sm_count,
+                                                ctx->wait_limit_ns));
     ctx->launches += 1;
     return OTT_OK;
 }

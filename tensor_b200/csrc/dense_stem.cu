@@ -171,7 +171,7 @@ template <int S, int ACT, bool OUT8>
 __global__ void __launch_bounds__(256, 4)
 dense_stem_pool_mma_kernel(const __grid_constant__ CUtensorMap image, const float* __restrict__ x, const __grid_constant__ StemParams P, float in_scale, float act_p0,
                            uint32_t half, void* __restrict__ out_any, ConvShape s, int ph_out, int pw_out, int tiles_x, int tiles_y, int tiles, FastDiv div_x, FastDiv div_y,
-                           int by_box, int pad_zero, uint32_t* __restrict__ status) {
+                           int by_box, int pad_zero, uint32_t* __restrict__ status, unsigned long long wait_ns) {
     using namespace umma;
     using Tile = StemTile<S>;
     constexpr int IH = Tile::IH, RP = Tile::RP, WORDS = Tile::WORDS;
@@ -247,7 +247,7 @@ dense_stem_pool_mma_kernel(const __grid_constant__ CUtensorMap image, const floa
     uint32_t phase = 0;
     for (int t = (int)blockIdx.x; t < tiles; t += (int)gridDim.x, phase ^= 1u) {
     if (by_box) {
-        if (!mbar_wait_warp(bar_x, phase, &abort_flag, status, 32u)) {
+        if (!mbar_wait_warp(bar_x, phase, &abort_flag, status, 32u, wait_ns)) {
             ok = false;
             const unsigned long long t0 = globaltimer_ns();
             while (globaltimer_ns() - t0 < 1000000ull) {}  // let the copy in flight land before its place is written
@@ -325,7 +325,7 @@ dense_stem_pool_mma_kernel(const __grid_constant__ CUtensorMap image, const floa
         }
         __syncwarp();
     }
-    if (!mbar_wait_warp(bar_d, phase, &abort_flag, status, 32u)) ok = false;
+    if (!mbar_wait_warp(bar_d, phase, &abort_flag, status, 32u, wait_ns)) ok = false;
     tc_fence_after();
     // the next tile's box takes the place of the taps, which the MMAs have read, while this tile is pooled
     if (by_box && threadIdx.x == 0 && ok && t + (int)gridDim.x < tiles) fetch(t + (int)gridDim.x);
@@ -464,14 +464,14 @@ static void fill_stem_params(StemParams& P, const ConvShape& s, const int8_t* w,
 
 template <int S, bool OUT8>
 static cudaError_t launch_pool_s(cudaStream_t stream, const float* x, const StemParams& P, float in_scale, const EpilogueParams& ep, void* out,
-                                 const ConvShape& s, int pad_zero, uint32_t* status) {
+                                 const ConvShape& s, int pad_zero, uint32_t* status, int sm_count, unsigned long long wait_ns) {
     using Tile = StemTile<S>;
     const int ph_out = (s.oh + 2 - 3) / 2 + 1, pw_out = (s.ow + 2 - 3) / 2 + 1;
     const int tiles_x = (pw_out + SP_PX - 1) / SP_PX, tiles_y = (ph_out + SP_PY - 1) / SP_PY;
     const long blocks = (long)s.n * tiles_x * tiles_y;
     if (blocks <= 0) return cudaSuccess;
     if (blocks > 0x7FFFFFFFl) return cudaErrorInvalidValue;
-    constexpr long kResident = 148 * 4;  // CTAs of the whole GPU at once; each walks over its tiles
+    const long resident = 4l * sm_count;  // CTAs of the whole GPU at once; each walks over its tiles
     // the halo tile as one box: rows of whole 16-byte words from a 16-byte boundary; any other image pixel by pixel
     CUtensorMap image{};
     const int by_box = s.w % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? 1 : 0;
@@ -491,9 +491,9 @@ static cudaError_t launch_pool_s(cudaStream_t stream, const float* x, const Stem
         auto kernel = dense_stem_pool_mma_kernel<S, ACT, OUT8>;                                                           \
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);            \
         if (e != cudaSuccess) return e;                                                                                   \
-        e = launch_overlapped(kernel, dim3((unsigned)(blocks < kResident ? blocks : kResident)), dim3(256), smem, stream, image, x, P, in_scale,  \
+        e = launch_overlapped(kernel, dim3((unsigned)(blocks < resident ? blocks : resident)), dim3(256), smem, stream, image, x, P, in_scale,  \
                               ep.act_param0, half_bits(ep.rounding), out, s, ph_out, pw_out, tiles_x, tiles_y, (int)blocks,             \
-                              make_fast_div((uint32_t)tiles_x), make_fast_div((uint32_t)tiles_y), by_box, pad_zero, status);            \
+                              make_fast_div((uint32_t)tiles_x), make_fast_div((uint32_t)tiles_y), by_box, pad_zero, status, wait_ns);            \
         if (e != cudaSuccess) return e;                                                                                   \
     }
     switch (ep.act_type) {
@@ -509,15 +509,15 @@ static cudaError_t launch_pool_s(cudaStream_t stream, const float* x, const Stem
 // first layer (fp32 output) + MaxPool 3x3 s2 p1 of its result; out is [n][cout][(oh+1)/2... pooled] fp32 NCHW
 cudaError_t launch_dense_stem_pool(cudaStream_t stream, const ConvShape& s, const float* x, const int8_t* w_oihw_host, const float* scale_in_host,
                                    const float* bias_host, const float* scale_out_host, float in_scale, const EpilogueParams& ep, void* out,
-                                   int out_dtype, int pad_zero, uint32_t* status) {
+                                   int out_dtype, int pad_zero, uint32_t* status, int sm_count, unsigned long long wait_ns) {
     StemParams P{};
     fill_stem_params(P, s, w_oihw_host, scale_in_host, bias_host, out_dtype == DT_S8_NHWC ? scale_out_host : nullptr);
     for (int o = 0; o < ST_COUT_MAX && !ep.has_bias; ++o) P.bias[o] = -0.f;  // (see epilogue.cuh)
     if (out_dtype == DT_S8_NHWC)
-        return s.sh == 1 ? launch_pool_s<1, true>(stream, x, P, in_scale, ep, out, s, pad_zero, status)
-                         : launch_pool_s<2, true>(stream, x, P, in_scale, ep, out, s, pad_zero, status);
-    return s.sh == 1 ? launch_pool_s<1, false>(stream, x, P, in_scale, ep, out, s, pad_zero, status)
-                     : launch_pool_s<2, false>(stream, x, P, in_scale, ep, out, s, pad_zero, status);
+        return s.sh == 1 ? launch_pool_s<1, true>(stream, x, P, in_scale, ep, out, s, pad_zero, status, sm_count, wait_ns)
+                         : launch_pool_s<2, true>(stream, x, P, in_scale, ep, out, s, pad_zero, status, sm_count, wait_ns);
+    return s.sh == 1 ? launch_pool_s<1, false>(stream, x, P, in_scale, ep, out, s, pad_zero, status, sm_count, wait_ns)
+                     : launch_pool_s<2, false>(stream, x, P, in_scale, ep, out, s, pad_zero, status, sm_count, wait_ns);
 }
 
 // Host-side parameter block: filters OIHW int8 [cout][3][3][3] and the per-channel epilogue vectors.

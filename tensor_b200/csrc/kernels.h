@@ -91,7 +91,7 @@ cudaError_t launch_dense_stem(cudaStream_t stream, const ConvShape& s, const flo
 // channel as an int8 NHWC tensor. Runs on the tensor cores; status: the word a timed-out wait is reported in.
 cudaError_t launch_dense_stem_pool(cudaStream_t stream, const ConvShape& s, const float* x, const int8_t* w_oihw_host, const float* scale_in_host,
                                    const float* bias_host, const float* scale_out_host, float in_scale, const EpilogueParams& ep, void* out,
-                                   int out_dtype, int pad_zero, uint32_t* status);
+                                   int out_dtype, int pad_zero, uint32_t* status, int sm_count, unsigned long long wait_ns);
 
 // fp32 convolution (the layers a mixed model keeps in floating point): x, out fp32 NCHW; weights packed by
 // conv_f32_pack_weights into [cin/groups][tap][conv_f32_channel_stride(cout)] (depthwise: [tap][stride]); bias padded to the same stride.

@@ -1,5 +1,6 @@
 """GPU: the 3-channel first layer, alone and with its max-pool, on an image that starts on every 4-byte offset from a 16-byte boundary:
-the bytes of the aligned run, both rounding rules."""
+the bytes of the aligned run, both rounding rules; and batches whose CTAs each walk over several tiles, the image by boxes and pixel
+by pixel."""
 import ctypes as C
 
 import numpy as np
@@ -41,3 +42,40 @@ def test_first_layer_on_a_misaligned_image(ctx, stride, rounding, offset):
     for p in (x, aligned, y):
         ctx.free(p)
     layer.close()
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("w,offset", [(72, 0), (70, 0), (71, 0), (72, 1)])
+def test_first_layer_and_maxpool_over_several_tiles(ctx, stride, w, offset):
+    """More than twice the tiles that the GPU's CTAs hold at once; the first, the middle and the last image against the checker."""
+    from gpu_support import bits
+    from graph_walk import maxpool_nchw
+    from support import nhwc_padded_to_nchw
+    from tensor_b200 import ConvInt8, nhwc_channels
+    n, h, cout = 91 if stride == 1 else 233, 50, 24
+    case = ConvCase("stem_tiles", 3, cout, 3, stride, 1, n=3, h=h, w=w, int8_scale_term=2, act_type=ACT_RELU, x_lo=0.0, seed=5).make()
+    conv = run_port(case, ROUND_ADD_HALF_TRUNC, want_acc=False)["y"]
+    want = maxpool_nchw(conv, 3, 2, 1, pad_zero=False)
+    scales = np.linspace(20.0, 60.0, cout).astype(np.float32)
+    t = want * scales[None, :, None, None]  # fp32 products, as in the kernel
+    want_s8 = np.clip(np.trunc(t.astype(np.float64) + 0.5), -127, 127).astype(np.int8)
+    oh, ow = want.shape[2:]
+    assert n * ((oh + 5) // 6) * ((ow + 15) // 16) > 2 * 4 * 148
+    x = np.tile(np.random.default_rng(6).uniform(0, 1, size=(5, 3, h, w)).astype(np.float32), (n // 5 + 1, 1, 1, 1))[:n]
+    at = [0, n // 2, n - 1]
+    x[at] = case.x_f32
+    kw = dict(cin=3, cout=cout, kh=3, kw=3, sh=stride, sw=stride, ph=1, pw=1, bias_term=1, act_type=ACT_RELU, weight=case.weight, bias=case.bias,
+              w_scales=case.w_scales, in_scales=case.in_scales)
+    f32_layer, s8_layer = ConvInt8(ctx, int8_scale_term=2, **kw), ConvInt8(ctx, int8_scale_term=101, out_scales=scales, **kw)
+    image = ctx.to_device(np.concatenate([np.zeros(offset, np.float32), x.reshape(-1)]))
+    f, q = ctx.malloc(n * cout * oh * ow * 4), ctx.malloc(n * oh * ow * nhwc_channels(cout))
+    ctx.check(ctx.lib.ott_conv_int8_forward_maxpool(ctx.h, f32_layer.h, C.c_void_p(image + 4 * offset), n, h, w, 0, C.c_void_p(f)))
+    ctx.check(ctx.lib.ott_conv_int8_forward_maxpool_s8(ctx.h, s8_layer.h, C.c_void_p(image + 4 * offset), n, h, w, 0, C.c_void_p(q)))
+    got, got_s8 = ctx.to_host(f, (n, cout, oh, ow), np.float32), ctx.to_host(q, (n, oh, ow, nhwc_channels(cout)), np.int8)
+    assert np.array_equal(bits(got[at]), bits(want)) and np.array_equal(nhwc_padded_to_nchw(got_s8[at], cout), want_s8)
+    rest = [i for i in range(n - 5) if i not in at and i + 5 not in at]  # images repeat every five
+    assert all(np.array_equal(got[i], got[i + 5]) and np.array_equal(got_s8[i], got_s8[i + 5]) for i in rest)
+    for p in (image, f, q):
+        ctx.free(p)
+    f32_layer.close()
+    s8_layer.close()
