@@ -1465,11 +1465,23 @@ UmmaChoice umma_choose(const UmmaVariant* v, int n, const ConvShape& s, int sm_c
 // back, and the planes can be fetched while other tiles are multiplied. us, other forms / this one: 256 -> 512 28x28 x128 (103 MB) 44.1 /
 // 38.7, 249 -> 61 192660 pixels 47.9 / 42.2, 620 -> 37 109800 pixels 59.7 / 54.0; but 105 -> 453 55200 pixels (23 MB) 16.6 / 18.8, 178 -> 58 54880
 // pixels (39 MB) 11.6 / 13.5, 120 -> 46 143000 pixels (69 MB) 18.3 / 20.7.
+// Its tiles of 64 pixels hold one image each, so that small planes leave them empty (43 -> 263 2x2 x143215 128 / 1773, 122 -> 382 6x4 x12099 66 / 155,
+// 170 -> 468 8x6 x4057 69.1 / 78.5): seven eighths full. Of 215 layers of 17 to 1024 channels, 40 to 400 MB, those whose tiles are: with few
+// input channels the accumulators are the longer half, and half-empty or many of them lose (92 -> 145 31x100 x359 151 / 181, 66 -> 137 55 / 64, 58 ->
+// 505 151 / 192, 83 -> 437 177 / 192; 101 -> 177 57 / 53, 80 -> 50 44.9 / 31.4); up to 384 they gain 1.00 to 1.58; above, the tile's operand and the weights
+// leave room for two or three stages, and only one narrow or full accumulators gain (434 -> 37 44.7 / 39.3, 624 -> 115 110 / 92; 511 -> 109 65 / 77, 612 -> 81
+// 42 / 51); above 640 none (700 -> 47 85 / 97, 722 -> 51 46.5 / 52.7).
 constexpr double kFillsL2 = 96.0 * (1 << 20);
+bool box_tiles_pay(const UmmaPlan& p, const ConvShape& s) {
+    const long hw = (long)s.h * s.w, in_tiles = (hw + p.rows - 1) / p.rows * p.rows;
+    if (4.0 * s.cin * s.n * hw < kFillsL2 || 8 * hw < 7 * in_tiles) return false;
+    if (p.k_total <= 128) return p.bn <= kTileM || (p.bn <= 3 * kTileM && 8 * s.cout_pad >= 7 * p.bn);
+    return p.k_total <= 384 || (p.k_total <= 640 && (p.bn <= 64 || 8 * s.cout_pad > 7 * p.bn));
+}
 UmmaChoice umma_choose_rows(const UmmaChoice& choice, const UmmaVariant* rows, int n_rows, const ConvShape& s, int sm_count, bool f32_input, bool may_box) {
     const PixelTiles t = tile_pixels(choice.variant->plan, s);
-    if (may_box && !choice.compact && t.flat && 4.0 * s.cin * s.n * s.h * s.w >= kFillsL2 && (double)s.n * s.h * s.w <= 2147483647.0 && n_rows > 0 &&
-        rows[n_rows - 1].plan.rows == rows_pixels(kRowsQuantBuild)) {
+    if (may_box && !choice.compact && t.flat && (double)s.n * s.h * s.w <= 2147483647.0 && n_rows > 0 &&
+        rows[n_rows - 1].plan.rows == rows_pixels(kRowsQuantBuild) && box_tiles_pay(rows[n_rows - 1].plan, s)) {
         UmmaChoice c = choice;
         c.variant = &rows[n_rows - 1];
         c.inside = true;

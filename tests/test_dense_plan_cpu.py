@@ -104,7 +104,7 @@ def test_int8_launches(plan, launch):
             assert k == 1 and not p["compact"] and p["halo"] == 0, (layer, p)
             if p["inside"]:  # the input quantized once, in front of all the channels
                 assert f32 and p["channel_rows"] == p["rows"] == 64 and p["panels"] == 1 and 4 * cin * n * h * w >= 96 << 20 and h * w % 4 == 0, (layer, p)
-                assert cout_pad <= p["columns"] <= 512, (layer, p)
+                assert cout_pad <= p["columns"] <= 512 and 8 * h * w >= 7 * ((h * w + 63) // 64 * 64) and k_total <= 640, (layer, p)
             else:
                 assert p["channel_rows"] == 128 and p["columns"] in (64, 128, 192, 256) and k_total <= 512 + 128, (layer, p)
                 last = cout_pad - (p["panels"] - 1) * p["columns"]
@@ -118,6 +118,11 @@ def test_int8_launches(plan, launch):
     ((256, 512, 1, 1, 128, 28, 28), 1, 1, 512, 1, 64),
     ((256, 512, 1, 1, 128, 28, 27), 1, 2, 256, 0, 128),  # 99.1 MB of input
     ((256, 512, 1, 1, 128, 28, 28), 0, 2, 256, 0, 128),
+    ((170, 468, 1, 1, 4057, 8, 6), 1, 2, 256, 0, 128),   # tiles of 64 pixels that 48 of an image fill
+    ((43, 263, 1, 1, 143215, 2, 2), 1, 2, 160, 0, 0),
+    ((700, 47, 1, 1, 42, 44, 80), 1, 1, 48, 1, 0),       # two stages of 768 channels
+    ((92, 145, 1, 1, 359, 31, 100), 1, 1, 160, 1, 0),    # three accumulators, one of them 17 channels
+    ((434, 37, 1, 1, 27, 54, 70), 1, 1, 64, 1, 64),
     ((64, 256, 1, 1, 128, 56, 56), 0, 1, 256, 0, 128),
     ((58, 58, 1, 1, 64, 40, 40), 0, 1, 64, 0, 128),
     ((600, 256, 1, 1, 128, 28, 28), 0, 1, 256, 0, 0),    # the MMAs are the longer half

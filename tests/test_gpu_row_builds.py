@@ -51,7 +51,7 @@ def test_epilogues(ctx, act, scale):
 
 
 @pytest.mark.parametrize("cin,cout,h,w", [(256, 512, 44, 20), (40, 330, 44, 21), (130, 240, 20, 44), (33, 64, 44, 20), (64, 100, 46, 22), (100, 16, 44, 20), (17, 40, 44, 20), (24, 24, 12, 10),
-                                          (32, 512, 20, 18)])
+                                          (32, 384, 20, 18)])
 @pytest.mark.parametrize("act", [ACT_RELU6, ACT_NONE])
 def test_quantized_inside(ctx, cin, cout, h, w, act):
     """fp32 input of 100 MB: one to four accumulators per tile of 64 pixels, the last tile of an image ragged; the first, the middle and
