@@ -362,7 +362,9 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
 // waves. The instruction counts are those of the inner loops: 26 per fp32 word loaded and quantized, 7 per 32 int8 quads
 // loaded and transposed, 46 / 75 per warp and output row of a 3x3 / 5x5 filter, 12 per row that only fills the ring. Counting the warps that
 // have no item in the last pass as if they issued kept eight-warp CTAs from launches that want them: 3x3 256 channels fp32 -> int8 56x56
-// x64 68.6 -> 65.7 us; fp32 -> fp32 from 15 us on 1.09 times as fast, the rest of 360 layers 0.99 to 1.03.
+// x64 68.6 -> 65.7 us; fp32 -> fp32 from 15 us on 1.09 times as fast, the rest of 360 layers 0.99 to 1.03. Low bands (below) are counted
+// that way all the same: what bounds them is the stores, and a count without idle warps picks bands that leave many of them (236 channels 57x72 x45 100 us, 74.9 this way;
+// 261 35x11 x78 37.6 / 33.4; 130 such layers on average the same).
 // fp32 output from int8, stride 1: a lane stores 16 bytes of its own channel's plane, half a sector (single pixels where the rows are not
 // aligned), and the rest of the sector and of the line comes from the next warps. An output that does not fit L2, or one of single
 // pixels, wants that to happen soon: low bands (planes of 128 words), eight warps side by side on the same rows. us, high bands / low:
@@ -398,7 +400,7 @@ inline Tile plan_tile(const ConvShape& s) {
             nrg = (ty + rpt - 1) / rpt;
             const int passes = (T.nxq * nrg + w - 1) / w;
             const double load = npos * (IN_F32 ? 26.0 : 7.0), item = rpt * (K == 3 ? 46.0 : 75.0) + (K - S) * 12.0;
-            const double issued = load + T.nxq * nrg * item, instr = load + passes * w * item;  // (a warp without an item in the last pass issues nothing)
+            const double instr = load + passes * w * item, issued = low ? instr : load + T.nxq * nrg * item;  // (a warp without an item in the last pass issues nothing)
             int resident = 65536 / ((K == 3 ? 64 : 80) * 32 * w);
             const int by_smem = 224 * 1024 / (CG * 4 * npos + 2048);
             if (by_smem < resident) resident = by_smem;
