@@ -39,6 +39,30 @@ int check_status_word(ott_ctx* ctx, bool copied = false) {
     return OTT_OK;
 }
 
+// Whether float2int8(act(v) * so), v = fma(acc, si, bias), with its two roundings equals trunc(fma(act(v), so, 0.5)) for every s32 sum: see
+// round2_nonneg. Only sums whose product lies within 2^-25 of 0.5 can tell the two apart; v does not decrease with the sum, so they are
+// neighbours, and both forms are worked out for the few around the one that gives 0.5.
+bool one_rounding_does(float si, float bias, bool has_bias, int act, float so, int rounding) {
+    if (!(so > 0.f) || !(std::isfinite(so) && std::isfinite(si) && std::isfinite(bias))) return so == 0.f;
+    const float h = rounding == OTT_ROUND_HALF_AWAY ? 0x1.fffffep-2f : 0.5f;
+    auto same = [&](float y) {
+        const volatile float product = y * so;
+        const volatile float sum = product + h;
+        return std::trunc(sum) == std::trunc(std::fma(y, so, 0.5f));
+    };
+    if (act == ACT_RELU6 && !same(6.f)) return false;
+    if (si == 0.f) return !(bias > 0.f) || same(act == ACT_RELU6 ? std::min(bias, 6.f) : bias);
+    const double at = (0.5 / (double)so - (double)bias) / (double)si, away = 4.0 + std::fabs(at) * 0x1p-21 + std::fabs((double)bias / si) * 0x1p-22;
+    if (std::fabs(at) > 4294967296.0) return true;  // (no s32 sum comes near)
+    if (away > 4096.0) return false;                // (so many that it is not worth a look)
+    for (double acc = std::floor(at - away); acc <= at + away; acc += 1.0) {
+        const volatile float a = (float)acc, plain = a * si;
+        const float v = has_bias ? std::fma((float)a, si, bias) : (float)plain;
+        if (v > 0.f && !same(act == ACT_RELU6 ? std::min(v, 6.f) : v)) return false;
+    }
+    return true;
+}
+
 // The launch of a dense layer on the tensor cores: the form of a stride-2 layer by its map, panels, tile and build for pixels as rows, and
 // for one int8 output channels as rows where that is faster.
 UmmaChoice choose_dense(const std::vector<UmmaVariant>& taps, const std::vector<UmmaVariant>& parity, const std::vector<UmmaVariant>& rows, const ConvShape& s,
@@ -615,20 +639,21 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
     c->scale_out_host = scale_out;
     c->in_scale0 = in_scales[0];
     if (requant) {
-        c->negative_scale = std::any_of(scale_out.begin(), scale_out.end(), [](float v) { return v < 0.f; }) ? 1 : 0;
+        const size_t per_cout = (size_t)(d->cin / d->groups) * d->kh * d->kw;
+        if (d->act_type == ACT_RELU || d->act_type == ACT_RELU6)
+            for (int p = 0; p < d->cout && !c->signed_rounding; ++p)
+                c->signed_rounding = scale_out[p] < 0.f || !one_rounding_does(scale_in[p], bias_p[p], d->bias_term != 0, d->act_type, scale_out[p], d->rounding) ? 1 : 0;
         c->one_scale_out = std::isfinite(scale_out[0]) && std::all_of(scale_out.begin(), scale_out.begin() + d->cout, [&](float v) { return v == scale_out[0]; }) ? 1 : 0;
         // whether the clamp of the int8 output can stand for the activation (EpilogueParams::int8_pos): the largest sum the
         // weights allow bounds what is requantized, and ReLU6 must have nothing to cut that the clamp would not
-        bool pos = d->act_type == ACT_RELU || d->act_type == ACT_RELU6;
-        const size_t per_cout = (size_t)(d->cin / d->groups) * d->kh * d->kw;
+        bool pos = (d->act_type == ACT_RELU || d->act_type == ACT_RELU6) && !c->signed_rounding;
         for (int p = 0; p < d->cout && pos; ++p) {
             long sum = 0;
             for (size_t i = 0; i < per_cout; ++i) sum += std::abs((int)w_oihw[p * per_cout + i]);
             const double top = (128.0 * (double)sum * std::fabs((double)scale_in[p]) + std::fabs((double)bias_p[p])) * scale_out[p];
             pos = scale_out[p] > 0.f && top < 32000.0;  // (false for NaN)
             if (d->act_type == ACT_RELU6) {
-                const volatile float six = 6.f * scale_out[p], sum_h = six + (d->rounding == OTT_ROUND_HALF_AWAY ? 0x1.fffffep-2f : 0.5f);
-                pos = pos && sum_h >= 127.f;
+                pos = pos && std::fma(6.f, scale_out[p], 0.5f) >= 127.f;
             }
         }
         c->int8_pos = pos ? 1 : 0;
@@ -725,7 +750,7 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
         rc = upload(ctx, wtiled.data(), wtiled.size() * 4, (void**)&c->w_tiled_dev);
     }
     if (rc == OTT_OK && depthwise && !gi && d->kh == 3 && d->kw == 3 && d->ph == 1 && d->pw == 1 && d->dh == 1 && d->dw == 1 && d->sh == d->sw &&
-        (d->sh == 1 || d->sh == 2) && d->rounding == OTT_ROUND_ADD_HALF_TRUNC && !c->negative_scale) {
+        (d->sh == 1 || d->sh == 2) && d->rounding == OTT_ROUND_ADD_HALF_TRUNC && !c->signed_rounding) {
         int smem_optin = 0;
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
         if (dw_umma_plan(d->cout, d->sh, smem_optin, &c->dw_plan)) {
@@ -1070,7 +1095,7 @@ int forward_maxpool_impl(ott_ctx* ctx, const ott_conv* c, const float* in_dev, i
     cudaSetDevice(ctx->device);
     EpilogueParams ep{};
     ep.scale_in = c->scale_in_dev; ep.bias = c->bias_dev; ep.scale_out = c->scale_out_dev;
-    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos; ep.negative_scale = c->negative_scale;
+    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos; ep.signed_rounding = c->signed_rounding;
     ep.has_bias = d.bias_term ? 1 : 0;
     ep.act_type = d.act_type; ep.act_param0 = d.act_param0; ep.rounding = d.rounding;
     OTT_CUDA_CHECK(ctx, launch_dense_stem_pool(ctx->stream, s, in_dev, c->w_host.data(), c->scale_in_host.data(), c->bias_host.data(),
@@ -1155,13 +1180,13 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
 
     EpilogueParams ep{};
     ep.scale_in = c->scale_in_dev; ep.bias = c->bias_dev; ep.scale_out = c->scale_out_dev;
-    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos; ep.negative_scale = c->negative_scale;
+    ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos; ep.signed_rounding = c->signed_rounding;
     ep.has_bias = d.bias_term ? 1 : 0;
     ep.act_type = d.act_type; ep.act_param0 = d.act_param0; ep.rounding = d.rounding;
 
-    // The CUDA-core depthwise kernel rounds what ReLU left as a number that is not negative. Under a negative scale the layer runs as
-    // the LeakyReLU of slope 0, whose results are the same int8 values (ReLU6: see the kernel).
-    if (c->kind == OTT_KERNEL_DEPTHWISE && c->negative_scale && out_dtype == OTT_S8_NHWC && d.act_type == ACT_RELU) {
+    // The CUDA-core depthwise kernel rounds what ReLU left as a number that is not negative, in one step. Where that does not do the layer runs
+    // as the LeakyReLU of slope 0, whose results are the same int8 values (ReLU6: a build of its own).
+    if (c->kind == OTT_KERNEL_DEPTHWISE && c->signed_rounding && out_dtype == OTT_S8_NHWC && d.act_type == ACT_RELU) {
         ep.act_type = ACT_LRELU;
         ep.act_param0 = 0.f;
     }

@@ -27,7 +27,7 @@ struct ott_conv {
     std::vector<int8_t> w_host;
     std::vector<float> scale_in_host, bias_host, scale_out_host;
     float in_scale0 = 1.f;
-    int one_scale_out = 0, int8_pos = 0, negative_scale = 0;  // see EpilogueParams
+    int one_scale_out = 0, int8_pos = 0, signed_rounding = 0;  // see EpilogueParams
     ottk::UmmaPlan plan{};
     std::vector<ottk::UmmaVariant> umma;  // tensor-core layers: `plan` and the narrower ones, each with its weight map
     std::vector<ottk::UmmaVariant> umma_parity;  // stride-2 layers: the other form, over weights packed for it

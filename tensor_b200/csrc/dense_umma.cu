@@ -780,12 +780,12 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         const float2 t = __ffma2_rn(make_float2(__int2float_rn(a[4 * g + 2 * j]), __int2float_rn(a[4 * g + 2 * j + 1])), si[h][j], bi[h][j]);
-                        y[j] = __fmul2_rn(make_float2(activate_t<ACT>(t.x, ep.act_param0), activate_t<ACT>(t.y, ep.act_param0)), so[h][j]);
+                        y[j] = make_float2(activate_t<ACT>(t.x, ep.act_param0), activate_t<ACT>(t.y, ep.act_param0));
                     }
                     if constexpr (ACT == ACT_POS) {
-                        w[g] = requant4_pos(y[0], y[1], half);
+                        w[g] = requant4_pos(y[0], so[h][0], y[1], so[h][1]);
                     } else {
-                        const int2 qa = round2(y[0], half), qb = round2(y[1], half);
+                        const int2 qa = round2(__fmul2_rn(y[0], so[h][0]), half), qb = round2(__fmul2_rn(y[1], so[h][1]), half);
                         w[g] = pack_sat_s8x4(qa.x, qa.y, qb.x, qb.y);
                     }
                 }
@@ -956,12 +956,12 @@ dense_umma_kernel(const __grid_constant__ InputOf<BUILD> maps, const __grid_cons
                         float4 so;
                         if constexpr (ONE_SCALE) so = make_float4(ep.scale_out0, ep.scale_out0, ep.scale_out0, ep.scale_out0);
                         else so = *reinterpret_cast<const float4*>(s_so + col0 + g * 4);
-                        const float2 ta = __fmul2_rn(make_float2(y[g * 4], y[g * 4 + 1]), make_float2(so.x, so.y));
-                        const float2 tb = __fmul2_rn(make_float2(y[g * 4 + 2], y[g * 4 + 3]), make_float2(so.z, so.w));
+                        const float2 ya = make_float2(y[g * 4], y[g * 4 + 1]), yb = make_float2(y[g * 4 + 2], y[g * 4 + 3]), sa = make_float2(so.x, so.y),
+                                     sb = make_float2(so.z, so.w);
                         if constexpr (ACT == ACT_POS) {
-                            wds[g] = requant4_pos(ta, tb, half);
+                            wds[g] = requant4_pos(ya, sa, yb, sb);
                         } else {
-                            const int2 qa = round2(ta, half), qb = round2(tb, half);  // (signed: a scale may be negative)
+                            const int2 qa = round2(__fmul2_rn(ya, sa), half), qb = round2(__fmul2_rn(yb, sb), half);  // (signed: a scale may be negative)
                             wds[g] = pack_sat_s8x4(qa.x, qa.y, qb.x, qb.y);
                         }
                     }

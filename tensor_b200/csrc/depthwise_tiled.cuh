@@ -114,28 +114,29 @@ struct RowRing {
     }
 };
 
+// Added to the activation of an int8 build: EpilogueParams::signed_rounding (ReLU6; such a layer with ReLU runs as the LeakyReLU of slope 0).
+constexpr int kSignedRounding = 8;
+
 // Four accumulators of one channel -> four int8 in one word, the arithmetic as packed pairs.
-// top, half: see the caller.
-template <int ACT>
-__device__ __forceinline__ uint32_t epi_s8x4(const int (&acc)[4], float si, float bi, float so, float p0, float top, uint32_t half) {
+template <int ACT, bool SIGNED>
+__device__ __forceinline__ uint32_t epi_s8x4(const int (&acc)[4], float si, float bi, float so, float p0, uint32_t half) {
     const float2 s2 = make_float2(si, si), b2 = make_float2(bi, bi), o2 = make_float2(so, so);
     int2 q[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const float2 v = __ffma2_rn(make_float2(__int2float_rn(acc[2 * h]), __int2float_rn(acc[2 * h + 1])), s2, b2);
-        const float2 y = ACT == ACT_RELU6 ? make_float2(fminf(fmaxf(v.x, 0.f), top), fminf(fmaxf(v.y, 0.f), top))
-                                          : make_float2(activate_t<ACT>(v.x, p0), activate_t<ACT>(v.y, p0));
-        q[h] = round2_act<ACT>(__fmul2_rn(y, o2), half);
+        q[h] = round2_act<ACT, SIGNED>(make_float2(activate_t<ACT>(v.x, p0), activate_t<ACT>(v.y, p0)), o2, half);
     }
     return pack_sat_s8x4(q[0].x, q[0].y, q[1].x, q[1].y);
 }
 
-template <int K, int S, bool IN_F32, int EPI, int ACT>
+template <int K, int S, bool IN_F32, int EPI, int ACT_BUILD>
 __global__ void __launch_bounds__(THREADS, K == 3 ? 4 : 3)
 depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ PlaneGather G, const uint32_t* __restrict__ wq,
                        const float* __restrict__ in_scales, int n_in_scales, EpilogueParams ep, void* __restrict__ out, ConvShape s, Tile T,
                        int aligned) {
-    constexpr int KK = Geo<K, S>::KK;
+    constexpr int KK = Geo<K, S>::KK, ACT = ACT_BUILD & ~kSignedRounding;
+    constexpr bool SIGNED = (ACT_BUILD & kSignedRounding) != 0;
     extern __shared__ uint32_t smem[];
     __shared__ const float* ch_ptr[CG];
     __shared__ float ch_scale[CG];
@@ -172,10 +173,6 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
     const float p_bi = c_ok ? bias_or_neutral(ep, c) : 0.f;
     const uint32_t half = half_bits(ep.rounding);
     const float p_so = c_ok && EPI != EPI_F32 ? __ldg(ep.scale_out + c) : 0.f;
-    // ReLU6 under a negative scale: nothing is above zero after the product, so the rounding constant changes its sign, and the product
-    // is kept above -127.5 by cutting the activation where it has reached -127.25
-    const float p_top = p_so < 0.f ? fminf(6.f, __fdiv_rn(-127.25f, p_so)) : 6.f;
-    const uint32_t half_out = ACT == ACT_RELU6 && p_so < 0.f ? half | 0x80000000u : half;
     if (IN_F32 && tid < CG && c0 + tid < s.cin) {
         ch_ptr[tid] = G.plane(c0 + tid, img, (long)s.h * s.w);
         ch_scale[tid] = n_in_scales == 1 ? __ldg(in_scales) : __ldg(in_scales + c0 + tid);
@@ -322,7 +319,7 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
             int acc[4] = {0, 0, 0, 0};
             ring.template advance<R>(p, T.rp, sh, wmod8, wk, wv, w44, acc);
             if (EPI != EPI_F32) {
-                uint32_t w = epi_s8x4<ACT>(acc, p_si, p_bi, p_so, ep.act_param0, p_top, half_out);
+                uint32_t w = epi_s8x4<ACT, SIGNED>(acc, p_si, p_bi, p_so, ep.act_param0, half);
                 w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 2), sel_a);
                 w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 1), sel_b);
                 if (store_ok) *reinterpret_cast<uint32_t*>(o8) = w;
@@ -455,6 +452,9 @@ cudaError_t launch_t(cudaStream_t stream, const ConvShape& s, const void* x, con
 template <int K, int S, bool IN_F32, int EPI>
 cudaError_t launch_act(cudaStream_t stream, const ConvShape& s, const void* x, const PlaneGather& G, const uint32_t* wq, const float* in_scales,
                        int n_in_scales, const EpilogueParams& ep, void* out) {
+    if constexpr (EPI != EPI_F32)
+        if (ep.signed_rounding && ep.act_type == ACT_RELU6)
+            return launch_t<K, S, IN_F32, EPI, ACT_RELU6 | kSignedRounding>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);
     switch (ep.act_type) {
         case ACT_RELU: return launch_t<K, S, IN_F32, EPI, ACT_RELU>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);
         case ACT_LRELU: return launch_t<K, S, IN_F32, EPI, ACT_LRELU>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);

@@ -153,7 +153,7 @@ int ott_dwpw_int8_forward_io(ott_ctx* ctx, const ott_dwpw* f, const ott_conv_io*
     ep.dw.has_bias = 1;
     ep.pw.scale_in = f->pw->scale_in_dev; ep.pw.bias = f->pw->bias_dev; ep.pw.scale_out = f->pw->scale_out_dev;
     ep.pw.has_bias = 1; ep.pw.act_type = f->pw->d.act_type; ep.pw.act_param0 = f->pw->d.act_param0;
-    ep.pw.negative_scale = f->pw->negative_scale;
+    ep.pw.signed_rounding = f->pw->signed_rounding;
     const char* err = launch_dwpw_umma(ctx->stream, ctx->sm_count, f->plan, f->maps, s, x, gathered ? &us : nullptr, f->cout2, ep, io->out_dev, io->out_dtype,
                                        status_word_dev ? status_word_dev : ctx->status_dev, io->out_f32_dev ? &mixed : nullptr, ctx->wait_limit_ns);
     if (err) return ctx->fail(OTT_ERR_CUDA, "%s: %s", err, cudaGetErrorString(cudaGetLastError()));

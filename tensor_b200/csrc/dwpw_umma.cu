@@ -481,8 +481,8 @@ const char* launch_dwpw_umma(cudaStream_t stream, int sm_count, const DwPwPlan& 
     }
     const int act = ep.pw.act_type;
     if (out_dtype == DT_F32_NCHW) { OTT_DWPW_ACT(DT_F32_NCHW) }
-    else if (ep.pw.negative_scale && act == ACT_RELU) OTT_DWPW_LAUNCH((ACT_RELU | kSignedScale), DT_S8_NHWC);
-    else if (ep.pw.negative_scale && act == ACT_RELU6) OTT_DWPW_LAUNCH((ACT_RELU6 | kSignedScale), DT_S8_NHWC);
+    else if (ep.pw.signed_rounding && act == ACT_RELU) OTT_DWPW_LAUNCH((ACT_RELU | kSignedScale), DT_S8_NHWC);
+    else if (ep.pw.signed_rounding && act == ACT_RELU6) OTT_DWPW_LAUNCH((ACT_RELU6 | kSignedScale), DT_S8_NHWC);
     else { OTT_DWPW_ACT(DT_S8_NHWC) }
 #undef OTT_DWPW_ACT
 #undef OTT_DWPW_LAUNCH

@@ -35,9 +35,11 @@ struct EpilogueParams {
     int one_scale_out;       // every channel's scale_out is scale_out0, and finite (padding channels, which hold 0, take it too)
     float scale_out0;
     // ReLU, or ReLU6 where f(6) is 127 in every channel, and |v * scale_out| + 1 stays below 2^15 in every channel whatever the int8
-    // input is: float2int8(act(v) * scale_out) is trunc(v * scale_out + h) clamped to [0, 127], see requant4_pos
+    // input is, and not signed_rounding: float2int8(act(v) * scale_out) is trunc(v * scale_out + h) clamped to [0, 127], see requant4_pos
     int int8_pos;
-    int negative_scale;      // some channel's scale_out is below zero
+    // ReLU or ReLU6, and some channel's scale_out is below zero, or some sum gives a product so close to 0.5 that one rounding would not do
+    // for two (round2_nonneg)
+    int signed_rounding;
 };
 
 __device__ __forceinline__ float dequant(int acc, float scale_in, float bias, int has_bias) {
@@ -118,25 +120,35 @@ __device__ __forceinline__ int2 round2(float2 v, uint32_t h) {
     return make_int2(__float2int_rz(fmaxf(r.x, -127.5f)), __float2int_rz(fmaxf(r.y, -127.5f)));
 }
 
-// the same for v >= 0 (after ReLU / ReLU6, times a scale that is not negative): copysign(h, v) is +h; v == -0 truncates to 0 either way
-__device__ __forceinline__ int2 round2_nonneg(float2 v, uint32_t h) {
-    const float2 r = __fadd2_rn(v, make_float2(__uint_as_float(h), __uint_as_float(h)));
+// Behind ReLU / ReLU6 and a scale that is not negative the product and the rounding are one fused multiply-add: trunc(fma(y, s, 0.5)). For
+// every integer n >= 1 that passes n + 0.5 at the same product as BOTH rules with their two roundings: RN(p) >= n + 0.5 and RN(p + 0.5) >= n + 1
+// each ask for p >= n + 0.5 - half a step of fp32, the steps below n + 0.5 and n + 1 being equal, ties going up in both (n + 0.5 and n + 1 have even
+// significands). Only below 0.5, where the steps differ, do they part, for products within 2^-25 of it; which sums give such a
+// product is known when the layer is created (EpilogueParams::signed_rounding), and a layer that has one does not come here.
+// The two roundings cannot be written as a product and a sum: the compiler contracts mul.rn.f32x2 with an add.rn.f32x2 that is its only
+// reader (it does, with -fmad=false and .rn alike), and with h = 0.5 - 2^-25 that moved one product in some millions across
+// n + 0.5. round2 is safe from that: the product has a second reader, half_signed.
+constexpr uint32_t kHalfFused = 0x3F000000u;
+
+__device__ __forceinline__ int2 round2_nonneg(float2 y, float2 s) {
+    const float2 r = __ffma2_rn(y, s, make_float2(__uint_as_float(kHalfFused), __uint_as_float(kHalfFused)));
     return make_int2(__float2int_rz(r.x), __float2int_rz(r.y));
 }
 
-// SIGNED: some output scale is below zero, so that what follows ReLU / ReLU6 may be too
+// float2int8(y * s), the clamp at +127 left to pack_sat_s8x4. SIGNED: EpilogueParams::signed_rounding
 template <int ACT, bool SIGNED = false>
-__device__ __forceinline__ int2 round2_act(float2 v, uint32_t h) {
-    return !SIGNED && (ACT == ACT_RELU || ACT == ACT_RELU6) ? round2_nonneg(v, h) : round2(v, h);
+__device__ __forceinline__ int2 round2_act(float2 y, float2 s, uint32_t h) {
+    if (!SIGNED && (ACT == ACT_RELU || ACT == ACT_RELU6)) return round2_nonneg(y, s);
+    return round2(__fmul2_rn(y, s), h);
 }
 
-// Four v * scale_out of an int8_pos layer -> four int8 of the activated values, a.x in byte 0. Adding 1.5 * 2^23 with rounding toward
-// zero leaves trunc(u + h) in the low bits of the sum (a floor below zero, which the clamp drops), so that neither the activation nor
+// Four sums v and scales s of an int8_pos layer -> four int8 of the activated values, va.x in byte 0. Adding 1.5 * 2^23 with rounding
+// toward zero leaves trunc(u) in the low bits of the sum (a floor below zero, which the clamp drops), so that neither the activation nor
 // a conversion to integer is an instruction of its own, and two values are clamped at a time: 2.3 logic instructions per value
-// less. Exact while |u| + h < 2^15, where the low 16 bits carry the sign.
-__device__ __forceinline__ uint32_t requant4_pos(float2 a, float2 b, uint32_t h) {
-    const float2 hh = make_float2(__uint_as_float(h), __uint_as_float(h)), magic = make_float2(12582912.f, 12582912.f);
-    const float2 ra = __fadd2_rz(__fadd2_rn(a, hh), magic), rb = __fadd2_rz(__fadd2_rn(b, hh), magic);
+// less. Exact while |u| < 2^15, where the low 16 bits carry the sign.
+__device__ __forceinline__ uint32_t requant4_pos(float2 va, float2 sa, float2 vb, float2 sb) {
+    const float2 hh = make_float2(__uint_as_float(kHalfFused), __uint_as_float(kHalfFused)), magic = make_float2(12582912.f, 12582912.f);
+    const float2 ra = __fadd2_rz(__ffma2_rn(va, sa, hh), magic), rb = __fadd2_rz(__ffma2_rn(vb, sb, hh), magic);
     uint32_t pa = __byte_perm(__float_as_uint(ra.x), __float_as_uint(ra.y), 0x5410), pb = __byte_perm(__float_as_uint(rb.x), __float_as_uint(rb.y), 0x5410);
     asm("min.relu.s16x2 %0, %0, %1;" : "+r"(pa) : "r"(0x007F007Fu));
     asm("min.relu.s16x2 %0, %0, %1;" : "+r"(pb) : "r"(0x007F007Fu));

@@ -8,7 +8,7 @@
 
 namespace ottk {
 
-// Added to the activation of a build of the fused kernels: some layer of it has an output scale below zero behind ReLU or ReLU6.
+// Added to the activation of a build of the fused kernels: some layer of it has EpilogueParams::signed_rounding.
 constexpr int kSignedScale = 8;
 
 // 16 accumulators -> 16 int8 (rounding rule: add half, truncate), packed into four words
@@ -26,8 +26,7 @@ __device__ __forceinline__ void requant16(const int (&v)[16], const float* __res
             const float2 a = make_float2(__int2float_rn(v[g * 4 + 2 * h]), __int2float_rn(v[g * 4 + 2 * h + 1]));
             const float2 t = __ffma2_rn(a, h ? make_float2(si.z, si.w) : make_float2(si.x, si.y), h ? make_float2(bi.z, bi.w) : make_float2(bi.x, bi.y));
             const float2 y = make_float2(activate_t<ACT>(t.x, p0), activate_t<ACT>(t.y, p0));
-            const float2 u = __fmul2_rn(y, h ? make_float2(so.z, so.w) : make_float2(so.x, so.y));
-            const int2 r = round2_act<ACT, SIGNED>(u, kHalfTrunc);
+            const int2 r = round2_act<ACT, SIGNED>(y, h ? make_float2(so.z, so.w) : make_float2(so.x, so.y), kHalfTrunc);
             qv[2 * h] = r.x;
             qv[2 * h + 1] = r.y;
         }
@@ -125,8 +124,7 @@ __device__ __forceinline__ void store_accumulator_row(uint32_t taddr, int ncols,
                 int qv[4];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const float2 u = __fmul2_rn(make_float2(y[g * 4 + 2 * h], y[g * 4 + 2 * h + 1]), h ? make_float2(o4.z, o4.w) : make_float2(o4.x, o4.y));
-                    const int2 r = round2_act<ACT, SIGNED>(u, kHalfTrunc);
+                    const int2 r = round2_act<ACT, SIGNED>(make_float2(y[g * 4 + 2 * h], y[g * 4 + 2 * h + 1]), h ? make_float2(o4.z, o4.w) : make_float2(o4.x, o4.y), kHalfTrunc);
                     qv[2 * h] = r.x;
                     qv[2 * h + 1] = r.y;
                 }

@@ -15,7 +15,7 @@ struct ott_unit {
     UnitWeights maps{};
     int cin1 = 0, cm = 0, cout2 = 0;
     bool requant2 = false;
-    int act = 0, negative1 = 0;  // the 1x1 layers' activation; the first one has an output scale below zero
+    int act = 0, signed1 = 0;  // the 1x1 layers' activation; EpilogueParams::signed_rounding of the first one
     float act_p1 = 0.f, act_p2 = 0.f;
     // the first layer's input: K block kb = 32 channels from block_x[kb] of source block_src[kb]
     std::vector<uint16_t> block_x;
@@ -77,7 +77,7 @@ int ott_unit_int8_create(ott_ctx* ctx, const ott_conv* pw1, const ott_conv* dw, 
     if (!u) return OTT_ERR_ALLOC;
     u->cin1 = d1.cin; u->cm = d1.cout; u->cout2 = d2.cout;
     u->requant2 = d2.int8_scale_term > 100;
-    u->negative1 = pw1->negative_scale;
+    u->signed1 = pw1->signed_rounding;
     u->act = d1.act_type; u->act_p1 = d1.act_param0; u->act_p2 = d2.act_param0;
     u->pw2 = pw2;
     std::vector<int8_t> wk;  // first layer's weights against its K order
@@ -169,12 +169,12 @@ int ott_unit_int8_forward_io(ott_ctx* ctx, const ott_unit* u, const ott_conv_io*
     const int cm = u->plan.cm;
     ep.e1.scale_in = u->params; ep.e1.bias = u->params + cm; ep.e1.scale_out = u->params + 2 * cm;
     ep.e1.has_bias = 1; ep.e1.act_type = u->act; ep.e1.act_param0 = u->act_p1;
-    ep.e1.negative_scale = u->negative1;
+    ep.e1.signed_rounding = u->signed1;
     ep.edw.scale_in = u->params + 3 * cm; ep.edw.bias = u->params + 4 * cm; ep.edw.scale_out = u->params + 5 * cm;
     ep.edw.has_bias = 1;
     ep.e2.scale_in = u->pw2->scale_in_dev; ep.e2.bias = u->pw2->bias_dev; ep.e2.scale_out = u->pw2->scale_out_dev;
     ep.e2.has_bias = 1; ep.e2.act_type = u->act; ep.e2.act_param0 = u->act_p2;
-    ep.e2.negative_scale = u->pw2->negative_scale;
+    ep.e2.signed_rounding = u->pw2->signed_rounding;
     const char* err = launch_unit_umma(ctx->stream, ctx->sm_count, u->plan, u->maps, us, n, h, w, u->cout2, ep, io->out_dev, io->out_dtype,
                                        status_word_dev ? status_word_dev : ctx->status_dev, io->out_f32_dev ? &mixed : nullptr, ctx->wait_limit_ns);
     if (err) return ctx->fail(OTT_ERR_CUDA, "%s: %s", err, cudaGetErrorString(cudaGetLastError()));

@@ -467,9 +467,9 @@ const char* launch_unit_umma(cudaStream_t stream, int sm_count, const UnitPlan& 
         if (out_dtype == DT_F32_NCHW) OTT_UNIT_LAUNCH((ACT | kSignedScale), DT_F32_NCHW);                    \
         else OTT_UNIT_LAUNCH((ACT | kSignedScale), DT_S8_NHWC);                                              \
     }
-    const bool negative = ep.e1.negative_scale || ep.e2.negative_scale;
-    if (negative && act == ACT_RELU) OTT_UNIT_SIGNED(ACT_RELU)
-    else if (negative && act == ACT_RELU6) OTT_UNIT_SIGNED(ACT_RELU6)
+    const bool signed_rounding = ep.e1.signed_rounding || ep.e2.signed_rounding;
+    if (signed_rounding && act == ACT_RELU) OTT_UNIT_SIGNED(ACT_RELU)
+    else if (signed_rounding && act == ACT_RELU6) OTT_UNIT_SIGNED(ACT_RELU6)
     else if (out_dtype == DT_F32_NCHW) { OTT_UNIT_ACT(DT_F32_NCHW) } else { OTT_UNIT_ACT(DT_S8_NHWC) }
 #undef OTT_UNIT_SIGNED
 #undef OTT_UNIT_ACT
