@@ -22,6 +22,7 @@ struct HostPipeline {
     void* dev_in = nullptr;
     std::vector<ott_net_graph*> graphs;
     int calls = 0;       // calls of this shape so far
+    int retry_at = 0;    // memory was refused to its capture: the call at which it is tried again
     bool plain = false;  // cannot be captured, or delivers a blob that has to be re-ordered on the host: runs layer by layer
 };
 // Shapes with captured graphs, and shapes remembered in all. The shape unused for longest goes: of those without graphs, or, when a
@@ -312,7 +313,7 @@ int ott_net_forward(ott_net* net, const char* input_blob, const void* in, int in
         const size_t img_bytes = (size_t)c * h * w * sizeof(float);
         const bool chunked = n >= 2 * chunk;
         pipe = net->pipeline(pipeline_key(net, "forward", input_blob, n, c, h, w, n_out, out_blobs));
-        if (chunked && pipe->graphs.empty() && !pipe->plain) {
+        if (chunked && pipe->graphs.empty() && !pipe->plain && pipe->calls >= pipe->retry_at) {
             const int rc = net->build(*pipe, input_blob, n, c, h, w, chunk, n_out, out_blobs, true);
             if (rc != OTT_OK) return rc;
         }
@@ -456,7 +457,7 @@ bool ott_net::release_graphs() {
         if (p.graphs.empty()) continue;
         any = true;
         drop(p);
-        p.calls = 0;
+        p.calls = p.retry_at = 0;
     }
     return any;
 }
@@ -484,7 +485,7 @@ HostPipeline* ott_net::pipeline(const std::string& key) {
 bool ott_net::may_capture(const HostPipeline& p) {
     size_t captured = 0;
     for (const HostPipeline& q : pipelines) captured += q.graphs.empty() ? 0 : 1;
-    return p.calls >= (captured < kMaxCaptured ? 2 : kCallsToReplace);
+    return p.calls >= p.retry_at && p.calls >= (captured < kMaxCaptured ? 2 : kCallsToReplace);
 }
 
 int ott_net::capture(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs, bool warm) {
@@ -505,22 +506,23 @@ int ott_net::capture(HostPipeline& p, const char* input_blob, int n, int c, int 
     return rc;
 }
 
-// Captures the pipeline's graphs. A wait that ran out is reported (the next call tries again). Any other failure, or an output that
-// is not dense NCHW, makes the shape a plain one: it runs layer by layer, as its first calls did. Memory that other shapes' graphs
-// hold is given back before that.
+// Captures the pipeline's graphs. A wait that ran out is reported (the next call tries again). Memory that is refused is asked for again
+// kCallsToReplace calls later, and at once when other shapes' graphs hold some. Any other failure, or an output that is not dense NCHW,
+// makes the shape a plain one: it runs layer by layer, as its first calls did.
 int ott_net::build(HostPipeline& p, const char* input_blob, int n, int c, int h, int w, int chunk, int n_out, const char* const* out_blobs, bool warm) {
     size_t captured = 0;
     for (const HostPipeline& q : pipelines) captured += q.graphs.empty() ? 0 : 1;
     for (HostPipeline& q : pipelines)
         if (captured >= kMaxCaptured && !q.graphs.empty()) {
             drop(q);
-            q.calls = 0;
+            q.calls = q.retry_at = 0;
             --captured;
         }
     int rc = capture(p, input_blob, n, c, h, w, chunk, n_out, out_blobs, warm);
     if (rc == OTT_ERR_ALLOC && release_graphs()) rc = capture(p, input_blob, n, c, h, w, chunk, n_out, out_blobs, warm);
     if (rc == OTT_OK || rc == OTT_ERR_DEVICE_WAIT) return rc;
-    p.plain = true;
+    if (rc == OTT_ERR_ALLOC) p.retry_at = p.calls + kCallsToReplace;
+    else p.plain = true;
     error.clear();
     return OTT_OK;
 }

@@ -87,6 +87,32 @@ def test_memory_refused_to_a_capture(small):
         ctx.check(ctx.lib.ott_debug_fail_alloc_after(ctx.h, 0))
 
 
+def test_a_capture_that_was_refused_memory_is_tried_again(small):
+    """Also of a batch in chunks, whose copies overlap its kernels only when it is captured."""
+    net, params, want = small
+    ctx = net.context()
+    for n, chunk, capturing in ((13, 64, 2), (12, 4, 1)):  # the call that captures: the second one, for chunks the first
+        x = np.random.default_rng(n).uniform(0, 1, size=(n, 3, 40, 48)).astype(np.float32)
+        expect = want(x, "conv5").view(np.int32)
+        taken = 0
+        for refuse in (False, True):
+            net.set_option("host_chunk", chunk)  # forgets all shapes
+            for _ in range(capturing - 1):
+                net.forward("data", x, ["conv5"])
+            before = _allocations(net)
+            ctx.check(ctx.lib.ott_debug_fail_alloc_after(ctx.h, taken))  # the last allocation of that call, a temporary of the capture
+            assert np.array_equal(net.forward("data", x, ["conv5"])[0].view(np.int32), expect)
+            ctx.check(ctx.lib.ott_debug_fail_alloc_after(ctx.h, 0))
+            taken = _allocations(net) - before
+        assert taken > 0
+        for _ in range(10):
+            assert np.array_equal(net.forward("data", x, ["conv5"])[0].view(np.int32), expect)
+        before = _allocations(net)
+        assert np.array_equal(net.forward("data", x, ["conv5"])[0].view(np.int32), expect)
+        assert _allocations(net) == before, (n, chunk)
+    net.set_option("host_chunk", 64)
+
+
 def test_an_output_that_does_not_exist_is_refused_on_every_call(small):
     net, params, want = small
     x = np.zeros((1, 3, 40, 48), np.float32)
