@@ -1098,6 +1098,25 @@ int forward_maxpool_impl(ott_ctx* ctx, const ott_conv* c, const float* in_dev, i
     ep.one_scale_out = c->one_scale_out; ep.scale_out0 = c->scale_out_host[0]; ep.int8_pos = c->int8_pos; ep.signed_rounding = c->signed_rounding;
     ep.has_bias = d.bias_term ? 1 : 0;
     ep.act_type = d.act_type; ep.act_param0 = d.act_param0; ep.rounding = d.rounding;
+    if (d.act_type == ACT_LRELU && !(d.act_param0 >= 0.f)) {
+        // The fused kernel pools the sums, which needs an activation that does not decrease: this one falls below zero, so each in its turn.
+        const int ph = (s.oh - 1) / 2 + 1, pw = (s.ow - 1) / 2 + 1;
+        DeviceBlock conv, pooled;
+        if (conv.alloc(ctx, (size_t)n * s.cout * s.oh * s.ow * 4) != cudaSuccess ||
+            (out_dtype == OTT_S8_NHWC && pooled.alloc(ctx, (size_t)n * s.cout * ph * pw * 4) != cudaSuccess)) {
+            (void)cudaGetLastError();
+            return ctx->fail(OTT_ERR_ALLOC, "scratch allocation for the unpooled layer failed");
+        }
+        OTT_CUDA_CHECK(ctx, launch_dense_stem(ctx->stream, s, in_dev, c->w_host.data(), c->scale_in_host.data(), c->bias_host.data(), c->scale_out_host.data(),
+                                               c->in_scale0, ep, conv.p, OTT_F32_NCHW));
+        ctx->launches += 1;
+        float* dst = static_cast<float*>(out_dtype == OTT_S8_NHWC ? pooled.p : out_dev);
+        const int rc = ott_maxpool_f32_nchw(ctx, static_cast<const float*>(conv.p), n, s.cout, s.oh, s.ow, 3, 3, 2, 2, 1, 1, pad_with_zero, dst);
+        if (rc != OTT_OK || out_dtype != OTT_S8_NHWC) return rc;
+        OTT_CUDA_CHECK(ctx, launch_quantize_dense(ctx->stream, dst, s.cout, static_cast<int8_t*>(out_dev), c->scale_out_dev, s.cout, n, s.cout, ph, pw, d.rounding));
+        ctx->launches += 1;
+        return OTT_OK;
+    }
     OTT_CUDA_CHECK(ctx, launch_dense_stem_pool(ctx->stream, s, in_dev, c->w_host.data(), c->scale_in_host.data(), c->bias_host.data(),
                                                 c->scale_out_host.data(), c->in_scale0, ep, out_dev, out_dtype, pad_with_zero, ctx->status_dev, ctx->sm_count,
                                                 ctx->wait_limit_ns));
