@@ -1446,7 +1446,7 @@ UmmaChoice umma_choose(const UmmaVariant* v, int n, const ConvShape& s, int sm_c
     return c;
 }
 
-// Channels as accumulator rows (the two builds at the end of the comment in front of the kernel). What they gain is the epilogue; an
+// Channels as accumulator rows (builds 6 and 7 of the comment in front of the kernel; 8 below). What they gain is the epilogue; an
 // MMA of 128 channels x 128 pixels reads as many bytes of shared memory as its port delivers in the time it takes, one of 128 pixels x
 // 256 channels three quarters of them, so with more input channels the order of the operands that keeps the port free is the better one.
 // us, pixels as rows / channels as rows: 64 -> 256 56x56 x128 41.8 / 26.0, 256 -> 512 28x28 x128 23.9 / 18.5, 116 -> 116 20x20 x256 9.3 / 6.5,

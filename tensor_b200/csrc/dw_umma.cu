@@ -32,12 +32,11 @@ namespace {
 using namespace umma;
 constexpr int kTileM = 128, kTw = 8, kTh = 16, kBlock = 32;
 // Builds of the kernel: 0 = one CTA per SM, 8 epilogue warps; 1 = two CTAs per SM (narrow layers); 2 = one CTA per SM with 16
-// epilogue warps and four issuing warps, for wide channel slices: a tile of 8 channel blocks is 72 MMAs, which one warp gets
-// out at one per 75 cycles however many of its lanes issue (two warps reach the pipe's 40), and holds more requantize work
-// than eight warps get through meanwhile.
+// epilogue warps, for wide channel slices: a tile of 8 channel blocks holds more requantize work than eight warps get through while
+// its 72 MMAs run. One elected thread issues them at the pipe's 40 cycles; with two or four issuing warps the layers of this
+// build take the same time (256 channels 56x56 x64 stride 2 15.2 us, 464 63x31 x40 15.7, fp32 output at stride 1 53.3).
 __host__ __device__ constexpr int epi_warps_of(int build) { return build == 2 ? 16 : 8; }
-__host__ __device__ constexpr int issue_warps_of(int build) { return build == 2 ? 4 : 1; }
-__host__ __device__ constexpr int threads_of(int build) { return 32 * (1 + issue_warps_of(build) + epi_warps_of(build)); }
+__host__ __device__ constexpr int threads_of(int build) { return 32 * (2 + epi_warps_of(build)); }
 constexpr int kWideCols = 128;  // channel-slice width from which build 2 is taken
 constexpr int kMaxStages = 3, kMaxAcc = 2;
 
@@ -57,7 +56,7 @@ template <int ACT, int OUT, int BUILD>
 __global__ void __launch_bounds__(threads_of(BUILD), BUILD == 1 ? 2 : 1)
 dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUtensorMap tmW, const DwPlan P, const DwGeom G, const EpilogueParams ep,
                void* __restrict__ out, uint32_t* __restrict__ status) {
-    constexpr int kEpiWarps = epi_warps_of(BUILD), kIssueWarps = issue_warps_of(BUILD);
+    constexpr int kEpiWarps = epi_warps_of(BUILD);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -74,17 +73,16 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
     const int cb0 = grp * P.ncb;
     const int nb = P.ncb_total - cb0 < P.ncb ? P.ncb_total - cb0 : P.ncb;
     const int c_base = cb0 * kBlock;
-    const int issuers = nb < kIssueWarps ? nb : kIssueWarps;
     if (threadIdx.x == 0) {
         prefetch_tensormap(&tmW);
         for (int cb = 0; cb < nb; ++cb) prefetch_tensormap(&maps.tm[maps.block_src[cb0 + cb]]);
         mbar_init(bar_w, 1);
         for (int i = 0; i < P.stages; ++i) {
             mbar_init(bar_full + 8u * i, 1);
-            mbar_init(bar_empty + 8u * i, (uint32_t)issuers);  // one commit per issuing warp
+            mbar_init(bar_empty + 8u * i, 1);
         }
         for (int i = 0; i < P.acc_bufs; ++i) {
-            mbar_init(bar_afull + 8u * i, (uint32_t)issuers);
+            mbar_init(bar_afull + 8u * i, 1);
             mbar_init(bar_aempty + 8u * i, kEpiWarps);
         }
         *abort_flag = 0;
@@ -136,9 +134,9 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
                 while (globaltimer_ns() - t0 < 1000000ull) {}  // let bulk copies in flight land before shared memory is released
             }
         }
-    } else if (warp <= kIssueWarps) {
-        if (warp <= issuers && elect_one()) {
-            // ---- MMA issuers: one thread per issuing warp, which takes every kIssueWarps-th channel block, nine taps each ----
+    } else if (warp == 1) {
+        if (elect_one()) {
+            // ---- MMA issuer: nine taps per channel block ----
             bool ok = mbar_wait(bar_w, 0, abort_flag, status, 16u, P.wait_ns);
             tc_fence_after();
             // The offset of a tap's shifted input view inside a block (16-byte units; stride 2: the taps kx = 1 read the second column set,
@@ -159,7 +157,7 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
                 if (!mbar_wait(bar_full + 8u * st, ph, abort_flag, status, 2u, P.wait_ns)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll 1
-                for (int cb = warp - 1; cb < nb; cb += kIssueWarps) {
+                for (int cb = 0; cb < nb; ++cb) {
                     const uint32_t d = tmem_base + buf * (uint32_t)P.cols + (uint32_t)(cb * kBlock);
                     // 8-row groups (one tile row of 8 pixels each) are `stride` input rows apart
                     const uint64_t a0 = make_smem_desc(sX + st * (uint32_t)P.stage_bytes + (uint32_t)(cb * P.block_bytes), kBlock, (int)sbo);
@@ -177,7 +175,7 @@ dw_umma_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ CUte
         }
     } else {
         // ---- epilogue warps ----
-        const int q = warp & 3, sub = (warp - (1 + kIssueWarps)) >> 2, nsub = kEpiWarps >> 2;
+        const int q = warp & 3, sub = (warp - 2) >> 2, nsub = kEpiWarps >> 2;
         const int row = q * 32 + lane;
         const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
         const long plane = (long)G.oh * G.ow;
