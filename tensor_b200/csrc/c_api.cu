@@ -43,7 +43,7 @@ int check_status_word(ott_ctx* ctx, bool copied = false) {
 // round2_nonneg. Only sums whose product lies within 2^-25 of 0.5 can tell the two apart; v does not decrease with the sum, so they are
 // neighbours, and both forms are worked out for the few around the one that gives 0.5.
 bool one_rounding_does(float si, float bias, bool has_bias, int act, float so, int rounding) {
-    if (!(so > 0.f) || !(std::isfinite(so) && std::isfinite(si) && std::isfinite(bias))) return so == 0.f;
+    if (!(so > 0.f) || !std::isfinite(so)) return so == 0.f;
     const float h = rounding == OTT_ROUND_HALF_AWAY ? 0x1.fffffep-2f : 0.5f;
     auto same = [&](float y) {
         const volatile float product = y * so;
@@ -51,6 +51,7 @@ bool one_rounding_does(float si, float bias, bool has_bias, int act, float so, i
         return std::trunc(sum) == std::trunc(std::fma(y, so, 0.5f));
     };
     if (act == ACT_RELU6 && !same(6.f)) return false;
+    if (!std::isfinite(si) || !std::isfinite(bias)) return true;  // (an activation leaves 0, 6 or infinity of such a v, 0 of a NaN)
     if (si == 0.f) return !(bias > 0.f) || same(act == ACT_RELU6 ? std::min(bias, 6.f) : bias);
     const double at = (0.5 / (double)so - (double)bias) / (double)si, away = 4.0 + std::fabs(at) * 0x1p-21 + std::fabs((double)bias / si) * 0x1p-22;
     if (std::fabs(at) > 4294967296.0) return true;  // (no s32 sum comes near)
@@ -1203,12 +1204,6 @@ int conv_forward_impl(ott_ctx* ctx, const ott_conv* c, const void* in_dev, const
     ep.has_bias = d.bias_term ? 1 : 0;
     ep.act_type = d.act_type; ep.act_param0 = d.act_param0; ep.rounding = d.rounding;
 
-    // The CUDA-core depthwise kernel rounds what ReLU left as a number that is not negative, in one step. Where that does not do the layer runs
-    // as the LeakyReLU of slope 0, whose results are the same int8 values (ReLU6: a build of its own).
-    if (c->kind == OTT_KERNEL_DEPTHWISE && c->signed_rounding && out_dtype == OTT_S8_NHWC && d.act_type == ACT_RELU) {
-        ep.act_type = ACT_LRELU;
-        ep.act_param0 = 0.f;
-    }
     uint32_t* status = status_word_dev ? status_word_dev : ctx->status_dev;
     PlaneGather groups8;  // depthwise over gathered int8 input: where each 16-channel group lies
     const bool dw_tensor = c->kind == OTT_KERNEL_DEPTHWISE && in_dtype == OTT_S8_NHWC && (!gathered || c->gather_group == 32) &&

@@ -114,7 +114,8 @@ struct RowRing {
     }
 };
 
-// Added to the activation of an int8 build: EpilogueParams::signed_rounding (ReLU6; such a layer with ReLU runs as the LeakyReLU of slope 0).
+// Added to the activation (ReLU, ReLU6) of an int8 build: EpilogueParams::signed_rounding. (ReLU is not the LeakyReLU of slope 0: a bias of
+// -infinity, a channel that is switched off, would become a NaN.)
 constexpr int kSignedRounding = 8;
 
 // Four accumulators of one channel -> four int8 in one word, the arithmetic as packed pairs.
@@ -452,9 +453,12 @@ cudaError_t launch_t(cudaStream_t stream, const ConvShape& s, const void* x, con
 template <int K, int S, bool IN_F32, int EPI>
 cudaError_t launch_act(cudaStream_t stream, const ConvShape& s, const void* x, const PlaneGather& G, const uint32_t* wq, const float* in_scales,
                        int n_in_scales, const EpilogueParams& ep, void* out) {
-    if constexpr (EPI != EPI_F32)
+    if constexpr (EPI != EPI_F32) {
+        if (ep.signed_rounding && ep.act_type == ACT_RELU)
+            return launch_t<K, S, IN_F32, EPI, ACT_RELU | kSignedRounding>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);
         if (ep.signed_rounding && ep.act_type == ACT_RELU6)
             return launch_t<K, S, IN_F32, EPI, ACT_RELU6 | kSignedRounding>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);
+    }
     switch (ep.act_type) {
         case ACT_RELU: return launch_t<K, S, IN_F32, EPI, ACT_RELU>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);
         case ACT_LRELU: return launch_t<K, S, IN_F32, EPI, ACT_LRELU>(stream, s, x, G, wq, in_scales, n_in_scales, ep, out);

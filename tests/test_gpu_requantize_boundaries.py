@@ -105,3 +105,21 @@ def test_quantized_input(ctx, rounding, k):
     case.x_f32 = (edge.view(np.int32) + rng.integers(-2, 3, size=edge.shape).astype(np.int32)).view(np.float32)
     got, want = run_gpu(ctx, case, rounding, want_acc=False)["y"], run_port(case, rounding, want_acc=False)["y"]
     assert np.array_equal(got, want) and np.unique(want).size > 200
+
+
+@pytest.mark.parametrize("act", [ACT_RELU, ACT_RELU6])
+@pytest.mark.parametrize("signs", [False, True])
+@pytest.mark.parametrize("name,c,k,stride,n,h,s8,depthwise", [("dw3", 48, 3, 1, 2, 17, True, True), ("dw3_f32", 48, 3, 1, 2, 17, False, True),
+                                                              ("dw3_tensor", 256, 3, 2, 20, 56, True, True), ("dw5", 48, 5, 2, 2, 17, True, True),
+                                                              ("dw7", 48, 7, 1, 2, 12, True, True), ("one_tile", 64, 1, 1, 1, 9, True, False),
+                                                              ("channel_rows", 64, 1, 1, 16, 50, True, False)])
+def test_channels_switched_off(ctx, name, c, k, stride, n, h, s8, depthwise, signs, act):
+    """A bias of -infinity leaves 0 of a channel behind ReLU and ReLU6, under scales of either sign."""
+    from gpu_support import run_gpu
+    case = _make(f"off_{name}", c, c, k, act, n, h, h, s8, c + k, stride, depthwise, 0.2 if depthwise else 0.05)
+    case.bias[::5] = -np.inf
+    scale = np.geomspace(5.0, 300.0, c).astype(np.float32)
+    case.out_scales = np.where(np.arange(c) % 3 == 0, -scale, scale) if signs else scale
+    got, want = run_gpu(ctx, case, ROUND_ADD_HALF_TRUNC, want_acc=False)["y"], run_port(case, ROUND_ADD_HALF_TRUNC, want_acc=False)["y"]
+    assert not want[:, ::5].any() and np.unique(want).size > 50
+    assert np.array_equal(got, want), np.argwhere(got != want)[:5]
