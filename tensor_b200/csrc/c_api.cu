@@ -751,7 +751,8 @@ int conv_create_impl(ott_ctx* ctx, const ott_conv_desc* d, const int8_t* w_oihw,
         rc = upload(ctx, wtiled.data(), wtiled.size() * 4, (void**)&c->w_tiled_dev);
     }
     if (rc == OTT_OK && depthwise && !gi && d->kh == 3 && d->kw == 3 && d->ph == 1 && d->pw == 1 && d->dh == 1 && d->dw == 1 && d->sh == d->sw &&
-        (d->sh == 1 || d->sh == 2) && d->rounding == OTT_ROUND_ADD_HALF_TRUNC && !c->signed_rounding) {
+        (d->sh == 1 || d->sh == 2) && d->rounding == OTT_ROUND_ADD_HALF_TRUNC && !c->signed_rounding &&
+        std::none_of(scale_out.begin(), scale_out.end(), [](float v) { return v < 0.f; })) {
         int smem_optin = 0;
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
         if (dw_umma_plan(d->cout, d->sh, smem_optin, &c->dw_plan)) {

@@ -68,6 +68,25 @@ def test_fused_layers(ctx, act, unit, f32_out):
         o.close()
 
 
+@pytest.mark.parametrize("negative", [False, True])
+def test_fused_pair_refuses_a_negative_depthwise_scale(ctx, negative):
+    from gpu_support import make_layer
+    from tensor_b200 import DwPwInt8, OtterB200Error
+    dw = ConvCase("refused_dw", 40, 40, 3, 1, 1, groups=40, bias_term=1, int8_scale_term=101, act_type=ACT_NONE, s8_input=True, n=1, h=8, w=8, seed=2).make()
+    pw = ConvCase("refused_pw", 40, 40, 1, 1, 0, bias_term=1, int8_scale_term=101, act_type=ACT_RELU, s8_input=True, n=1, h=8, w=8, seed=3).make()
+    dw.out_scales = np.linspace(1.0, 40.0, 40).astype(np.float32)
+    if negative:
+        dw.out_scales[7] = -3.0
+    layers = [make_layer(ctx, x, ROUND_ADD_HALF_TRUNC) for x in (dw, pw)]
+    if negative:
+        with pytest.raises(OtterB200Error):
+            DwPwInt8(ctx, *layers)
+    else:
+        DwPwInt8(ctx, *layers).close()
+    for layer in layers:
+        layer.close()
+
+
 def test_first_layer_maxpool_with_negative_scales(ctx):
     """Against the fp32 form of the same kernel, rounded half away from zero."""
     from tensor_b200 import ConvInt8, nhwc_channels
