@@ -119,14 +119,24 @@ struct RowRing {
 constexpr int kSignedRounding = 8;
 
 // Four accumulators of one channel -> four int8 in one word, the arithmetic as packed pairs.
-template <int ACT, bool SIGNED>
+// LONG: the constant of the fused product and sum takes the sum's sign, which is + (or that of a -0, and the result 0 all the same), in one value of
+// each pair. That instruction makes the compiler keep 80 registers where it makes do with 71, and the latency of a band, which bounds the
+// smaller launches, is shorter. For the one instance that had 80 before its rounding was mended (5x5, ReLU6; us with 71 / this / two
+// roundings: 96 channels 40x40 x32 9.92 / 7.93 / 8.27, 75 66x15 x25 5.55 / 4.99 / 5.20, x100 13.2 / 13.7 / 14.4, 96 40x40 x128 24.8 / 27.3 / 29.3).
+template <int ACT, bool SIGNED, bool LONG>
 __device__ __forceinline__ uint32_t epi_s8x4(const int (&acc)[4], float si, float bi, float so, float p0, uint32_t half) {
     const float2 s2 = make_float2(si, si), b2 = make_float2(bi, bi), o2 = make_float2(so, so);
     int2 q[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const float2 v = __ffma2_rn(make_float2(__int2float_rn(acc[2 * h]), __int2float_rn(acc[2 * h + 1])), s2, b2);
-        q[h] = round2_act<ACT, SIGNED>(make_float2(activate_t<ACT>(v.x, p0), activate_t<ACT>(v.y, p0)), o2, half);
+        const float2 y = make_float2(activate_t<ACT>(v.x, p0), activate_t<ACT>(v.y, p0));
+        if (LONG) {
+            const float2 r = __ffma2_rn(y, o2, make_float2(half_signed(y.x, kHalfFused), __uint_as_float(kHalfFused)));
+            q[h] = make_int2(__float2int_rz(r.x), __float2int_rz(r.y));
+        } else {
+            q[h] = round2_act<ACT, SIGNED>(y, o2, half);
+        }
     }
     return pack_sat_s8x4(q[0].x, q[0].y, q[1].x, q[1].y);
 }
@@ -138,6 +148,7 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
                        int aligned) {
     constexpr int KK = Geo<K, S>::KK, ACT = ACT_BUILD & ~kSignedRounding;
     constexpr bool SIGNED = (ACT_BUILD & kSignedRounding) != 0;
+    constexpr bool LONG = K == 5 && S == 1 && !IN_F32 && EPI == EPI_S8 && ACT_BUILD == ACT_RELU6;
     extern __shared__ uint32_t smem[];
     __shared__ const float* ch_ptr[CG];
     __shared__ float ch_scale[CG];
@@ -320,7 +331,7 @@ depthwise_tiled_kernel(const void* __restrict__ xin, const __grid_constant__ Pla
             int acc[4] = {0, 0, 0, 0};
             ring.template advance<R>(p, T.rp, sh, wmod8, wk, wv, w44, acc);
             if (EPI != EPI_F32) {
-                uint32_t w = epi_s8x4<ACT, SIGNED>(acc, p_si, p_bi, p_so, ep.act_param0, half);
+                uint32_t w = epi_s8x4<ACT, SIGNED, LONG>(acc, p_si, p_bi, p_so, ep.act_param0, half);
                 w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 2), sel_a);
                 w = __byte_perm(w, __shfl_xor_sync(0xFFFFFFFFu, w, 1), sel_b);
                 if (store_ok) *reinterpret_cast<uint32_t*>(o8) = w;
